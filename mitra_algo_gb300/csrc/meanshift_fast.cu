@@ -1,5 +1,6 @@
 // SPDX-License-Identifier: MPL-2.0
 // SIMT mean-shift (FP32 and FP64) over a Morton-chunked 6-D vote set.
+#include "chunk_lists.cuh"
 #include "meanshift_fast.cuh"
 #include "primitives.cuh"
 
@@ -153,162 +154,386 @@ __global__ void __launch_bounds__(kBlockChunks) block_boxes(const float *cbox, u
 }
 
 // ------------------------------------------------------------ mean shift
-__device__ __forceinline__ float box_gap2(const float *a_lo, const float *a_hi, const float *b) {
-  float g = 0;
-  for (int k = 0; k < 6; ++k) {
-    float d = fmaxf(fmaxf(b[k] - a_hi[k], a_lo[k] - b[6 + k]), 0.f);
-    g += d * d;
-  }
-  return g;
+// Summation layout of one iteration: the chunks are cut into `splits` runs of
+// `cps`, and a seed's sums are its splits' partial sums added in the fixed
+// order of ms_reduce.  touched: one bit per (tile, split) that had a chunk to
+// evaluate, kGroups x words 32-bit words per tile (split p: bit p / kGroups of
+// group p % kGroups); an untouched split has no partial sums -- they would be
+// zeros, which change no sum -- and is skipped by ms_reduce.
+constexpr int kGroups = 8;
+struct Grid {
+  uint64_t tiles, splits, cps, slots;
+  uint32_t words;  // 32-bit words of `touched` per group of a tile
+};
+
+__device__ __forceinline__ bool touch(uint32_t *touched, uint32_t words, uint32_t tile, uint32_t p) {
+  uint32_t *w = touched + (uint64_t(tile) * kGroups + p % kGroups) * words + (p / kGroups) / 32;
+  const uint32_t bit = 1u << ((p / kGroups) % 32);
+  return !(atomicOr(w, bit) & bit);
 }
 
-// One block = one tile of up to kChunk active seeds (ids[tile*kChunk + t])
-// x one split of the chunk range.  Each thread accumulates, for its seed,
-// sum w x and sum w over the votes of the chunks its tile cannot skip, and
-// for a kNear seed also the unweighted in-window sums of d = v - x and
-// d d^T (the Jacobian of the Newton step).
-// COUNT: count the votes within the bandwidth instead.
-// NEWTON: some seed of the launch is kNear (the plain instance keeps its
-// register footprint small).  The FP32 instances are held to 64 registers,
-// eight CTAs per SM (measured: the polish 0.4 ms faster on the benchmark).
-template <typename T, bool COUNT, bool NEWTON>
-__global__ void __launch_bounds__(kChunk, sizeof(T) == 4 ? 8 : 1)
-    ms_tile(const T *desc, const float *cbox, const float *bbox, const float *sbox,
-            uint64_t nchunks, uint64_t q, const T *means, const uint8_t *state,
-            const int32_t *ids, uint64_t nactive, T h2, T gk, float skip_gap2,
-            uint64_t chunks_per_split, T *partial, unsigned long long *evals) {
-  constexpr int stride = COUNT ? 8 : kPartial;
-  constexpr bool kFine = NEWTON || COUNT;  // sub-box tests
-  __shared__ T xs[kChunk * 8];
-  __shared__ float sb[kFine ? kSubs * 12 : 1];
-  __shared__ float tlo[6][4], thi[6][4];
-  // NEWTON: the 27 unweighted in-window sums of each thread's seed, in
-  // shared memory (in-window votes are rare; registers stay free)
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+
+// Work items of the SIMT kernel.  split_items: for every tile, the chunks
+// within the bandwidth of some of its seeds (bits[t * bwords + c / 32]) and
+// the (tile, split) pairs that hold one (pairs, in no particular order).
+// weigh_items: an item (quarter of the tile, split) per quarter with active
+// seeds, queued by the split's number of chunks, so the warps of ms_tile draw
+// the longest items first (a warp that meets one of them last keeps the launch
+// waiting: the first Newton iteration of the 20,000-sample motif sphere took
+// 4.0 ms in the list's order, 3.0 with the longest first).
+// bits, touched and work are zeroed before.  CTAs shared among the tiles.
+constexpr int kQueues = 8;  // queue k: items of more than (kQueues - 1 - k) / kQueues of cps chunks
+enum { kWorkPairs = 0, kWorkNext = 1, kWorkQueue = 2, kWorkSize = 2 + kQueues };
+template <typename T>
+__global__ void __launch_bounds__(kListThreads) split_items(
+    const float *boxes, const T *means, const int32_t *ids, const unsigned *nact, const float *cbox,
+    const float *bbox, uint32_t nchunks, const uint32_t *sblk, const uint32_t *nsurv, uint32_t nblk,
+    float skip_gap2, uint32_t cps, uint32_t words, uint32_t bwords, uint32_t *bits,
+    uint32_t *touched, uint2 *pairs, uint32_t *work) {
+  __shared__ TileSeeds seeds;
+  uint32_t t, sub, per;
+  if (!list_share(nact, t, sub, per)) return;
+  const uint32_t ns = nsurv[t];
+  if (sub >= ns) return;
+  load_tile(seeds, t, nact[0], boxes, means, ids);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (uint32_t j = sub; j < ns; j += per) {
+    const uint32_t blk = sblk[uint64_t(t) * nblk + j];
+    const bool keep = chunk_needed(seeds, blk, bbox, cbox, nchunks, skip_gap2);
+    const unsigned bal = __ballot_sync(0xffffffffu, keep);
+    if (lane == 0) bits[uint64_t(t) * bwords + blk * (kBlockChunks / 32) + warp] = bal;
+    if (keep) {  // the first kept chunk of each split in the warp lists it
+      const uint32_t p = (blk * kBlockChunks + threadIdx.x) / cps;
+      const unsigned peers = __match_any_sync(bal, p);
+      if (lane == __ffs(int(peers)) - 1 && touch(touched, words, t, p))
+        pairs[atomicAdd(&work[kWorkPairs], 1u)] = make_uint2(t, p);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256) weigh_items(const uint2 *pairs, const unsigned *nact,
+                                                   const uint32_t *bits, uint32_t bwords,
+                                                   uint32_t cps, uint32_t nchunks, uint32_t room,
+                                                   uint2 *items, uint32_t *work) {
+  const uint32_t n = work[kWorkPairs];
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint32_t t = pairs[i].x, p = pairs[i].y;
+    const uint32_t c0 = p * cps, c1 = min(nchunks, c0 + cps);
+    uint32_t weight = 0;
+    for (uint32_t base = c0 & ~31u; base < c1; base += 32) {
+      uint32_t word = bits[uint64_t(t) * bwords + base / 32];
+      if (base < c0) word &= ~0u << (c0 - base);
+      if (c1 - base < 32) word &= (1u << (c1 - base)) - 1u;
+      weight += __popc(word);
+    }
+    const uint32_t k = kQueues - 1 - min(uint32_t(kQueues - 1), (weight - 1) * kQueues / cps);
+    const uint32_t quarters = min((nact[0] - t * kChunk + 31) / 32, uint32_t(kChunk / 32));
+    const uint32_t at = atomicAdd(&work[kWorkQueue + k], quarters);
+    for (uint32_t x = 0; x < quarters; ++x)
+      items[uint64_t(k) * room + at + x] = make_uint2(t * (kChunk / 32) + x, p);
+  }
+}
+
+// Two values at once: packed FP32 arithmetic rounds each like the scalar
+// instruction.
+template <typename T>
+struct Two {
+  T x, y;
+};
+__device__ __forceinline__ unsigned long long bits_of(Two<float> a) {
+  unsigned long long r;
+  memcpy(&r, &a, 8);
+  return r;
+}
+__device__ __forceinline__ Two<float> two_of(unsigned long long r) {
+  Two<float> a;
+  memcpy(&a, &r, 8);
+  return a;
+}
+__device__ __forceinline__ Two<float> add2(Two<float> a, Two<float> b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits_of(a)), "l"(bits_of(b)));
+  return two_of(r);
+}
+__device__ __forceinline__ Two<float> mul2(Two<float> a, Two<float> b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits_of(a)), "l"(bits_of(b)));
+  return two_of(r);
+}
+__device__ __forceinline__ Two<float> fma2(Two<float> a, Two<float> b, Two<float> c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(bits_of(a)), "l"(bits_of(b)), "l"(bits_of(c)));
+  return two_of(r);
+}
+__device__ __forceinline__ Two<double> add2(Two<double> a, Two<double> b) {
+  return {add_rn(a.x, b.x), add_rn(a.y, b.y)};
+}
+__device__ __forceinline__ Two<double> mul2(Two<double> a, Two<double> b) {
+  return {mul_rn(a.x, b.x), mul_rn(a.y, b.y)};
+}
+__device__ __forceinline__ Two<double> fma2(Two<double> a, Two<double> b, Two<double> c) {
+  return {fma(a.x, b.x, c.x), fma(a.y, b.y, c.y)};
+}
+
+// a / b, correctly rounded, from r = 1 / b correctly rounded (a <= b): two
+// residual corrections q + (a - b q) r.  The first leaves q within one unit in
+// the last place; from there the second rounds correctly (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// 1990).  No branch, unlike the general division, so several overlap.  (A
+// quotient so small that its residual underflows is far below the weights'
+// rounding.)
+__device__ __forceinline__ float ratio(float a, float b, float r) {
+  float q = a * r;
+  q = fmaf(fmaf(-b, q, a), r, q);
+  return fmaf(fmaf(-b, q, a), r, q);
+}
+__device__ __forceinline__ double ratio(double a, double b, double) { return a / b; }
+__device__ __forceinline__ float reciprocal(float b) { return __frcp_rn(b); }
+__device__ __forceinline__ double reciprocal(double) { return 0.0; }
+
+// A run of kSubVotes votes in shared memory: coordinate d of vote j at
+// (j / 2) * kPairStride + 2 d + j % 2, so a pair's coordinates are adjacent
+// (packed arithmetic) and lanes reading different votes meet different banks.
+constexpr int kPairStride = 20, kRunValues = kSubVotes / 2 * kPairStride;
+
+// A warp takes 32 active seeds (a quarter of a tile of kChunk, a lane each) and
+// one split of the chunk range: each lane accumulates, for its seed, sum
+// w (v - x) and sum w over the split's votes in order, and for a kNear seed
+// also the unweighted in-window sums of d = v - x and d d^T (the Jacobian of
+// the Newton step).
+// COUNT: the votes within the bandwidth of each seed are added to
+// counts[seed] instead.
+// NEWTON: some seed of the launch is kNear; its 27 sums are kept in shared
+// memory (in-window votes are rare, and registers would halve the warps).
+// GAUSS: the shifted Gaussian weights instead of Epanechnikov's.
+// With `items`, the warps draw (quarter, split) items of split_items' list
+// and take the chunks whose bits are set; without, block
+// (tile, split) takes every chunk of its split, a quarter per warp.
+//
+// Of the chunks, the lanes test the boxes of four chunks' runs of kSubVotes
+// votes (kSubs each) against the box of the warp's seeds at once; a run that
+// passes is tested against each seed and then evaluated: first which of the
+// votes lie within the bandwidth of the lane's seed (two votes per packed
+// instruction, a bit each, no branches), then every lane takes its own
+// members in turn.  Votes outside the bandwidth add nothing, so no test
+// changes a sum.  Which products of a sum are rounded before they are
+// added is spelt out, so every instance rounds alike whatever the compiler
+// would contract.
+//
+// No barrier joins the warps: a form whose four warps shared each chunk
+// through shared memory spent 10 to 14 issue slots of stall per instruction
+// at its barriers, with 40% of the issue slots used and a third of the time in
+// the tail of its CTAs (first Newton iteration of the 20,000-sample motif
+// sphere, 2,048 seeds, 2.5e7 votes: 5.2 ms, 2.9 ms here).  The next run's
+// 512 bytes are loaded while the current one is evaluated.
+template <typename T, bool COUNT, bool NEWTON, bool GAUSS>
+__global__ void __launch_bounds__(kChunk, sizeof(T) == 4 ? 8 : 2)
+    ms_tile(const T *desc, const float *sbox, uint32_t nchunks, uint64_t q, const T *means,
+            const uint8_t *state, const int32_t *ids, uint32_t nactive, T h2, T gk, float skip_gap2,
+            Grid grid, uint32_t *touched, const uint32_t *bits, uint32_t bwords, const uint2 *items,
+            uint32_t room, uint32_t *work, T *partial, unsigned long long *counts, unsigned long long *evals) {
+  constexpr int kWords = int(sizeof(T)) / 4;  // 16-byte words per lane of a run
+  __shared__ __align__(16) T runs[kChunk / 32][2][kRunValues];
   __shared__ T nsum[NEWTON ? 27 * kChunk : 1];
-  uint64_t slot = uint64_t(blockIdx.x) * kChunk + threadIdx.x, split = blockIdx.y;
-  uint64_t slots = uint64_t(gridDim.x) * kChunk;
-  bool live = slot < nactive;
-  int32_t seed = live ? ids[slot] : 0;
-  const bool newton = NEWTON && !COUNT && live && is_near(state[seed]);
-  T m[6];
-  for (int d = 0; d < 6; ++d) m[d] = live ? means[uint64_t(seed) * 8 + d] : T(0);
-  float lo[6], hi[6];
-  for (int d = 0; d < 6; ++d) {
-    lo[d] = live ? float(m[d]) : INFINITY;
-    hi[d] = live ? float(m[d]) : -INFINITY;
-  }
-  int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int o = 16; o; o >>= 1)
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t queue_end[kQueues];  // items of the queues up to and including each
+  for (int k = 0; k < kQueues; ++k)
+    queue_end[k] = (k ? queue_end[k - 1] : 0u) + (items ? work[kWorkQueue + k] : 0u);
+  T *const ns = nsum + threadIdx.x;
+  const T rcp = reciprocal(h2), floor_w = GAUSS ? exp2(-gk) : T(0);
+  for (;;) {
+    uint32_t tile = blockIdx.x, split = blockIdx.y, quarter = warp;
+    if (items) {
+      uint32_t it = 0;
+      if (lane == 0) it = atomicAdd(&work[kWorkNext], 1u);
+      it = __shfl_sync(0xffffffffu, it, 0);
+      if (it >= queue_end[kQueues - 1]) return;
+      uint64_t at = it;
+      for (int k = 1; k < kQueues; ++k)
+        if (it >= queue_end[k - 1]) at = uint64_t(k) * room + (it - queue_end[k - 1]);
+      const uint2 x = items[at];
+      tile = x.x / (kChunk / 32), quarter = x.x % (kChunk / 32), split = x.y;
+    }
+    const uint32_t slot = tile * kChunk + quarter * 32 + lane;
+    const bool live = slot < nactive;
+    if (!__any_sync(0xffffffffu, live)) return;  // without items only
+    const int32_t seed = live ? ids[slot] : 0;
+    const bool newton = NEWTON && !COUNT && live && is_near(state[seed]);
+    T m[6];
+    float mf[6], lo[6], hi[6];
     for (int d = 0; d < 6; ++d) {
-      lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
-      hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+      m[d] = live ? means[uint64_t(seed) * 8 + d] : T(0);
+      mf[d] = float(m[d]);
+      lo[d] = live ? mf[d] : INFINITY;
+      hi[d] = live ? mf[d] : -INFINITY;
     }
-  if (lane == 0)
-    for (int d = 0; d < 6; ++d) tlo[d][warp] = lo[d], thi[d][warp] = hi[d];
-  __syncthreads();
-  for (int d = 0; d < 6; ++d) {
-    lo[d] = fminf(fminf(tlo[d][0], tlo[d][1]), fminf(tlo[d][2], tlo[d][3]));
-    hi[d] = fmaxf(fmaxf(thi[d][0], thi[d][1]), fmaxf(thi[d][2], thi[d][3]));
-  }
-  T acc[7] = {0, 0, 0, 0, 0, 0, 0};
-  if (NEWTON)
-    for (int j = 0; j < 27; ++j) nsum[j * kChunk + threadIdx.x] = T(0);
-  uint64_t c0 = split * chunks_per_split;
-  uint64_t c1 = c0 + chunks_per_split < nchunks ? c0 + chunks_per_split : nchunks;
-  unsigned long long done = 0;
-  for (uint64_t c = c0; c < c1; ++c) {
-    if (c == c0 || c % kBlockChunks == 0) {  // the block's box first (one test for the CTA)
-      const uint64_t blk = c / kBlockChunks;
-      if (box_gap2(lo, hi, bbox + blk * 12) > skip_gap2) {
-        c = (blk + 1) * kBlockChunks - 1;
-        continue;
-      }
-    }
-    if (box_gap2(lo, hi, cbox + c * 12) > skip_gap2) continue;
-    // skip the chunk unless some seed of the block lies within the bandwidth
-    // of its box (exact for Epanechnikov weights)
-    const float *cb = cbox + c * 12;
-    float g = 0;
-    for (int d = 0; d < 6; ++d) {
-      const float x = float(m[d]);
-      const float e = fmaxf(fmaxf(cb[d] - x, x - cb[6 + d]), 0.f);
-      g += e * e;
-    }
-    if (!__syncthreads_or(live && g <= skip_gap2)) continue;
-    uint64_t v = c * kChunk + threadIdx.x;
-    for (int d = 0; d < 8; ++d) xs[threadIdx.x * 8 + d] = v < q ? desc[v * 8 + d] : T(1e30);
-    if (kFine)
-      for (int i = threadIdx.x; i < kSubs * 12; i += kChunk) sb[i] = sbox[c * kSubs * 12 + i];
-    __syncthreads();
-    uint64_t rest = q - c * kChunk;
-    int n = rest < uint64_t(kChunk) ? int(rest) : kChunk;
-    done += n;
-    auto eval = [&](int j) {
-      T e[6], d2 = 0;
-#pragma unroll
+    for (int o = 16; o; o >>= 1)
       for (int d = 0; d < 6; ++d) {
-        e[d] = xs[j * 8 + d] - m[d];
-        d2 += e[d] * e[d];
+        lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+        hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
       }
-      if (d2 < h2) {
-        if (COUNT) {
-          acc[6] += T(1);
-        } else {
-          const T floor_w = gk > T(0) ? exp2(-gk) : T(0);
-          const T w = gk > T(0) ? exp2(-gk * (d2 / h2)) - floor_w : T(1) - d2 / h2;
+    T acc[7] = {0, 0, 0, 0, 0, 0, 0};
+    unsigned members = 0;
+    if (NEWTON)
+      for (int j = 0; j < 27; ++j) ns[j * kChunk] = T(0);
+    const uint32_t c0 = split * uint32_t(grid.cps);
+    const uint32_t c1 = c0 + uint32_t(grid.cps) < nchunks ? c0 + uint32_t(grid.cps) : nchunks;
+    const uint32_t *mine = items ? bits + uint64_t(tile) * bwords : nullptr;
+    unsigned long long done = 0;
+
+    uint4 held[kWords];
+    uint32_t held_run = 0;
+    auto fetch = [&](uint32_t run) {
+      const uint4 *src = reinterpret_cast<const uint4 *>(desc);
+      const uint64_t first = uint64_t(run) * 32 * kWords, last = q * 2 * kWords;
+      for (int k = 0; k < kWords; ++k) {
+        const uint64_t w = first + uint64_t(lane) * kWords + k;
+        held[k] = w < last ? src[w] : make_uint4(0, 0, 0, 0);
+      }
+      held_run = run;
+    };
+    // the run in `held` goes to shared memory (lane: half a vote), then is evaluated
+    int buf = 0;
+    auto store = [&]() {
+      T v[4];
+      memcpy(v, held, 4 * sizeof(T));
+      T *dst = runs[warp][buf] + (lane >> 2) * kPairStride + (lane & 1) * 8 + ((lane >> 1) & 1);
+      for (int k = 0; k < 4; ++k) dst[2 * k] = v[k];
+      __syncwarp();
+    };
+    auto eval = [&](uint32_t run, const T *vs) {
+      const uint64_t rest = q - uint64_t(run) * kSubVotes;
+      unsigned in = 0;
+#pragma unroll
+      for (int p = 0; p < kSubVotes / 2; ++p) {
+        Two<T> v[6], d2{T(0), T(0)};
+        memcpy(v, __builtin_assume_aligned(vs + p * kPairStride, 16), 6 * sizeof(Two<T>));
+#pragma unroll
+        for (int d = 0; d < 6; ++d) {
+          const Two<T> e = add2(v[d], Two<T>{-m[d], -m[d]});
+          d2 = NEWTON && !GAUSS ? add2(d2, mul2(e, e)) : fma2(e, e, d2);
+        }
+        in |= unsigned(d2.x < h2) << (2 * p) | unsigned(d2.y < h2) << (2 * p + 1);
+      }
+      if (rest < uint64_t(kSubVotes)) in &= (1u << unsigned(rest)) - 1u;
+      if (!live) in = 0;
+      if (COUNT) {
+        members += __popc(in);
+        return;
+      }
+      // the lane's members, in vote order, the weights of kAhead at a time (their
+      // latencies overlap; past the last member it stands in again, unused)
+      constexpr int kAhead = NEWTON ? 2 : 4;
+      while (in) {
+        T w[kAhead];
+        int at[kAhead];
+        const int n = __popc(in);
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
+          const int j = __ffs(int(in)) - 1;
+          if (k + 1 < n || k + 1 == kAhead) in &= in - 1;
+          at[k] = (j >> 1) * kPairStride + (j & 1);
+          T d2 = 0;
+#pragma unroll
+          for (int d = 0; d < 6; ++d) {
+            const T e = vs[at[k] + 2 * d] - m[d];
+            d2 = NEWTON && !GAUSS ? add_rn(d2, mul_rn(e, e)) : fma(e, e, d2);
+          }
+          const T x = ratio(d2, h2, rcp);
+          w[k] = GAUSS ? exp2(-gk * x) - floor_w : T(1) - x;
+          if (k >= n) w[k] = T(0);  // adds nothing
+        }
+        if (n <= kAhead) in = 0;
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
           // sums of w (v - x), not of w v: the step m - x comes out without
           // the cancellation of a mean of large coordinates (votes moved
           // to their own cell of vote space lie up to 14 from the origin)
+          T e[6];
 #pragma unroll
-          for (int d = 0; d < 6; ++d) acc[d] += w * e[d];
-          acc[6] += w;
-          if (newton) {  // Epanechnikov: unweighted sums; Gaussian: by 2^(-k d^2/h^2)
-            const T wn = gk > T(0) ? w + floor_w : T(1);
-            T *ns = nsum + threadIdx.x;
-            int at = 6;
+          for (int d = 0; d < 6; ++d) {
+            e[d] = vs[at[k] + 2 * d] - m[d];
+            acc[d] = fma(w[k], e[d], acc[d]);
+          }
+          acc[6] += w[k];
+          if (NEWTON && newton && k < n) {  // Epanechnikov: unweighted sums; Gaussian: by 2^(-k d^2/h^2)
+            const T wn = w[k] + floor_w;
+            int i = 6;
 #pragma unroll
             for (int d = 0; d < 6; ++d) {
-              const T we = wn * e[d];
+              const T we = GAUSS ? wn * e[d] : e[d];
               ns[d * kChunk] += we;
 #pragma unroll
-              for (int l = d; l < 6; ++l, ++at) ns[at * kChunk] += we * e[l];
+              for (int l = d; l < 6; ++l, ++i) {
+                T &sum = ns[i * kChunk];
+                sum = !GAUSS && l == d ? add_rn(sum, mul_rn(we, we)) : fma(we, e[l], sum);
+              }
             }
           }
         }
       }
     };
-    if (kFine) {
-      // the polish (NEWTON) and the support count (COUNT) also skip per
-      // warp, by runs of kSubVotes votes: a run none of the warp's 32 seeds
-      // lies within the bandwidth of would only add zeros.  The approach
-      // instance keeps the tile granularity of the tensor kernel (one
-      // 128-seed tile per chunk), so the two forms of the approach make the
-      // same seed-vote evaluations.
-      if (!__any_sync(0xffffffffu, live && g <= skip_gap2)) continue;
-#pragma unroll 1
-      for (int r = 0; r < kSubs && r * kSubVotes < n; ++r) {
-        const float *b = sb + r * 12;
-        float gr = 0;
-        for (int d = 0; d < 6; ++d) {
-          const float x = float(m[d]);
-          const float e = fmaxf(fmaxf(b[d] - x, x - b[6 + d]), 0.f);
-          gr += e * e;
-        }
-        if (!__any_sync(0xffffffffu, live && gr <= skip_gap2)) continue;
-        const int j1 = min(n, (r + 1) * kSubVotes);
-        for (int j = r * kSubVotes; j < j1; ++j) eval(j);
+    bool pending = false;
+    auto finish = [&](bool more, uint32_t run) {  // evaluates the held run, with the next one on its way
+      const uint32_t cur = held_run;
+      if (pending) store();
+      if (more) fetch(run);
+      if (pending) {
+        if (__any_sync(0xffffffffu, live && point_gap2_16(mf, sbox + uint64_t(cur) * 12) <= skip_gap2))
+          eval(cur, runs[warp][buf]);
+        buf ^= 1;
       }
-    } else {
-      for (int j = 0; j < n; ++j) eval(j);
+      pending = more;
+    };
+    for (uint32_t base = c0 & ~31u; base < c1; base += 32) {
+      uint32_t word = mine ? mine[base / 32] : ~0u;
+      if (base < c0) word &= ~0u << (c0 - base);
+      if (c1 - base < 32) word &= (1u << (c1 - base)) - 1u;
+      if (quarter == 0 && evals && lane == 0 && word) {
+        done += uint64_t(__popc(word)) * kChunk;
+        if (c1 == nchunks && c1 - base <= 32 && (word >> (nchunks - 1 - base) & 1u) && q % kChunk)
+          done -= kChunk - q % kChunk;  // the last chunk is not full
+      }
+      while (word) {  // four chunks at a time: a run box per lane
+        uint32_t w = word;
+        for (int k = 0; k < 3; ++k) w = k < (lane >> 3) ? w & (w - 1) : w;
+        for (int k = 0; k < 4; ++k) word &= word - 1;
+        bool keep = false;
+        uint32_t run = 0;
+        if (w) {
+          run = (base + uint32_t(__ffs(int(w)) - 1)) * kSubs + (lane & 7);
+          if (uint64_t(run) * kSubVotes < q) {
+            const float4 *b4 = reinterpret_cast<const float4 *>(sbox + uint64_t(run) * 12);
+            const float4 a = b4[0], b = b4[1], c = b4[2];
+            const float box[12] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w};
+            keep = box_gap2(lo, hi, box) <= skip_gap2;
+          }
+        }
+        for (unsigned todo = __ballot_sync(0xffffffffu, keep); todo; todo &= todo - 1)
+          finish(true, __shfl_sync(0xffffffffu, run, __ffs(int(todo)) - 1));
+      }
+    }
+    finish(false, 0);
+    if (COUNT) {
+      if (live && members) atomicAdd(&counts[seed], (unsigned long long)members);
+    } else if (live) {
+      // split-major layout: value d of slot s of split p at (p * kPartial + d) *
+      // slots + s, so the reduction reads consecutive seeds contiguously
+      T *out = partial + uint64_t(split) * kPartial * grid.slots + slot;
+      for (int d = 0; d < 7; ++d) out[d * grid.slots] = acc[d];
+      if (newton)
+        for (int j = 0; j < 27; ++j) out[(8 + j) * grid.slots] = ns[j * kChunk];
+    }
+    if (done) atomicAdd(evals, done * (unsigned long long)kChunk);
+    if (!items) {
+      if (!COUNT && quarter == 0 && lane == 0) touch(touched, grid.words, tile, split);
+      return;
     }
   }
-  // split-major layout: value d of slot s of split p at (p * stride + d) *
-  // slots + s, so the reduction reads consecutive seeds contiguously
-  T *out = partial + split * stride * slots + slot;
-  for (int d = 0; d < 7; ++d) out[d * slots] = acc[d];
-  if (newton)
-    for (int j = 0; j < 27; ++j) out[(8 + j) * slots] = nsum[j * kChunk + threadIdx.x];
-  if (threadIdx.x == 0 && done && evals) atomicAdd(evals, done * (unsigned long long)kChunk);
 }
 
 // b <- M^-1 b by Gaussian elimination with partial pivoting; false when a
@@ -359,23 +584,60 @@ __device__ bool solve6(T (&M)[6][6], T (&b)[6], T tiny) {
 // Sum of the splits of one value of a tile's seeds: block (tile, j, g) adds
 // value d = j (j < 7) or j + 1 (the Newton sums) over split group g (splits
 // g, g + kGroups, ...), one thread per seed slot, so each split's row of 128
-// values is read contiguously.  red[(g * kPartial + d) * slots + slot] = the
-// group's sum; ms_update adds the groups in order.
-constexpr int kGroups = 8;
+// values is read contiguously.  The i-th split of the group goes into the
+// sum i % 2, and only the touched splits are read: their positions come
+// from the set bits of the group's words.  red[(g * kPartial + d) * slots +
+// slot] = the group's sum; ms_update adds the groups in order.  Each half of
+// the block takes one of the two sums.  Bound by the latency of the loads: 16
+// are in flight per thread.  (Reading every split, two loads in flight, took
+// 148 us per iteration on the 5.1e6-pair torus with 256 seeds, 70 MB of zeros
+// mostly; 21 us now.)
+constexpr int kReduceWords = 32;  // words of touched splits listed at a time
 template <typename T>
-__global__ void __launch_bounds__(kChunk) ms_reduce(const T *partial, uint64_t splits, uint64_t slots,
-                                                    uint64_t nactive, T *red) {
-  const uint64_t slot = uint64_t(blockIdx.x) * kChunk + threadIdx.x;
-  if (slot >= nactive) return;
+__global__ void __launch_bounds__(2 * kChunk) ms_reduce(const T *partial, Grid grid, uint64_t nactive,
+                                                        const uint32_t *touched, T *red) {
+  __shared__ uint16_t list[2][kReduceWords * 16];
+  __shared__ int count[2];
+  __shared__ T other[kChunk];
+  const int half = threadIdx.x >= kChunk, t = threadIdx.x % kChunk, lane = threadIdx.x & 31;
+  const uint64_t slot = uint64_t(blockIdx.x) * kChunk + t;
   const int d = blockIdx.y < 7 ? int(blockIdx.y) : int(blockIdx.y) + 1;
   const uint64_t g = blockIdx.z;
-  const T *in = partial + uint64_t(d) * slots + slot;
-  const uint64_t step = uint64_t(kPartial) * slots;
-  T s0 = 0, s1 = 0;  // two interleaved sums, added in a fixed order
-  uint64_t p = g;
-  for (; p + kGroups < splits; p += 2 * kGroups) s0 += in[p * step], s1 += in[(p + kGroups) * step];
-  if (p < splits) s0 += in[p * step];
-  red[(g * kPartial + d) * slots + slot] = s0 + s1;
+  const T *in = partial + (g * kPartial + uint64_t(d)) * grid.slots + slot;
+  const uint64_t step = uint64_t(kGroups) * kPartial * grid.slots;
+  const uint32_t *words = touched + (uint64_t(blockIdx.x) * kGroups + g) * grid.words;
+  const bool live = slot < nactive;
+  T sum = 0;
+  for (uint32_t w0 = 0; w0 < grid.words; w0 += kReduceWords) {
+    if (t < 32) {  // one warp per half lists its touched splits, ascending
+      const uint32_t i = w0 + lane;
+      uint32_t m = (i < grid.words ? words[i] : 0u) & (half ? 0xAAAAAAAAu : 0x55555555u);
+      const int n = __popc(m);
+      int incl = n;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      for (int at = incl - n; m; m &= m - 1) list[half][at++] = uint16_t(lane * 32 + __ffs(int(m)) - 1);
+      if (lane == 31) count[half] = incl;
+    }
+    __syncthreads();
+    const int n = count[half];
+    const T *base = in + uint64_t(w0) * 32 * step;
+    constexpr int kAhead = 16;  // loads in flight per thread
+    if (live)
+      for (int k = 0; k < n; k += kAhead) {
+        T v[kAhead];
+#pragma unroll
+        for (int a = 0; a < kAhead; ++a) v[a] = k + a < n ? base[list[half][k + a] * step] : T(0);
+#pragma unroll
+        for (int a = 0; a < kAhead; ++a) sum += v[a];  // past the end: zeros, which change nothing
+      }
+    __syncthreads();
+  }
+  if (half) other[t] = sum;
+  __syncthreads();
+  if (!half && live) red[(g * kPartial + d) * grid.slots + slot] = sum + other[t];
 }
 
 // One thread per seed: the step from the summed values (ms_reduce).
@@ -434,6 +696,8 @@ __global__ void __launch_bounds__(kChunk) ms_update(T *means, const T *red, uint
     state[s] = polish_it < kNewtonCap && st_s == kNear ? kNearRetry1 : kSettled;
   }
 }
+
+constexpr uint64_t kListedPairs = 32768;  // (tile, chunk) pairs from which the items pay (listed)
 
 constexpr int kRetile = 2048;  // seeds sorted in one block (static shared memory)
 
@@ -568,19 +832,6 @@ __global__ void gather_seeds(const T *desc, const int64_t *pos, uint64_t k, T *m
   for (int d = 0; d < 8; ++d) means[i * 8 + d] = desc[uint64_t(pos[i]) * 8 + d];
 }
 
-__global__ void sum_counts(const float *partial, uint64_t splits, uint64_t slots, const int32_t *ids,
-                           uint64_t n, unsigned long long *counts) {
-  uint64_t slot = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (slot >= n) return;
-  unsigned long long c = 0;
-  for (uint64_t p = 0; p < splits; ++p) c += (unsigned long long)partial[(p * 8 + 6) * slots + slot];
-  counts[ids[slot]] = c;
-}
-
-struct Grid {
-  uint64_t tiles, splits, cps, slots;
-};
-
 Grid grid_for(uint64_t nactive, uint64_t nchunks, int blocks_per_sm) {
   Grid g;
   g.tiles = (nactive + kChunk - 1) / kChunk;
@@ -589,7 +840,96 @@ Grid grid_for(uint64_t nactive, uint64_t nchunks, int blocks_per_sm) {
   g.cps = (nchunks + g.splits - 1) / g.splits;
   g.splits = (nchunks + g.cps - 1) / g.cps;
   g.slots = g.tiles * kChunk;
+  g.words = uint32_t(((g.splits + kGroups - 1) / kGroups + 31) / 32);
   return g;
+}
+
+// Whether an iteration draws its work from split_items' list: with few
+// (tile, chunk) pairs the direct grid's own tests cost less than the three list
+// kernels (us per iteration, direct and listed: 44 and 61 at 940 pairs, 71 and
+// 80 at 18,750 pairs, 300 and 160 at 160,000 pairs).
+bool listed(const Grid &g, uint64_t nchunks) { return g.tiles * nchunks >= kListedPairs; }
+
+// Scratch of one ms_tile launch, sized for `k` seeds.
+struct TileWork {
+  uint32_t *work = nullptr;     // [items, next item], then `touched`, then `bits`: zeroed together
+  uint32_t *touched = nullptr, *bits = nullptr;
+  uint32_t bwords = 0, nblk = 0;
+  uint64_t max_splits = 0;      // tiles x splits never exceeds it
+  float *boxes = nullptr;
+  uint32_t *sblk = nullptr, *nsurv = nullptr;
+  uint2 *pairs = nullptr, *items = nullptr;
+  unsigned list_ctas = 0;
+};
+
+template <typename T>
+TileWork tile_work(Call &call, const VoteSet &v, uint64_t k) {
+  TileWork w;
+  const uint64_t tiles = (k + kChunk - 1) / kChunk;
+  w.nblk = uint32_t(v.nblocks);
+  w.bwords = w.nblk * (kBlockChunks / 32);
+  // splits <= blocks * 152 / tiles + 1 each; a group's words round up
+  w.max_splits = uint64_t(v.tuning.simt_blocks_per_sm) * 152 + 2 * tiles;
+  const uint64_t touch_words = w.max_splits / 32 + (tiles + 1) * kGroups * 2;
+  w.work = call.alloc<uint32_t>(kWorkSize + touch_words + tiles * w.bwords);
+  w.touched = w.work + kWorkSize;
+  w.boxes = call.alloc<float>(tiles * kBoxFloats);
+  w.sblk = call.alloc<uint32_t>(tiles * w.nblk);
+  w.nsurv = call.alloc<uint32_t>(tiles);
+  w.pairs = call.alloc<uint2>(w.max_splits);
+  w.items = call.alloc<uint2>(w.max_splits * (kChunk / 32) * kQueues);
+  static const int per_sm = [] {
+    int a = 0;
+    SYM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, split_items<T>, kListThreads, 0));
+    return std::max(1, a);
+  }();
+  w.list_ctas = unsigned(std::max<uint64_t>(tiles, uint64_t(152) * per_sm));
+  return w;
+}
+
+// One ms_tile launch (and, listed, the work items before it) over n seeds.
+template <typename T, bool COUNT, bool NEWTON, bool GAUSS>
+void run_tiles(Call &call, const VoteSet &v, const T *desc, const T *means, const uint8_t *state,
+               const int32_t *ids, const unsigned *nact, uint64_t n, double h2, const Grid &g,
+               TileWork &w, T *partial, unsigned long long *counts, unsigned long long *evals) {
+  cudaStream_t st = call.stream();
+  const float gap = float(std::sqrt(h2)) + 1e-6f, gap2 = gap * gap;
+  const uint64_t touch_words = g.tiles * kGroups * g.words;
+  const bool list = listed(g, v.nchunks);
+  w.bits = w.touched + touch_words;
+  SYM_CUDA(cudaMemsetAsync(w.work, 0, (kWorkSize + touch_words + (list ? g.tiles * w.bwords : 0)) * 4, st));
+  const T k = T(v.kernel_k);
+  if (!list) {
+    ms_tile<T, COUNT, NEWTON, GAUSS><<<dim3(unsigned(g.tiles), unsigned(g.splits)), kChunk, 0, st>>>(
+        desc, v.sbox, uint32_t(v.nchunks), v.q, means, state, ids, uint32_t(n), T(h2), k, gap2, g,
+        w.touched, nullptr, 0, nullptr, 0, nullptr, partial, counts, evals);
+    check_launch();
+    call.launched();
+    return;
+  }
+  tile_boxes<T><<<unsigned(g.tiles), kCullThreads, 0, st>>>(means, ids, nact, v.bbox, w.nblk, gap2,
+                                                            w.boxes, w.sblk, w.nsurv, nullptr);
+  check_launch();
+  split_items<T><<<w.list_ctas, kListThreads, 0, st>>>(
+      w.boxes, means, ids, nact, v.cbox, v.bbox, uint32_t(v.nchunks), w.sblk, w.nsurv, w.nblk, gap2,
+      uint32_t(g.cps), g.words, w.bwords, w.bits, w.touched, w.pairs, w.work);
+  check_launch();
+  const uint32_t room = uint32_t(w.max_splits * (kChunk / 32));
+  weigh_items<<<blocks_for(g.tiles * g.splits), kThreads, 0, st>>>(
+      w.pairs, nact, w.bits, w.bwords, uint32_t(g.cps), uint32_t(v.nchunks), room, w.items, w.work);
+  check_launch();
+  static const int per_sm = [] {
+    int a = 0;
+    SYM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, ms_tile<T, COUNT, NEWTON, GAUSS>,
+                                                           kChunk, 0));
+    return std::max(1, a);
+  }();
+  const unsigned ctas = unsigned(std::min<uint64_t>(g.tiles * g.splits, uint64_t(152) * per_sm));
+  ms_tile<T, COUNT, NEWTON, GAUSS><<<ctas, kChunk, 0, st>>>(
+      desc, v.sbox, uint32_t(v.nchunks), v.q, means, state, ids, uint32_t(n), T(h2), k, gap2, g,
+      w.touched, w.bits, w.bwords, w.items, room, w.work, partial, counts, evals);
+  check_launch();
+  call.launched(4);
 }
 
 template <typename T>
@@ -604,7 +944,7 @@ int shift_impl(Call &call, const VoteSet &v, const T *desc, T *means, uint8_t *s
   uint64_t cap = (uint64_t(bps) * 152 + 2) * uint64_t(kChunk) + std::max<uint64_t>(k, kChunk) * 2;
   T *partial = call.alloc<T>(cap * kPartial);
   T *red = call.alloc<T>(uint64_t(kGroups) * kPartial * std::max<uint64_t>(k, kChunk) * 2);
-  float gap = float(std::sqrt(h2)) + 1e-6f;
+  TileWork work = tile_work<T>(call, v, k);
   int it = 0;
   for (; it < max_iter; ++it) {
     retile<T><<<1, 1024, 0, st>>>(means, state, k, v.gbox, polish, ids, nact);
@@ -617,25 +957,20 @@ int shift_impl(Call &call, const VoteSet &v, const T *desc, T *means, uint8_t *s
     if (!n) break;
     if (seed_iterations) *seed_iterations += n;
     if (trace && it < trace_len) trace[it] = n;
-    Grid g = grid_for(n, v.nchunks, bps);
-    if (g.splits * g.slots > cap) fail(SYM_RUNTIME_ERROR, "mean-shift partial buffer too small");
-    const dim3 grid(unsigned(g.tiles), unsigned(g.splits));
-    if (counts[1])
-      ms_tile<T, false, true><<<grid, kChunk, 0, st>>>(desc, v.cbox, v.bbox, v.sbox, v.nchunks, v.q, means, state, ids,
-                                                      n, T(h2), T(v.kernel_k), gap * gap, g.cps,
-                                                      partial, evals);
-    else
-      ms_tile<T, false, false><<<grid, kChunk, 0, st>>>(desc, v.cbox, v.bbox, v.sbox, v.nchunks, v.q, means, state,
-                                                       ids, n, T(h2), T(v.kernel_k), gap * gap,
-                                                       g.cps, partial, evals);
-    check_launch();
-    ms_reduce<T><<<dim3(unsigned(g.tiles), counts[1] ? 34u : 7u, kGroups), kChunk, 0, st>>>(
-        partial, g.splits, g.slots, n, red);
+    const Grid g = grid_for(n, v.nchunks, bps);
+    if (g.splits * g.slots > cap || g.splits * g.tiles > work.max_splits)
+      fail(SYM_RUNTIME_ERROR, "mean-shift partial buffer too small");
+    const bool gauss = v.kernel_k > 0;
+    const auto tiles = counts[1] ? (gauss ? run_tiles<T, false, true, true> : run_tiles<T, false, true, false>)
+                                 : (gauss ? run_tiles<T, false, false, true> : run_tiles<T, false, false, false>);
+    tiles(call, v, desc, means, state, ids, nact, n, h2, g, work, partial, nullptr, evals);
+    ms_reduce<T><<<dim3(unsigned(g.tiles), counts[1] ? 34u : 7u, kGroups), 2 * kChunk, 0, st>>>(
+        partial, g, n, work.touched, red);
     check_launch();
     ms_update<T><<<unsigned(g.tiles), kChunk, 0, st>>>(means, red, g.slots, ids, n, T(h2),
                                                        T(v.kernel_k), polish ? it : -1, state);
     check_launch();
-    call.launched(3);
+    call.launched(2);
   }
   return it;
 }
@@ -736,16 +1071,12 @@ void count_within(Call &call, const VoteSet &v, const float *points, uint64_t nm
   unsigned *nact = call.alloc<unsigned>(2);
   retile<float><<<1, 1024, 0, st>>>(points, state, nm, v.gbox, false, ids, nact);
   check_launch();
-  Grid g = grid_for(nm, v.nchunks, v.tuning.simt_blocks_per_sm);
-  float *partial = call.alloc<float>(g.splits * g.slots * 8);
-  float gap = float(std::sqrt(h2)) + 1e-6f;
-  ms_tile<float, true, false><<<dim3(unsigned(g.tiles), unsigned(g.splits)), kChunk, 0, st>>>(
-      v.desc, v.cbox, v.bbox, v.sbox, v.nchunks, v.q, points, nullptr, ids, nm, float(h2), 0.f, gap * gap, g.cps,
-      partial, nullptr);
-  check_launch();
-  sum_counts<<<blocks_for(nm), kThreads, 0, st>>>(partial, g.splits, g.slots, ids, nm, counts);
-  check_launch();
-  call.launched(3);
+  const Grid g = grid_for(nm, v.nchunks, v.tuning.simt_blocks_per_sm);
+  TileWork work = tile_work<float>(call, v, nm);
+  SYM_CUDA(cudaMemsetAsync(counts, 0, nm * sizeof(*counts), st));
+  run_tiles<float, true, false, false>(call, v, v.desc, points, nullptr, ids, nact, nm, h2, g, work,
+                                static_cast<float *>(nullptr), counts, nullptr);
+  call.launched();
 }
 
 }  // namespace sym

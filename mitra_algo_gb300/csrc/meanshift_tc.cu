@@ -22,6 +22,7 @@
 // (cp.async.bulk + mbarrier complete_tx) stages a chunk.  Every mbarrier wait
 // is bounded; on timeout the CTA records a status, drains its copies and
 // MMAs, and frees its TMEM.
+#include "chunk_lists.cuh"
 #include "meanshift_fast.cuh"
 #include "primitives.cuh"
 
@@ -323,131 +324,12 @@ __global__ void build_images(const float *desc, uint64_t q, uint64_t nchunks, co
   for (int w = t; w < int(kImage / 16); w += kChunk) dst[w] = src[w];
 }
 
-__device__ __forceinline__ float box_gap2_tc(const float *lo, const float *hi, const float *b) {
-  float g = 0;
-  for (int k = 0; k < 6; ++k) {
-    float d = fmaxf(fmaxf(b[k] - hi[k], lo[k] - b[6 + k]), 0.f);
-    g += d * d;
-  }
-  return g;
-}
-
 // ------------------------------------------------- work lists per tile
-// The number of active seeds n = nact[0] is read on the device by every
-// kernel of an iteration, so the host never waits for it: grids are sized
-// for all k seeds and blocks past the active tiles return at once.
-__device__ __forceinline__ uint32_t active_tiles(const unsigned *nact) {
-  return (nact[0] + kChunk - 1) / kChunk;
-}
-
-// boxes[t * kBoxFloats ..]: the box of tile t's active seeds (12 floats:
-// lo, hi), then the boxes of its eight groups of 16 seeds (one block per
-// tile).  Then the block cull: sblk[t * nblk ..] lists, in ascending order,
-// the blocks of kBlockChunks chunks whose box lies within the bandwidth of
-// the tile's box and of some group's box (exact, as the chunk tests), and
-// nsurv[t] counts them; their counts bcount[t * nblk + j] are zeroed.
-constexpr int kGroupSeeds = 16, kBoxFloats = 12 * (1 + kChunk / kGroupSeeds);
-constexpr int kCullThreads = 512;  // threads of tile_boxes (the first kChunk hold the seeds)
-__global__ void __launch_bounds__(kCullThreads) tile_boxes(const float *means, const int32_t *ids,
-                                                           const unsigned *nact, const float *bbox,
-                                                           uint32_t nblk, float skip_gap2,
-                                                           float *boxes, uint32_t *sblk,
-                                                           uint32_t *nsurv, uint32_t *bcount) {
-  __shared__ float part[kChunk / kGroupSeeds][12];
-  __shared__ float tb[kBoxFloats];
-  __shared__ uint32_t warp_cnt[kCullThreads / 32], base_s;
-  if (blockIdx.x >= active_tiles(nact)) return;
-  if (threadIdx.x < kChunk) {  // whole warps
-    const uint64_t slot = uint64_t(blockIdx.x) * kChunk + threadIdx.x;
-    const bool live = slot < nact[0];
-    float lo[6], hi[6];
-    for (int d = 0; d < 6; ++d) {
-      float m = live ? means[uint64_t(ids[slot]) * 8 + d] : 0.f;
-      lo[d] = live ? m : INFINITY, hi[d] = live ? m : -INFINITY;
-    }
-    for (int o = kGroupSeeds / 2; o; o >>= 1)  // within each group of 16 lanes
-      for (int d = 0; d < 6; ++d) {
-        lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
-        hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
-      }
-    const int group = threadIdx.x / kGroupSeeds;
-    if (threadIdx.x % kGroupSeeds == 0)
-      for (int d = 0; d < 6; ++d) part[group][d] = lo[d], part[group][6 + d] = hi[d];
-  }
-  if (threadIdx.x == 0) base_s = 0;
-  __syncthreads();
-  float *out = boxes + uint64_t(blockIdx.x) * kBoxFloats;
-  constexpr int kGroups = kChunk / kGroupSeeds;
-  if (threadIdx.x < 12) {
-    float v = part[0][threadIdx.x];
-    for (int w = 1; w < kGroups; ++w)
-      v = threadIdx.x < 6 ? fminf(v, part[w][threadIdx.x]) : fmaxf(v, part[w][threadIdx.x]);
-    out[threadIdx.x] = v, tb[threadIdx.x] = v;
-  } else if (threadIdx.x < kBoxFloats) {
-    const float v = part[(threadIdx.x - 12) / 12][(threadIdx.x - 12) % 12];
-    out[threadIdx.x] = v, tb[threadIdx.x] = v;
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t *mine = sblk + uint64_t(blockIdx.x) * nblk;
-  for (uint32_t b0 = 0; b0 < nblk; b0 += kCullThreads) {
-    const uint32_t b = b0 + threadIdx.x;
-    bool keep = false;
-    if (b < nblk) {
-      float bb[12];
-      for (int d = 0; d < 12; ++d) bb[d] = bbox[uint64_t(b) * 12 + d];
-      if (box_gap2_tc(tb, tb + 6, bb) <= skip_gap2)
-        for (int g = 0; g < kGroups && !keep; ++g)
-          keep = box_gap2_tc(tb + 12 + 12 * g, tb + 18 + 12 * g, bb) <= skip_gap2;
-    }
-    const uint32_t bal = __ballot_sync(0xffffffffu, keep);
-    if (lane == 0) warp_cnt[warp] = __popc(bal);
-    __syncthreads();
-    uint32_t before = base_s, total = 0;
-    for (int w = 0; w < kCullThreads / 32; ++w) {
-      if (w < warp) before += warp_cnt[w];
-      total += warp_cnt[w];
-    }
-    if (keep) {
-      const uint32_t at = before + __popc(bal & ((1u << lane) - 1u));
-      mine[at] = b;
-      bcount[uint64_t(blockIdx.x) * nblk + at] = 0;  // tile_count adds the block's kept chunks
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) base_s += total;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) nsurv[blockIdx.x] = base_s;
-}
-
-// The CTAs of a list kernel's grid shared among the active tiles: CTA i
-// serves tile i % tiles and takes every per-th of its surviving blocks,
-// starting at i / tiles (per = CTAs / tiles); false for a CTA left over.
-__device__ __forceinline__ bool list_share(const unsigned *nact, uint32_t &t, uint32_t &sub,
-                                           uint32_t &per) {
-  const uint32_t tiles = active_tiles(nact), i = blockIdx.x;
-  if (!tiles) return false;
-  per = gridDim.x / tiles;
-  if (!per || i >= per * tiles) return false;
-  t = i % tiles, sub = i / tiles;
-  return true;
-}
-
-constexpr int kListThreads = 256;  // chunks per block of the list kernels
-static_assert(kListThreads == kBlockChunks, "one thread per chunk of a block box");
-
 // need[t * nchunks + c]: some seed of tile t lies within the bandwidth of
-// chunk c's box, for the chunks of tile t's surviving blocks: tested
-// against the tile's box, each group's box (16 seeds), each quad's box (4
-// consecutive seeds), then the quad's seeds, among the seeds within the
-// bandwidth of the block's box only (a mask per block).  Exact for Epanechnikov
-// weights: every vote of a skipped chunk is farther than the bandwidth from
-// every seed of the tile; and a box holds its seeds' coordinates, so in
-// FP32 too its gap (monotone in every operation) is never above a seed's.
+// chunk c's box (chunk_needed), for the chunks of tile t's surviving blocks.
 // bcount[t * nblk + j] (zeroed by tile_boxes) gains the kept chunks of the
 // tile's j-th surviving block, one integer atomic per warp: no barrier
 // between blocks, and the counts do not depend on the order.
-constexpr int kQuads = kChunk / 4;
 __global__ void __launch_bounds__(kListThreads) tile_count(const float *boxes, const float *means,
                                                            const int32_t *ids, const unsigned *nact,
                                                            const float *cbox, const float *bbox,
@@ -455,86 +337,19 @@ __global__ void __launch_bounds__(kListThreads) tile_count(const float *boxes, c
                                                            const uint32_t *nsurv, uint32_t nblk,
                                                            float skip_gap2, uint8_t *need,
                                                            uint32_t *bcount) {
-  __shared__ float seed[kChunk * 6];
-  __shared__ float gb[kBoxFloats];
-  __shared__ float qb[kQuads * 12];
-  __shared__ bool alive[kChunk];
-  __shared__ uint32_t reach[kChunk / 32];  // seeds within the bandwidth of the block's box
+  __shared__ TileSeeds seeds;
   uint32_t t, sub, per;
   if (!list_share(nact, t, sub, per)) return;
-  const unsigned nactive = nact[0];
   const uint32_t ns = nsurv[t];
   if (sub >= ns) return;
-  for (int i = threadIdx.x; i < kChunk; i += blockDim.x) {
-    const uint64_t slot = uint64_t(t) * kChunk + i;
-    const bool live = slot < nactive;
-    alive[i] = live;
-    for (int d = 0; d < 6; ++d) seed[i * 6 + d] = live ? means[uint64_t(ids[slot]) * 8 + d] : 1e30f;
-  }
-  if (threadIdx.x < kBoxFloats) gb[threadIdx.x] = boxes[uint64_t(t) * kBoxFloats + threadIdx.x];
-  __syncthreads();
-  if (threadIdx.x < kQuads) {  // a quad without live seeds gets an empty box (gap infinite)
-    float lo[6], hi[6];
-    for (int d = 0; d < 6; ++d) lo[d] = INFINITY, hi[d] = -INFINITY;
-    for (int i = 4 * threadIdx.x; i < 4 * threadIdx.x + 4; ++i)
-      if (alive[i])
-        for (int d = 0; d < 6; ++d) lo[d] = fminf(lo[d], seed[i * 6 + d]), hi[d] = fmaxf(hi[d], seed[i * 6 + d]);
-    for (int d = 0; d < 6; ++d) qb[threadIdx.x * 12 + d] = lo[d], qb[threadIdx.x * 12 + 6 + d] = hi[d];
-  }
-  __syncthreads();
+  load_tile(seeds, t, nact[0], boxes, means, ids);
   const int lane = threadIdx.x & 31;
   uint32_t *bc = bcount + uint64_t(t) * nblk;
   for (uint32_t j = sub; j < ns; j += per) {
     const uint32_t blk = sblk[uint64_t(t) * nblk + j];
-    // the seeds that can reach the block at all: a seed beyond the
-    // bandwidth of the block's box is beyond it for each of its chunks
-    // (their boxes lie inside it), so the chunk tests skip it
-    __syncthreads();  // the previous block's mask is no longer read
-    if (threadIdx.x < kChunk) {  // whole warps
-      bool ok = false;
-      if (alive[threadIdx.x]) {
-        const float *bb = bbox + uint64_t(blk) * 12;
-        float q = 0;
-        for (int d = 0; d < 6; ++d) {
-          const float x = seed[threadIdx.x * 6 + d];
-          const float e = fmaxf(fmaxf(bb[d] - x, x - bb[6 + d]), 0.f);
-          q += e * e;
-        }
-        ok = q <= skip_gap2;
-      }
-      const unsigned bal = __ballot_sync(0xffffffffu, ok);
-      if (lane == 0) reach[threadIdx.x >> 5] = bal;
-    }
-    __syncthreads();
+    const bool keep = chunk_needed(seeds, blk, bbox, cbox, nchunks, skip_gap2);
     const uint64_t c = uint64_t(blk) * kBlockChunks + threadIdx.x;
-    bool keep = false;
-    if (c < nchunks) {
-      float cb[12];
-      for (int d = 0; d < 12; ++d) cb[d] = cbox[c * 12 + d];
-      if (box_gap2_tc(gb, gb + 6, cb) <= skip_gap2)
-        for (int g = 0; g < kChunk / kGroupSeeds && !keep; ++g) {
-          const uint32_t gm = (reach[g >> 1] >> ((g & 1) * kGroupSeeds)) & 0xffffu;
-          if (!gm) continue;
-          const float *b = gb + 12 + 12 * g;
-          if (box_gap2_tc(b, b + 6, cb) > skip_gap2) continue;
-          for (int qd = 4 * g; qd < 4 * g + 4 && !keep; ++qd) {
-            const uint32_t qm = (gm >> (4 * (qd - 4 * g))) & 0xfu;
-            if (!qm) continue;
-            if (box_gap2_tc(qb + 12 * qd, qb + 12 * qd + 6, cb) > skip_gap2) continue;
-            for (int i = 4 * qd; i < 4 * qd + 4 && !keep; ++i) {
-              if (!((qm >> (i - 4 * qd)) & 1u)) continue;
-              float q = 0;
-              for (int d = 0; d < 6; ++d) {
-                const float x = seed[i * 6 + d];
-                const float e = fmaxf(fmaxf(cb[d] - x, x - cb[6 + d]), 0.f);
-                q += e * e;
-              }
-              keep = q <= skip_gap2;
-            }
-          }
-        }
-      need[uint64_t(t) * nchunks + c] = keep;
-    }
+    if (c < nchunks) need[uint64_t(t) * nchunks + c] = keep;
     const unsigned bal = __ballot_sync(0xffffffffu, keep);
     if (lane == 0 && bal) atomicAdd(&bc[j], unsigned(__popc(bal)));
   }
