@@ -73,12 +73,13 @@ HostBvh::HostBvh(const sym_mesh_view &m) {
   } builder{*this, coord};
   if (!ids.empty()) builder.build(0, int(ids.size()), 0);
   if (depth > 31) throw Error(SYM_RUNTIME_ERROR, "verification: BVH too deep");
-  path.assign(nodes.size(), 0);
-  leaf_slot.assign(nodes.size(), -1);
-  face_leaf.assign(ids.size(), -1);
-  face_pos.assign(ids.size(), -1);
+  order.assign(ids.size(), FaceOrder{0, -1, -1, 0});
+  std::vector<uint32_t> path(nodes.size(), 0);
   std::vector<int32_t> node_depth(nodes.size(), 0), parent(nodes.size(), -1);
   int32_t leaves = 0;
+  for (size_t n = 0; n < nodes.size(); ++n) leaves += nodes[n].left < 0;
+  ancestors.assign(size_t(leaves) * 32, -1);
+  leaves = 0;
   for (size_t n = 0; n < nodes.size(); ++n) {  // parents precede their children
     const BvhNode &b = nodes[n];
     if (b.left >= 0) {
@@ -88,15 +89,21 @@ HostBvh::HostBvh(const sym_mesh_view &m) {
       path[b.left] = path[n];
       path[b.right] = path[n] | (1u << (31 - d));
     } else {
-      leaf_slot[n] = leaves++;
-      for (int32_t i = b.begin; i < b.end; ++i) face_leaf[ids[i]] = int32_t(n), face_pos[ids[i]] = i;
+      const int32_t leaf = leaves++;
+      for (int32_t i = b.begin; i < b.end; ++i) order[ids[i]] = FaceOrder{path[n], leaf, i, 0};
+      for (int32_t a = int32_t(n); a >= 0; a = parent[a]) ancestors[size_t(leaf) * 32 + node_depth[a]] = a;
     }
   }
-  ancestors.assign(size_t(leaves) * 32, -1);
-  for (size_t n = 0; n < nodes.size(); ++n)
-    if (leaf_slot[n] >= 0)
-      for (int32_t a = int32_t(n); a >= 0; a = parent[a])
-        ancestors[size_t(leaf_slot[n]) * 32 + node_depth[a]] = a;
+}
+
+// boxes32 of RefBvh: the boxes of a node's children in FP32 (an inner node's).
+__global__ void ref_boxes32(const BvhNode *nodes, uint64_t n, float4 *out) {
+  const uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= n || nodes[i].left < 0) return;
+  const BvhNode &l = nodes[nodes[i].left], &r = nodes[nodes[i].right];
+  out[3 * i] = make_float4(float(l.lo[0]), float(l.lo[1]), float(l.lo[2]), float(l.hi[0]));
+  out[3 * i + 1] = make_float4(float(l.hi[1]), float(l.hi[2]), float(r.lo[0]), float(r.lo[1]));
+  out[3 * i + 2] = make_float4(float(r.lo[2]), float(r.hi[0]), float(r.hi[1]), float(r.hi[2]));
 }
 
 RefBvh ref_bvh_upload(const HostBvh &bvh, cudaStream_t stream) {
@@ -104,9 +111,9 @@ RefBvh ref_bvh_upload(const HostBvh &bvh, cudaStream_t stream) {
   b.depth = bvh.depth;
   auto pad = [](size_t x) { return (x + 255) & ~size_t(255); };
   const size_t nn = bvh.nodes.size(), nf = bvh.ids.size(), na = bvh.ancestors.size();
-  const size_t s_nodes = pad(nn * sizeof(BvhNode)), s_face = pad(nf * 4), s_node = pad(nn * 4),
-               s_anc = pad(na * 4);
-  SYM_CUDA(cudaMalloc(&b.block, s_nodes + 3 * s_face + 2 * s_node + s_anc + 256));
+  const size_t s_nodes = pad(nn * sizeof(BvhNode)), s_ids = pad(nf * 4),
+               s_order = pad(nf * sizeof(FaceOrder)), s_anc = pad(na * 4);
+  SYM_CUDA(cudaMalloc(&b.block, s_nodes + s_ids + s_order + s_anc + nn * 48 + 256));
   char *at = b.block;
   auto put = [&](const void *src, size_t bytes, size_t room) {
     if (bytes) SYM_CUDA(cudaMemcpyAsync(at, src, bytes, cudaMemcpyHostToDevice, stream));
@@ -115,12 +122,14 @@ RefBvh ref_bvh_upload(const HostBvh &bvh, cudaStream_t stream) {
     return here;
   };
   b.nodes = reinterpret_cast<const BvhNode *>(put(bvh.nodes.data(), nn * sizeof(BvhNode), s_nodes));
-  b.ids = reinterpret_cast<const int32_t *>(put(bvh.ids.data(), nf * 4, s_face));
-  b.face_leaf = reinterpret_cast<const int32_t *>(put(bvh.face_leaf.data(), nf * 4, s_face));
-  b.face_pos = reinterpret_cast<const int32_t *>(put(bvh.face_pos.data(), nf * 4, s_face));
-  b.path = reinterpret_cast<const uint32_t *>(put(bvh.path.data(), nn * 4, s_node));
-  b.leaf_slot = reinterpret_cast<const int32_t *>(put(bvh.leaf_slot.data(), nn * 4, s_node));
+  b.ids = reinterpret_cast<const int32_t *>(put(bvh.ids.data(), nf * 4, s_ids));
+  b.order = reinterpret_cast<const FaceOrder *>(put(bvh.order.data(), nf * sizeof(FaceOrder), s_order));
   b.ancestors = reinterpret_cast<const int32_t *>(put(bvh.ancestors.data(), na * 4, s_anc));
+  b.boxes32 = reinterpret_cast<const float4 *>(at);
+  if (nn) {
+    ref_boxes32<<<blocks_for(nn), kThreads, 0, stream>>>(b.nodes, nn, reinterpret_cast<float4 *>(at));
+    check_launch();
+  }
   SYM_CUDA(cudaStreamSynchronize(stream));
   return b;
 }

@@ -79,6 +79,11 @@ __device__ inline double box_d2(D3 p, const BvhNode &n) {
   return s;
 }
 
+struct __align__(16) FaceOrder {
+  uint32_t path;
+  int32_t leaf, pos, pad;
+};
+
 // Host build in the reference's construction order (surface.h:16-50:
 // median split by std::nth_element on the longest axis, leaves of <= 8
 // faces), so that a near-first strict-< traversal visits faces in the
@@ -86,12 +91,12 @@ __device__ inline double box_d2(D3 p, const BvhNode &n) {
 struct HostBvh {
   std::vector<BvhNode> nodes;
   std::vector<int32_t> ids;
-  // the visiting order's bookkeeping: each node's path from the root (bit
-  // 31 - k = 1 when the step from depth k went to the right child), each
-  // face's leaf and position in `ids`, and each leaf's ancestors by depth
-  // (32 slots per leaf, leaf_slot[node] = the leaf's row, -1 inside)
-  std::vector<uint32_t> path;
-  std::vector<int32_t> leaf_slot, ancestors, face_leaf, face_pos;
+  // the visiting order's bookkeeping: of each face its leaf's path from the
+  // root (bit 31 - k = 1 when the step from depth k went to the right child),
+  // its leaf's row of `ancestors` and its position in `ids`; and each leaf's
+  // ancestors by depth (32 slots per leaf)
+  std::vector<FaceOrder> order;
+  std::vector<int32_t> ancestors;
   int depth = 0;
   explicit HostBvh(const sym_mesh_view &m);
 };
@@ -100,9 +105,9 @@ struct HostBvh {
 struct RefBvh {
   const BvhNode *nodes = nullptr;
   const int32_t *ids = nullptr;
-  const uint32_t *path = nullptr;
-  const int32_t *leaf_slot = nullptr, *ancestors = nullptr, *face_leaf = nullptr,
-                *face_pos = nullptr;
+  const FaceOrder *order = nullptr;
+  const int32_t *ancestors = nullptr;
+  const float4 *boxes32 = nullptr;  // 3 per node: the two children's lo[3], hi[3] in FP32
   char *block = nullptr;
   int depth = 0;
 };
@@ -117,13 +122,55 @@ void ref_bvh_free(RefBvh &b);
 // node holding a face at the minimum distance is farther than it.
 __device__ inline int32_t first_in_reference_order(const RefBvh &t, D3 q, int32_t a, int32_t b) {
   if (a == b) return a;
-  const int32_t la = t.face_leaf[a], lb = t.face_leaf[b];
-  if (la == lb) return t.face_pos[a] < t.face_pos[b] ? a : b;
-  const uint32_t pa = t.path[la], pb = t.path[lb];
-  const int depth = __clz(pa ^ pb);  // depth of the lowest common ancestor
-  const BvhNode &lca = t.nodes[t.ancestors[t.leaf_slot[la] * 32 + depth]];
+  const FaceOrder oa = t.order[a], ob = t.order[b];
+  if (oa.leaf == ob.leaf) return oa.pos < ob.pos ? a : b;
+  const int depth = __clz(oa.path ^ ob.path);  // depth of the lowest common ancestor
+  const BvhNode &lca = t.nodes[t.ancestors[int64_t(oa.leaf) * 32 + depth]];
   const bool right_first = box_d2(q, t.nodes[lca.left]) > box_d2(q, t.nodes[lca.right]);
-  const bool a_right = (pa >> (31 - depth)) & 1u;
+  const bool a_right = (oa.path >> (31 - depth)) & 1u;
+  return a_right == right_first ? a : b;
+}
+
+// A box distance in FP32 for a comparison with FP64's outcome: 0 when the
+// point lies inside by more than `margin`, the distance (good to well below
+// `margin`) when it lies outside by more than that, -1 when undecided.
+__device__ __forceinline__ float box_distance_f(float px, float py, float pz, const float *b,
+                                                float margin) {
+  const float gx = fmaxf(b[0] - px, px - b[3]), gy = fmaxf(b[1] - py, py - b[4]),
+              gz = fmaxf(b[2] - pz, pz - b[5]);
+  const float g = fmaxf(gx, fmaxf(gy, gz));
+  if (g < -margin) return 0.f;
+  if (g <= margin) return -1.f;
+  const float x = fmaxf(gx, 0.f), y = fmaxf(gy, 0.f), z = fmaxf(gz, 0.f);
+  return sqrtf(x * x + y * y + z * z);
+}
+
+// The same with the two box distances compared in FP32 where that decides
+// (um = u M, the FP32 unit at the largest coordinate magnitude: a box corner
+// and the image are each within u M of their FP64 values, so a distance is
+// within 8 u M; the margin is 32), in FP64 otherwise.
+__device__ inline int32_t first_in_reference_order_f(const RefBvh &t, D3 q, float um, int32_t a,
+                                                     int32_t b) {
+  if (a == b) return a;
+  const FaceOrder oa = t.order[a], ob = t.order[b];
+  if (oa.leaf == ob.leaf) return oa.pos < ob.pos ? a : b;
+  const int depth = __clz(oa.path ^ ob.path);
+  const int32_t node = t.ancestors[int64_t(oa.leaf) * 32 + depth];
+  const float4 *r = t.boxes32 + 3 * int64_t(node);
+  const float4 x = r[0], y = r[1], z = r[2];
+  const float left[6] = {x.x, x.y, x.z, x.w, y.x, y.y}, right[6] = {y.z, y.w, z.x, z.y, z.z, z.w};
+  const float margin = 32.f * um;
+  const float px = float(q.x), py = float(q.y), pz = float(q.z);
+  const float dl = box_distance_f(px, py, pz, left, margin),
+              dr = box_distance_f(px, py, pz, right, margin);
+  bool right_first;
+  if (dl < 0.f || dr < 0.f || (dl > 0.f && dr > 0.f && fabsf(dl - dr) <= margin)) {
+    const BvhNode &lca = t.nodes[node];
+    right_first = box_d2(q, t.nodes[lca.left]) > box_d2(q, t.nodes[lca.right]);
+  } else {
+    right_first = dl > dr;  // both inside: equal, the left one
+  }
+  const bool a_right = (oa.path >> (31 - depth)) & 1u;
   return a_right == right_first ? a : b;
 }
 
@@ -300,10 +347,10 @@ struct Lbvh {
   uint64_t nv = 0, nf = 0;
   const int32_t *faces = nullptr;  // 3 x nf (the mesh's)
   float *xyz = nullptr;            // 3 x nv, FP32 copy of the vertices
-  int32_t *child = nullptr;        // (nf - 1) x 2: >= 0 internal node, < 0 leaf ~face
-  float *box = nullptr;            // (nf - 1) x 12: the two children's lo[3], hi[3]
+  float4 *node = nullptr;          // (nf - 1) x 4: the two children's lo[3], hi[3], then their
+                                   // ids (>= 0 internal node, < 0 leaf ~face) and padding
+  float4 *face = nullptr;          // nf x 4: corners, edge and normal data (verify_fast.cu, Face)
   float *vn = nullptr;             // 3 x nv, FP32 copy of the vertex normals
-  float4 *fn = nullptr;            // nf: unit face normals from the FP64 corners, w = 1 (0: none)
   int32_t *order = nullptr;        // nv: the vertices in Morton order of their position
   double *fn64 = nullptr;          // nf x 3: unit(cross(b - a, c - a)) of each face, FP64
   char *block = nullptr;           // owns every array above (cudaMalloc)

@@ -148,7 +148,11 @@ __device__ __forceinline__ int lcp(const uint64_t *keys, int64_t n, int64_t i, i
 
 // Internal node i of n - 1 (Karras 2012): its range, split and children;
 // child < 0 encodes the leaf ~sorted position; parent_* = 2 * parent + slot.
-__global__ void lbvh_internal(const uint64_t *keys, int64_t n, int32_t *child, int32_t *parent_in,
+// A node is 64 bytes (16 words: the children's boxes lo0 hi0 lo1 hi1, then
+// their ids in words 12 and 13), so a traversal step reads it with four
+// 16-byte loads instead of 14 4-byte ones.
+constexpr int kNodeWords = 16, kNodeChild = 12;
+__global__ void lbvh_internal(const uint64_t *keys, int64_t n, int32_t *node, int32_t *parent_in,
                               int32_t *parent_leaf) {
   int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n - 1) return;
@@ -170,7 +174,7 @@ __global__ void lbvh_internal(const uint64_t *keys, int64_t n, int32_t *child, i
   const int64_t lo = i < j ? i : j, hi = i < j ? j : i;
   int32_t left = lo == gamma ? ~int32_t(gamma) : int32_t(gamma);
   int32_t right = hi == gamma + 1 ? ~int32_t(gamma + 1) : int32_t(gamma + 1);
-  child[2 * i] = left, child[2 * i + 1] = right;
+  node[i * kNodeWords + kNodeChild] = left, node[i * kNodeWords + kNodeChild + 1] = right;
   if (left < 0) parent_leaf[gamma] = int32_t(2 * i);
   else parent_in[gamma] = int32_t(2 * i);
   if (right < 0) parent_leaf[gamma + 1] = int32_t(2 * i + 1);
@@ -182,8 +186,8 @@ __global__ void lbvh_internal(const uint64_t *keys, int64_t n, int32_t *child, i
 // and carries it one level up.  Leaves are renamed from sorted positions to
 // face ids on the way.
 __global__ void lbvh_boxes(const float *xyz, uint64_t nv, const int32_t *faces, int64_t n,
-                           const int32_t *sorted_ids, int32_t *child, const int32_t *parent_in,
-                           const int32_t *parent_leaf, float *box, unsigned *arrivals) {
+                           const int32_t *sorted_ids, int32_t *nodes, const int32_t *parent_in,
+                           const int32_t *parent_leaf, unsigned *arrivals) {
   int64_t leaf = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (leaf >= n) return;
   const int32_t f = sorted_ids[leaf];
@@ -197,14 +201,15 @@ __global__ void lbvh_boxes(const float *xyz, uint64_t nv, const int32_t *faces, 
   }
   int32_t node = parent_leaf[leaf] >> 1;
   int slot = parent_leaf[leaf] & 1;
-  child[2 * node + slot] = ~f;  // leaves now name faces
+  float *box = reinterpret_cast<float *>(nodes);
+  nodes[int64_t(node) * kNodeWords + kNodeChild + slot] = ~f;  // leaves now name faces
   for (int guard = 0; guard < 128; ++guard) {
-    volatile float *dst = box + int64_t(node) * 12 + slot * 6;
+    volatile float *dst = box + int64_t(node) * kNodeWords + slot * 6;
     for (int k = 0; k < 6; ++k) dst[k] = b[k];
     __threadfence();
     if (atomicAdd(&arrivals[node], 1u) == 0) return;  // the sibling finishes the node
     __threadfence();
-    volatile const float *src = box + int64_t(node) * 12;
+    volatile const float *src = box + int64_t(node) * kNodeWords;
     for (int a = 0; a < 3; ++a) {
       b[a] = fminf(src[a], src[6 + a]);
       b[3 + a] = fmaxf(src[3 + a], src[9 + a]);
@@ -218,20 +223,28 @@ __global__ void lbvh_boxes(const float *xyz, uint64_t nv, const int32_t *faces, 
 // ------------------------------------------------------------ verification
 constexpr int kStackFast = 96;
 
-__device__ __forceinline__ float box_d2f(F3 p, const float *b) {
-  float dx = fmaxf(fmaxf(b[0] - p.x, p.x - b[3]), 0.f);
-  float dy = fmaxf(fmaxf(b[1] - p.y, p.y - b[4]), 0.f);
-  float dz = fmaxf(fmaxf(b[2] - p.z, p.z - b[5]), 0.f);
+__device__ __forceinline__ float box_d2f(F3 p, float lx, float ly, float lz, float hx, float hy,
+                                         float hz) {
+  float dx = fmaxf(fmaxf(lx - p.x, p.x - hx), 0.f);
+  float dy = fmaxf(fmaxf(ly - p.y, p.y - hy), 0.f);
+  float dz = fmaxf(fmaxf(lz - p.z, p.z - hz), 0.f);
   return dx * dx + dy * dy + dz * dz;
 }
+
+// A face as the searches read it, 64 bytes: corners a, b, c in FP32, the
+// reciprocal squared lengths of the edges ab, bc, ca, the unit normal from the
+// FP64 corners and `reach`, a bound on the edge lengths (0: no usable normal).
+struct Face {
+  F3 a, b, c, n;
+  float inv_ab, inv_bc, inv_ca, reach;
+};
 
 struct BvhView {
   uint64_t nv, nf;
   const int32_t *faces;
   const float *xyz;
-  const int32_t *child;
-  const float *box;
-  const float4 *fn;  // nf: unit face normal from the FP64 corners, w = 1 (0: none usable)
+  const float4 *node;    // nf - 1 records of four (lbvh_internal)
+  const float4 *face;    // nf records of four: (a, inv_ab), (b, inv_bc), (c, inv_ca), (n, reach)
   const int32_t *order;  // nv: query order of the vertices (Morton order of their position)
   const double *fn64;    // nf x 3: the faces' FP64 unit normals of the normal test
 };
@@ -239,9 +252,34 @@ struct BvhView {
 __device__ __forceinline__ F3 vtx(const BvhView &b, int32_t v) {
   return {b.xyz[v], b.xyz[b.nv + v], b.xyz[2 * b.nv + v]};
 }
-__device__ __forceinline__ float face_d2(const BvhView &b, F3 p, int32_t f) {
-  return triangle_d2f(p, vtx(b, b.faces[f]), vtx(b, b.faces[b.nf + f]), vtx(b, b.faces[2 * b.nf + f]));
+__device__ __forceinline__ Face load_face(const BvhView &b, int32_t f) {
+  const float4 *r = b.face + 4 * int64_t(f);
+  const float4 x = r[0], y = r[1], z = r[2], w = r[3];
+  return {{x.x, x.y, x.z}, {y.x, y.y, y.z}, {z.x, z.y, z.z}, {w.x, w.y, w.z}, x.w, y.w, z.w, w.w};
 }
+__device__ __forceinline__ float face_d2(const BvhView &b, F3 p, int32_t f) {
+  const float4 *r = b.face + 4 * int64_t(f);
+  const float4 x = r[0], y = r[1], z = r[2];
+  return triangle_d2f(p, {x.x, x.y, x.z}, {y.x, y.y, y.z}, {z.x, z.y, z.z});
+}
+
+// The children of a node and p's squared distances to their boxes.
+struct Children {
+  int32_t c0, c1;
+  float d0, d1;
+};
+__device__ __forceinline__ Children load_children(const BvhView &b, F3 p, int32_t node) {
+  const float4 *r = b.node + 4 * int64_t(node);
+  const float4 x = r[0], y = r[1], z = r[2], w = r[3];
+  return {__float_as_int(w.x), __float_as_int(w.y), box_d2f(p, x.x, x.y, x.z, x.w, y.x, y.y),
+          box_d2f(p, y.z, y.w, z.x, z.y, z.z, z.w)};
+}
+
+// A stack entry: a node and its box's squared distance, moved as one word.
+struct __align__(8) Pending {
+  int32_t node;
+  float d2;
+};
 
 // Nearest face within `best` (FP32), near-first; -1 when none.
 __device__ int32_t nearest_face_fast(const BvhView &b, F3 p, float &best, int *status) {
@@ -251,39 +289,30 @@ __device__ int32_t nearest_face_fast(const BvhView &b, F3 p, float &best, int *s
     if (d < best) best = d, face = 0;
     return face;
   }
-  int32_t stack[kStackFast];
-  float dist[kStackFast];
+  Pending stack[kStackFast];
   int top = 0;
-  stack[top] = 0, dist[top++] = 0.f;
+  stack[top++] = {0, 0.f};
   while (top) {
-    --top;
-    if (dist[top] >= best) continue;
-    const int32_t node = stack[top];
-    const float *bx = b.box + int64_t(node) * 12;
-    const int32_t c0 = b.child[2 * node], c1 = b.child[2 * node + 1];
-    float d0 = box_d2f(p, bx), d1 = box_d2f(p, bx + 6);
-    if (c0 < 0 && d0 < best) {
-      float d = face_d2(b, p, ~c0);
-      if (d < best) best = d, face = ~c0;
+    const Pending at = stack[--top];
+    if (at.d2 >= best) continue;
+    const Children k = load_children(b, p, at.node);
+    if (k.c0 < 0 && k.d0 < best) {
+      float d = face_d2(b, p, ~k.c0);
+      if (d < best) best = d, face = ~k.c0;
     }
-    if (c1 < 0 && d1 < best) {
-      float d = face_d2(b, p, ~c1);
-      if (d < best) best = d, face = ~c1;
+    if (k.c1 < 0 && k.d1 < best) {
+      float d = face_d2(b, p, ~k.c1);
+      if (d < best) best = d, face = ~k.c1;
     }
-    const bool p0 = c0 >= 0 && d0 < best, p1 = c1 >= 0 && d1 < best;
+    const bool p0 = k.c0 >= 0 && k.d0 < best, p1 = k.c1 >= 0 && k.d1 < best;
     if (top + 2 > kStackFast) {
       atomicExch(status, DS_CAPACITY);
       return face;
     }
-    if (p0 && p1) {  // the nearer child is popped first
-      bool first0 = d0 <= d1;
-      stack[top] = first0 ? c1 : c0, dist[top++] = first0 ? d1 : d0;
-      stack[top] = first0 ? c0 : c1, dist[top++] = first0 ? d0 : d1;
-    } else if (p0) {
-      stack[top] = c0, dist[top++] = d0;
-    } else if (p1) {
-      stack[top] = c1, dist[top++] = d1;
-    }
+    const bool first0 = k.d0 <= k.d1;  // the nearer child is popped first
+    if (p0 && !first0) stack[top++] = {k.c0, k.d0};
+    if (p1) stack[top++] = {k.c1, k.d1};
+    if (p0 && first0) stack[top++] = {k.c0, k.d0};
   }
   return face;
 }
@@ -316,9 +345,8 @@ __device__ __forceinline__ int32_t support_query(const BvhView &b, const double 
   const F3 qf{float(q[0]), float(q[1]), float(q[2])};
   const int32_t face = nearest_face_fast(b, qf, best, status);
   if (face < 0) return -1;
-  const F3 a = vtx(b, b.faces[face]), bb = vtx(b, b.faces[b.nf + face]),
-           cc = vtx(b, b.faces[2 * b.nf + face]);
-  F3 fn = crossf(bb - a, cc - a);
+  const Face at = load_face(b, face);
+  F3 fn = crossf(at.b - at.a, at.c - at.a);
   float len = sqrtf(dotf(fn, fn));
   if (!(len > 0.f)) return -1;
   const double ni[3] = {vn[i], vn[nv + i], vn[2 * nv + i]};
@@ -350,36 +378,49 @@ constexpr float kErr = 1.0f / 32768.0f;
 constexpr float kNormalBand = 1.0f / 1024.0f;
 constexpr int kCandidates = 16;
 
-// FP32 squared distance from p to the face (a, b, c) with unit normal n;
-// um = u M, the FP32 unit at the query's magnitude.  The plane distance
-// when p projects inside all three edges by more than their rounding band
-// (p then projects into the face), the nearest of the three edge segments
-// when it projects outside one of them by more than its band (the nearest
-// point then lies on the boundary).  Otherwise `d2` receives min(plane,
-// segments), a lower bound of the distance, and the function returns
-// false.  Band of an edge function E = (n x e) . (p - v): with |dn| <= u,
+// FP32 squared distance from p to a face with a usable normal; um = u M, the
+// FP32 unit at the query's magnitude.  The plane distance when p projects
+// inside all three edges by more than their rounding band (p then projects
+// into the face), the nearest of the edge segments when it projects outside
+// one of them by more than its band (the nearest point then lies on an edge p
+// is outside of, so edges p is inside of by more than the band need no
+// distance).  Otherwise `d2` receives min(plane, segments), a lower bound of
+// the distance, and the function returns false; also, with the plane
+// distance, when that alone is above `lim` (the caller drops the face).
+// Band of an edge function E = (n x e) . (p - v): with |dn| <= u,
 // corners within 1.8 u M and the image within 30 u M of their FP64 values,
 // and the cross and dot products' rounding, |dE| <= u (11 |e| |p - v| +
-// 3.6 M |p - v| + 32 M |e|) <= 42 u M (|p - v| + |e|) for |e| <= 3.5 M; the
-// band is 64 u M (|p - v| + |e|).
-__device__ bool face_d2n(F3 p, F3 a, F3 b, F3 c, F3 n, float um, float &d2) {
-  const F3 ab = b - a, bc = c - b, ca = a - c, ap = p - a, bp = p - b, cp = p - c;
-  const float k = 64.f * um;
-  const float ba = k * (sqrtf(dotf(ap, ap)) + sqrtf(dotf(ab, ab)));
-  const float bb = k * (sqrtf(dotf(bp, bp)) + sqrtf(dotf(bc, bc)));
-  const float bcb = k * (sqrtf(dotf(cp, cp)) + sqrtf(dotf(ca, ca)));
-  const float ea = dotf(crossf(n, ab), ap), eb = dotf(crossf(n, bc), bp), ec = dotf(crossf(n, ca), cp);
-  const float seg = fminf(segment_d2f(p, a, b), fminf(segment_d2f(p, b, c), segment_d2f(p, c, a)));
-  if (ea < -ba || eb < -bb || ec < -bcb) {
+// 3.6 M |p - v| + 32 M |e|) <= 42 u M (|p - v| + |e|) for |e| <= 3.5 M; one
+// band serves the three, 64 u M (|p - a|_1 + 2 reach) with |p - v| <= |p - a| +
+// reach and |e| <= reach (a band too wide only leaves more to FP64): six
+// square roots and three divisions fewer per face than bands and segments of
+// their own (verify_fp32 on the 1e6-triangle torus, 2e7 queries, with the
+// 64-byte nodes and faces: 72 -> 48 ms, 41 with four CTAs per SM).
+__device__ __forceinline__ bool face_d2n(F3 p, const Face &f, float um, float lim, float &d2) {
+  const F3 ap = p - f.a;
+  const float h = dotf(f.n, ap), h2 = h * h;
+  d2 = h2;
+  if (h2 > lim) return false;
+  const F3 ab = f.b - f.a, bc = f.c - f.b, ca = f.a - f.c, bp = p - f.b, cp = p - f.c;
+  const float band = 64.f * um * (fabsf(ap.x) + fabsf(ap.y) + fabsf(ap.z) + 2.f * f.reach);
+  const float ea = dotf(crossf(f.n, ab), ap), eb = dotf(crossf(f.n, bc), bp),
+              ec = dotf(crossf(f.n, ca), cp);
+  const float least = fminf(ea, fminf(eb, ec));
+  if (least > band) return true;  // inside
+  float seg = INFINITY;
+  auto segment = [&](F3 q, F3 e, float inv) {
+    const float t = __saturatef(dotf(q, e) * inv);
+    const F3 r = q - e * t;
+    seg = fminf(seg, dotf(r, r));
+  };
+  if (ea <= band) segment(ap, ab, f.inv_ab);
+  if (eb <= band) segment(bp, bc, f.inv_bc);
+  if (ec <= band) segment(cp, ca, f.inv_ca);
+  if (least < -band) {
     d2 = seg;
     return true;
   }
-  const float h = dotf(n, ap);
-  if (ea > ba && eb > bb && ec > bcb) {
-    d2 = h * h;
-    return true;
-  }
-  d2 = fminf(h * h, seg);
+  d2 = fminf(h2, seg);
   return false;
 }
 
@@ -389,10 +430,16 @@ __device__ bool face_d2n(F3 p, F3 a, F3 b, F3 c, F3 n, float um, float &d2) {
 // distance) is within 2 error bounds of min(best FP32 distance, tau +
 // bound) -- the face of smallest FP64 distance is at most 2 bounds farther
 // in FP32 than the best FP32 face.  Nodes are pruned with a slightly larger
-// radius, for the rounding of their boxes' distances.  Undecided faces are
-// listed as ~face.  Returns the count (N + 1 on overflow: faces and keys
-// hold N entries); `best` receives the smallest FP32 squared distance of a
-// decided face (INFINITY when none lies within tau + 3 bounds).
+// radius, for the rounding of their boxes' distances.  The search's window is
+// generous; the faces returned are held to the error of a decided distance
+// itself: 30 u M for the image, 2 u M for the corners, 14 u M for the normal and
+// the rounding of the products, 64 u M taken, so 128 u M from the best (with
+// the search's window, 1,024 u M, eight times as many queries found
+// neighbouring faces in it that disagree on the normal test, and went to
+// FP64).  Undecided faces are listed as ~face.  Returns the count (N + 1 on
+// overflow: faces and keys hold N entries); `best` receives the smallest FP32
+// squared distance of a decided face (INFINITY when none lies within tau + 3
+// bounds).
 template <int N = kCandidates>
 __device__ int candidate_faces(const BvhView &b, F3 p, float tau_err, float err, int32_t *faces,
                                float *keys, float &best, int *status) {
@@ -403,13 +450,10 @@ __device__ int candidate_faces(const BvhView &b, F3 p, float tau_err, float err,
   bool overflow = false;
   const float um = err * (1.f / 512.f);  // err = kErr M = 512 u M
   auto consider = [&](int32_t f, float box) {
-    const float4 fn = b.fn[f];
+    const Face face = load_face(b, f);
     float key = box;
     int32_t id = ~f;
-    if (fn.w != 0.f) {
-      const F3 a = vtx(b, b.faces[f]), bb = vtx(b, b.faces[b.nf + f]), cc = vtx(b, b.faces[2 * b.nf + f]);
-      if (face_d2n(p, a, bb, cc, F3{fn.x, fn.y, fn.z}, um, key)) id = f;
-    }
+    if (face.reach != 0.f && face_d2n(p, face, um, lim, key)) id = f;
     if (id >= 0) {
       if (key < best) {
         best = key;
@@ -434,36 +478,30 @@ __device__ int candidate_faces(const BvhView &b, F3 p, float tau_err, float err,
   if (b.nf == 1) {
     consider(0, 0.f);
   } else {
-    int32_t stack[kStackFast];
-    float dist[kStackFast];
+    Pending stack[kStackFast];
     int top = 0;
-    stack[top] = 0, dist[top++] = 0.f;
+    stack[top++] = {0, 0.f};
     while (top) {
-      --top;
-      if (dist[top] > lim_box) continue;
-      const int32_t node = stack[top];
-      const float *bx = b.box + int64_t(node) * 12;
-      const int32_t c0 = b.child[2 * node], c1 = b.child[2 * node + 1];
-      const float d0 = box_d2f(p, bx), d1 = box_d2f(p, bx + 6);
-      if (c0 < 0 && d0 <= lim_box) consider(~c0, d0);
-      if (c1 < 0 && d1 <= lim_box) consider(~c1, d1);
-      const bool p0 = c0 >= 0 && d0 <= lim_box, p1 = c1 >= 0 && d1 <= lim_box;
+      const Pending at = stack[--top];
+      if (at.d2 > lim_box) continue;
+      const Children k = load_children(b, p, at.node);
+      if (k.c0 < 0 && k.d0 <= lim_box) consider(~k.c0, k.d0);
+      if (k.c1 < 0 && k.d1 <= lim_box) consider(~k.c1, k.d1);
+      const bool p0 = k.c0 >= 0 && k.d0 <= lim_box, p1 = k.c1 >= 0 && k.d1 <= lim_box;
       if (top + 2 > kStackFast) {
         atomicExch(status, DS_CAPACITY);
         return N + 1;
       }
-      if (p0 && p1) {  // the nearer child is popped first
-        const bool first0 = d0 <= d1;
-        stack[top] = first0 ? c1 : c0, dist[top++] = first0 ? d1 : d0;
-        stack[top] = first0 ? c0 : c1, dist[top++] = first0 ? d0 : d1;
-      } else if (p0) {
-        stack[top] = c0, dist[top++] = d0;
-      } else if (p1) {
-        stack[top] = c1, dist[top++] = d1;
-      }
+      const bool first0 = k.d0 <= k.d1;  // the nearer child is popped first
+      if (p0 && !first0) stack[top++] = {k.c0, k.d0};
+      if (p1) stack[top++] = {k.c1, k.d1};
+      if (p0 && first0) stack[top++] = {k.c0, k.d0};
     }
   }
   if (overflow) return N + 1;
+  // what is left by a decided distance's own error, 64 u M
+  radius = fminf(tau_err, sqrtf(best)) + 128.f * um;
+  lim = fminf(lim, radius * radius);
   int m = 0;
   for (int j = 0; j < n; ++j)
     if (keys[j] <= lim) faces[m] = faces[j], keys[m++] = keys[j];
@@ -496,6 +534,7 @@ struct RowLists {
   uint8_t *mark;        // per query: 1 = left to the next kernel (FP64, then reference order)
   int32_t *fp64;        // queries decided in FP64, ascending
   int32_t *reference;   // queries left to the wide list, then to the reference-order BVH
+  int32_t *open;        // FP64 queries the first FP64 pass leaves to the second
   // the FP32 candidates of an FP64 query (kCandidates per slot, kNoFace
   // padded), so the FP64 decisions need no search of their own; slot_of[qid]
   // = kNoSlot for a query sent on before its candidates were known,
@@ -503,7 +542,7 @@ struct RowLists {
   uint32_t *slot_of;
   int32_t *cand;
   unsigned long long slots;    // capacity of cand, in slots
-  unsigned long long *counts;  // [forward, slots used, unused, tie]
+  unsigned long long *counts;  // [forward, slots used, open, tie]
 };
 
 // Decisions in FP32 (verify_fp32).  The reference's tests are made with
@@ -512,9 +551,9 @@ struct RowLists {
 // candidates that disagree on the normal test, or a candidate overflow send
 // the row to the FP64 decisions.  An accepted forward row is listed with its
 // candidates, the faces its FP64 distance is the smallest of.
-__global__ void verify_fp32(BvhView b, const float *vn32, const MotionF *motions, uint64_t nc,
-                            float tau, float scale, uint8_t *flags, double *err, RowLists lists,
-                            int *status) {
+__global__ void __launch_bounds__(kThreads, 4)
+    verify_fp32(BvhView b, const float *vn32, const MotionF *motions, uint64_t nc, float tau,
+                float scale, uint8_t *flags, double *err, RowLists lists, int *status) {
   // query q = (c, direction, j) takes vertex i = order[j]: the warps walk
   // neighbouring vertices; flags and errors stay per vertex (row)
   const uint64_t qid = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -587,7 +626,7 @@ __global__ void verify_fp32(BvhView b, const float *vn32, const MotionF *motions
   for (int j = 0; j < n; ++j) {
     // the face's unit normal from its FP64 corners (every candidate here
     // has one): the cosine is good to a few u
-    const float4 fn = b.fn[faces[j]];
+    const float4 fn = b.face[4 * int64_t(faces[j]) + 3];
     const float v = dotf(rn, F3{fn.x, fn.y, fn.z});
     if (fabsf(v - 0.5f) <= kNormalBand) return to_fp64_listed();
     if (v >= 0.5f) ++agree;
@@ -601,26 +640,6 @@ __global__ void verify_fp32(BvhView b, const float *vn32, const MotionF *motions
     lists.forward[k] = uint32_t(row);
     for (int j = 0; j < kCandidates; ++j) lists.faces[k * kCandidates + j] = j < n ? faces[j] : -1;
   }
-}
-
-// The reference's FP64 squared distance of each listed forward row: the
-// smallest over its candidate faces (the face it keeps is among them).
-__global__ void forward_errors(Surface s, const ClusterMotion *motions, RowLists lists,
-                               unsigned long long count, double *err) {
-  const uint64_t k = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k >= count) return;
-  const uint64_t row = lists.forward[k], nv = s.nv;
-  const uint64_t c = row / (2 * nv), i = row % (2 * nv);
-  const ClusterMotion &m = motions[c];
-  const M3 r = query_rotation(m, false);
-  const D3 q = mul(r, vertex(s, int32_t(i))) + D3{m.t[0], m.t[1], m.t[2]};
-  double dmin = INFINITY;
-  for (int j = 0; j < kCandidates; ++j) {
-    const int32_t f = lists.faces[k * kCandidates + j];
-    if (f < 0) break;
-    dmin = fmin(dmin, triangle_d2(q, corner(s, f, 0), corner(s, f, 1), corner(s, f, 2)));
-  }
-  err[c * nv + i] = dmin;
 }
 
 // The reference's normal test (verification.cpp:70-73, normal_agrees) with
@@ -685,107 +704,221 @@ __device__ int hybrid_query(const BvhView &b, const Surface &s, const double *vn
   return agree ? 1 : 0;
 }
 
+// Which corner of the face is the nearest point to p, by the region tests of
+// triangle_d2, when FP32 decides them: 0, 1, 2 for a, b, c, else -1.  p is
+// within 1.8 u M of its FP64 value, as the corners are, so a product e . (p - v)
+// is within 3.6 u M (|e| + |p - v|) of its own and its rounding within 5 u |e|
+// |p - v|; the band takes twice that and more, in 1-norms.  A decided corner
+// is the nearest point by that margin, and for faces with a usable normal
+// (corner angles with sin above 1e-6) the FP64 tests, good to 1e-16 of the same
+// products, then choose its region too: the distance is triangle_d2's
+// |p - v|^2, the same FP64 expression.
+__device__ __forceinline__ int corner_region(F3 p, const Face &f, float um) {
+  const F3 ab = f.b - f.a, ac = f.c - f.a, bc = f.c - f.b;
+  const F3 ap = p - f.a, bp = p - f.b, cp = p - f.c;
+  auto norm1 = [](F3 x) { return fabsf(x.x) + fabsf(x.y) + fabsf(x.z); };
+  const float lab = norm1(ab), lac = norm1(ac), lbc = norm1(bc);
+  const float lap = norm1(ap), lbp = norm1(bp), lcp = norm1(cp);
+  // e . v beyond its band, to the + or the - side
+  auto above = [&](float x, float le, float lv) { return x > 8.f * um * (le + lv) + 1e-6f * le * lv; };
+  if (above(-dotf(ab, ap), lab, lap) && above(-dotf(ac, ap), lac, lap)) return 0;
+  if (above(dotf(ab, bp), lab, lbp) && above(-dotf(bc, bp), lbc, lbp)) return 1;
+  if (above(dotf(ac, cp), lac, lcp) && above(dotf(bc, cp), lbc, lcp)) return 2;
+  return -1;
+}
+
+// The reference's FP64 squared distance of each listed forward row: the
+// smallest over its candidate faces (the face it keeps is among them).
+__global__ void forward_errors(Surface s, const ClusterMotion *motions, RowLists lists,
+                               unsigned long long count, double *err) {
+  const uint64_t k = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (k >= count) return;
+  const uint64_t row = lists.forward[k], nv = s.nv;
+  const uint64_t c = row / (2 * nv), i = row % (2 * nv);
+  const ClusterMotion &m = motions[c];
+  const M3 r = query_rotation(m, false);
+  const D3 q = mul(r, vertex(s, int32_t(i))) + D3{m.t[0], m.t[1], m.t[2]};
+  double dmin = INFINITY;
+  for (int j = 0; j < kCandidates; ++j) {
+    const int32_t f = lists.faces[k * kCandidates + j];
+    if (f < 0) break;
+    dmin = fmin(dmin, triangle_d2(q, corner(s, f, 0), corner(s, f, 1), corner(s, f, 2)));
+  }
+  err[c * nv + i] = dmin;
+}
+
 // The FP64 decisions of the rows verify_fp32 listed.  Where the faces at
 // the minimum disagree on the normal test, the first of them the reference's
 // search reaches takes the test (first_in_reference_order); rows whose
 // candidates overflow the list are listed for verify_listed_ref.
-__global__ void verify_rows_fp64(BvhView b, Surface s, RefBvh t, const double *vn,
-                                 const ClusterMotion *motions, double tau, float scale,
-                                 uint8_t *flags, double *err, RowLists lists,
-                                 unsigned long long count, int *status) {
+//
+// Eight lanes serve a row, two candidates each.  FP64 runs at 1/64 of the
+// FP32 rate, so it is kept to what FP32 cannot decide: a face whose nearest
+// point is one of its corners (most of a rough mesh's rows: the faces around
+// a vertex at exactly one distance) takes that vertex's |q - v|^2, eight FP64
+// operations instead of some eighty; another face is evaluated only when its
+// FP32 distance does not already put it beyond the smallest of those; the
+// normal test and the visiting order go through FP32 with a band.  A warp pays
+// for a whole distance when one of its four rows needs one, so the first pass
+// (ALL = false) leaves such rows, and those without candidates, in lists.open
+// for a second pass over them alone.  On the 1e6-triangle torus (1.1e7 rows)
+// the two take 17 and 11 ms; every candidate's distance, normal and order in
+// FP64 took 56 ms.
+template <bool ALL>
+__global__ void verify_rows_fp64(BvhView b, Surface s, RefBvh t, const double *vn, const float *vn32,
+                                 const ClusterMotion *motions, const MotionF *motions32, double tau,
+                                 float scale, uint8_t *flags, double *err, RowLists lists,
+                                 unsigned long long rows, int *status) {
   constexpr int kGroup = 8;  // lanes per row: candidates j = sub and sub + 8
-  const uint64_t gid = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  const uint64_t k = gid / kGroup;
   const int sub = threadIdx.x % kGroup;
   const unsigned group_mask = 0xffu << (threadIdx.x & 31 & ~(kGroup - 1));
-  if (k >= count) return;  // whole groups (count rows x 8 lanes)
-  const uint64_t qid = uint64_t(lists.fp64[k]), nv = b.nv;  // a query, as verify_fp32's
+  const unsigned long long count = ALL ? lists.counts[2] : rows;
+  const int32_t *list = ALL ? lists.open : lists.fp64;
+  const uint64_t nv = b.nv;
+  for (uint64_t k = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / kGroup; k < count;
+       k += uint64_t(gridDim.x) * blockDim.x / kGroup) {  // whole groups
+  const uint64_t qid = uint64_t(list[k]);  // a query, as verify_fp32's
   const uint64_t c = qid / (2 * nv), rem = qid % (2 * nv);
   const bool inverse = rem >= nv;
   const uint64_t i = uint64_t(b.order[rem % nv]);
   const uint64_t row = qid - rem % nv + i;
   const uint32_t slot = lists.slot_of[qid];
-  if (slot == kWideSlot) return;  // left marked for verify_rows_wide
+  if (slot == kWideSlot) continue;  // left marked for verify_rows_wide
+  auto leave_open = [&]() {
+    if (sub == 0) lists.open[atomicAdd(&lists.counts[2], 1ull)] = int32_t(qid);
+  };
   if (slot == kNoSlot) {  // no candidates yet: the search, on one lane
-    if (sub) return;
-    double d = 0;
-    int32_t tied[kCandidates];
-    int v = hybrid_query(b, s, vn, motions[c], inverse, i, tau, scale, d, tied, status);
-    if (v == 3) {
-      atomicAdd(&lists.counts[3], 1ull);
-      const M3 r = query_rotation(motions[c], inverse);
-      D3 q;
-      query_skipped(motions[c], r, inverse, vertex(s, int32_t(i)), tau, q);
-      int32_t first = tied[0];
-      for (int x = 1; x < kCandidates && tied[x] >= 0; ++x)
-        first = first_in_reference_order(t, q, first, tied[x]);
-      v = normal_agrees_t(b, first, r, D3{vn[i], vn[nv + i], vn[2 * nv + i]}) ? 1 : 0;
+    if (!ALL) {
+      leave_open();
+    } else if (sub == 0) {
+      double d = 0;
+      int32_t tied[kCandidates];
+      int v = hybrid_query(b, s, vn, motions[c], inverse, i, tau, scale, d, tied, status);
+      if (v == 3) {
+        atomicAdd(&lists.counts[3], 1ull);
+        const M3 r = query_rotation(motions[c], inverse);
+        D3 q;
+        query_skipped(motions[c], r, inverse, vertex(s, int32_t(i)), tau, q);
+        int32_t first = tied[0];
+        for (int x = 1; x < kCandidates && tied[x] >= 0; ++x)
+          first = first_in_reference_order(t, q, first, tied[x]);
+        v = normal_agrees_t(b, first, r, D3{vn[i], vn[nv + i], vn[2 * nv + i]}) ? 1 : 0;
+      }
+      flags[row] = v == 1;
+      if (!inverse) err[c * nv + i] = v == 1 ? d : 0.0;
+      if (v != 2) lists.mark[qid] = 0;  // marked queries go on to the reference-order search
     }
-    flags[row] = v == 1;
-    if (!inverse) err[c * nv + i] = v == 1 ? d : 0.0;
-    if (v != 2) lists.mark[qid] = 0;  // marked queries go on to the reference-order search
-    return;
+    continue;
   }
+  // the image; verify_fp32 decided the 2 tau and side tests of a row with candidates
   const ClusterMotion &m = motions[c];
   const M3 r = query_rotation(m, inverse);
-  D3 q;
-  const bool skipped = query_skipped(m, r, inverse, vertex(s, int32_t(i)), tau, q);
-  int v = 0;
-  double dmin = INFINITY;
-  if (!skipped) {
-    // the reference's FP64 distance of each candidate, and the minimum
-    const int32_t *cl = lists.cand + uint64_t(slot) * kCandidates;
-    int32_t f[2];
-    double d[2];
-    for (int h = 0; h < 2; ++h) {
-      const int32_t x = cl[sub + kGroup * h];
-      f[h] = x == kNoFace ? -1 : (x < 0 ? ~x : x);
-      d[h] = f[h] < 0 ? INFINITY
-                      : triangle_d2(q, corner(s, f[h], 0), corner(s, f[h], 1), corner(s, f[h], 2));
-      dmin = fmin(dmin, d[h]);
+  const D3 p = vertex(s, int32_t(i)), mt{m.t[0], m.t[1], m.t[2]};
+  const D3 q = inverse ? mul(r, p - mt) : mul(r, p) + mt;
+  const F3 qf{float(q.x), float(q.y), float(q.z)};
+  const float mag = fmaxf(scale, fmaxf(fabsf(qf.x), fmaxf(fabsf(qf.y), fabsf(qf.z))));
+  const float um = kErr * (1.f / 512.f) * mag;
+  // distances compare as their bits: none is negative
+  constexpr unsigned long long kNone = 0x7ff0000000000000ull;
+  auto smallest = [&](unsigned long long x) {
+    for (int o = kGroup / 2; o; o >>= 1) {
+      const unsigned long long y = __shfl_xor_sync(group_mask, x, o);
+      if (y < x) x = y;
     }
-    for (int o = kGroup / 2; o; o >>= 1) dmin = fmin(dmin, __shfl_xor_sync(group_mask, dmin, o));
-    if (dmin <= tau * tau) {
-      // the normal test of the faces at exactly the minimum
-      const D3 ni{vn[i], vn[nv + i], vn[2 * nv + i]};
-      int agree = 0, disagree = 0;
-      bool ok[2] = {false, false};
-      int32_t first = -1;  // this lane's face at the minimum the reference visits first
-      for (int h = 0; h < 2; ++h)
-        if (f[h] >= 0 && d[h] == dmin) {
-          ok[h] = normal_agrees_t(b, f[h], r, ni);
-          if (ok[h]) ++agree;
-          else ++disagree;
-          first = first < 0 ? f[h] : first_in_reference_order(t, q, first, f[h]);
-        }
+    return x;
+  };
+  const int32_t *cl = lists.cand + uint64_t(slot) * kCandidates;
+  int32_t f[2];
+  unsigned long long d[2] = {kNone, kNone};
+  bool open[2] = {false, false};
+  float key[2] = {0.f, 0.f};
+  F3 fn[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int32_t x = cl[sub + kGroup * h];
+    f[h] = x == kNoFace ? -1 : (x < 0 ? ~x : x);
+    if (f[h] < 0) continue;
+    const Face face = load_face(b, f[h]);
+    fn[h] = face.n;
+    open[h] = true;
+    if (face.reach == 0.f) continue;
+    const int v = corner_region(qf, face, um);
+    if (v >= 0) {
+      const D3 e = q - corner(s, f[h], v);
+      d[h] = __double_as_longlong(dot(e, e));
+      open[h] = false;
+    } else if (!face_d2n(qf, face, um, INFINITY, key[h])) {
+      key[h] = 0.f;
+    }
+  }
+  unsigned long long dmin = smallest(d[0] < d[1] ? d[0] : d[1]);
+  // a decided FP32 distance is within 32 u M of FP64's
+  const float beyond = dmin == kNone ? INFINITY : sqrtf(float(__longlong_as_double(dmin))) + 64.f * um;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) open[h] = open[h] && !(sqrtf(key[h]) > beyond);
+  if (ALL) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (open[h])
+        d[h] = __double_as_longlong(
+            triangle_d2(q, corner(s, f[h], 0), corner(s, f[h], 1), corner(s, f[h], 2)));
+    dmin = smallest(d[0] < d[1] ? d[0] : d[1]);
+  } else if (__ballot_sync(group_mask, open[0] || open[1]) & group_mask) {
+    leave_open();
+    continue;
+  }
+  int v = 0;
+  if (dmin <= (unsigned long long)__double_as_longlong(tau * tau)) {
+    // the normal test of the faces at exactly the minimum
+    const MotionF &mf = motions32[c];
+    float rf[9];
+    for (int j = 0; j < 9; ++j) rf[j] = inverse ? mf.r[(j % 3) * 3 + j / 3] : mf.r[j];
+    const F3 ni{vn32[i], vn32[nv + i], vn32[2 * nv + i]};
+    const F3 rn{rf[0] * ni.x + rf[1] * ni.y + rf[2] * ni.z, rf[3] * ni.x + rf[4] * ni.y + rf[5] * ni.z,
+                rf[6] * ni.x + rf[7] * ni.y + rf[8] * ni.z};
+    int agree = 0, disagree = 0;
+    bool ok[2] = {false, false};
+    int32_t first = -1;  // this lane's face at the minimum the reference visits first
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (f[h] >= 0 && d[h] == dmin) {
+        const float cosine = dotf(rn, fn[h]);
+        const bool sure = b.face[4 * int64_t(f[h]) + 3].w != 0.f && fabsf(cosine - 0.5f) > kNormalBand;
+        ok[h] = sure ? cosine > 0.5f
+                     : normal_agrees_t(b, f[h], r, D3{vn[i], vn[nv + i], vn[2 * nv + i]});
+        if (ok[h]) ++agree;
+        else ++disagree;
+        first = first < 0 ? f[h] : first_in_reference_order_f(t, q, um, first, f[h]);
+      }
+    for (int o = kGroup / 2; o; o >>= 1) {
+      agree += __shfl_xor_sync(group_mask, agree, o);
+      disagree += __shfl_xor_sync(group_mask, disagree, o);
+    }
+    if (agree && disagree) {
+      // faces at the minimum disagree: the one the reference visits first
+      // (its visiting order is a total order on the faces for this
+      // query, so the group reduces it like a minimum)
       for (int o = kGroup / 2; o; o >>= 1) {
-        agree += __shfl_xor_sync(group_mask, agree, o);
-        disagree += __shfl_xor_sync(group_mask, disagree, o);
+        const int32_t other = __shfl_xor_sync(group_mask, first, o);
+        if (other >= 0)
+          first = first < 0 ? other : first_in_reference_order_f(t, q, um, first, other);
       }
-      if (agree && disagree) {
-        // faces at the minimum disagree: the one the reference visits first
-        // (its visiting order is a total order on the faces for this
-        // query, so the group reduces it like a minimum)
-        for (int o = kGroup / 2; o; o >>= 1) {
-          const int32_t other = __shfl_xor_sync(group_mask, first, o);
-          if (other >= 0) first = first < 0 ? other : first_in_reference_order(t, q, first, other);
-        }
-        const bool mine_agrees = (f[0] == first && first >= 0 && ok[0]) || (f[1] == first && first >= 0 && ok[1]);
-        v = (__ballot_sync(group_mask, mine_agrees) & group_mask) ? 1 : 0;
-        if (sub == 0) {  // one count per converged set of groups
-          const unsigned active = __activemask();
-          const unsigned leaders = active & 0x01010101u;
-          if ((threadIdx.x & 31) == __ffs(leaders) - 1) atomicAdd(&lists.counts[3], __popc(leaders));
-        }
-      } else {
-        v = agree ? 1 : 0;
+      const bool mine_agrees = (f[0] == first && first >= 0 && ok[0]) || (f[1] == first && first >= 0 && ok[1]);
+      v = (__ballot_sync(group_mask, mine_agrees) & group_mask) ? 1 : 0;
+      if (sub == 0) {  // one count per converged set of groups
+        const unsigned active = __activemask();
+        const unsigned leaders = active & 0x01010101u;
+        if ((threadIdx.x & 31) == __ffs(leaders) - 1) atomicAdd(&lists.counts[3], __popc(leaders));
       }
+    } else {
+      v = agree ? 1 : 0;
     }
   }
   if (sub == 0) {
     flags[row] = v == 1;
-    if (!inverse) err[c * nv + i] = v == 1 ? dmin : 0.0;
+    if (!inverse) err[c * nv + i] = v == 1 ? __longlong_as_double(dmin) : 0.0;
     lists.mark[qid] = 0;
+  }
   }
 }
 
@@ -1150,29 +1283,40 @@ __global__ void count_roots(int32_t *parent_all, uint64_t nv, uint64_t sets, uns
 
 // Unit normal of every face, (b - a) x (c - a) normalised in FP64 as the
 // reference's normal test forms it (src/cpu/verification.cpp:71-75), rounded
-// to FP32, w = 1.  w = 0 when that FP64 normal is not accurate to well below
+// to FP32.  Not usable when that FP64 normal is not accurate to well below
 // an FP32 unit (|ab x ac| <= 1e-6 |ab| |ac|: its direction error is about
 // 1e-16 / sin of the corner angle), and near the reference's cut-off of
 // unit() (a cross product of norm <= 1e-14 becomes the zero vector, which
 // fails the test): those faces leave their rows to the FP64 decisions.
-__global__ void lbvh_face_normals(const double *xyz, uint64_t nv, const int32_t *faces,
-                                  uint64_t nf, float4 *fn, double *fn64) {
+// The FP32 record of the face (Face) goes with it: its corners, reciprocal
+// squared edge lengths and, where the normal is usable, a bound on its edge
+// lengths.
+__global__ void lbvh_face_records(const double *xyz, uint64_t nv, const int32_t *faces, uint64_t nf,
+                                  float4 *face, double *fn64) {
   const uint64_t f = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (f >= nf) return;
   D3 c[3];
-  for (int k = 0; k < 3; ++k) {
-    const int32_t v = faces[k * nf + f];
-    c[k] = D3{xyz[v], xyz[nv + v], xyz[2 * nv + v]};
+  F3 k[3];
+  for (int i = 0; i < 3; ++i) {
+    const int32_t v = faces[i * nf + f];
+    c[i] = D3{xyz[v], xyz[nv + v], xyz[2 * nv + v]};
+    k[i] = F3{float(c[i].x), float(c[i].y), float(c[i].z)};
   }
   const D3 ab = c[1] - c[0], ac = c[2] - c[0], n = cross(ab, ac);
   const D3 u = unit(n);  // the normal test's expression (normal_agrees), once per face
   fn64[3 * f] = u.x, fn64[3 * f + 1] = u.y, fn64[3 * f + 2] = u.z;
   const double n2 = dot(n, n), l2 = dot(ab, ab) * dot(ac, ac);
-  if (!(n2 > 1e-12 * l2) || !(n2 > 4e-28)) {
-    fn[f] = make_float4(0.f, 0.f, 0.f, 0.f);
-    return;
+  const bool usable = n2 > 1e-12 * l2 && n2 > 4e-28;
+  float inv[3], longest = 0;
+  for (int i = 0; i < 3; ++i) {
+    const F3 e = k[(i + 1) % 3] - k[i];
+    const float l = dotf(e, e);
+    inv[i] = l > 0.f ? 1.f / l : 0.f;
+    longest = fmaxf(longest, l);
   }
-  fn[f] = make_float4(float(u.x), float(u.y), float(u.z), 1.f);
+  for (int i = 0; i < 3; ++i) face[4 * f + i] = make_float4(k[i].x, k[i].y, k[i].z, inv[i]);
+  face[4 * f + 3] = make_float4(float(u.x), float(u.y), float(u.z),
+                                usable ? fmaxf(sqrtf(longest) * 1.0001f, 1e-30f) : 0.f);
 }
 
 Lbvh lbvh_build(Call &call, const double *xyz, const double *vn, uint64_t nv,
@@ -1183,21 +1327,26 @@ Lbvh lbvh_build(Call &call, const double *xyz, const double *vn, uint64_t nv,
   cudaStream_t st = call.stream();
   const uint64_t ni = nf - 1;
   auto pad = [](uint64_t x) { return (x + 255) & ~uint64_t(255); };
-  const uint64_t s_xyz = pad(12 * nv), s_child = pad(8 * ni + 8), s_box = pad(48 * ni + 48);
-  const uint64_t s_fn = pad(16 * nf), s_order = pad(4 * nv), s_fn64 = pad(24 * nf);
-  SYM_CUDA(cudaMalloc(&b.block, 2 * s_xyz + s_child + s_box + s_fn + s_order + s_fn64));
-  b.xyz = reinterpret_cast<float *>(b.block);
-  b.child = reinterpret_cast<int32_t *>(b.block + s_xyz);
-  b.box = reinterpret_cast<float *>(b.block + s_xyz + s_child);
-  b.vn = reinterpret_cast<float *>(b.block + s_xyz + s_child + s_box);
-  b.fn = reinterpret_cast<float4 *>(b.block + 2 * s_xyz + s_child + s_box);
-  b.order = reinterpret_cast<int32_t *>(b.block + 2 * s_xyz + s_child + s_box + s_fn);
-  b.fn64 = reinterpret_cast<double *>(b.block + 2 * s_xyz + s_child + s_box + s_fn + s_order);
+  const uint64_t s_xyz = pad(12 * nv), s_node = pad(4 * kNodeWords * (ni + 1)),
+                 s_face = pad(64 * nf), s_order = pad(4 * nv), s_fn64 = pad(24 * nf);
+  SYM_CUDA(cudaMalloc(&b.block, 2 * s_xyz + s_node + s_face + s_order + s_fn64));
+  char *at = b.block;
+  auto take = [&](uint64_t bytes) {
+    char *r = at;
+    at += bytes;
+    return r;
+  };
+  b.node = reinterpret_cast<float4 *>(take(s_node));
+  b.face = reinterpret_cast<float4 *>(take(s_face));
+  b.xyz = reinterpret_cast<float *>(take(s_xyz));
+  b.vn = reinterpret_cast<float *>(take(s_xyz));
+  b.order = reinterpret_cast<int32_t *>(take(s_order));
+  b.fn64 = reinterpret_cast<double *>(take(s_fn64));
   lbvh_vertices<<<blocks_for(3 * nv), kThreads, 0, st>>>(xyz, nv, b.xyz);
   check_launch();
   lbvh_vertices<<<blocks_for(3 * nv), kThreads, 0, st>>>(vn, nv, b.vn);
   check_launch();
-  lbvh_face_normals<<<blocks_for(nf), kThreads, 0, st>>>(xyz, nv, faces, nf, b.fn, b.fn64);
+  lbvh_face_records<<<blocks_for(nf), kThreads, 0, st>>>(xyz, nv, faces, nf, b.face, b.fn64);
   check_launch();
   // the mesh box, for the Morton quantisation
   std::vector<float> h(3 * nv);
@@ -1230,11 +1379,12 @@ Lbvh lbvh_build(Call &call, const double *xyz, const double *vn, uint64_t nv,
     int32_t *parent_in = call.alloc<int32_t>(ni), *parent_leaf = call.alloc<int32_t>(nf);
     unsigned *arrivals = call.alloc<unsigned>(ni);
     SYM_CUDA(cudaMemsetAsync(arrivals, 0, 4 * ni, st));
-    lbvh_internal<<<blocks_for(ni), kThreads, 0, st>>>(skeys, int64_t(nf), b.child, parent_in,
+    int32_t *nodes = reinterpret_cast<int32_t *>(b.node);
+    lbvh_internal<<<blocks_for(ni), kThreads, 0, st>>>(skeys, int64_t(nf), nodes, parent_in,
                                                         parent_leaf);
     check_launch();
-    lbvh_boxes<<<blocks_for(nf), kThreads, 0, st>>>(b.xyz, nv, faces, int64_t(nf), sids, b.child,
-                                                     parent_in, parent_leaf, b.box, arrivals);
+    lbvh_boxes<<<blocks_for(nf), kThreads, 0, st>>>(b.xyz, nv, faces, int64_t(nf), sids, nodes,
+                                                     parent_in, parent_leaf, arrivals);
     check_launch();
   }
   call.launched(ni ? 8 : 6);
@@ -1248,6 +1398,10 @@ void lbvh_free(Lbvh &b) {
 }
 
 namespace {
+
+BvhView view_of(const Lbvh &b) {
+  return {b.nv, b.nf, b.faces, b.xyz, b.node, b.face, b.order, b.fn64};
+}
 
 // `refine` passes of FP64 least-squares refinement of the nc modes' motions
 // against the mesh (ICP: forward correspondences under the current motion,
@@ -1341,8 +1495,7 @@ uint64_t exact_flags(Call &call, const ResidentSurface &m, const ClusterMotion *
   lists.counts = call.alloc<unsigned long long>(4);
   uint64_t *listed = call.alloc<uint64_t>(2);
   SYM_CUDA(cudaMemsetAsync(lists.counts, 0, 32, st));
-  const BvhView view{bvh.nv, bvh.nf, bvh.faces, bvh.xyz, bvh.child, bvh.box, bvh.fn, bvh.order,
-                     bvh.fn64};
+  const BvhView view = view_of(bvh);
   Surface s{m.xyz, nv, m.faces, m.nf, nullptr, nullptr};
   verify_fp32<<<blocks_for(rows), kThreads, 0, st>>>(view, bvh.vn, dmf, nc, float(tau), bvh.scale,
                                                       flags, err, lists, call.status());
@@ -1361,11 +1514,16 @@ uint64_t exact_flags(Call &call, const ResidentSurface &m, const ClusterMotion *
   if (counts[1]) {
     ensure_ref_bvh(call, m);
     s.nodes = m.ref->dev.nodes, s.ids = m.ref->dev.ids;
-    verify_rows_fp64<<<blocks_for(counts[1] * 8), kThreads, 0, st>>>(view, s, m.ref->dev, m.vn, dm, tau,
-                                                                  bvh.scale, flags, err, lists,
-                                                                  counts[1], call.status());
+    lists.open = lists.reference;  // free until the next compaction
+    verify_rows_fp64<false><<<blocks_for(counts[1] * 8), kThreads, 0, st>>>(
+        view, s, m.ref->dev, m.vn, bvh.vn, dm, dmf, tau, bvh.scale, flags, err, lists, counts[1],
+        call.status());
     check_launch();
-    call.launched();
+    verify_rows_fp64<true><<<unsigned(std::min<uint64_t>(blocks_for(counts[1] * 8), 152 * 8)), kThreads,
+                             0, st>>>(view, s, m.ref->dev, m.vn, bvh.vn, dm, dmf, tau, bvh.scale, flags,
+                                      err, lists, 0, call.status());
+    check_launch();
+    call.launched(2);
     compact_indices(call, lists.mark, rows, lists.reference, listed + 1);
     call.d2h(&counts[2], listed + 1, 8);
     call.d2h(&counts[3], lists.counts + 3, 8);
@@ -1414,8 +1572,7 @@ void verification_fast(Call &call, const ResidentSurface &m, sym_cluster_record 
   ClusterMotion *dm = call.upload(motions.data(), nc);
   if (refine > 0 && m.nf) {
     const Lbvh &bvh = *m.lbvh;
-    const BvhView view{bvh.nv, bvh.nf, bvh.faces, bvh.xyz, bvh.child, bvh.box, bvh.fn, bvh.order,
-                     bvh.fn64};
+    const BvhView view = view_of(bvh);
     refine_motions(call, view, m.xyz, m.vn, m.w, dm, nc, tau, refine, origin);
     call.d2h(motions.data(), dm, nc * sizeof(ClusterMotion));
     call.check_status("transform refinement");
