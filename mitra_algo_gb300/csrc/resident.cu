@@ -1237,15 +1237,10 @@ sym_status sym_verification_resident(sym_context *ctx, sym_mesh_handle *mesh,
     const uint64_t nc = clusters->count;
     if (nc && (!mesh->nv || !mesh->nf))
       sym::fail(SYM_INVALID_ARGUMENT, "verification requires a nonempty surface");
-    std::vector<std::vector<int32_t>> side;
-    std::vector<std::vector<std::vector<int32_t>>> patches;
-    std::vector<double> coverage, rms;
     uint64_t n = 0;
     sym::verification_resident(call, mesh->surface(), clusters->records, nc,
-                               options->verify_threshold * mesh->model.box_size, side, patches,
-                               coverage, rms, &n);
+                               options->verify_threshold * mesh->model.box_size, *out, std::malloc, &n);
     if (undecided) *undecided = n;
-    sym::fill_verification_result(nc, side, patches, coverage, rms, *out, std::malloc);
     return SYM_OK;
   } catch (const sym::Error &e) {
     sym_error_text = e.what();

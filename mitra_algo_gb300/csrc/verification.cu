@@ -12,19 +12,22 @@
 //    near-first, strict-< traversal returns the same face on distance ties
 //    and the normal test agrees; the traversal itself runs on the GPU;
 //  * ONE launch covers every cluster, both directions and every vertex;
-//  * rms / coverage use the reference's serial summation order (one thread
-//    per cluster), so coverage is bit-exact;
+//  * rms / coverage are the reference's serial sums bit for bit, computed in
+//    parallel (serial_sum);
 //  * patches are connected components grown on the GPU with lock-free
 //    union-find that always links the larger root under the smaller one, so
 //    a component's root is its smallest vertex; a stable sort by (cluster,
 //    side, root) then yields the reference's breadth-first patch order
-//    (patches by smallest vertex, members ascending).
+//    (patches by smallest vertex, members ascending), which the device writes
+//    in the result's layout (20 clusters of an 80,000-vertex torus, 1.6e6
+//    members: building the lists on the host took some 35 ms of the call's 58).
 #include "common.cuh"
 #include "primitives.cuh"
 #include "verification.cuh"
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <limits>
 #include <numeric>
 #include <vector>
@@ -176,63 +179,188 @@ __global__ void verify_vertices(Surface s, const double *vn, const int32_t *orde
   if (!inverse) err[c * nv + i] = d;
 }
 
-// One warp per cluster (block c < nc) or for the total weight (block nc):
-// rows are staged 32 at a time in shared memory and lane 0 adds them in
-// vertex order; a group of 32 rows with no flag set is skipped (adding
-// nothing leaves the sums unchanged).
-__global__ void __launch_bounds__(32) ordered_sums_warp(const uint8_t *flags, const double *err,
-                                                         const double *w, uint64_t nv, uint64_t nc,
-                                                         double *error, double *area,
-                                                         uint64_t *count, double *total) {
-  __shared__ double sv[32], sw[32];
-  const uint64_t c = blockIdx.x;
-  const unsigned lane = threadIdx.x;
-  if (c == nc) {
-    double t = 0;
-    for (uint64_t base = 0; base < nv; base += 32) {
-      const uint64_t i = base + lane;
-      sw[lane] = i < nv ? w[i] : 0.0;
-      __syncwarp();
-      if (lane == 0) {
-        const unsigned m = nv - base < 32 ? unsigned(nv - base) : 32u;
-        for (unsigned j = 0; j < m; ++j) t += sw[j];
+// The serial sum s = ((x0 + x1) + x2) + ... in parallel, bit for bit.  While
+// the running sum stays in one binade [2^E, 2^(E+1)) it is an integer S times
+// u = 2^(E - 52), and adding x >= 0 turns S into S + k + c: k = floor(x / u), and
+// c = 1 when the rest of x / u exceeds a half, 0 when it is less, and for a
+// tie the parity of S + k (round half to even).  So an addend is a map that
+// depends only on the parity of S, two increments (even, odd), and such maps
+// compose associatively: a block-wide scan gives every prefix of a tile of
+// addends.  The first addend whose exact sum leaves the binade (S + k >= 2^53) is
+// added as it is, and the rest of the tile starts over from there: one more
+// round per binade the sum passes.  Addends that are negative or not finite, and
+// sums without a binade (infinite, not a number, next to zero), are added one by
+// one, kSerial at a time.
+struct Increment {
+  long long even, odd;  // what S gains, by its parity; at most kBeyond
+};
+constexpr long long kBeyond = 1ll << 54;  // past the end of any binade
+__device__ __forceinline__ Increment then(Increment a, Increment b) {
+  const long long even = a.even + (a.even & 1 ? b.odd : b.even);
+  const long long odd = a.odd + (a.odd & 1 ? b.even : b.odd);
+  return {even < kBeyond ? even : kBeyond, odd < kBeyond ? odd : kBeyond};
+}
+
+// floor(x / u) and the increment of x >= 0 in the binade of exponent E
+// (biased, normal).
+__device__ __forceinline__ Increment increment(double x, int E, long long &k) {
+  const unsigned long long bits = (unsigned long long)__double_as_longlong(x) & ~(1ull << 63);
+  const int e = int(bits >> 52);
+  const unsigned long long m = (bits & ((1ull << 52) - 1)) | (e ? 1ull << 52 : 0ull);
+  const int d = E - (e ? e : 1);  // x / u = m 2^-d
+  if (d <= 0) {
+    k = d > -2 ? (long long)(m << -d) : kBeyond;
+    return {k, k};
+  }
+  if (d > 53) {
+    k = 0;
+    return {0, 0};
+  }
+  k = (long long)(m >> d);
+  const unsigned long long rest = m & ((1ull << d) - 1), half = 1ull << (d - 1);
+  if (rest == half) return {k + (k & 1), k + ((k + 1) & 1)};
+  const long long up = rest > half;
+  return {k + up, k + up};
+}
+
+constexpr int kSumThreads = 1024, kSumItems = 4, kSumTile = kSumThreads * kSumItems, kSerial = 256;
+
+// The serial sum of value(0), ..., value(n - 1) by a block of kSumThreads.
+template <class Value>
+__device__ double serial_sum(uint64_t n, Value &&value) {
+  __shared__ Increment warp_sum[kSumThreads / 32];
+  __shared__ double s_shared;
+  __shared__ unsigned event_s;
+  __shared__ int rough_s;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double s = 0;
+  int rough = 0;  // the last addend was irregular: go on one by one
+  for (uint64_t pos = 0; pos < n;) {
+    const unsigned long long sb = (unsigned long long)__double_as_longlong(s);
+    const int E = int(sb >> 52);  // sign included: negative sums are not regular
+    const bool zero = sb == 0, regular = E > 64 && E < 0x7ff;
+    if (rough || !(zero || regular)) {
+      if (threadIdx.x == 0) {
+        const uint64_t end = pos + kSerial < n ? pos + kSerial : n;
+        for (uint64_t j = pos; j < end; ++j) s += value(j);
+        s_shared = s;
       }
-      __syncwarp();
+      __syncthreads();
+      s = s_shared;
+      pos += kSerial, rough = 0;
+      __syncthreads();
+      continue;
     }
-    if (lane == 0) *total = t;
-    return;
-  }
-  double e = 0, a = 0;
-  unsigned long long n = 0;
-  for (int dir = 0; dir < 2; ++dir) {
-    const uint8_t *f = flags + (c * 2 + dir) * nv;
-    for (uint64_t base = 0; base < nv; base += 32) {
-      const uint64_t i = base + lane;
-      const bool on = i < nv && f[i];
-      const unsigned mask = __ballot_sync(0xffffffffu, on);
-      if (!mask) continue;
-      sw[lane] = on ? w[i] : 0.0;
-      if (dir == 0) sv[lane] = on ? err[c * nv + i] : 0.0;
-      __syncwarp();
-      if (lane == 0)
-        for (unsigned j = 0; j < 32; ++j)
-          if (mask >> j & 1u) {
-            if (dir == 0) e += sv[j], ++n;
-            a += sw[j];
-          }
-      __syncwarp();
+    // this thread's addends
+    const uint64_t first = pos + uint64_t(threadIdx.x) * kSumItems;
+    double x[kSumItems];
+    long long k[kSumItems];
+    Increment each[kSumItems], mine{0, 0};
+#pragma unroll
+    for (int j = 0; j < kSumItems; ++j) {
+      x[j] = first + j < n ? value(first + j) : 0.0;
+      const bool odd_one = !(x[j] >= 0.0 && x[j] < INFINITY);
+      if (zero) k[j] = x[j] != 0.0 || odd_one ? kBeyond : 0, each[j] = {0, 0};
+      else if (odd_one) k[j] = kBeyond, each[j] = {0, 0};
+      else each[j] = increment(x[j], E, k[j]);
+      mine = then(mine, each[j]);
     }
+    // exclusive scan over the block
+    Increment incl = mine;
+    for (int o = 1; o < 32; o <<= 1) {
+      const Increment before{__shfl_up_sync(0xffffffffu, incl.even, o),
+                             __shfl_up_sync(0xffffffffu, incl.odd, o)};
+      if (lane >= o) incl = then(before, incl);
+    }
+    if (lane == 31) warp_sum[warp] = incl;
+    if (threadIdx.x == 0) event_s = kSumTile;
+    __syncthreads();
+    if (warp == 0) {
+      Increment w = warp_sum[lane];
+      for (int o = 1; o < 32; o <<= 1) {
+        const Increment before{__shfl_up_sync(0xffffffffu, w.even, o),
+                               __shfl_up_sync(0xffffffffu, w.odd, o)};
+        if (lane >= o) w = then(before, w);
+      }
+      warp_sum[lane] = w;  // inclusive over warps
+    }
+    __syncthreads();
+    Increment lane_before{__shfl_up_sync(0xffffffffu, incl.even, 1),
+                          __shfl_up_sync(0xffffffffu, incl.odd, 1)};
+    if (lane == 0) lane_before = {0, 0};
+    const Increment before = warp ? then(warp_sum[warp - 1], lane_before) : lane_before;
+    const unsigned long long S0 = zero ? 0 : (sb & ((1ull << 52) - 1)) | (1ull << 52);
+    // the first addend that leaves the binade
+    unsigned long long S = S0 + (unsigned long long)(S0 & 1 ? before.odd : before.even);
+    unsigned long long at_event = 0;
+    double x_event = 0;
+    unsigned event = kSumTile;
+#pragma unroll
+    for (int j = 0; j < kSumItems; ++j)
+      if (event == kSumTile) {
+        if (S + (unsigned long long)k[j] >= (1ull << 53))
+          event = threadIdx.x * kSumItems + j, at_event = S, x_event = x[j];
+        S += (unsigned long long)(S & 1 ? each[j].odd : each[j].even);
+      }
+    if (event < kSumTile) atomicMin(&event_s, event);
+    __syncthreads();
+    const double u = __longlong_as_double((long long)(E - 52) << 52);
+    if (event_s == kSumTile) {
+      if (threadIdx.x == kSumThreads - 1) s_shared = zero ? 0.0 : double(S) * u, rough_s = 0;
+    } else if (event == event_s) {
+      s_shared = (zero ? 0.0 : double(at_event) * u) + x_event;
+      rough_s = !(x_event >= 0.0 && x_event < INFINITY);
+    }
+    __syncthreads();
+    s = s_shared, rough = rough_s;
+    pos += event_s == kSumTile ? uint64_t(kSumTile) : uint64_t(event_s) + 1;
+    __syncthreads();
   }
-  if (lane == 0) error[c] = e, area[c] = a, count[c] = n;
+  return s;
+}
+
+// Block b < nc: the forward errors of cluster b (and their count); block nc + c:
+// the supporting weight of cluster c, forward vertices, then inverse ones;
+// block 2 nc: the total weight.  A vertex that does not support the cluster
+// adds zero, which leaves a sum as it is.
+__global__ void __launch_bounds__(kSumThreads) ordered_sums(const uint8_t *flags, const double *err,
+                                                            const double *w, uint64_t nv, uint64_t nc,
+                                                            double *error, double *area,
+                                                            uint64_t *count, double *total) {
+  const uint64_t b = blockIdx.x;
+  if (b == 2 * nc) {
+    const double t = serial_sum(nv, [&](uint64_t i) { return w[i]; });
+    if (threadIdx.x == 0) *total = t;
+  } else if (b >= nc) {
+    const uint64_t c = b - nc;
+    const uint8_t *f = flags + c * 2 * nv;
+    const double a =
+        serial_sum(2 * nv, [&](uint64_t i) { return f[i] ? w[i < nv ? i : i - nv] : 0.0; });
+    if (threadIdx.x == 0) area[c] = a;
+  } else {
+    __shared__ unsigned long long n_s;
+    const uint8_t *f = flags + b * 2 * nv;
+    if (threadIdx.x == 0) n_s = 0;
+    __syncthreads();
+    unsigned n = 0;
+    for (uint64_t i = threadIdx.x; i < nv; i += kSumThreads) n += f[i] != 0;
+    n = __reduce_add_sync(0xffffffffu, n);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&n_s, (unsigned long long)n);
+    const double e = serial_sum(nv, [&](uint64_t i) { return f[i] ? err[b * nv + i] : 0.0; });
+    if (threadIdx.x == 0) error[b] = e, count[b] = n_s;
+  }
 }
 
 }  // namespace
 
+// Latency-bound: some 50 scans of 4,096 addends per sum (20 clusters of an
+// 80,000-vertex torus: 0.31 ms; one warp per cluster adding in order, whose
+// every addition waits for the one before, 13.9 ms).
 void ordered_verification_sums(Call &call, const uint8_t *flags, const double *err,
                                const double *w, uint64_t nv, uint64_t nc, double *error,
                                double *area, uint64_t *count, double *total) {
-  ordered_sums_warp<<<unsigned(nc + 1), 32, 0, call.stream()>>>(flags, err, w, nv, nc, error, area,
-                                                                 count, total);
+  ordered_sums<<<unsigned(2 * nc + 1), kSumThreads, 0, call.stream()>>>(flags, err, w, nv, nc, error,
+                                                                        area, count, total);
   check_launch();
   call.launched();
 }
@@ -278,27 +406,56 @@ __global__ void unite_edges(const uint64_t *nbr_off, const int32_t *nbr, uint64_
 
 namespace {
 
-// keys for the grouping sort: (set << 32) | root, values: vertex.
-__global__ void root_keys(int32_t *parent_all, uint64_t nv, uint64_t sets, uint64_t *keys,
-                          int32_t *vals, uint8_t *allowed) {
-  uint64_t k = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k >= sets * nv) return;
-  uint64_t set = k / nv;
-  int32_t *parent = parent_all + set * nv;
-  int32_t i = int32_t(k % nv);
-  allowed[k] = parent[i] >= 0;
-  int32_t r = parent[i] >= 0 ? find_root(parent, i) : 0;
-  keys[k] = (set << 32) | uint64_t(uint32_t(r));
+// Of the k-th kept row (set * nv + vertex, ascending): its component as set *
+// nv + root, and the vertex.
+__global__ void root_keys(const int32_t *pos, uint64_t n, int32_t *parent_all, uint64_t nv,
+                          uint64_t *keys, int32_t *vals) {
+  const uint64_t k = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const uint64_t at = uint64_t(uint32_t(pos[k])), set = at / nv;
+  const int32_t i = int32_t(at - set * nv);
+  keys[k] = set * nv + uint64_t(uint32_t(find_root(parent_all + set * nv, i)));
   vals[k] = i;
 }
 
-__global__ void gather_kept(const int32_t *pos, uint64_t n, const uint64_t *keys, uint64_t nv,
-                            uint64_t *out_keys, int32_t *out_vals) {
-  uint64_t k = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+// starts[s] = the first kept row of set s, s in [0, sets].
+__global__ void set_starts(const int32_t *pos, uint64_t n, uint64_t nv, uint64_t sets,
+                           uint64_t *starts) {
+  const uint64_t s = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (s > sets) return;
+  uint64_t lo = 0, hi = n;
+  while (lo < hi) {
+    const uint64_t mid = (lo + hi) / 2;
+    if (uint64_t(uint32_t(pos[mid])) < s * nv) lo = mid + 1;
+    else hi = mid;
+  }
+  starts[s] = lo;
+}
+
+// The result's order: the forward sets' members (a) cluster by cluster, then
+// the inverse ones' (b).  sides: each set's vertices, ascending; members: the
+// same grouped by component (keys and vals sorted by component), with first[k]
+// = 1 where a component begins.
+__global__ void result_order(const int32_t *pos, const uint64_t *keys, const int32_t *vals,
+                             uint64_t n, uint64_t nv, uint64_t sets, const uint64_t *starts,
+                             const uint64_t *dest, int32_t *sides, int32_t *members,
+                             uint8_t *first) {
+  const uint64_t k = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k >= n) return;
-  uint64_t at = uint64_t(uint32_t(pos[k]));
-  out_keys[k] = keys[at];
-  out_vals[k] = int32_t(at % nv);
+  const uint64_t at = uint64_t(uint32_t(pos[k])), set = at / nv;
+  const uint64_t to = dest[set] + (k - starts[set]);
+  sides[to] = int32_t(at - set * nv);
+  members[to] = vals[k];  // a set's rows keep their places in the sort
+  first[to] = k == starts[set] || keys[k] != keys[k - 1];
+}
+
+// dest[s] = the place of set s's first member in the result's order.
+__global__ void set_places(const uint64_t *starts, uint64_t nc, uint64_t *dest) {
+  if (threadIdx.x || blockIdx.x) return;
+  uint64_t at = 0;
+  for (int dir = 0; dir < 2; ++dir)
+    for (uint64_t c = 0; c < nc; ++c)
+      dest[2 * c + dir] = at, at += starts[2 * c + dir + 1] - starts[2 * c + dir];
 }
 
 __global__ void triangle_query(const double *q, uint64_t n, double *out) {
@@ -366,69 +523,120 @@ ClusterMotion cluster_motion(const sym_cluster_record &r) {
 
 void finish_verification(Call &call, const uint8_t *flags, const double *err, const double *w,
                          const uint64_t *nbr_off, const int32_t *nbr, uint64_t nv, uint64_t nc,
-                         std::vector<std::vector<int32_t>> &side,
-                         std::vector<std::vector<std::vector<int32_t>>> &patches,
-                         std::vector<double> &coverage, std::vector<double> &rms) {
+                         sym_verification_result &out, void *(*allocate)(size_t)) {
   cudaStream_t st = call.stream();
-  side.assign(2 * nc, {});
-  patches.assign(2 * nc, {});
-  coverage.assign(nc, 0);
-  rms.assign(nc, 0);
-  if (!nc) return;
-  const uint64_t rows = nc * 2 * nv;
-  double *error = call.alloc<double>(nc), *area = call.alloc<double>(nc), *total = call.alloc<double>(1);
-  uint64_t *na = call.alloc<uint64_t>(nc);
-  ordered_verification_sums(call, flags, err, w, nv, nc, error, area, na, total);
-  int32_t *parent = call.alloc<int32_t>(rows);
-  init_parents<<<blocks_for(rows), kThreads, 0, st>>>(flags, rows, parent, nv);
-  check_launch();
-  unite_edges<<<blocks_for(rows), kThreads, 0, st>>>(nbr_off, nbr, nv, 2 * nc, parent, call.status(),
-                                                      kUniteRetries);
-  check_launch();
-  uint64_t *keys = call.alloc<uint64_t>(rows), *skeys = call.alloc<uint64_t>(rows);
-  int32_t *vals = call.alloc<int32_t>(rows), *svals = call.alloc<int32_t>(rows);
-  uint8_t *allowed = call.alloc<uint8_t>(rows);
-  root_keys<<<blocks_for(rows), kThreads, 0, st>>>(parent, nv, 2 * nc, keys, vals, allowed);
-  check_launch();
-  uint64_t *kept = call.alloc<uint64_t>(1);
-  int32_t *pos = call.alloc<int32_t>(rows);
-  compact_indices(call, allowed, rows, pos, kept);
-  uint64_t nkept = 0;
-  call.d2h(&nkept, kept, 8);
-  call.sync();
-  call.launched(3);
-  std::vector<uint64_t> hkeys(nkept);
-  std::vector<int32_t> hvals(nkept);
-  if (nkept) {
-    uint64_t *dk = call.alloc<uint64_t>(nkept);
-    int32_t *dv = call.alloc<int32_t>(nkept);
-    gather_kept<<<blocks_for(nkept), kThreads, 0, st>>>(pos, nkept, keys, nv, dk, dv);
+  const uint64_t rows = nc * 2 * nv, sets = 2 * nc;
+  uint64_t n = 0, patches = 0;  // members of all sets; their components
+  std::vector<uint64_t> starts(sets + 1, 0);
+  std::vector<int32_t> begins;  // where the components begin, in the result's order
+  int32_t *lists = nullptr, *dbegins = nullptr;
+  double *sums = nullptr;
+  if (nc) {
+    sums = call.alloc<double>(3 * nc + 1);  // error, area, count (as bits), total
+    uint64_t *na = reinterpret_cast<uint64_t *>(sums + 2 * nc);
+    ordered_verification_sums(call, flags, err, w, nv, nc, sums, sums + nc, na, sums + 3 * nc);
+    int32_t *parent = call.alloc<int32_t>(rows), *pos = call.alloc<int32_t>(rows);
+    init_parents<<<blocks_for(rows), kThreads, 0, st>>>(flags, rows, parent, nv);
     check_launch();
-    call.launched();
-    int bits = 32;
-    while ((uint64_t(1) << (bits - 32)) < 2 * nc) ++bits;
-    radix_sort_pairs(call, dk, dv, skeys, svals, nkept, bits);
-    call.d2h(hkeys.data(), skeys, nkept * 8);
-    call.d2h(hvals.data(), svals, nkept * 4);
+    unite_edges<<<blocks_for(rows), kThreads, 0, st>>>(nbr_off, nbr, nv, sets, parent, call.status(),
+                                                        kUniteRetries);
+    check_launch();
+    uint64_t *counts = call.alloc<uint64_t>(2), *dstarts = call.alloc<uint64_t>(sets + 1),
+             *dest = call.alloc<uint64_t>(sets);
+    compact_indices(call, flags, rows, pos, counts);
+    call.d2h(&n, counts, 8);
+    call.sync();
+    call.launched(2);
+    set_starts<<<blocks_for(sets + 1), kThreads, 0, st>>>(pos, n, nv, sets, dstarts);
+    check_launch();
+    set_places<<<1, 32, 0, st>>>(dstarts, nc, dest);
+    check_launch();
+    call.launched(2);
+    call.d2h(starts.data(), dstarts, (sets + 1) * 8);
+    if (n) {
+      uint64_t *keys = call.alloc<uint64_t>(n), *skeys = call.alloc<uint64_t>(n);
+      int32_t *vals = call.alloc<int32_t>(n), *svals = call.alloc<int32_t>(n);
+      lists = call.alloc<int32_t>(2 * n), dbegins = call.alloc<int32_t>(n);
+      uint8_t *first = call.alloc<uint8_t>(n);
+      root_keys<<<blocks_for(n), kThreads, 0, st>>>(pos, n, parent, nv, keys, vals);
+      check_launch();
+      int bits = 1;
+      while (bits < 64 && (rows >> bits)) ++bits;
+      radix_sort_pairs(call, keys, vals, skeys, svals, n, bits);
+      result_order<<<blocks_for(n), kThreads, 0, st>>>(pos, skeys, svals, n, nv, sets, dstarts, dest,
+                                                       lists, lists + n, first);
+      check_launch();
+      compact_indices(call, first, n, dbegins, counts + 1);
+      call.launched(2);
+      call.d2h(&patches, counts + 1, 8);
+    }
   }
-  std::vector<double> herr(nc), harea(nc);
-  std::vector<uint64_t> hna(nc);
-  double htotal = 0;
-  call.d2h(herr.data(), error, nc * 8);
-  call.d2h(harea.data(), area, nc * 8);
-  call.d2h(hna.data(), na, nc * 8);
-  call.d2h(&htotal, total, 8);
+  std::vector<double> hs(3 * nc + 1, 0.0);
+  if (nc) call.d2h(hs.data(), sums, hs.size() * 8);
   call.check_status("verification");
-  for (uint64_t k = 0; k < nkept; ++k) {
-    uint64_t set = hkeys[k] >> 32;
-    side[set].push_back(hvals[k]);
-    if (k == 0 || hkeys[k] != hkeys[k - 1]) patches[set].emplace_back();
-    patches[set].back().push_back(hvals[k]);
+  if (patches) {
+    begins.resize(patches);
+    call.d2h(begins.data(), dbegins, patches * 4);
+    call.sync();
   }
-  for (auto &sv : side) std::sort(sv.begin(), sv.end());
+  // the result block
+  uint64_t na = 0;
+  for (uint64_t c = 0; c < nc; ++c) na += starts[2 * c + 1] - starts[2 * c];
+  const uint64_t ra = uint64_t(std::lower_bound(begins.begin(), begins.end(), int64_t(na),
+                                                [](int32_t x, int64_t y) { return int64_t(uint32_t(x)) < y; }) -
+                               begins.begin());
+  const uint64_t nb = n - na, rb = patches - ra;
+  const size_t bytes = (4 * (nc + 1) + (ra + 1) + (rb + 1)) * 8 + 2 * n * 4 + 2 * nc * 8 + 256;
+  char *block = static_cast<char *>(allocate(bytes));
+  if (!block) fail(SYM_RUNTIME_ERROR, "host allocation failed");
+  out.storage = block;
+  out.cluster_count = nc;
+  uint64_t *u = reinterpret_cast<uint64_t *>(block);
+  out.side_a_offsets = u, u += nc + 1;
+  out.side_b_offsets = u, u += nc + 1;
+  out.patches_a.groups = u, u += nc + 1;
+  out.patches_b.groups = u, u += nc + 1;
+  out.patches_a.offsets = u, u += ra + 1;
+  out.patches_b.offsets = u, u += rb + 1;
+  double *dd = reinterpret_cast<double *>(u);
+  out.coverage = dd, dd += nc;
+  out.rms = dd, dd += nc;
+  int32_t *ii = reinterpret_cast<int32_t *>(dd);
+  out.side_a = ii, ii += na;
+  out.side_b = ii, ii += nb;
+  out.patches_a.indices = ii, ii += na;
+  out.patches_b.indices = ii;
+  if (n) {
+    try {
+      call.d2h(out.side_a, lists, 2 * n * 4);  // sides a, b, then members a, b
+      call.sync();
+    } catch (...) {
+      std::free(block);
+      out = sym_verification_result{};
+      throw;
+    }
+  }
+  auto fill = [&](int dir, uint64_t *off, sym_grouped_csr &pg, uint64_t base, uint64_t first,
+                  uint64_t last, uint64_t members) {
+    off[0] = 0, pg.groups[0] = 0;
+    uint64_t row = first;
+    for (uint64_t c = 0; c < nc; ++c) {
+      off[c + 1] = off[c] + starts[2 * c + dir + 1] - starts[2 * c + dir];
+      while (row < last && uint64_t(uint32_t(begins[row])) - base < off[c + 1]) ++row;
+      pg.groups[c + 1] = row - first;
+    }
+    for (uint64_t k = first; k < last; ++k) pg.offsets[k - first] = uint64_t(uint32_t(begins[k])) - base;
+    pg.offsets[last - first] = members;
+    pg.rows = last - first;
+  };
+  fill(0, out.side_a_offsets, out.patches_a, 0, 0, ra, na);
+  fill(1, out.side_b_offsets, out.patches_b, na, ra, patches, nb);
   for (uint64_t c = 0; c < nc; ++c) {
-    rms[c] = hna[c] ? std::sqrt(herr[c] / double(hna[c])) : 0;
-    coverage[c] = htotal > 0 ? std::min(1.0, harea[c] / htotal) : 0;
+    uint64_t count;
+    std::memcpy(&count, &hs[2 * nc + c], 8);
+    const double total = hs[3 * nc];
+    out.rms[c] = count ? std::sqrt(hs[c] / double(count)) : 0;
+    out.coverage[c] = total > 0 ? std::min(1.0, hs[nc + c] / total) : 0;
   }
 }
 
@@ -462,20 +670,13 @@ static std::vector<int32_t> morton_order(const sym_mesh_view &m) {
 
 // Device core of sym_verification.  Mesh arrays are device pointers; `m` is
 // the host mesh (the BVH is built on the host with the reference's
-// construction order).  Fills per (cluster, side) vertex lists, patches,
-// rms and coverage.
+// construction order).
 void verification_core(Call &call, const sym_mesh_view &m, const double *xyz, const int32_t *faces,
                        const double *vn, const double *w, const uint64_t *nbr_off,
                        const int32_t *nbr, const sym_cluster_record *records, uint64_t nc,
-                       double tau, std::vector<std::vector<int32_t>> &side,
-                       std::vector<std::vector<std::vector<int32_t>>> &patches,
-                       std::vector<double> &coverage, std::vector<double> &rms) {
+                       double tau, sym_verification_result &out, void *(*allocate)(size_t)) {
   const uint64_t nv = m.vertices.count, nf = m.faces.count;
   cudaStream_t st = call.stream();
-  if (!nc) {
-    finish_verification(call, nullptr, nullptr, w, nbr_off, nbr, nv, 0, side, patches, coverage, rms);
-    return;
-  }
   HostBvh bvh(m);
   if (2 * bvh.depth + 4 > kRefStack) fail(SYM_RUNTIME_ERROR, "verification: BVH too deep");
   Surface s;
@@ -498,61 +699,7 @@ void verification_core(Call &call, const sym_mesh_view &m, const double *xyz, co
                                                          err, call.status());
   check_launch();
   call.launched();
-  finish_verification(call, flags, err, w, nbr_off, nbr, nv, nc, side, patches, coverage, rms);
-}
-
-void fill_verification_result(uint64_t nc, const std::vector<std::vector<int32_t>> &side,
-                              const std::vector<std::vector<std::vector<int32_t>>> &patches,
-                              const std::vector<double> &coverage, const std::vector<double> &rms,
-                              sym_verification_result &out, void *(*allocate)(size_t)) {
-  uint64_t na = 0, nb = 0, ra = 0, rb = 0;
-  for (uint64_t c = 0; c < nc; ++c) {
-    na += side[2 * c].size(), nb += side[2 * c + 1].size();
-    ra += patches[2 * c].size(), rb += patches[2 * c + 1].size();
-  }
-  size_t bytes = (2 * (nc + 1) + 2 * (nc + 1) + (ra + 1) + (rb + 1)) * 8 + 2 * (na + nb) * 4 +
-                 2 * nc * 8 + 256;
-  char *block = static_cast<char *>(allocate(bytes));
-  if (!block) fail(SYM_RUNTIME_ERROR, "host allocation failed");
-  out.storage = block;
-  out.cluster_count = nc;
-  uint64_t *u = reinterpret_cast<uint64_t *>(block);
-  out.side_a_offsets = u, u += nc + 1;
-  out.side_b_offsets = u, u += nc + 1;
-  out.patches_a.groups = u, u += nc + 1;
-  out.patches_b.groups = u, u += nc + 1;
-  out.patches_a.offsets = u, u += ra + 1;
-  out.patches_b.offsets = u, u += rb + 1;
-  double *dd = reinterpret_cast<double *>(u);
-  out.coverage = dd, dd += nc;
-  out.rms = dd, dd += nc;
-  int32_t *ii = reinterpret_cast<int32_t *>(dd);
-  out.side_a = ii, ii += na;
-  out.side_b = ii, ii += nb;
-  out.patches_a.indices = ii, ii += na;
-  out.patches_b.indices = ii, ii += nb;
-  auto fill = [&](int dir, uint64_t *off, int32_t *idx, sym_grouped_csr &pg) {
-    off[0] = 0;
-    pg.groups[0] = 0;
-    pg.offsets[0] = 0;
-    uint64_t row = 0, at = 0;
-    for (uint64_t c = 0; c < nc; ++c) {
-      auto &sv = side[2 * c + dir];
-      std::copy(sv.begin(), sv.end(), idx + off[c]);
-      off[c + 1] = off[c] + sv.size();
-      for (auto &p : patches[2 * c + dir]) {
-        std::copy(p.begin(), p.end(), pg.indices + at);
-        at += p.size();
-        pg.offsets[++row] = at;
-      }
-      pg.groups[c + 1] = row;
-    }
-    pg.rows = row;
-  };
-  fill(0, out.side_a_offsets, out.side_a, out.patches_a);
-  fill(1, out.side_b_offsets, out.side_b, out.patches_b);
-  std::copy(coverage.begin(), coverage.end(), out.coverage);
-  std::copy(rms.begin(), rms.end(), out.rms);
+  finish_verification(call, flags, err, w, nbr_off, nbr, nv, nc, out, allocate);
 }
 
 void verification_host(Call &call, const sym_mesh_view &m, const sym_topology_view &g,
@@ -560,10 +707,9 @@ void verification_host(Call &call, const sym_mesh_view &m, const sym_topology_vi
                        const sym_options &o, sym_verification_result &out,
                        void *(*allocate)(size_t)) {
   const uint64_t nv = m.vertices.count, nf = m.faces.count, nc = cl.count;
-  std::vector<std::vector<int32_t>> side;
-  std::vector<std::vector<std::vector<int32_t>>> patches;
-  std::vector<double> coverage, rms;
-  if (nc) {
+  if (!nc) {
+    finish_verification(call, nullptr, nullptr, nullptr, nullptr, nullptr, nv, 0, out, allocate);
+  } else {
     if (!nv || !nf) fail(SYM_INVALID_ARGUMENT, "verification requires a nonempty surface");
     if (g.normals.count != nv || g.weight_count != nv || g.neighbors.rows != nv)
       fail(SYM_INVALID_ARGUMENT, "SoA component lengths differ");
@@ -581,9 +727,8 @@ void verification_host(Call &call, const sym_mesh_view &m, const sym_topology_vi
     uint64_t *nbr_off = call.upload(g.neighbors.offsets, nv + 1);
     int32_t *nbr = call.upload(g.neighbors.indices, nbr_count);
     verification_core(call, m, xyz, faces, vn, w, nbr_off, nbr, cl.records, nc,
-                      o.verify_threshold * ctx.box_size, side, patches, coverage, rms);
+                      o.verify_threshold * ctx.box_size, out, allocate);
   }
-  fill_verification_result(nc, side, patches, coverage, rms, out, allocate);
 }
 
 }  // namespace sym

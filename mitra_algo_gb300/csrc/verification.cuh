@@ -318,29 +318,20 @@ __global__ void unite_edges(const uint64_t *nbr_off, const int32_t *nbr, uint64_
 // Sums of the reference's verification in its serial order
 // (verification.cpp:75-77, :93-96, :98-99): per cluster the forward
 // squared distances and the supporting weight (forward vertices in vertex
-// order, then inverse ones), the forward count, and the total weight.  One
-// warp per cluster stages 32 rows at a time and adds them in order, so the
-// results equal the reference's bit for bit.  flags[(c * 2 + dir) * nv + i],
-// err[c * nv + i].
+// order, then inverse ones), the forward count, and the total weight, equal to
+// the reference's bit for bit.  flags[(c * 2 + dir) * nv + i], err[c * nv + i].
 void ordered_verification_sums(Call &call, const uint8_t *flags, const double *err,
                                const double *w, uint64_t nv, uint64_t nc, double *error,
                                double *area, uint64_t *count, double *total);
 
-// From the flags and forward errors of nc clusters: patches (connected
-// components of the supporting vertices, in the reference's breadth-first
-// order), side lists, coverage and rms, all as the reference computes them.
+// From the flags and forward errors of nc clusters: side lists, patches
+// (connected components of the supporting vertices, in the reference's
+// breadth-first order), coverage and rms, all as the reference computes them,
+// in one host block from `allocate` (malloc or like it).  The lists are put in
+// the result's order on the device and copied straight into the block.
 void finish_verification(Call &call, const uint8_t *flags, const double *err, const double *w,
                          const uint64_t *nbr_off, const int32_t *nbr, uint64_t nv, uint64_t nc,
-                         std::vector<std::vector<int32_t>> &side,
-                         std::vector<std::vector<std::vector<int32_t>>> &patches,
-                         std::vector<double> &coverage, std::vector<double> &rms);
-
-// Writes side lists, patches, coverage and rms into a library-owned
-// sym_verification_result (one host block from `allocate`).
-void fill_verification_result(uint64_t nc, const std::vector<std::vector<int32_t>> &side,
-                              const std::vector<std::vector<std::vector<int32_t>>> &patches,
-                              const std::vector<double> &coverage, const std::vector<double> &rms,
-                              sym_verification_result &out, void *(*allocate)(size_t));
+                         sym_verification_result &out, void *(*allocate)(size_t));
 
 // Linear BVH over the faces of a resident mesh, FP32 (throughput path).
 struct Lbvh {
@@ -400,10 +391,8 @@ void verification_fast(Call &call, const ResidentSurface &m, sym_cluster_record 
 
 // The reference's full verification of nc records on a resident mesh.
 void verification_resident(Call &call, const ResidentSurface &m, const sym_cluster_record *records,
-                           uint64_t nc, double tau, std::vector<std::vector<int32_t>> &side,
-                           std::vector<std::vector<std::vector<int32_t>>> &patches,
-                           std::vector<double> &coverage, std::vector<double> &rms,
-                           uint64_t *undecided);
+                           uint64_t nc, double tau, sym_verification_result &out,
+                           void *(*allocate)(size_t), uint64_t *undecided);
 
 // Builds the LBVH on the device (synchronises); release with lbvh_free.
 Lbvh lbvh_build(Call &call, const double *xyz, const double *vn, uint64_t nv,

@@ -1619,25 +1619,22 @@ void verification_fast(Call &call, const ResidentSurface &m, sym_cluster_record 
 // The reference's verification of `records` on a resident mesh: side
 // lists, patches, coverage and rms identical to verification_core's.
 void verification_resident(Call &call, const ResidentSurface &m, const sym_cluster_record *records,
-                           uint64_t nc, double tau, std::vector<std::vector<int32_t>> &side,
-                           std::vector<std::vector<std::vector<int32_t>>> &patches,
-                           std::vector<double> &coverage, std::vector<double> &rms,
-                           uint64_t *undecided) {
+                           uint64_t nc, double tau, sym_verification_result &out,
+                           void *(*allocate)(size_t), uint64_t *undecided) {
   const uint64_t nv = m.nv;
   if (undecided) *undecided = 0;
-  if (!nc) {
-    finish_verification(call, nullptr, nullptr, m.w, m.nbr_off, m.nbr, nv, 0, side, patches,
-                        coverage, rms);
-    return;
+  uint8_t *flags = nullptr;
+  double *err = nullptr;
+  if (nc) {
+    std::vector<ClusterMotion> motions(nc);
+    for (uint64_t c = 0; c < nc; ++c) motions[c] = cluster_motion(records[c]);
+    ClusterMotion *dm = call.upload(motions.data(), nc);
+    flags = call.alloc<uint8_t>(nc * 2 * nv);
+    err = call.alloc<double>(nc * nv);
+    const uint64_t n = exact_flags(call, m, dm, records, nc, tau, flags, err, nullptr);
+    if (undecided) *undecided = n;
   }
-  std::vector<ClusterMotion> motions(nc);
-  for (uint64_t c = 0; c < nc; ++c) motions[c] = cluster_motion(records[c]);
-  ClusterMotion *dm = call.upload(motions.data(), nc);
-  uint8_t *flags = call.alloc<uint8_t>(nc * 2 * nv);
-  double *err = call.alloc<double>(nc * nv);
-  const uint64_t n = exact_flags(call, m, dm, records, nc, tau, flags, err, nullptr);
-  if (undecided) *undecided = n;
-  finish_verification(call, flags, err, m.w, m.nbr_off, m.nbr, nv, nc, side, patches, coverage, rms);
+  finish_verification(call, flags, err, m.w, m.nbr_off, m.nbr, nv, nc, out, allocate);
 }
 
 }  // namespace sym
