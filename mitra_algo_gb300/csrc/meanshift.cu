@@ -11,24 +11,21 @@
 // reference evaluator only reads the seed descriptor and the vote set), so:
 //   1. one launch runs the trajectory of EVERY vote as a seed, a warp per
 //      seed, and records its final mean, its converged/exhausted flags and
-//      its support as a bitmask over same-kind votes;
+//      per same-kind vote the iterations that counted it (its support);
 //   2. the host replays the reference's host loop verbatim (RNG draw per seed,
 //      visited set, merge test, budgets) on those results - no device round
 //      trip per trajectory;
-//   3. one launch re-runs only the trajectories the host loop used and adds
-//      each member's per-iteration hit into its cluster's support counts;
-//      one launch picks each vote's winning cluster (largest count, first
+//   3. the hits of the trajectories the host loop used are added up per
+//      cluster, and each vote takes the cluster with the most (the first
 //      cluster on ties).
 // Distances, weights and products are the reference's FP64 expressions (no
 // FMA contraction), and the weighted sums add the members' contributions in
 // vote order, as the reference's serial loop does: each lane evaluates one
-// vote of a group of 32, then every lane adds the members' shuffled weights
-// and products in lane order.  The means are therefore the reference's bit
+// vote of a group of 32, then a lane per sum adds the members' values in order.  The means are therefore the reference's bit
 // for bit, and so is every decision that depends on them (d^2 < h^2, the
 // stop test, the merge test): no rounding band exists to be checked.
-// Memory: seeds run in batches whose support bitmasks fit a fixed device
-// budget (the supports go to the host as sparse member lists), and the
-// members' hit counts are accumulated over batches of clusters.
+// Memory: seeds run in batches whose hit counts fit a fixed device budget (the
+// supports are kept as sparse lists), and so do the clusters' hit counts.
 #include "common.cuh"
 #include "primitives.cuh"
 #include "rng.hpp"
@@ -43,13 +40,6 @@ namespace {
 
 constexpr double kExhausted = 1e-14;  // clustering.cpp:15,169
 
-__global__ void split_kinds(const uint8_t *kind, uint64_t q, uint8_t *is_refl, uint8_t *is_rigid) {
-  uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= q) return;
-  is_refl[i] = kind[i] == SYM_REFLECTION;
-  is_rigid[i] = kind[i] != SYM_REFLECTION;
-}
-
 // AoS descriptors of one kind: out[j*D + k] = lanes[k][ids[j]].
 template <int D>
 __global__ void gather_desc(const double *lanes, uint64_t q, const int32_t *ids, uint64_t n,
@@ -60,181 +50,274 @@ __global__ void gather_desc(const double *lanes, uint64_t q, const int32_t *ids,
   for (int k = 0; k < D; ++k) out[j * D + k] = lanes[uint64_t(k) * q + v];
 }
 
+// Lanes of the descriptors rounded to FP32: out[k * n + j] = desc[j * D + k].
+template <int D>
 __global__ void round_desc(const double *desc, uint64_t n, float *out) {
-  uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = float(desc[i]);
+  const uint64_t j = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (j >= n) return;
+  for (int k = 0; k < D; ++k) out[uint64_t(k) * n + j] = float(desc[j * D + k]);
 }
 
-template <int D>
-struct Traj {
-  double mean[D];
-  bool converged, exhausted;
-};
-
-// One trajectory per warp.  RECORD: write the support bitmask row; else add
-// every member hit to counts[cluster * n + j].
+// The trajectory of every vote of [first, first + nseeds) as a seed, a warp
+// each; counts[s * n + j] += the iterations in which vote j was within the
+// bandwidth (the support is where it is not 0).
 //
-// Culling: `desc32` holds the descriptors rounded to FP32 and `reach` the
+// Culling: `lanes32` holds the descriptors rounded to FP32 and `reach` the
 // bandwidth plus a bound on how far an FP32 distance can fall below the FP64
 // one (the rounding of the mean and of every coordinate, D times 2^-22 of the
 // largest coordinate magnitude, and of the FP32 arithmetic).  A vote whose
 // FP32 squared distance exceeds reach^2 lies outside the bandwidth in FP64
 // as well; only the others take the reference's FP64 test.
-template <int D, bool RECORD>
-__global__ void __launch_bounds__(128) trajectories(const double *desc, const float *desc32,
-                                                    float reach, uint64_t n,
-                                                    const int32_t *seeds, const int32_t *cluster,
-                                                    uint64_t nseeds, double h2, int max_iter,
-                                                    double *final_mean, uint8_t *flags,
-                                                    uint32_t *support, uint64_t words,
-                                                    uint32_t *counts) {
-  uint64_t si = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  int lane = threadIdx.x & 31;
+//
+// A mean moves little, so the votes are not all tested in every iteration: the
+// warp lists, in vote order, those within reach + `slack` of the mean in FP32, and
+// a vote within the bandwidth of a later mean is among them as long as that mean
+// is within `slack` of the listed one; then the list is made anew (a list longer
+// than kListed is not kept: every vote is tested).  The listed votes that pass
+// the FP32 test are gathered 32 at a time, so FP64 (1/64 of the FP32 rate) runs
+// with full warps: each lane makes one vote's distance, weight and products,
+// then lane d adds the d-th sum's members in vote order -- one addition per
+// member and warp, where every lane adding every sum took D + 1.
+// (8,900 votes of the mirrored 128 x 128 height field, 1,500 of them planes:
+// trajectories and counts 15.7 ms, 1.0 ms now.)
+constexpr int kListed = 1024, kTrajWarps = 4;
+template <int D>
+__global__ void __launch_bounds__(32 * kTrajWarps) trajectories(
+    const double *desc, const float *lanes32, float reach, float slack, uint64_t n, uint64_t first,
+    uint64_t nseeds, double h2, int max_iter, double *final_mean, uint8_t *flags, uint32_t *counts) {
+  __shared__ uint32_t list_s[kTrajWarps][kListed];
+  __shared__ uint32_t near_s[kTrajWarps][64];
+  __shared__ double term_s[kTrajWarps][32 * (D + 1)];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint64_t si = uint64_t(blockIdx.x) * kTrajWarps + warp;
   if (si >= nseeds) return;
-  int32_t s = seeds[si];
-  uint64_t crow = RECORD ? 0 : uint64_t(cluster[si]) * n;
-  double mean[D];
-  for (int k = 0; k < D; ++k) mean[k] = desc[uint64_t(s) * D + k];
+  uint32_t *list = list_s[warp], *near = near_s[warp];
+  double *term = term_s[warp];
+  uint32_t *row = counts + si * n;
+  double mean[D];  // the same in every lane, as `converged` and `exhausted`
+  float mean32[D], listed32[D];
+  for (int k = 0; k < D; ++k) mean[k] = desc[(first + si) * D + k], listed32[k] = INFINITY;
   bool converged = false, exhausted = false;
   const double stop = 1e-6 * h2;
+  const float reach2 = reach * reach, wide = (reach + slack) * (1 + 1e-5f), wide2 = wide * wide;
+  const float slack2 = slack * slack * (1 - 1e-4f);
+  uint64_t listed = 0;  // entries; n: every vote, no list
   for (int it = 0; it < max_iter; ++it) {
-    double wt = 0, ws[D];  // the same values in every lane
-    for (int k = 0; k < D; ++k) ws[k] = 0;
-    float mean32[D];
-    for (int k = 0; k < D; ++k) mean32[k] = float(mean[k]);
-    const float reach2 = reach * reach;
-    for (uint64_t base = 0; base < n; base += 32) {
-      uint64_t j = base + lane;
-      bool in = false;
-      double w = 0, x[D];
-      for (int k = 0; k < D; ++k) x[k] = 0;
-      bool near = false;
-      if (j < n) {
-        float d32 = 0;
-        for (int k = 0; k < D; ++k) {
-          const float e = mean32[k] - desc32[j * D + k];
-          d32 += e * e;
+    float moved = 0;
+    for (int k = 0; k < D; ++k) {
+      mean32[k] = float(mean[k]);
+      const float e = mean32[k] - listed32[k];
+      moved += e * e;
+    }
+    if (!(moved < slack2)) {  // list the votes around the mean
+      listed = 0;
+      for (int k = 0; k < D; ++k) listed32[k] = mean32[k];
+      __syncwarp();
+      for (uint64_t base = 0; base < n; base += 32) {
+        const uint64_t j = base + lane;
+        float d32 = j < n ? 0.f : INFINITY;
+        constexpr int kSome = D < 6 ? D : 3;  // the last ones (a rigid vote's translation) first
+        if (j < n)
+          for (int k = D - kSome; k < D; ++k) {
+            const float e = mean32[k] - lanes32[uint64_t(k) * n + j];
+            d32 += e * e;
+          }
+        if (!__any_sync(0xffffffffu, j < n && !(d32 > wide2))) continue;
+        if (kSome < D && j < n && !(d32 > wide2))
+          for (int k = 0; k < D - kSome; ++k) {
+            const float e = mean32[k] - lanes32[uint64_t(k) * n + j];
+            d32 += e * e;
+          }
+        const unsigned keep = __ballot_sync(0xffffffffu, !(d32 > wide2) && j < n);
+        if (listed + __popc(keep) > kListed) {
+          listed = n;
+          break;
         }
-        near = !(d32 > reach2);
+        if (keep >> lane & 1u) list[listed + __popc(keep & ((1u << lane) - 1u))] = uint32_t(j);
+        listed += __popc(keep);
       }
-      if (near) {
-        double dist = 0;
+      if (listed == n && n > kListed) {
+        for (int k = 0; k < D; ++k) listed32[k] = INFINITY;  // no list: try again next time
+      }
+      __syncwarp();
+    }
+    const bool all = listed == n && n > kListed;
+    double sum = 0;  // lane 0: the weights; lane d: coordinate d - 1 of the weighted sum
+    int pending = 0;
+    auto take = [&](int count) {  // the first `count` gathered votes
+      const bool mine = lane < count;
+      const uint64_t j = mine ? near[lane] : 0;
+      bool in = false;
+      if (mine) {
+        double x[D], dist = 0;
         for (int k = 0; k < D; ++k) {
           x[k] = desc[j * D + k];
-          double d = mean[k] - x[k];
+          const double d = mean[k] - x[k];
           dist += d * d;
         }
         if (dist < h2) {
           in = true;
-          w = 1 - dist / h2;
+          const double w = 1 - dist / h2;
+          term[lane * (D + 1)] = w;
+          for (int k = 0; k < D; ++k) term[lane * (D + 1) + 1 + k] = w * x[k];
+          atomicAdd(&row[j], 1u);
         }
       }
       const unsigned bits = __ballot_sync(0xffffffffu, in);
-      // the members of this group in vote order: weight, then w * x
-      for (unsigned m = bits; m; m &= m - 1) {
-        const int src = __ffs(int(m)) - 1;
-        wt += __shfl_sync(0xffffffffu, w, src);
-        for (int k = 0; k < D; ++k) ws[k] += __shfl_sync(0xffffffffu, w * x[k], src);
+      __syncwarp();
+      for (unsigned m = bits; m; m &= m - 1)  // in vote order
+        if (lane <= D) sum += term[(__ffs(int(m)) - 1) * (D + 1) + lane];
+      __syncwarp();
+    };
+    for (uint64_t base = 0; base < listed; base += 32) {
+      uint64_t j = base + lane;
+      float d32 = INFINITY;
+      if (j < listed) {
+        if (!all) j = list[j];
+        d32 = 0;
+        for (int k = 0; k < D; ++k) {
+          const float e = mean32[k] - lanes32[uint64_t(k) * n + j];
+          d32 += e * e;
+        }
       }
-      if (RECORD) {
-        if (lane == 0 && bits) support[si * words + base / 32] |= bits;
-      } else if (in) {
-        atomicAdd(&counts[crow + j], 1u);
+      const bool close = base + lane < listed && !(d32 > reach2);
+      const unsigned bits = __ballot_sync(0xffffffffu, close);
+      if (close) near[pending + __popc(bits & ((1u << lane) - 1u))] = uint32_t(j);
+      pending += __popc(bits);
+      __syncwarp();
+      if (pending >= 32) {
+        take(32);
+        const uint32_t rest = lane < pending - 32 ? near[32 + lane] : 0u;
+        __syncwarp();
+        near[lane] = rest;
+        pending -= 32;
+        __syncwarp();
       }
     }
+    if (pending) take(pending);
+    const double wt = __shfl_sync(0xffffffffu, sum, 0);
     if (wt <= kExhausted) {
       exhausted = true;
       break;
     }
-    double movement = 0;
+    double next = lane && lane <= D ? sum / wt : 0.0, movement = 0;
     for (int k = 0; k < D; ++k) {
-      double next = ws[k] / wt;
-      double d = mean[k] - next;
+      const double to = __shfl_sync(0xffffffffu, next, k + 1);
+      const double d = mean[k] - to;
       movement += d * d;
-      mean[k] = next;
+      mean[k] = to;
     }
     if (movement < stop) {
       converged = true;
       break;
     }
   }
-  if (RECORD && lane == 0) {
+  if (lane == 0) {
     for (int k = 0; k < D; ++k) final_mean[si * D + k] = mean[k];
     flags[si] = uint8_t((converged ? 1 : 0) | (exhausted ? 2 : 0));
   }
 }
 
-// Winner per vote over one batch of clusters (in creation order): the
-// cluster with the largest count so far, the earliest one on ties (a later
-// cluster must count strictly more); best/winner carry over batches.
-__global__ void winners(const uint32_t *counts, uint64_t nclusters, uint64_t n,
-                        const int32_t *cluster_id, uint32_t *best, int32_t *winner) {
-  uint64_t j = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  uint32_t b = best[j];
-  int32_t w = winner[j];
-  for (uint64_t c = 0; c < nclusters; ++c) {
-    uint32_t v = counts[c * n + j];
-    if (v > b) b = v, w = cluster_id[c];
+// Row s of the counts as a list: the votes with hits, ascending, and their
+// hits; a warp per row.  size[s] (entries null) or entries[off[s] ..].
+__global__ void list_hits(const uint32_t *counts, uint64_t n, uint64_t nseeds, uint64_t *size,
+                          const uint64_t *off, uint2 *entries) {
+  const uint64_t s = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (s >= nseeds) return;
+  uint64_t at = entries ? off[s] : 0;
+  for (uint64_t base = 0; base < n; base += 32) {
+    const uint64_t j = base + lane;
+    const uint32_t hits = j < n ? counts[s * n + j] : 0u;
+    const unsigned bits = __ballot_sync(0xffffffffu, hits != 0);
+    if (entries && hits) entries[at + __popc(bits & ((1u << lane) - 1u))] = make_uint2(uint32_t(j), hits);
+    at += __popc(bits);
   }
-  best[j] = b, winner[j] = w;
+  if (!entries && lane == 0) size[s] = at;
 }
 
-// Device bytes for one batch of seeds' support bitmasks, and for one batch
-// of clusters' hit counts.
+// The used seeds' hits added up per cluster (PICK = false), then per vote the
+// cluster with the most, the earliest on ties (PICK): best[j] = the count, then
+// the complement of the cluster's id, so a plain maximum decides.
+template <bool PICK>
+__global__ void cluster_hits(const uint2 *used, uint64_t nused, const uint64_t *off,
+                             const uint2 *entries, const int32_t *cluster_id, uint64_t n,
+                             uint32_t *counts, unsigned long long *best) {
+  const uint64_t i = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  if (i >= nused) return;
+  const uint32_t s = used[i].x, c = used[i].y;  // seed of the batch, cluster of the batch
+  for (uint64_t e = off[s] + (threadIdx.x & 31); e < off[s + 1]; e += 32) {
+    const uint2 x = entries[e];
+    uint32_t *sum = &counts[uint64_t(c) * n + x.x];
+    if (!PICK) atomicAdd(sum, x.y);
+    else atomicMax(&best[x.x], (unsigned long long)*sum << 32 | (0xffffffffu - uint32_t(cluster_id[c])));
+  }
+}
+
+// Device bytes for one batch of seeds' hit counts, and for one batch of
+// clusters'.
 constexpr uint64_t kBatchBytes = uint64_t(1) << 30;
+
+// A batch of seeds' supports on the device: off[s] .. off[s + 1] of entries
+// (vote, hits).
+struct SeedBatch {
+  uint64_t first = 0, count = 0;
+  const uint64_t *off = nullptr;
+  const uint2 *entries = nullptr;
+};
 
 struct KindData {
   int dim = 0;
-  uint64_t n = 0, words = 0;
+  uint64_t n = 0;
   std::vector<int32_t> ids;          // global vote id of each local index
   double *desc = nullptr;            // device AoS
-  float *desc32 = nullptr;           // the same rounded to FP32
+  float *lanes32 = nullptr;          // the same rounded to FP32, lane-major
   float reach = 0;                   // the culling radius (trajectories)
   std::vector<double> mean;          // n x dim final means
   std::vector<uint8_t> flags;        // bit0 converged, bit1 exhausted
   std::vector<uint64_t> sup_off;     // n + 1: each seed's support (kind-local
-  std::vector<uint32_t> sup_idx;     //   member ids, ascending)
+  std::vector<uint2> sup;            //   member ids, ascending, and their hits)
+  std::vector<SeedBatch> batches;
 };
 
 template <int D>
 void run_all_seeds(Call &call, KindData &k, double h2, int max_iter) {
   if (!k.n) return;
   cudaStream_t st = call.stream();
-  k.words = (k.n + 31) / 32;
-  const uint64_t batch = std::max<uint64_t>(1, std::min<uint64_t>(k.n, kBatchBytes / (k.words * 4)));
-  int32_t *seeds = call.alloc<int32_t>(batch);
+  const uint64_t batch = std::max<uint64_t>(1, std::min<uint64_t>(k.n, kBatchBytes / (k.n * 4)));
   double *mean = call.alloc<double>(batch * D);
   uint8_t *flags = call.alloc<uint8_t>(batch);
-  uint32_t *support = call.alloc<uint32_t>(batch * k.words);
+  uint32_t *counts = call.alloc<uint32_t>(batch * k.n);
+  uint64_t *size = call.alloc<uint64_t>(batch);
   k.mean.resize(k.n * D);
   k.flags.resize(k.n);
   k.sup_off.assign(1, 0);
-  k.sup_idx.clear();
-  std::vector<int32_t> iota(batch);
-  std::vector<uint32_t> rows(batch * k.words);
+  k.sup.clear();
   for (uint64_t first = 0; first < k.n; first += batch) {
     const uint64_t cnt = std::min(batch, k.n - first);
-    for (uint64_t i = 0; i < cnt; ++i) iota[i] = int32_t(first + i);
-    call.h2d(seeds, iota.data(), cnt * 4);
-    SYM_CUDA(cudaMemsetAsync(support, 0, cnt * k.words * 4, st));
-    const unsigned blocks = unsigned((cnt * 32 + 127) / 128);
-    trajectories<D, true><<<blocks, 128, 0, st>>>(k.desc, k.desc32, k.reach, k.n, seeds, nullptr,
-                                                  cnt, h2, max_iter,
-                                                  mean, flags, support, k.words, nullptr);
+    SYM_CUDA(cudaMemsetAsync(counts, 0, cnt * k.n * 4, st));
+    trajectories<D><<<blocks_for(cnt, kTrajWarps), 32 * kTrajWarps, 0, st>>>(
+        k.desc, k.lanes32, k.reach, float(0.5 * std::sqrt(h2)), k.n, first, cnt, h2, max_iter, mean,
+        flags, counts);
     check_launch();
-    call.launched();
+    uint64_t *off = call.alloc<uint64_t>(cnt + 1);
+    list_hits<<<blocks_for(cnt * 32), kThreads, 0, st>>>(counts, k.n, cnt, size, nullptr, nullptr);
+    check_launch();
+    exclusive_scan(call, size, off, cnt);
+    std::vector<uint64_t> hoff(cnt + 1);
+    call.d2h(hoff.data(), off, (cnt + 1) * 8);
     call.d2h(k.mean.data() + first * D, mean, cnt * D * 8);
     call.d2h(k.flags.data() + first, flags, cnt);
-    call.d2h(rows.data(), support, cnt * k.words * 4);
     call.sync();
-    for (uint64_t i = 0; i < cnt; ++i) {
-      const uint32_t *row = &rows[i * k.words];
-      for (uint64_t w = 0; w < k.words; ++w)
-        for (uint32_t m = row[w]; m; m &= m - 1)
-          k.sup_idx.push_back(uint32_t(w * 32 + __builtin_ctz(m)));
-      k.sup_off.push_back(k.sup_idx.size());
-    }
+    const uint64_t total = hoff[cnt], at = k.sup.size();
+    uint2 *entries = call.alloc<uint2>(total);
+    list_hits<<<blocks_for(cnt * 32), kThreads, 0, st>>>(counts, k.n, cnt, nullptr, off, entries);
+    check_launch();
+    call.launched(3);
+    k.sup.resize(at + total);
+    call.d2h(k.sup.data() + at, entries, total * sizeof(uint2));
+    for (uint64_t s = 0; s < cnt; ++s) k.sup_off.push_back(at + hoff[s + 1]);
+    k.batches.push_back({first, cnt, off, entries});
   }
 }
 
@@ -246,9 +329,8 @@ struct Center {
   std::vector<int32_t> seeds;  // kind-local seeds merged into this cluster
 };
 
-template <int D>
-void count_members(Call &call, KindData &k, const std::vector<Center> &centers, int kind_index,
-                   double h2, int max_iter, std::vector<int32_t> &winner_global) {
+void count_members(Call &call, const KindData &k, const std::vector<Center> &centers, int kind_index,
+                   std::vector<int32_t> &winner_global) {
   std::vector<int32_t> cluster_ids;
   for (size_t c = 0; c < centers.size(); ++c)
     if (centers[c].kind == kind_index) cluster_ids.push_back(int32_t(c));
@@ -257,33 +339,39 @@ void count_members(Call &call, KindData &k, const std::vector<Center> &centers, 
   const uint64_t batch = std::max<uint64_t>(1, std::min<uint64_t>(cluster_ids.size(),
                                                                    kBatchBytes / (k.n * 4)));
   uint32_t *counts = call.alloc<uint32_t>(batch * k.n);
-  uint32_t *best = call.alloc<uint32_t>(k.n);
-  int32_t *win = call.alloc<int32_t>(k.n);
-  SYM_CUDA(cudaMemsetAsync(best, 0, k.n * 4, st));
-  SYM_CUDA(cudaMemsetAsync(win, 0xff, k.n * 4, st));  // -1: no cluster counted the vote
+  unsigned long long *best = call.alloc<unsigned long long>(k.n);
+  SYM_CUDA(cudaMemsetAsync(best, 0, k.n * 8, st));
+  std::vector<std::vector<uint2>> used(k.batches.size());  // kept until the copies are done
   for (uint64_t first = 0; first < cluster_ids.size(); first += batch) {
     const uint64_t nc = std::min<uint64_t>(batch, cluster_ids.size() - first);
-    std::vector<int32_t> seeds, cluster;
+    if (first) call.sync();
+    for (auto &u : used) u.clear();
     for (uint64_t c = 0; c < nc; ++c)
-      for (int32_t s : centers[cluster_ids[first + c]].seeds)
-        seeds.push_back(s), cluster.push_back(int32_t(c));
+      for (int32_t s : centers[cluster_ids[first + c]].seeds) {
+        const uint64_t b = uint64_t(s) / k.batches[0].count;
+        used[b].push_back(make_uint2(uint32_t(uint64_t(s) - k.batches[b].first), uint32_t(c)));
+      }
     SYM_CUDA(cudaMemsetAsync(counts, 0, nc * k.n * 4, st));
-    int32_t *dseeds = call.upload(seeds.data(), seeds.size());
-    int32_t *dcluster = call.upload(cluster.data(), cluster.size());
-    int32_t *dids = call.upload(cluster_ids.data() + first, nc);
-    const unsigned blocks = unsigned((seeds.size() * 32 + 127) / 128);
-    trajectories<D, false><<<blocks, 128, 0, st>>>(k.desc, k.desc32, k.reach, k.n, dseeds,
-                                                   dcluster, seeds.size(), h2,
-                                                   max_iter, nullptr, nullptr, nullptr, 0, counts);
-    check_launch();
-    winners<<<blocks_for(k.n), kThreads, 0, st>>>(counts, nc, k.n, dids, best, win);
-    check_launch();
-    call.launched(2);
+    const int32_t *dids = call.upload(cluster_ids.data() + first, nc);
+    std::vector<const uint2 *> dused(used.size(), nullptr);
+    for (size_t b = 0; b < used.size(); ++b)
+      if (!used[b].empty()) dused[b] = call.upload(used[b].data(), used[b].size());
+    for (int pick = 0; pick < 2; ++pick)
+      for (size_t b = 0; b < used.size(); ++b) {
+        if (used[b].empty()) continue;
+        const uint64_t m = used[b].size();
+        const auto kernel = pick ? cluster_hits<true> : cluster_hits<false>;
+        kernel<<<blocks_for(m * 32), kThreads, 0, st>>>(dused[b], m, k.batches[b].off,
+                                                        k.batches[b].entries, dids, k.n, counts, best);
+        check_launch();
+        call.launched();
+      }
   }
-  std::vector<int32_t> local(k.n);
-  call.d2h(local.data(), win, k.n * 4);
+  std::vector<unsigned long long> local(k.n);
+  call.d2h(local.data(), best, k.n * 8);
   call.sync();
-  for (uint64_t j = 0; j < k.n; ++j) winner_global[k.ids[j]] = local[j];
+  for (uint64_t j = 0; j < k.n; ++j)
+    winner_global[k.ids[j]] = local[j] >> 32 ? int32_t(0xffffffffu - uint32_t(local[j])) : -1;
 }
 
 // Index of the centers for the merge test (clustering.cpp:68-73: the first
@@ -385,9 +473,11 @@ void clustering_host(Call &call, const sym_votes_view &votes, const sym_model_co
       else
         gather_desc<12><<<blocks_for(k.n), kThreads, 0, call.stream()>>>(lanes, q, ids, k.n, k.desc);
       check_launch();
-      k.desc32 = call.alloc<float>(k.n * k.dim);
-      round_desc<<<blocks_for(k.n * k.dim), kThreads, 0, call.stream()>>>(k.desc, k.n * k.dim,
-                                                                         k.desc32);
+      k.lanes32 = call.alloc<float>(k.n * k.dim);
+      if (k.dim == 4)
+        round_desc<4><<<blocks_for(k.n), kThreads, 0, call.stream()>>>(k.desc, k.n, k.lanes32);
+      else
+        round_desc<12><<<blocks_for(k.n), kThreads, 0, call.stream()>>>(k.desc, k.n, k.lanes32);
       check_launch();
       call.launched(2);
       // the culling radius: h plus the FP32 shortfall of a distance (rounding
@@ -434,9 +524,9 @@ void clustering_host(Call &call, const sym_votes_view &votes, const sym_model_co
     int t = kind_of[seed];
     KindData &k = kinds[t];
     uint64_t s = uint64_t(local_of[seed]);
-    const uint32_t *members = k.sup_idx.data() + k.sup_off[s];
+    const uint2 *members = k.sup.data() + k.sup_off[s];
     const uint64_t size = k.sup_off[s + 1] - k.sup_off[s];
-    for (uint64_t m = 0; m < size; ++m) visit(uint64_t(k.ids[members[m]]));
+    for (uint64_t m = 0; m < size; ++m) visit(uint64_t(k.ids[members[m].x]));
     bool converged = k.flags[s] & 1, exhausted = k.flags[s] & 2;
     if (exhausted) visit(seed);
     if (!converged) ++limited;
@@ -447,8 +537,8 @@ void clustering_host(Call &call, const sym_votes_view &votes, const sym_model_co
     auto add_keys = [&](Center &c) {  // the support's members into the union
       uint64_t added = 0;
       for (uint64_t m = 0; m < size; ++m) {
-        uint64_t &w = c.keys[members[m] >> 6];
-        const uint64_t bit = uint64_t(1) << (members[m] & 63);
+        uint64_t &w = c.keys[members[m].x >> 6];
+        const uint64_t bit = uint64_t(1) << (members[m].x & 63);
         if (!(w & bit)) w |= bit, ++added;
       }
       c.key_count += added;
@@ -484,8 +574,8 @@ void clustering_host(Call &call, const sym_votes_view &votes, const sym_model_co
 
   // ---- support counts and winners (clustering.cpp:97-108) on the GPU
   std::vector<int32_t> winner(q, -1);
-  count_members<4>(call, kinds[0], centers, 0, h2, o.max_iterations, winner);
-  count_members<12>(call, kinds[1], centers, 1, h2, o.max_iterations, winner);
+  count_members(call, kinds[0], centers, 0, winner);
+  count_members(call, kinds[1], centers, 1, winner);
   std::vector<std::vector<int32_t>> members(centers.size());
   for (uint64_t i = 0; i < q; ++i)
     if (winner[i] >= 0) members[winner[i]].push_back(int32_t(i));
