@@ -32,7 +32,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <unordered_map>
 #include <vector>
 
 namespace sym {
@@ -324,7 +323,7 @@ void run_all_seeds(Call &call, KindData &k, double h2, int max_iter) {
 struct Center {
   double v[12];
   int kind;                    // index into kinds[]
-  std::vector<uint64_t> keys;  // union of supports, kind-local bitmask
+  std::vector<uint64_t> keys;  // union of supports, kind-local bitmask (from the second seed on)
   uint64_t key_count = 0;
   std::vector<int32_t> seeds;  // kind-local seeds merged into this cluster
 };
@@ -381,37 +380,53 @@ void count_members(Call &call, const KindData &k, const std::vector<Center> &cen
 // lowest-numbered center among those that pass the reference's test is the
 // reference's choice.  Centers with coordinates too large for the grid stay
 // in a list that every query scans.
+// The cells are hashed into chains of center numbers (an array each of chain
+// heads, links and cells: 27 probes per query are 27 array reads).
 class CenterGrid {
 public:
-  CenterGrid(double h, const int dims[3]) : scale_(2.0 / h * (1 - 1e-9)) {
+  CenterGrid(double h, const int dims[3]) : scale_(2.0 / h * (1 - 1e-9)), head_(1024, -1) {
     for (int i = 0; i < 3; ++i) dims_[i] = dims[i];
   }
   void insert(int32_t id, const double *v) {
     uint64_t key;
-    if (cell(v, 0, 0, 0, key)) map_[key].push_back(id);
-    else loose_.push_back(id);
+    if (!cell(v, 0, 0, 0, key)) {
+      loose_.push_back(id);
+      return;
+    }
+    if (size_t(id) >= cells_.size()) cells_.resize(id + 1), links_.resize(id + 1, -1);
+    if (++count_ > head_.size()) {  // twice the heads, the chains made anew
+      std::vector<int32_t> ids;
+      for (int32_t at : head_)
+        for (; at >= 0; at = links_[at]) ids.push_back(at);
+      head_.assign(2 * head_.size(), -1);
+      for (int32_t at : ids) link(at);
+    }
+    cells_[id] = key;
+    link(id);
   }
   void erase(int32_t id, const double *v) {
     uint64_t key;
-    std::vector<int32_t> &list = cell(v, 0, 0, 0, key) ? map_[key] : loose_;
-    list.erase(std::find(list.begin(), list.end(), id));
+    if (!cell(v, 0, 0, 0, key)) {
+      loose_.erase(std::find(loose_.begin(), loose_.end(), id));
+      return;
+    }
+    int32_t *at = &head_[slot(key)];
+    while (*at != id) at = &links_[*at];
+    *at = links_[id];
+    --count_;
   }
   template <class Test>
   int32_t first(const double *v, Test &&passes) const {
     int32_t best = -1;
-    auto scan = [&](const std::vector<int32_t> &list) {
-      for (int32_t id : list)
-        if ((best < 0 || id < best) && passes(id)) best = id;
-    };
-    scan(loose_);
+    for (int32_t id : loose_)
+      if ((best < 0 || id < best) && passes(id)) best = id;
     uint64_t key;
     for (int a = -1; a <= 1; ++a)
       for (int b = -1; b <= 1; ++b)
         for (int c = -1; c <= 1; ++c)
-          if (cell(v, a, b, c, key)) {
-            auto it = map_.find(key);
-            if (it != map_.end()) scan(it->second);
-          }
+          if (cell(v, a, b, c, key))
+            for (int32_t id = head_[slot(key)]; id >= 0; id = links_[id])
+              if (cells_[id] == key && (best < 0 || id < best) && passes(id)) best = id;
     return best;
   }
 
@@ -426,10 +441,20 @@ private:
     }
     return true;
   }
+  size_t slot(uint64_t key) const {  // splitmix64's finaliser
+    key = (key ^ (key >> 30)) * 0xBF58476D1CE4E5B9ull;
+    key = (key ^ (key >> 27)) * 0x94D049BB133111EBull;
+    return size_t(key ^ (key >> 31)) & (head_.size() - 1);
+  }
+  void link(int32_t id) {
+    int32_t &head = head_[slot(cells_[id])];
+    links_[id] = head, head = id;
+  }
   double scale_;
   int dims_[3];
-  std::unordered_map<uint64_t, std::vector<int32_t>> map_;
-  std::vector<int32_t> loose_;
+  size_t count_ = 0;
+  std::vector<int32_t> head_, links_, loose_;
+  std::vector<uint64_t> cells_;
 };
 
 double desc_d2(const double *a, const double *b, int dim) {
@@ -534,22 +559,20 @@ void clustering_host(Call &call, const sym_votes_view &votes, const sym_model_co
     const int merge = grids[t].first(mean, [&](int32_t c) {
       return desc_d2(mean, centers[c].v, k.dim) < h2 / 4;
     });
-    auto add_keys = [&](Center &c) {  // the support's members into the union
+    auto add_keys = [&](Center &c, uint64_t seed_of) {  // a support's members into the union
       uint64_t added = 0;
-      for (uint64_t m = 0; m < size; ++m) {
-        uint64_t &w = c.keys[members[m].x >> 6];
-        const uint64_t bit = uint64_t(1) << (members[m].x & 63);
+      for (uint64_t m = k.sup_off[seed_of]; m < k.sup_off[seed_of + 1]; ++m) {
+        uint64_t &w = c.keys[k.sup[m].x >> 6];
+        const uint64_t bit = uint64_t(1) << (k.sup[m].x & 63);
         if (!(w & bit)) w |= bit, ++added;
       }
-      c.key_count += added;
       return added;
     };
     if (merge < 0) {
       Center c;
       for (int i = 0; i < 12; ++i) c.v[i] = i < k.dim ? mean[i] : 0;
       c.kind = t;
-      c.keys.assign((k.n + 63) / 64, 0);
-      add_keys(c);
+      c.key_count = size;
       c.seeds.push_back(int32_t(s));
       support_entries += c.key_count;
       grids[t].insert(int32_t(centers.size()), c.v);
@@ -562,7 +585,13 @@ void clustering_host(Call &call, const sym_votes_view &votes, const sym_model_co
         for (int i = 0; i < k.dim; ++i) c.v[i] = (old * c.v[i] + now * mean[i]) / (old + now);
         grids[t].insert(merge, c.v);
       }
-      support_entries += add_keys(c);
+      if (c.keys.empty()) {
+        c.keys.assign((k.n + 63) / 64, 0);
+        add_keys(c, uint64_t(c.seeds[0]));
+      }
+      const uint64_t added = add_keys(c, s);
+      c.key_count += added;
+      support_entries += added;
       c.seeds.push_back(int32_t(s));
     }
     if (support_entries > 5000000)

@@ -16,7 +16,7 @@
 //  6. the edge table: the corner edges stably sorted by (lo, hi), one edge per
 //     run of equal keys with its first two corners - the order and content of
 //     the reference's std::map, plus its non-manifold / winding checks;
-//  7. the vertex centroid as one sequential sum.
+//  7. the vertex centroid as one sequential sum (on the host, meanwhile).
 // FP64 without FMA contraction in the reference's operation order, so every
 // output is bit-exact with the CPU path.
 #include "common.cuh"
@@ -176,14 +176,6 @@ __global__ void edge_records(const int32_t *faces, uint64_t nf, const uint64_t *
   edges[e] = sym_edge{int32_t(key / nv), int32_t(key % nv), a0, b0, f0, t - s == 2 ? f1 : -1};
 }
 
-__global__ void centroid(const double *xyz, uint64_t nv, double *out) {
-  if (blockIdx.x || threadIdx.x > 2) return;
-  const int k = threadIdx.x;
-  double s = 0;
-  for (uint64_t v = 0; v < nv; ++v) s += xyz[k * nv + v];  // the reference's order
-  out[k] = s;
-}
-
 int key_bits(uint64_t max_key) {
   int b = 8;
   while (b < 64 && (max_key >> b)) b += 8;
@@ -332,16 +324,16 @@ PreparedDevice prepare_device(Call &call, const sym_mesh_view &m, const sym_opti
   edge_records<<<blocks_for(ne), kThreads, 0, st>>>(p.faces, nf, sekey, secorner, pos, ne, nc, nv,
                                                     p.edges, diag, diag + 1);
   check_launch();
-  // 7. centroid
-  double *csum = call.alloc<double>(3);
-  centroid<<<1, 32, 0, st>>>(p.xyz, nv, csum);
-  check_launch();
+  // 7. centroid: one addition waits for the one before, so the host, which has
+  // the vertices, takes the serial sums while the device works (500,000
+  // vertices: 33 ms in a kernel of three threads)
+  double hc[3] = {0, 0, 0};
+  for (uint64_t v = 0; v < nv; ++v)
+    hc[0] += m.vertices.x[v], hc[1] += m.vertices.y[v], hc[2] += m.vertices.z[v];
   unsigned long long hd[2];
-  double hc[3];
   call.d2h(hd, diag, 16);
-  call.d2h(hc, csum, 24);
   call.sync();
-  call.launched(12);  // own kernels; the primitives count theirs
+  call.launched(11);  // own kernels; the primitives count theirs
   p.nonmanifold = hd[0], p.conflicts = hd[1];
   if (hd[0] || hd[1])
     fail(SYM_RUNTIME_ERROR,

@@ -28,75 +28,163 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <functional>
 #include <limits>
 #include <numeric>
+#include <system_error>
+#include <utility>
 #include <vector>
 
 namespace sym {
 
-HostBvh::HostBvh(const sym_mesh_view &m) {
-  ids.resize(m.faces.count);
-  for (uint64_t i = 0; i < ids.size(); ++i) ids[i] = int32_t(i);
-  auto coord = [&](int f, int corner, int axis) {
-    const int32_t *col = corner == 0 ? m.faces.v0 : (corner == 1 ? m.faces.v1 : m.faces.v2);
-    const double *c = axis == 0 ? m.vertices.x : (axis == 1 ? m.vertices.y : m.vertices.z);
-    return c[col[f]];
+// The reference's build (surface.h:16-50) gives its nodes in preorder and
+// halves every range by count, so the number of nodes, of leaves and the depth of
+// a subtree follow from its number of faces alone: each subtree knows where its
+// nodes and leaves go, and the subtrees build at the same time on host threads.
+// std::nth_element sees the same comparisons as the reference's (of the same
+// centroids, made once per face and laid out next to the ids it permutes), so it
+// leaves the same permutation.  (One thread that formed centroids and boxes
+// from the vertices at every comparison kept the first detection on a
+// 1e6-triangle torus waiting: 454 ms, 110 ms now.)
+namespace {
+
+struct SubtreeSize {
+  int64_t nodes, leaves;
+  int depth;
+};
+SubtreeSize joined(const SubtreeSize &l, const SubtreeSize &r) {
+  return {1 + l.nodes + r.nodes, l.leaves + r.leaves, 1 + std::max(l.depth, r.depth)};
+}
+// of n faces and of n + 1: the halves of both are n / 2 and n / 2 + 1 faces
+std::pair<SubtreeSize, SubtreeSize> subtree_sizes(int64_t n) {
+  const SubtreeSize one{1, 1, 0};
+  if (n + 1 <= 8) return {one, one};
+  const auto h = subtree_sizes(n / 2);
+  const SubtreeSize odd = joined(h.first, h.second);
+  if (n & 1) return {odd, joined(h.second, h.second)};
+  return {n <= 8 ? one : joined(h.first, h.first), odd};
+}
+SubtreeSize subtree_size(int64_t n) { return subtree_sizes(n).first; }
+
+// f on a thread of its own, or here when there is none to be had
+template <class F>
+std::future<void> launch(F f) {
+  try {
+    return std::async(std::launch::async, f);
+  } catch (const std::system_error &) {
+    f();
+    return {};
+  }
+}
+
+struct FaceBox {
+  double lo[3], hi[3];
+};
+
+struct BvhBuilder {
+  HostBvh &t;
+  std::vector<FaceBox> box;
+  std::vector<double> centroid[3];
+  struct Keyed {
+    double at;
+    int32_t face;
   };
-  struct Builder {
-    HostBvh &t;
-    decltype(coord) &co;
-    int build(int begin, int end, int level) {
-      t.depth = std::max(t.depth, level);
-      BvhNode n;
-      for (int k = 0; k < 3; ++k) n.lo[k] = 1e300, n.hi[k] = -1e300;
-      for (int i = begin; i < end; ++i)
-        for (int corner = 0; corner < 3; ++corner)
-          for (int k = 0; k < 3; ++k) {
-            double x = co(t.ids[i], corner, k);
-            n.lo[k] = std::min(n.lo[k], x);
-            n.hi[k] = std::max(n.hi[k], x);
-          }
-      n.begin = begin, n.end = end, n.left = -1, n.right = -1;
-      int index = int(t.nodes.size());
-      t.nodes.push_back(n);
-      if (end - begin > 8) {
-        double ext[3] = {n.hi[0] - n.lo[0], n.hi[1] - n.lo[1], n.hi[2] - n.lo[2]};
-        int axis = ext[1] > ext[0] ? 1 : 0;
-        if (ext[2] > ext[axis]) axis = 2;
-        int mid = (begin + end) / 2;
-        auto centroid = [&](int f) { return (co(f, 0, axis) + co(f, 1, axis) + co(f, 2, axis)) / 3; };
-        std::nth_element(t.ids.begin() + begin, t.ids.begin() + mid, t.ids.begin() + end,
-                         [&](int a, int b) { return centroid(a) < centroid(b); });
-        int l = build(begin, mid, level + 1), r = build(mid, end, level + 1);
-        t.nodes[index].left = l;
-        t.nodes[index].right = r;
-      }
-      return index;
+  std::vector<Keyed> keyed;  // each subtree works in its own range
+
+  // the subtrees that get a thread: at most 2^kSpawnLevels, of at least kSpawn faces
+  static constexpr int64_t kSpawn = 2048;
+  static constexpr int kSpawnLevels = 5;
+
+  void run(int64_t n, int64_t grain, const std::function<void(int64_t, int64_t)> &part) {
+    std::vector<std::future<void>> jobs;
+    for (int64_t at = grain; at < n; at += grain) {
+      const int64_t end = std::min(n, at + grain);
+      jobs.push_back(launch([&part, at, end] { part(at, end); }));
     }
-  } builder{*this, coord};
-  if (!ids.empty()) builder.build(0, int(ids.size()), 0);
-  if (depth > 31) throw Error(SYM_RUNTIME_ERROR, "verification: BVH too deep");
-  order.assign(ids.size(), FaceOrder{0, -1, -1, 0});
-  std::vector<uint32_t> path(nodes.size(), 0);
-  std::vector<int32_t> node_depth(nodes.size(), 0), parent(nodes.size(), -1);
-  int32_t leaves = 0;
-  for (size_t n = 0; n < nodes.size(); ++n) leaves += nodes[n].left < 0;
-  ancestors.assign(size_t(leaves) * 32, -1);
-  leaves = 0;
-  for (size_t n = 0; n < nodes.size(); ++n) {  // parents precede their children
-    const BvhNode &b = nodes[n];
-    if (b.left >= 0) {
-      const int d = node_depth[n];
-      parent[b.left] = parent[b.right] = int32_t(n);
-      node_depth[b.left] = node_depth[b.right] = d + 1;
-      path[b.left] = path[n];
-      path[b.right] = path[n] | (1u << (31 - d));
+    part(0, std::min(n, grain));
+    for (auto &j : jobs)
+      if (j.valid()) j.get();
+  }
+
+  FaceBox bounds(int64_t begin, int64_t end) const {
+    FaceBox b{{1e300, 1e300, 1e300}, {-1e300, -1e300, -1e300}};
+    for (int64_t i = begin; i < end; ++i) {
+      const FaceBox &f = box[t.ids[i]];
+      for (int k = 0; k < 3; ++k) b.lo[k] = std::min(b.lo[k], f.lo[k]), b.hi[k] = std::max(b.hi[k], f.hi[k]);
+    }
+    return b;
+  }
+
+  // chain[0 .. level): the ancestors; path: their steps
+  void build(int64_t begin, int64_t end, int level, int64_t index, int64_t leaf, uint32_t path,
+             int32_t *chain) {
+    const FaceBox b = bounds(begin, end);
+    BvhNode n;
+    for (int k = 0; k < 3; ++k) n.lo[k] = b.lo[k], n.hi[k] = b.hi[k];
+    n.begin = int32_t(begin), n.end = int32_t(end), n.left = -1, n.right = -1;
+    chain[level] = int32_t(index);
+    if (end - begin <= 8) {
+      t.nodes[index] = n;
+      for (int64_t i = begin; i < end; ++i) t.order[t.ids[i]] = FaceOrder{path, int32_t(leaf), int32_t(i), 0};
+      std::copy(chain, chain + level + 1, t.ancestors.begin() + leaf * 32);
+      return;
+    }
+    const double ext[3] = {n.hi[0] - n.lo[0], n.hi[1] - n.lo[1], n.hi[2] - n.lo[2]};
+    int axis = ext[1] > ext[0] ? 1 : 0;
+    if (ext[2] > ext[axis]) axis = 2;
+    const int64_t mid = (begin + end) / 2;
+    for (int64_t i = begin; i < end; ++i) keyed[i] = {centroid[axis][t.ids[i]], t.ids[i]};
+    std::nth_element(keyed.begin() + begin, keyed.begin() + mid, keyed.begin() + end,
+                     [](const Keyed &x, const Keyed &y) { return x.at < y.at; });
+    for (int64_t i = begin; i < end; ++i) t.ids[i] = keyed[i].face;
+    const SubtreeSize l = subtree_size(mid - begin);
+    n.left = int32_t(index + 1), n.right = int32_t(index + 1 + l.nodes);
+    t.nodes[index] = n;
+    const uint32_t right_path = path | (1u << (31 - level));
+    auto right = [&, right_path](int32_t *c) {
+      build(mid, end, level + 1, n.right, leaf + l.leaves, right_path, c);
+    };
+    if (level < kSpawnLevels && end - begin >= 2 * kSpawn) {
+      int32_t other[32];
+      std::copy(chain, chain + level + 1, other);
+      auto job = launch([&] { right(other); });
+      build(begin, mid, level + 1, n.left, leaf, path, chain);
+      if (job.valid()) job.get();
     } else {
-      const int32_t leaf = leaves++;
-      for (int32_t i = b.begin; i < b.end; ++i) order[ids[i]] = FaceOrder{path[n], leaf, i, 0};
-      for (int32_t a = int32_t(n); a >= 0; a = parent[a]) ancestors[size_t(leaf) * 32 + node_depth[a]] = a;
+      build(begin, mid, level + 1, n.left, leaf, path, chain);
+      right(chain);
     }
   }
+};
+
+}  // namespace
+
+HostBvh::HostBvh(const sym_mesh_view &m) {
+  const int64_t nf = int64_t(m.faces.count);
+  ids.resize(nf);
+  for (int64_t i = 0; i < nf; ++i) ids[i] = int32_t(i);
+  if (!nf) return;
+  const SubtreeSize size = subtree_size(nf);
+  depth = size.depth;
+  if (depth > 31) throw Error(SYM_RUNTIME_ERROR, "verification: BVH too deep");
+  nodes.resize(size.nodes);
+  order.resize(nf);
+  ancestors.assign(size_t(size.leaves) * 32, -1);
+  BvhBuilder build{*this, std::vector<FaceBox>(nf), {}, std::vector<BvhBuilder::Keyed>(nf)};
+  for (auto &c : build.centroid) c.resize(nf);
+  const int32_t *cols[3] = {m.faces.v0, m.faces.v1, m.faces.v2};
+  const double *axes[3] = {m.vertices.x, m.vertices.y, m.vertices.z};
+  build.run(nf, 1 << 16, [&](int64_t begin, int64_t end) {
+    for (int64_t f = begin; f < end; ++f)
+      for (int k = 0; k < 3; ++k) {
+        const double a = axes[k][cols[0][f]], b = axes[k][cols[1][f]], c = axes[k][cols[2][f]];
+        build.box[f].lo[k] = std::min(std::min(std::min(1e300, a), b), c);
+        build.box[f].hi[k] = std::max(std::max(std::max(-1e300, a), b), c);
+        build.centroid[k][f] = (a + b + c) / 3;
+      }
+  });
+  int32_t chain[32];
+  build.build(0, nf, 0, 0, 0, 0, chain);
 }
 
 // boxes32 of RefBvh: the boxes of a node's children in FP32 (an inner node's).
