@@ -142,7 +142,16 @@ __device__ __forceinline__ float box_distance_f(float px, float py, float pz, co
   if (g < -margin) return 0.f;
   if (g <= margin) return -1.f;
   const float x = fmaxf(gx, 0.f), y = fmaxf(gy, 0.f), z = fmaxf(gz, 0.f);
-  return sqrtf(x * x + y * y + z * z);
+  const float d2 = x * x + y * y + z * z;
+  return d2 > 1e-30f && d2 < 1e30f ? sqrtf(d2) : -1.f;  // not where the squares leave FP32
+}
+
+// Whether the right of two boxes at distances dl and dr (box_distance_f) is
+// strictly nearer; `exact` decides in FP64 where FP32 does not.
+template <class Exact>
+__device__ __forceinline__ bool right_nearer(float dl, float dr, float margin, Exact &&exact) {
+  if (dl < 0.f || dr < 0.f || (dl > 0.f && dr > 0.f && fabsf(dl - dr) <= margin)) return exact();
+  return dl > dr;  // both inside: equal, the left one
 }
 
 // The same with the two box distances compared in FP32 where that decides
@@ -163,13 +172,10 @@ __device__ inline int32_t first_in_reference_order_f(const RefBvh &t, D3 q, floa
   const float px = float(q.x), py = float(q.y), pz = float(q.z);
   const float dl = box_distance_f(px, py, pz, left, margin),
               dr = box_distance_f(px, py, pz, right, margin);
-  bool right_first;
-  if (dl < 0.f || dr < 0.f || (dl > 0.f && dr > 0.f && fabsf(dl - dr) <= margin)) {
+  const bool right_first = right_nearer(dl, dr, margin, [&] {
     const BvhNode &lca = t.nodes[node];
-    right_first = box_d2(q, t.nodes[lca.left]) > box_d2(q, t.nodes[lca.right]);
-  } else {
-    right_first = dl > dr;  // both inside: equal, the left one
-  }
+    return box_d2(q, t.nodes[lca.left]) > box_d2(q, t.nodes[lca.right]);
+  });
   const bool a_right = (oa.path >> (31 - depth)) & 1u;
   return a_right == right_first ? a : b;
 }
@@ -275,22 +281,31 @@ __device__ inline bool normal_agrees(const Surface &s, int32_t f, const M3 &r, D
 }
 
 // One (cluster, direction, vertex) query of the reference's verification
-// through the reference-order BVH: returns whether the vertex supports the
-// cluster in that direction, and its squared distance in `d2`.
-__device__ inline bool exact_query(const Surface &s, const double *vn, const ClusterMotion &m,
-                                   bool inverse, uint64_t i, double tau, double limit, double &d2,
-                                   int *status) {
+// through a search for the nearest face: returns whether the vertex supports
+// the cluster in that direction, and its squared distance in `d2`.
+template <class Search>
+__device__ inline bool exact_query_by(const Surface &s, const double *vn, const ClusterMotion &m,
+                                      bool inverse, uint64_t i, double tau, double &d2,
+                                      Search &&search) {
   const M3 r = query_rotation(m, inverse);
   const D3 p = vertex(s, int32_t(i));
   D3 q;
   if (query_skipped(m, r, inverse, p, tau, q)) return false;
   int32_t face;
-  const double d = nearest_face(s, q, limit, face, status);
+  const double d = search(q, face);
   if (d > tau * tau || face < 0) return false;
   const D3 ni{vn[i], vn[s.nv + i], vn[2 * s.nv + i]};
   if (!normal_agrees(s, face, r, ni)) return false;
   d2 = d;
   return true;
+}
+
+__device__ inline bool exact_query(const Surface &s, const double *vn, const ClusterMotion &m,
+                                   bool inverse, uint64_t i, double tau, double limit, double &d2,
+                                   int *status) {
+  return exact_query_by(s, vn, m, inverse, i, tau, d2, [&](D3 q, int32_t &face) {
+    return nearest_face(s, q, limit, face, status);
+  });
 }
 
 // Union-find over rows (set * nv + vertex): parent = own vertex for the

@@ -25,6 +25,7 @@
 // whose candidates overflow the list, is re-run through the reference-order
 // BVH (verification.cuh), built on the host once per resident mesh when the
 // first such query appears.  Sums use the reference's serial order.
+#include "face32.cuh"
 #include "primitives.cuh"
 #include "verification.cuh"
 
@@ -35,17 +36,6 @@
 
 namespace sym {
 namespace {
-
-struct F3 {
-  float x, y, z;
-};
-__device__ __forceinline__ F3 operator-(F3 a, F3 b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
-__device__ __forceinline__ F3 operator+(F3 a, F3 b) { return {a.x + b.x, a.y + b.y, a.z + b.z}; }
-__device__ __forceinline__ F3 operator*(F3 a, float s) { return {a.x * s, a.y * s, a.z * s}; }
-__device__ __forceinline__ float dotf(F3 a, F3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-__device__ __forceinline__ F3 crossf(F3 a, F3 b) {
-  return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
-}
 
 __device__ float segment_d2f(F3 p, F3 a, F3 b) {
   F3 d = b - a;
@@ -231,14 +221,6 @@ __device__ __forceinline__ float box_d2f(F3 p, float lx, float ly, float lz, flo
   return dx * dx + dy * dy + dz * dz;
 }
 
-// A face as the searches read it, 64 bytes: corners a, b, c in FP32, the
-// reciprocal squared lengths of the edges ab, bc, ca, the unit normal from the
-// FP64 corners and `reach`, a bound on the edge lengths (0: no usable normal).
-struct Face {
-  F3 a, b, c, n;
-  float inv_ab, inv_bc, inv_ca, reach;
-};
-
 struct BvhView {
   uint64_t nv, nf;
   const int32_t *faces;
@@ -252,11 +234,7 @@ struct BvhView {
 __device__ __forceinline__ F3 vtx(const BvhView &b, int32_t v) {
   return {b.xyz[v], b.xyz[b.nv + v], b.xyz[2 * b.nv + v]};
 }
-__device__ __forceinline__ Face load_face(const BvhView &b, int32_t f) {
-  const float4 *r = b.face + 4 * int64_t(f);
-  const float4 x = r[0], y = r[1], z = r[2], w = r[3];
-  return {{x.x, x.y, x.z}, {y.x, y.y, y.z}, {z.x, z.y, z.z}, {w.x, w.y, w.z}, x.w, y.w, z.w, w.w};
-}
+__device__ __forceinline__ Face load_face(const BvhView &b, int32_t f) { return sym::load_face(b.face, f); }
 __device__ __forceinline__ float face_d2(const BvhView &b, F3 p, int32_t f) {
   const float4 *r = b.face + 4 * int64_t(f);
   const float4 x = r[0], y = r[1], z = r[2];
@@ -377,52 +355,6 @@ __device__ __forceinline__ int32_t support_query(const BvhView &b, const double 
 constexpr float kErr = 1.0f / 32768.0f;
 constexpr float kNormalBand = 1.0f / 1024.0f;
 constexpr int kCandidates = 16;
-
-// FP32 squared distance from p to a face with a usable normal; um = u M, the
-// FP32 unit at the query's magnitude.  The plane distance when p projects
-// inside all three edges by more than their rounding band (p then projects
-// into the face), the nearest of the edge segments when it projects outside
-// one of them by more than its band (the nearest point then lies on an edge p
-// is outside of, so edges p is inside of by more than the band need no
-// distance).  Otherwise `d2` receives min(plane, segments), a lower bound of
-// the distance, and the function returns false; also, with the plane
-// distance, when that alone is above `lim` (the caller drops the face).
-// Band of an edge function E = (n x e) . (p - v): with |dn| <= u,
-// corners within 1.8 u M and the image within 30 u M of their FP64 values,
-// and the cross and dot products' rounding, |dE| <= u (11 |e| |p - v| +
-// 3.6 M |p - v| + 32 M |e|) <= 42 u M (|p - v| + |e|) for |e| <= 3.5 M; one
-// band serves the three, 64 u M (|p - a|_1 + 2 reach) with |p - v| <= |p - a| +
-// reach and |e| <= reach (a band too wide only leaves more to FP64): six
-// square roots and three divisions fewer per face than bands and segments of
-// their own (verify_fp32 on the 1e6-triangle torus, 2e7 queries, with the
-// 64-byte nodes and faces: 72 -> 48 ms, 41 with four CTAs per SM).
-__device__ __forceinline__ bool face_d2n(F3 p, const Face &f, float um, float lim, float &d2) {
-  const F3 ap = p - f.a;
-  const float h = dotf(f.n, ap), h2 = h * h;
-  d2 = h2;
-  if (h2 > lim) return false;
-  const F3 ab = f.b - f.a, bc = f.c - f.b, ca = f.a - f.c, bp = p - f.b, cp = p - f.c;
-  const float band = 64.f * um * (fabsf(ap.x) + fabsf(ap.y) + fabsf(ap.z) + 2.f * f.reach);
-  const float ea = dotf(crossf(f.n, ab), ap), eb = dotf(crossf(f.n, bc), bp),
-              ec = dotf(crossf(f.n, ca), cp);
-  const float least = fminf(ea, fminf(eb, ec));
-  if (least > band) return true;  // inside
-  float seg = INFINITY;
-  auto segment = [&](F3 q, F3 e, float inv) {
-    const float t = __saturatef(dotf(q, e) * inv);
-    const F3 r = q - e * t;
-    seg = fminf(seg, dotf(r, r));
-  };
-  if (ea <= band) segment(ap, ab, f.inv_ab);
-  if (eb <= band) segment(bp, bc, f.inv_bc);
-  if (ec <= band) segment(cp, ca, f.inv_ca);
-  if (least < -band) {
-    d2 = seg;
-    return true;
-  }
-  d2 = fminf(h2, seg);
-  return false;
-}
 
 // Faces whose FP64 distance to the image can be the smallest: every face
 // whose FP32 distance (or, for a face face_d2n leaves undecided or one
@@ -1304,7 +1236,7 @@ __global__ void lbvh_face_records(const double *xyz, uint64_t nv, const int32_t 
   }
   const D3 ab = c[1] - c[0], ac = c[2] - c[0], n = cross(ab, ac);
   const D3 u = unit(n);  // the normal test's expression (normal_agrees), once per face
-  fn64[3 * f] = u.x, fn64[3 * f + 1] = u.y, fn64[3 * f + 2] = u.z;
+  if (fn64) fn64[3 * f] = u.x, fn64[3 * f + 1] = u.y, fn64[3 * f + 2] = u.z;
   const double n2 = dot(n, n), l2 = dot(ab, ab) * dot(ac, ac);
   const bool usable = n2 > 1e-12 * l2 && n2 > 4e-28;
   float inv[3], longest = 0;
