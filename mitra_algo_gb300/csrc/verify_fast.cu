@@ -466,7 +466,10 @@ struct RowLists {
   uint8_t *mark;        // per query: 1 = left to the next kernel (FP64, then reference order)
   int32_t *fp64;        // queries decided in FP64, ascending
   int32_t *reference;   // queries left to the wide list, then to the reference-order BVH
-  int32_t *open;        // FP64 queries the first FP64 pass leaves to the second
+  // FP64 queries the first FP64 pass leaves to the second: with candidates
+  // from the front, without from the back of `capacity` entries
+  int32_t *open;
+  uint64_t capacity;
   // the FP32 candidates of an FP64 query (kCandidates per slot, kNoFace
   // padded), so the FP64 decisions need no search of their own; slot_of[qid]
   // = kNoSlot for a query sent on before its candidates were known,
@@ -474,7 +477,7 @@ struct RowLists {
   uint32_t *slot_of;
   int32_t *cand;
   unsigned long long slots;    // capacity of cand, in slots
-  unsigned long long *counts;  // [forward, slots used, open, tie]
+  unsigned long long *counts;  // [forward, slots used, open with candidates, tie, open without]
 };
 
 // Decisions in FP32 (verify_fp32).  The reference's tests are made with
@@ -684,173 +687,179 @@ __global__ void forward_errors(Surface s, const ClusterMotion *motions, RowLists
 // search reaches takes the test (first_in_reference_order); rows whose
 // candidates overflow the list are listed for verify_listed_ref.
 //
-// Eight lanes serve a row, two candidates each.  FP64 runs at 1/64 of the
-// FP32 rate, so it is kept to what FP32 cannot decide: a face whose nearest
-// point is one of its corners (most of a rough mesh's rows: the faces around
-// a vertex at exactly one distance) takes that vertex's |q - v|^2, eight FP64
-// operations instead of some eighty; another face is evaluated only when its
-// FP32 distance does not already put it beyond the smallest of those; the
-// normal test and the visiting order go through FP32 with a band.  A warp pays
-// for a whole distance when one of its four rows needs one, so the first pass
-// (ALL = false) leaves such rows, and those without candidates, in lists.open
-// for a second pass over them alone.  On the 1e6-triangle torus (1.1e7 rows)
-// the two take 17 and 11 ms; every candidate's distance, normal and order in
-// FP64 took 56 ms.
+// FP64 runs at 1/64 of the FP32 rate, and a warp pays for an FP64 operation
+// whether one of its lanes needs it or all: a lane serves a row (so the image
+// costs a warp its twenty operations once per 32 rows), and FP64 is kept to
+// what FP32 cannot decide.  A face whose nearest point is one of its corners
+// (most of a rough mesh's rows: the faces around a vertex at exactly one
+// distance) takes that vertex's |q - v|^2, eight FP64 operations and none for
+// the next face around the same vertex; another face is evaluated only when
+// its FP32 distance does not already put it beyond the smallest of those; the
+// normal test and the visiting order go through FP32 with a band.  Rows with a
+// face to evaluate, and those without candidates, are left by the first pass
+// (ALL = false) in lists.open for a second pass over them alone, from its two
+// ends: the searches of the latter take much longer and fill warps of their own.
+// On the 1e6-triangle torus (1.1e7 rows, 3.3e6 of them in the second pass) the
+// two take 4.4 and 4.2 ms; with eight lanes per row, each with its own copy of the
+// image, they took 17 and 11.
 template <bool ALL>
 __global__ void verify_rows_fp64(BvhView b, Surface s, RefBvh t, const double *vn, const float *vn32,
                                  const ClusterMotion *motions, const MotionF *motions32, double tau,
                                  float scale, uint8_t *flags, double *err, RowLists lists,
                                  unsigned long long rows, int *status) {
-  constexpr int kGroup = 8;  // lanes per row: candidates j = sub and sub + 8
-  const int sub = threadIdx.x % kGroup;
-  const unsigned group_mask = 0xffu << (threadIdx.x & 31 & ~(kGroup - 1));
-  const unsigned long long count = ALL ? lists.counts[2] : rows;
-  const int32_t *list = ALL ? lists.open : lists.fp64;
+  const unsigned long long searches = ALL ? lists.counts[4] : 0;
+  // the second pass's warps hold searches or rows with candidates, not both
+  const unsigned long long listed_from = (searches + 31) / 32 * 32;
+  const unsigned long long count = ALL ? listed_from + lists.counts[2] : rows;
   const uint64_t nv = b.nv;
-  for (uint64_t k = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / kGroup; k < count;
-       k += uint64_t(gridDim.x) * blockDim.x / kGroup) {  // whole groups
-  const uint64_t qid = uint64_t(list[k]);  // a query, as verify_fp32's
-  const uint64_t c = qid / (2 * nv), rem = qid % (2 * nv);
-  const bool inverse = rem >= nv;
-  const uint64_t i = uint64_t(b.order[rem % nv]);
-  const uint64_t row = qid - rem % nv + i;
-  const uint32_t slot = lists.slot_of[qid];
-  if (slot == kWideSlot) continue;  // left marked for verify_rows_wide
-  auto leave_open = [&]() {
-    if (sub == 0) lists.open[atomicAdd(&lists.counts[2], 1ull)] = int32_t(qid);
-  };
-  if (slot == kNoSlot) {  // no candidates yet: the search, on one lane
-    if (!ALL) {
-      leave_open();
-    } else if (sub == 0) {
-      double d = 0;
-      int32_t tied[kCandidates];
-      int v = hybrid_query(b, s, vn, motions[c], inverse, i, tau, scale, d, tied, status);
-      if (v == 3) {
-        atomicAdd(&lists.counts[3], 1ull);
-        const M3 r = query_rotation(motions[c], inverse);
-        D3 q;
-        query_skipped(motions[c], r, inverse, vertex(s, int32_t(i)), tau, q);
-        int32_t first = tied[0];
-        for (int x = 1; x < kCandidates && tied[x] >= 0; ++x)
-          first = first_in_reference_order(t, q, first, tied[x]);
-        v = normal_agrees_t(b, first, r, D3{vn[i], vn[nv + i], vn[2 * nv + i]}) ? 1 : 0;
+  const int lane = threadIdx.x & 31;
+  for (uint64_t k0 = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32 * 32; k0 < count;
+       k0 += uint64_t(gridDim.x) * blockDim.x) {  // whole warps
+    const uint64_t k = k0 + lane;
+    int32_t left = -1;      // the row to list for the second pass
+    bool search = false;    // ... which has to search
+    bool tie = false;
+    if (k < count && !(ALL && k >= searches && k < listed_from)) {
+      const uint64_t qid =  // a query, as verify_fp32's
+          uint64_t(!ALL              ? lists.fp64[k]
+                   : k < searches    ? lists.open[lists.capacity - 1 - k]
+                                     : lists.open[k - listed_from]);
+      const uint64_t c = qid / (2 * nv), rem = qid % (2 * nv);
+      const bool inverse = rem >= nv;
+      const uint64_t i = uint64_t(b.order[rem % nv]);
+      const uint64_t row = qid - rem % nv + i;
+      const uint32_t slot = lists.slot_of[qid];
+      if (slot == kWideSlot) {
+        // left marked for verify_rows_wide
+      } else if (slot == kNoSlot) {  // no candidates yet
+        if (!ALL) {
+          left = int32_t(qid), search = true;
+        } else {
+          double d = 0;
+          int32_t tied[kCandidates];
+          int v = hybrid_query(b, s, vn, motions[c], inverse, i, tau, scale, d, tied, status);
+          if (v == 3) {
+            tie = true;
+            const M3 r = query_rotation(motions[c], inverse);
+            D3 q;
+            query_skipped(motions[c], r, inverse, vertex(s, int32_t(i)), tau, q);
+            int32_t first = tied[0];
+            for (int x = 1; x < kCandidates && tied[x] >= 0; ++x)
+              first = first_in_reference_order(t, q, first, tied[x]);
+            v = normal_agrees_t(b, first, r, D3{vn[i], vn[nv + i], vn[2 * nv + i]}) ? 1 : 0;
+          }
+          flags[row] = v == 1;
+          if (!inverse) err[c * nv + i] = v == 1 ? d : 0.0;
+          if (v != 2) lists.mark[qid] = 0;  // marked queries go on to the reference-order search
+        }
+      } else {
+        // the image; verify_fp32 decided the 2 tau and side tests of a row with candidates
+        const ClusterMotion &m = motions[c];
+        const M3 r = query_rotation(m, inverse);
+        const D3 p = vertex(s, int32_t(i)), mt{m.t[0], m.t[1], m.t[2]};
+        const D3 q = inverse ? mul(r, p - mt) : mul(r, p) + mt;
+        const F3 qf{float(q.x), float(q.y), float(q.z)};
+        const float mag = fmaxf(scale, fmaxf(fabsf(qf.x), fmaxf(fabsf(qf.y), fabsf(qf.z))));
+        const float um = kErr * (1.f / 512.f) * mag;
+        const MotionF &mf = motions32[c];
+        float rf[9];
+        for (int j = 0; j < 9; ++j) rf[j] = inverse ? mf.r[(j % 3) * 3 + j / 3] : mf.r[j];
+        const F3 ni{vn32[i], vn32[nv + i], vn32[2 * nv + i]};
+        const F3 rn{rf[0] * ni.x + rf[1] * ni.y + rf[2] * ni.z, rf[3] * ni.x + rf[4] * ni.y + rf[5] * ni.z,
+                    rf[6] * ni.x + rf[7] * ni.y + rf[8] * ni.z};
+        const int32_t *cl = lists.cand + uint64_t(slot) * kCandidates;
+        auto candidate = [&](int j) {
+          const int32_t x = cl[j];
+          return x < 0 ? ~x : x;
+        };
+        // sets of candidates, a bit each: at the smallest distance so far, in
+        // no corner's region, with the normal, with the normal test undecided
+        unsigned at_min = 0, open = 0, agrees = 0, unsure = 0;
+        double dmin = INFINITY, dv = 0;
+        int32_t at_vertex = -1;  // of which dv is the squared distance
+        auto take = [&](double d, int j) {
+          if (d < dmin) dmin = d, at_min = 0;
+          if (d == dmin) at_min |= 1u << j;
+        };
+        for (int j = 0; j < kCandidates && cl[j] != kNoFace; ++j) {
+          const int32_t f = candidate(j);
+          const Face face = load_face(b, f);
+          const float cosine = dotf(rn, face.n);
+          if (face.reach == 0.f || !(fabsf(cosine - 0.5f) > kNormalBand)) unsure |= 1u << j;
+          else if (cosine > 0.5f) agrees |= 1u << j;
+          const int v = face.reach == 0.f ? -1 : corner_region(qf, face, um);
+          if (v < 0) {
+            open |= 1u << j;
+            continue;
+          }
+          const int32_t id = s.faces[uint64_t(v) * s.nf + f];
+          if (id != at_vertex) {
+            const D3 e = q - vertex(s, id);
+            dv = dot(e, e), at_vertex = id;
+          }
+          take(dv, j);
+        }
+        bool leave = false;
+        for (unsigned rest = open; rest && !leave; rest &= rest - 1) {
+          const int j = __ffs(rest) - 1;
+          const int32_t f = candidate(j);
+          if (dmin < INFINITY) {  // a decided FP32 distance is within 32 u M of FP64's
+            const Face face = load_face(b, f);
+            float key;
+            if (face.reach != 0.f && face_d2n(qf, face, um, INFINITY, key) &&
+                sqrtf(key) > sqrtf(float(dmin)) + 64.f * um)
+              continue;
+          }
+          if (ALL) take(triangle_d2(q, corner(s, f, 0), corner(s, f, 1), corner(s, f, 2)), j);
+          else leave = true;
+        }
+        if (leave) {
+          left = int32_t(qid);
+        } else {
+          bool ok = false;
+          if (dmin <= tau * tau) {  // the normal test of the faces at exactly the minimum
+            for (unsigned rest = at_min & unsure; rest; rest &= rest - 1) {
+              const int j = __ffs(rest) - 1;
+              if (normal_agrees_t(b, candidate(j), r, D3{vn[i], vn[nv + i], vn[2 * nv + i]}))
+                agrees |= 1u << j;
+            }
+            tie = (at_min & agrees) && (at_min & ~agrees);
+            if (tie) {
+              // they disagree: the one the reference visits first (its
+              // visiting order is a total order on the faces for this query)
+              int jf = __ffs(at_min) - 1;
+              int32_t first = candidate(jf);
+              for (unsigned rest = at_min & (at_min - 1); rest; rest &= rest - 1) {
+                const int j = __ffs(rest) - 1;
+                const int32_t f = candidate(j);
+                if (first_in_reference_order_f(t, q, um, first, f) != first) first = f, jf = j;
+              }
+              ok = agrees >> jf & 1u;
+            } else {
+              ok = (at_min & agrees) != 0;
+            }
+          }
+          flags[row] = ok;
+          if (!inverse) err[c * nv + i] = ok ? dmin : 0.0;
+          lists.mark[qid] = 0;
+        }
       }
-      flags[row] = v == 1;
-      if (!inverse) err[c * nv + i] = v == 1 ? d : 0.0;
-      if (v != 2) lists.mark[qid] = 0;  // marked queries go on to the reference-order search
     }
-    continue;
-  }
-  // the image; verify_fp32 decided the 2 tau and side tests of a row with candidates
-  const ClusterMotion &m = motions[c];
-  const M3 r = query_rotation(m, inverse);
-  const D3 p = vertex(s, int32_t(i)), mt{m.t[0], m.t[1], m.t[2]};
-  const D3 q = inverse ? mul(r, p - mt) : mul(r, p) + mt;
-  const F3 qf{float(q.x), float(q.y), float(q.z)};
-  const float mag = fmaxf(scale, fmaxf(fabsf(qf.x), fmaxf(fabsf(qf.y), fabsf(qf.z))));
-  const float um = kErr * (1.f / 512.f) * mag;
-  // distances compare as their bits: none is negative
-  constexpr unsigned long long kNone = 0x7ff0000000000000ull;
-  auto smallest = [&](unsigned long long x) {
-    for (int o = kGroup / 2; o; o >>= 1) {
-      const unsigned long long y = __shfl_xor_sync(group_mask, x, o);
-      if (y < x) x = y;
+    const unsigned ties = __ballot_sync(0xffffffffu, tie);
+    if (ties && lane == 0) atomicAdd(&lists.counts[3], (unsigned long long)__popc(ties));
+    if (!ALL) {  // one atomic per warp and list
+      const unsigned rows_left = __ballot_sync(0xffffffffu, left >= 0 && !search),
+                     to_search = __ballot_sync(0xffffffffu, left >= 0 && search);
+      unsigned long long at = 0;
+      if (lane == 0 && rows_left) at = atomicAdd(&lists.counts[2], (unsigned long long)__popc(rows_left));
+      if (lane == 1 && to_search) at = atomicAdd(&lists.counts[4], (unsigned long long)__popc(to_search));
+      const unsigned long long rows_at = __shfl_sync(0xffffffffu, at, 0),
+                               search_at = __shfl_sync(0xffffffffu, at, 1);
+      const unsigned lt = (1u << lane) - 1;
+      if (left >= 0 && !search) lists.open[rows_at + __popc(rows_left & lt)] = left;
+      if (left >= 0 && search)
+        lists.open[lists.capacity - 1 - (search_at + __popc(to_search & lt))] = left;
     }
-    return x;
-  };
-  const int32_t *cl = lists.cand + uint64_t(slot) * kCandidates;
-  int32_t f[2];
-  unsigned long long d[2] = {kNone, kNone};
-  bool open[2] = {false, false};
-  float key[2] = {0.f, 0.f};
-  F3 fn[2];
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int32_t x = cl[sub + kGroup * h];
-    f[h] = x == kNoFace ? -1 : (x < 0 ? ~x : x);
-    if (f[h] < 0) continue;
-    const Face face = load_face(b, f[h]);
-    fn[h] = face.n;
-    open[h] = true;
-    if (face.reach == 0.f) continue;
-    const int v = corner_region(qf, face, um);
-    if (v >= 0) {
-      const D3 e = q - corner(s, f[h], v);
-      d[h] = __double_as_longlong(dot(e, e));
-      open[h] = false;
-    } else if (!face_d2n(qf, face, um, INFINITY, key[h])) {
-      key[h] = 0.f;
-    }
-  }
-  unsigned long long dmin = smallest(d[0] < d[1] ? d[0] : d[1]);
-  // a decided FP32 distance is within 32 u M of FP64's
-  const float beyond = dmin == kNone ? INFINITY : sqrtf(float(__longlong_as_double(dmin))) + 64.f * um;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) open[h] = open[h] && !(sqrtf(key[h]) > beyond);
-  if (ALL) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-      if (open[h])
-        d[h] = __double_as_longlong(
-            triangle_d2(q, corner(s, f[h], 0), corner(s, f[h], 1), corner(s, f[h], 2)));
-    dmin = smallest(d[0] < d[1] ? d[0] : d[1]);
-  } else if (__ballot_sync(group_mask, open[0] || open[1]) & group_mask) {
-    leave_open();
-    continue;
-  }
-  int v = 0;
-  if (dmin <= (unsigned long long)__double_as_longlong(tau * tau)) {
-    // the normal test of the faces at exactly the minimum
-    const MotionF &mf = motions32[c];
-    float rf[9];
-    for (int j = 0; j < 9; ++j) rf[j] = inverse ? mf.r[(j % 3) * 3 + j / 3] : mf.r[j];
-    const F3 ni{vn32[i], vn32[nv + i], vn32[2 * nv + i]};
-    const F3 rn{rf[0] * ni.x + rf[1] * ni.y + rf[2] * ni.z, rf[3] * ni.x + rf[4] * ni.y + rf[5] * ni.z,
-                rf[6] * ni.x + rf[7] * ni.y + rf[8] * ni.z};
-    int agree = 0, disagree = 0;
-    bool ok[2] = {false, false};
-    int32_t first = -1;  // this lane's face at the minimum the reference visits first
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-      if (f[h] >= 0 && d[h] == dmin) {
-        const float cosine = dotf(rn, fn[h]);
-        const bool sure = b.face[4 * int64_t(f[h]) + 3].w != 0.f && fabsf(cosine - 0.5f) > kNormalBand;
-        ok[h] = sure ? cosine > 0.5f
-                     : normal_agrees_t(b, f[h], r, D3{vn[i], vn[nv + i], vn[2 * nv + i]});
-        if (ok[h]) ++agree;
-        else ++disagree;
-        first = first < 0 ? f[h] : first_in_reference_order_f(t, q, um, first, f[h]);
-      }
-    for (int o = kGroup / 2; o; o >>= 1) {
-      agree += __shfl_xor_sync(group_mask, agree, o);
-      disagree += __shfl_xor_sync(group_mask, disagree, o);
-    }
-    if (agree && disagree) {
-      // faces at the minimum disagree: the one the reference visits first
-      // (its visiting order is a total order on the faces for this
-      // query, so the group reduces it like a minimum)
-      for (int o = kGroup / 2; o; o >>= 1) {
-        const int32_t other = __shfl_xor_sync(group_mask, first, o);
-        if (other >= 0)
-          first = first < 0 ? other : first_in_reference_order_f(t, q, um, first, other);
-      }
-      const bool mine_agrees = (f[0] == first && first >= 0 && ok[0]) || (f[1] == first && first >= 0 && ok[1]);
-      v = (__ballot_sync(group_mask, mine_agrees) & group_mask) ? 1 : 0;
-      if (sub == 0) {  // one count per converged set of groups
-        const unsigned active = __activemask();
-        const unsigned leaders = active & 0x01010101u;
-        if ((threadIdx.x & 31) == __ffs(leaders) - 1) atomicAdd(&lists.counts[3], __popc(leaders));
-      }
-    } else {
-      v = agree ? 1 : 0;
-    }
-  }
-  if (sub == 0) {
-    flags[row] = v == 1;
-    if (!inverse) err[c * nv + i] = v == 1 ? __longlong_as_double(dmin) : 0.0;
-    lists.mark[qid] = 0;
-  }
   }
 }
 
@@ -1424,9 +1433,10 @@ uint64_t exact_flags(Call &call, const ResidentSurface &m, const ClusterMotion *
   lists.slot_of = call.alloc<uint32_t>(rows);
   lists.slots = std::min<uint64_t>(rows, uint64_t(1) << 24);  // at most 1 GiB of candidates
   lists.cand = call.alloc<int32_t>(lists.slots * kCandidates);
-  lists.counts = call.alloc<unsigned long long>(4);
+  lists.counts = call.alloc<unsigned long long>(5);
+  lists.capacity = rows;
   uint64_t *listed = call.alloc<uint64_t>(2);
-  SYM_CUDA(cudaMemsetAsync(lists.counts, 0, 32, st));
+  SYM_CUDA(cudaMemsetAsync(lists.counts, 0, 40, st));
   const BvhView view = view_of(bvh);
   Surface s{m.xyz, nv, m.faces, m.nf, nullptr, nullptr};
   verify_fp32<<<blocks_for(rows), kThreads, 0, st>>>(view, bvh.vn, dmf, nc, float(tau), bvh.scale,
@@ -1447,11 +1457,11 @@ uint64_t exact_flags(Call &call, const ResidentSurface &m, const ClusterMotion *
     ensure_ref_bvh(call, m);
     s.nodes = m.ref->dev.nodes, s.ids = m.ref->dev.ids;
     lists.open = lists.reference;  // free until the next compaction
-    verify_rows_fp64<false><<<blocks_for(counts[1] * 8), kThreads, 0, st>>>(
+    verify_rows_fp64<false><<<blocks_for(counts[1]), kThreads, 0, st>>>(
         view, s, m.ref->dev, m.vn, bvh.vn, dm, dmf, tau, bvh.scale, flags, err, lists, counts[1],
         call.status());
     check_launch();
-    verify_rows_fp64<true><<<unsigned(std::min<uint64_t>(blocks_for(counts[1] * 8), 152 * 8)), kThreads,
+    verify_rows_fp64<true><<<unsigned(std::min<uint64_t>(blocks_for(counts[1] + 32), 152 * 8)), kThreads,
                              0, st>>>(view, s, m.ref->dev, m.vn, bvh.vn, dm, dmf, tau, bvh.scale, flags,
                                       err, lists, 0, call.status());
     check_launch();
