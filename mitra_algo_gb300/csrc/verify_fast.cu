@@ -921,31 +921,74 @@ __global__ void verify_listed_ref(Surface s, const double *vn, const int32_t *or
   if (!inverse) err[c * nv + i] = ok ? d : 0.0;
 }
 
-// Block c < nc: sum of the forward errors, supporting weight (both
-// directions) and forward count of cluster c; block nc: the total weight.
-// Fixed-order strided partials and a fixed tree: reproducible, and within
-// a few units of rounding of the reference's serial sums.
-__global__ void __launch_bounds__(256) tree_sums(const uint8_t *flags, const double *err,
-                                                 const double *w, uint64_t nv, uint64_t nc,
-                                                 double *error, double *area, uint64_t *count,
-                                                 double *total) {
-  __shared__ double se[256], sa[256];
-  __shared__ unsigned long long sn[256];
-  const uint64_t c = blockIdx.x;
-  double e = 0, a = 0;
-  unsigned long long n = 0;
-  if (c == nc) {
-    for (uint64_t i = threadIdx.x; i < nv; i += 256) a += w[i];
-  } else {
-    const uint8_t *fa = flags + c * 2 * nv, *fb = fa + nv;
-    for (uint64_t i = threadIdx.x; i < nv; i += 256) {
-      if (fa[i]) e += err[c * nv + i], a += w[i], ++n;
-      if (fb[i]) a += w[i];
+// Cluster c < nc: sum of the forward errors, supporting weight (both
+// directions) and forward count; c == nc: the total weight.  kTreeThreads
+// fixed-order strided partials and a fixed tree: reproducible, and within a
+// few units of rounding of the reference's serial sums.  A partial is a chain
+// of FP64 additions, which one SM runs at 1/64 of its FP32 rate, so the chains
+// are spread: a warp of 32 strides takes one of the two sums
+// (tree_partials, one-warp blocks), with kTreeAhead elements' loads in flight,
+// and the trees follow in a kernel of their own.  1e6-triangle torus, 20
+// clusters: 490 us; a block of all 256 strides per cluster took 1,570 us.
+constexpr int kTreeThreads = 256, kTreeAhead = 8;
+
+__global__ void __launch_bounds__(32) tree_partials(const uint8_t *flags, const double *err,
+                                                    const double *w, uint64_t nv, uint64_t nc,
+                                                    double *partial, unsigned *partial_count) {
+  const uint64_t c = blockIdx.z, kind = blockIdx.y;  // 0: the errors, 1: the weights
+  const unsigned stride0 = blockIdx.x * 32 + threadIdx.x;
+  const uint8_t *fa = flags + c * 2 * nv, *fb = fa + nv;
+  double sum = 0;
+  unsigned n = 0;
+  for (uint64_t i0 = stride0; i0 < nv; i0 += kTreeThreads * kTreeAhead) {
+    if (c == nc) {
+      if (kind == 0) break;
+      double v[kTreeAhead];
+#pragma unroll
+      for (int k = 0; k < kTreeAhead; ++k) {
+        const uint64_t i = i0 + uint64_t(k) * kTreeThreads;
+        v[k] = i < nv ? w[i] : 0.0;
+      }
+#pragma unroll
+      for (int k = 0; k < kTreeAhead; ++k)
+        if (i0 + uint64_t(k) * kTreeThreads < nv) sum += v[k];
+      continue;
+    }
+    bool a[kTreeAhead], b[kTreeAhead];
+    double v[kTreeAhead];
+#pragma unroll
+    for (int k = 0; k < kTreeAhead; ++k) {
+      const uint64_t i = i0 + uint64_t(k) * kTreeThreads;
+      a[k] = i < nv && fa[i], b[k] = i < nv && kind == 1 && fb[i];
+    }
+#pragma unroll
+    for (int k = 0; k < kTreeAhead; ++k) {
+      const uint64_t i = i0 + uint64_t(k) * kTreeThreads;
+      v[k] = a[k] || b[k] ? (kind == 0 ? err[c * nv + i] : w[i]) : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < kTreeAhead; ++k) {
+      if (a[k]) sum += v[k], ++n;
+      if (b[k]) sum += v[k];
     }
   }
-  se[threadIdx.x] = e, sa[threadIdx.x] = a, sn[threadIdx.x] = n;
+  const uint64_t at = (c * 2 + kind) * kTreeThreads + stride0;
+  partial[at] = sum;
+  if (kind == 0) partial_count[c * kTreeThreads + stride0] = n;
+}
+
+__global__ void __launch_bounds__(kTreeThreads) tree_sums(const double *partial,
+                                                          const unsigned *partial_count, uint64_t nc,
+                                                          double *error, double *area,
+                                                          uint64_t *count, double *total) {
+  __shared__ double se[kTreeThreads], sa[kTreeThreads];
+  __shared__ unsigned long long sn[kTreeThreads];
+  const uint64_t c = blockIdx.x;
+  se[threadIdx.x] = partial[c * 2 * kTreeThreads + threadIdx.x];
+  sa[threadIdx.x] = partial[(c * 2 + 1) * kTreeThreads + threadIdx.x];
+  sn[threadIdx.x] = partial_count[c * kTreeThreads + threadIdx.x];
   __syncthreads();
-  for (int h = 128; h; h >>= 1) {
+  for (int h = kTreeThreads / 2; h; h >>= 1) {
     if (int(threadIdx.x) < h) {
       se[threadIdx.x] += se[threadIdx.x + h];
       sa[threadIdx.x] += sa[threadIdx.x + h];
@@ -1055,40 +1098,116 @@ __global__ void refine_pairs(BvhView b, const double *xyz, const double *vn,
   ok[row] = 1;
 }
 
-constexpr int kRefineSums = 28, kRefineThreads = 128;
+constexpr int kRefineSums = 28, kRefineThreads = 128, kRefineGroups = 9, kRefineAhead = 4;
 
-// Block c: the weighted sums of mode c's correspondences (p the vertex, q its
-// target, both relative to o; weights = vertex weights): W, W p, W q,
-// W p q^T (row-major), W p p^T and W q q^T (upper triangles).  Fixed-order
-// strided partials and a fixed tree.
-__global__ void __launch_bounds__(kRefineThreads) refine_sums(const double *xyz, const double *w,
-                                                              uint64_t nv, const uint8_t *ok,
-                                                              const double *target, Origin o,
-                                                              double *sums) {
-  __shared__ double part[kRefineSums][kRefineThreads];
-  const uint64_t c = blockIdx.x;
-  double acc[kRefineSums];
-  for (int k = 0; k < kRefineSums; ++k) acc[k] = 0;
-  for (uint64_t i = threadIdx.x; i < nv; i += kRefineThreads) {
-    if (!ok[c * nv + i]) continue;
-    const double wi = w[i];
-    double p[3], q[3];
-    for (int a = 0; a < 3; ++a) p[a] = xyz[a * nv + i] - o.x[a], q[a] = target[(c * nv + i) * 3 + a];
-    acc[0] += wi;
-    for (int a = 0; a < 3; ++a) acc[1 + a] += wi * p[a], acc[4 + a] += wi * q[a];
-    for (int a = 0; a < 3; ++a)
-      for (int e = 0; e < 3; ++e) acc[7 + a * 3 + e] += wi * p[a] * q[e];
-    for (int a = 0, at = 0; a < 3; ++a)
-      for (int e = a; e < 3; ++e, ++at) acc[16 + at] += wi * p[a] * p[e], acc[22 + at] += wi * q[a] * q[e];
+// The strided partials of N sums over the correspondences of one cluster: a
+// thread takes vertices i0, i0 + kRefineThreads, ... in order.  `terms` adds a
+// correspondence's terms from its weight and those of the coordinates of p
+// (the vertex) and q (its target) that the masks P and Q name; the loads of
+// kRefineAhead vertices are in flight together.
+template <unsigned P, unsigned Q, int N, class Terms>
+__device__ __forceinline__ void refine_partials(const double *xyz, const double *w, uint64_t nv,
+                                                const uint8_t *ok, const double *target,
+                                                const Origin &o, uint64_t i0, double *out,
+                                                Terms &&terms) {
+  double acc[N];
+  for (int k = 0; k < N; ++k) acc[k] = 0;
+  for (uint64_t at = i0; at < nv; at += kRefineThreads * kRefineAhead) {
+    bool use[kRefineAhead];
+    double wi[kRefineAhead], p[kRefineAhead][3], q[kRefineAhead][3];
+#pragma unroll
+    for (int k = 0; k < kRefineAhead; ++k) {
+      const uint64_t i = at + uint64_t(k) * kRefineThreads;
+      use[k] = i < nv && ok[i];
+    }
+#pragma unroll
+    for (int k = 0; k < kRefineAhead; ++k) {
+      if (!use[k]) continue;
+      const uint64_t i = at + uint64_t(k) * kRefineThreads;
+      wi[k] = w[i];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        if (P >> a & 1) p[k][a] = xyz[a * nv + i];
+        if (Q >> a & 1) q[k][a] = target[i * 3 + a];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kRefineAhead; ++k) {
+      if (!use[k]) continue;
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+        if (P >> a & 1) p[k][a] -= o.x[a];
+      terms(acc, wi[k], p[k], q[k]);
+    }
   }
-  for (int k = 0; k < kRefineSums; ++k) part[k][threadIdx.x] = acc[k];
-  __syncthreads();
-  for (int s = kRefineThreads / 2; s; s >>= 1) {
-    if (int(threadIdx.x) < s)
-      for (int k = 0; k < kRefineSums; ++k) part[k][threadIdx.x] += part[k][threadIdx.x + s];
-    __syncthreads();
+  for (int k = 0; k < N; ++k) out[k * kRefineThreads] = acc[k];
+}
+
+// The weighted sums of mode c's correspondences (p the vertex, q its target,
+// both relative to o; weights = vertex weights): W, W p, W q, W p q^T
+// (row-major), W p p^T and W q q^T (upper triangles), as kRefineThreads
+// fixed-order strided partials each; refine_solve adds them by a fixed tree.
+// Bound by FP64 additions and products at 1/64 of the FP32 rate, so they are
+// spread over the SMs: one-warp blocks (32 strides, one of kRefineGroups
+// groups of three or four sums with a common factor, cluster).  16k vertices,
+// 8 clusters: 56 us; one block per cluster took 318.
+__global__ void __launch_bounds__(32) refine_sums(const double *xyz, const double *w, uint64_t nv,
+                                                  const uint8_t *ok_all, const double *target_all,
+                                                  Origin o, double *partial) {
+  const uint64_t c = blockIdx.z;
+  const unsigned stride0 = blockIdx.x * 32 + threadIdx.x;
+  const uint8_t *ok = ok_all + c * nv;
+  const double *target = target_all + c * nv * 3;
+  double *out = partial + c * kRefineSums * kRefineThreads + stride0;
+  auto sums_at = [&](int k) { return out + k * kRefineThreads; };
+  // w x[A] (y0, y1, y2) into acc[0..2]
+  auto row = [](double *acc, double wx, const double *y) {
+    for (int e = 0; e < 3; ++e) acc[e] += wx * y[e];
+  };
+  switch (blockIdx.y) {
+    case 0:
+      refine_partials<7, 0, 4>(xyz, w, nv, ok, target, o, stride0, sums_at(0),
+                               [&](double *acc, double wi, const double *p, const double *) {
+                                 acc[0] += wi;
+                                 for (int a = 0; a < 3; ++a) acc[1 + a] += wi * p[a];
+                               });
+      break;
+    case 1:
+      refine_partials<0, 7, 3>(xyz, w, nv, ok, target, o, stride0, sums_at(4),
+                               [&](double *acc, double wi, const double *, const double *q) { row(acc, wi, q); });
+      break;
+    case 2:
+      refine_partials<1, 7, 3>(xyz, w, nv, ok, target, o, stride0, sums_at(7),
+                               [&](double *acc, double wi, const double *p, const double *q) { row(acc, wi * p[0], q); });
+      break;
+    case 3:
+      refine_partials<2, 7, 3>(xyz, w, nv, ok, target, o, stride0, sums_at(10),
+                               [&](double *acc, double wi, const double *p, const double *q) { row(acc, wi * p[1], q); });
+      break;
+    case 4:
+      refine_partials<4, 7, 3>(xyz, w, nv, ok, target, o, stride0, sums_at(13),
+                               [&](double *acc, double wi, const double *p, const double *q) { row(acc, wi * p[2], q); });
+      break;
+    case 5:
+      refine_partials<7, 0, 3>(xyz, w, nv, ok, target, o, stride0, sums_at(16),
+                               [&](double *acc, double wi, const double *p, const double *) { row(acc, wi * p[0], p); });
+      break;
+    case 6:
+      refine_partials<6, 0, 3>(xyz, w, nv, ok, target, o, stride0, sums_at(19),
+                               [&](double *acc, double wi, const double *p, const double *) {
+                                 acc[0] += wi * p[1] * p[1], acc[1] += wi * p[1] * p[2], acc[2] += wi * p[2] * p[2];
+                               });
+      break;
+    case 7:
+      refine_partials<0, 7, 3>(xyz, w, nv, ok, target, o, stride0, sums_at(22),
+                               [&](double *acc, double wi, const double *, const double *q) { row(acc, wi * q[0], q); });
+      break;
+    default:
+      refine_partials<0, 6, 3>(xyz, w, nv, ok, target, o, stride0, sums_at(25),
+                               [&](double *acc, double wi, const double *, const double *q) {
+                                 acc[0] += wi * q[1] * q[1], acc[1] += wi * q[1] * q[2], acc[2] += wi * q[2] * q[2];
+                               });
   }
-  if (threadIdx.x < kRefineSums) sums[c * kRefineSums + threadIdx.x] = part[threadIdx.x][0];
 }
 
 // Eigen-decomposition of a symmetric 3x3 matrix (row-major) by cyclic
@@ -1137,7 +1256,8 @@ __device__ void jacobi3(const double m[9], double val[3], double vec[9]) {
       }
 }
 
-// One thread per mode: the least-squares motion of its correspondences.
+// A block per mode adds the partials of refine_sums, one thread of it finds
+// the least-squares motion of the correspondences.
 // Rigid: the rotation R maximising tr(R H), H = sum w (p - pbar)(q - qbar)^T,
 // from H's singular vectors (Kabsch: H = U S V^T, R = V diag(1, 1, d) U^T
 // with d making det R = +1), t = qbar - R pbar.  Reflection: the plane
@@ -1145,10 +1265,21 @@ __device__ void jacobi3(const double m[9], double val[3], double vec[9]) {
 // run along it), oriented like the previous one, and the plane passes
 // through the weighted mean of the midpoints (p + q) / 2.  A mode with too
 // few or degenerate correspondences keeps its motion.
-__global__ void refine_solve(const double *sums, uint64_t nc, Origin o, ClusterMotion *motions) {
-  const uint64_t c = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (c >= nc) return;
-  const double *s = sums + c * kRefineSums;
+__global__ void __launch_bounds__(kRefineThreads) refine_solve(const double *partial, Origin o,
+                                                               ClusterMotion *motions) {
+  __shared__ double part[kRefineSums][kRefineThreads];
+  const uint64_t c = blockIdx.x;
+  for (int k = 0; k < kRefineSums; ++k)
+    part[k][threadIdx.x] = partial[(c * kRefineSums + k) * kRefineThreads + threadIdx.x];
+  __syncthreads();
+  for (int h = kRefineThreads / 2; h; h >>= 1) {
+    if (int(threadIdx.x) < h)
+      for (int k = 0; k < kRefineSums; ++k) part[k][threadIdx.x] += part[k][threadIdx.x + h];
+    __syncthreads();
+  }
+  if (threadIdx.x) return;
+  double s[kRefineSums];
+  for (int k = 0; k < kRefineSums; ++k) s[k] = part[k][0];
   const double W = s[0];
   if (!(W > 0)) return;
   double pb[3], qb[3];
@@ -1355,16 +1486,18 @@ void refine_motions(Call &call, const BvhView &view, const double *xyz, const do
   if (refine <= 0 || !nc || !nv || !view.nf) return;
   cudaStream_t st = call.stream();
   const Origin o{{origin[0], origin[1], origin[2]}};
-  double *target = call.alloc<double>(nc * nv * 3), *sums = call.alloc<double>(nc * kRefineSums);
+  double *target = call.alloc<double>(nc * nv * 3);
+  double *partial = call.alloc<double>(nc * kRefineSums * kRefineThreads);
   uint8_t *ok = call.alloc<uint8_t>(nc * nv);
   for (int it = 0; it < refine; ++it) {
     refine_pairs<<<blocks_for(nc * nv), kThreads, 0, st>>>(view, xyz, vn, dm, nc, tau,
                                                            float(tau * tau), o, target, ok,
                                                            call.status());
     check_launch();
-    refine_sums<<<unsigned(nc), kRefineThreads, 0, st>>>(xyz, w, nv, ok, target, o, sums);
+    refine_sums<<<dim3(kRefineThreads / 32, kRefineGroups, unsigned(nc)), 32, 0, st>>>(
+        xyz, w, nv, ok, target, o, partial);
     check_launch();
-    refine_solve<<<unsigned((nc + 31) / 32), 32, 0, st>>>(sums, nc, o, dm);
+    refine_solve<<<unsigned(nc), kRefineThreads, 0, st>>>(partial, o, dm);
     check_launch();
     call.launched(3);
   }
@@ -1527,9 +1660,14 @@ void verification_fast(Call &call, const ResidentSurface &m, sym_cluster_record 
   if (undecided) *undecided = n;
   double *error = call.alloc<double>(nc), *area = call.alloc<double>(nc), *total = call.alloc<double>(1);
   uint64_t *na = call.alloc<uint64_t>(nc);
-  tree_sums<<<unsigned(nc + 1), 256, 0, st>>>(flags, err, m.w, nv, nc, error, area, na, total);
+  double *partial = call.alloc<double>((nc + 1) * 2 * kTreeThreads);
+  unsigned *partial_count = call.alloc<unsigned>((nc + 1) * kTreeThreads);
+  tree_partials<<<dim3(kTreeThreads / 32, 2, unsigned(nc + 1)), 32, 0, st>>>(flags, err, m.w, nv, nc,
+                                                                            partial, partial_count);
   check_launch();
-  call.launched();
+  tree_sums<<<unsigned(nc + 1), kTreeThreads, 0, st>>>(partial, partial_count, nc, error, area, na, total);
+  check_launch();
+  call.launched(2);
   int32_t *parent = call.alloc<int32_t>(rows);
   unsigned *dpatch = call.alloc<unsigned>(2 * nc);
   SYM_CUDA(cudaMemsetAsync(dpatch, 0, 8 * nc, st));
