@@ -279,22 +279,6 @@ __device__ __forceinline__ Two<double> fma2(Two<double> a, Two<double> b, Two<do
   return {fma(a.x, b.x, c.x), fma(a.y, b.y, c.y)};
 }
 
-// a / b, correctly rounded, from r = 1 / b correctly rounded (a <= b): two
-// residual corrections q + (a - b q) r.  The first leaves q within one unit in
-// the last place; from there the second rounds correctly (P. Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000 processor",
-// 1990).  No branch, unlike the general division, so several overlap.  (A
-// quotient so small that its residual underflows is far below the weights'
-// rounding.)
-__device__ __forceinline__ float ratio(float a, float b, float r) {
-  float q = a * r;
-  q = fmaf(fmaf(-b, q, a), r, q);
-  return fmaf(fmaf(-b, q, a), r, q);
-}
-__device__ __forceinline__ double ratio(double a, double b, double) { return a / b; }
-__device__ __forceinline__ float reciprocal(float b) { return __frcp_rn(b); }
-__device__ __forceinline__ double reciprocal(double) { return 0.0; }
-
 // A run of kSubVotes votes in shared memory: coordinate d of vote j at
 // (j / 2) * kPairStride + 2 d + j % 2, so a pair's coordinates are adjacent
 // (packed arithmetic) and lanes reading different votes meet different banks.
@@ -555,7 +539,7 @@ __device__ bool solve6(T (&M)[6][6], T (&b)[6], T tiny) {
       b[c] = b[piv], b[piv] = t;
     }
     for (int r = c + 1; r < 6; ++r) {
-      T f = M[r][c] / M[c][c];
+      T f = quotient(M[r][c], M[c][c]);
       for (int j = c; j < 6; ++j) M[r][j] -= f * M[c][j];
       b[r] -= f * b[c];
     }
@@ -563,7 +547,7 @@ __device__ bool solve6(T (&M)[6][6], T (&b)[6], T tiny) {
   for (int c = 5; c >= 0; --c) {
     T s = b[c];
     for (int j = c + 1; j < 6; ++j) s -= M[c][j] * b[j];
-    b[c] = s / M[c][c];
+    b[c] = quotient(s, M[c][c]);
   }
   return true;
 }
@@ -665,7 +649,7 @@ __global__ void __launch_bounds__(kChunk) ms_update(T *means, const T *red, uint
   T x[6], delta[6], move = 0;
   for (int d = 0; d < 6; ++d) {
     x[d] = means[uint64_t(s) * 8 + d];
-    delta[d] = acc[d] / acc[6];  // m - x from the sums of w (v - x)
+    delta[d] = quotient(acc[d], acc[6]);  // m - x from the sums of w (v - x)
     move += delta[d] * delta[d];
   }
   if (!near) {
@@ -699,129 +683,118 @@ __global__ void __launch_bounds__(kChunk) ms_update(T *means, const T *red, uint
 
 constexpr uint64_t kListedPairs = 32768;  // (tile, chunk) pairs from which the items pay (listed)
 
-constexpr int kRetile = 2048;  // seeds sorted in one block (static shared memory)
-
-__device__ __forceinline__ bool pair_less(unsigned long long ka, int32_t va, unsigned long long kb,
-                                          int32_t vb) {
-  return ka < kb || (ka == kb && va < vb);
+// Active seeds (kMoving, and kNear when include_near): in seed order, sorted
+// by the Morton key of their current mean (ties by seed id) when k <= kRetile.
+// nactive[0] = the number of active seeds, nactive[1] = how many of them are
+// kNear.  With `iter`, an iteration that finds active seeds records their
+// number in trace[*iter] (while *iter < trace_cap) and counts itself in *iter.
+//
+// Runs in every iteration between two kernels that wait for it, so its own
+// latency counts.  A block lists the active seeds for itself from their state
+// bytes.  Sorted, it makes every key and places kRankSeeds seeds by counting
+// the keys below each, a part of the keys per warp, where a bitonic network in
+// one block had up to 66 dependent steps (2,048 seeds: 15 us, 128: 5; the
+// network took 30 and 10).  Not sorted, a block places kRetile
+// seeds behind the active ones it counts before them.
+constexpr int kRetile = 2048;  // seeds a block lists
+constexpr int kRetileThreads = 256, kRankSeeds = 32;
+static_assert(kRetile == kRetileThreads * 8, "eight state bytes per thread");
+unsigned retile_blocks(uint64_t k) {
+  const uint64_t per = k <= kRetile ? kRankSeeds : kRetile;
+  return unsigned(std::max<uint64_t>(1, (k + per - 1) / per));  // one reports that there are none
 }
 
-// Sorts the n (<= kRetile) pairs keys[0..n), vals[0..n) of shared memory by
-// (key, value) and writes the values in that order to out[0..n); one block
-// of kRetile / 2 threads.  A bitonic network over the next power of two (at
-// least 64; padding pairs (~0, INT32_MAX) sort last): thread t holds
-// elements 2t and 2t + 1 in registers, so the stride-1 steps stay in the
-// thread, strides 2-32 are shuffles within a warp, and only the strides of
-// 64 and more go through the shared arrays.  The pairs are distinct (the
-// values are seed ids), so the order is the sorted order whatever the
-// network.
-__device__ void sort_pairs(unsigned long long *keys, int32_t *vals, unsigned n, int32_t *out) {
-  unsigned p2 = 64;
-  while (p2 < n) p2 <<= 1;
-  const unsigned t = threadIdx.x;
-  const bool on = t < p2 / 2;  // whole warps: p2 / 2 is a multiple of 32
-  unsigned long long k[2];
-  int32_t v[2];
-  for (int j = 0; j < 2; ++j) {
-    const unsigned i = 2 * t + j;
-    k[j] = on && i < n ? keys[i] : ~0ull;
-    v[j] = on && i < n ? vals[i] : 0x7fffffff;
-  }
-  __syncthreads();  // every pair read before the shared steps write
-  // element i keeps the smaller of (i, i ^ s) when it is the lower index of
-  // an ascending pair or the upper index of a descending one
-  auto step = [&](int j, unsigned size, unsigned s, unsigned long long pk, int32_t pv) {
-    const unsigned i = 2 * t + j;
-    const bool keep_min = ((i & s) == 0) == ((i & size) == 0);
-    if (pair_less(pk, pv, k[j], v[j]) == keep_min) k[j] = pk, v[j] = pv;
-  };
-  for (unsigned size = 2; size <= p2; size <<= 1)
-    for (unsigned s = size >> 1; s; s >>= 1) {
-      if (s >= 64) {
-        if (on)
-          for (int j = 0; j < 2; ++j) keys[2 * t + j] = k[j], vals[2 * t + j] = v[j];
-        __syncthreads();
-        if (on)
-          for (int j = 0; j < 2; ++j) {
-            const unsigned p = (2 * t + j) ^ s;
-            step(j, size, s, keys[p], vals[p]);
-          }
-        __syncthreads();
-      } else if (on && s == 1) {
-        const bool up = ((2 * t) & size) == 0;
-        if (pair_less(k[1], v[1], k[0], v[0]) == up) {
-          const unsigned long long tk = k[0];
-          const int32_t tv = v[0];
-          k[0] = k[1], v[0] = v[1], k[1] = tk, v[1] = tv;
-        }
-      } else if (on) {  // partner thread t ^ (s / 2), in the same warp
-        for (int j = 0; j < 2; ++j) {
-          const unsigned long long pk = __shfl_xor_sync(0xffffffffu, k[j], s >> 1);
-          const int32_t pv = __shfl_xor_sync(0xffffffffu, v[j], s >> 1);
-          step(j, size, s, pk, pv);
-        }
-      }
-    }
-  if (on)
-    for (int j = 0; j < 2; ++j)
-      if (2 * t + j < n) out[2 * t + j] = v[j];
-}
-
-// Active seeds (kMoving, and kNear when include_near) in seed order, then
-// sorted by the Morton key of
-// their current mean (ties by seed id) when k <= kRetile.  nactive[0] = the
-// number of active seeds, nactive[1] = how many of them are kNear.  With
-// `iter`, an iteration that finds active seeds records their number in
-// trace[*iter] (while *iter < trace_cap) and counts itself in *iter.
 template <typename T>
-__global__ void __launch_bounds__(1024) retile(const T *means, const uint8_t *state, uint64_t k,
-                                               const float *box, bool include_near, int32_t *ids,
-                                               unsigned *nactive, unsigned *iter = nullptr,
-                                               uint32_t *trace = nullptr, unsigned trace_cap = 0) {
+__global__ void __launch_bounds__(kRetileThreads) retile(const T *means, const uint8_t *state, uint64_t k,
+                                                         const float *box, bool include_near,
+                                                         int32_t *ids, unsigned *nactive,
+                                                         unsigned *iter = nullptr,
+                                                         uint32_t *trace = nullptr,
+                                                         unsigned trace_cap = 0) {
+  constexpr int kWarps = kRetileThreads / 32;
   __shared__ unsigned long long keys[kRetile];
-  __shared__ int32_t vals[kRetile];
-  __shared__ unsigned warp_tot[32];
-  __shared__ unsigned base_s, near_s;
-  if (threadIdx.x == 0) base_s = 0, near_s = 0;
-  __syncthreads();
-  bool sort = k <= kRetile;
-  for (uint64_t at = 0; at < k; at += blockDim.x) {
-    uint64_t s = at + threadIdx.x;
-    bool act = s < k && (state[s] == kMoving || (include_near && is_near(state[s])));
-    unsigned bal = __ballot_sync(0xffffffffu, act);
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) warp_tot[warp] = __popc(bal);
-    __syncthreads();
-    unsigned before = 0, total = 0;
-    for (int w = 0; w < int(blockDim.x >> 5); ++w) {
-      if (w < warp) before += warp_tot[w];
-      total += warp_tot[w];
-    }
-    unsigned pos = base_s + before + __popc(bal & ((1u << lane) - 1));
-    if (act && is_near(state[s])) atomicAdd(&near_s, 1u);
-    if (act) {
-      if (sort) {
-        float x[6];
-        for (int d = 0; d < 6; ++d) x[d] = float(means[s * 8 + d]);
-        keys[pos] = morton6(x, box);
-        vals[pos] = int32_t(s);
-      } else {
-        ids[pos] = int32_t(s);
+  __shared__ uint16_t seeds[kRetile];
+  __shared__ unsigned warp_active[kWarps], warp_near[kWarps], below[kWarps][kRankSeeds];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool sort = k <= kRetile;
+  const uint64_t first = sort ? 0 : uint64_t(blockIdx.x) * kRetile;
+  // the states of seeds s..s + 7 (zero bits: not active), `near` of them
+  unsigned mask = 0, near = 0, before = 0;
+  auto look = [&](uint64_t s, unsigned &m) {
+    for (int j = 0; j < 8; ++j)
+      if (s + j < k) {
+        const uint8_t st = state[s + j];
+        const bool close = include_near && is_near(st);
+        m |= unsigned(st == kMoving || close) << j;
+        near += close;
       }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) base_s += total;
-    __syncthreads();
+  };
+  for (uint64_t s = threadIdx.x * 8; s < first; s += kRetile) {  // (not sorted: the blocks before)
+    unsigned m = 0;
+    look(s, m);
+    before += __popc(m);
   }
-  unsigned n = base_s;
-  if (sort) sort_pairs(keys, vals, n, ids);
+  look(first + threadIdx.x * 8, mask);
+  // exclusive scan of the counts, with those of the blocks before on top
+  unsigned incl = __popc(mask);
+  const unsigned mine = incl;
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) warp_active[warp] = incl;
+  for (int o = 16; o; o >>= 1) {
+    near += __shfl_xor_sync(0xffffffffu, near, o);
+    before += __shfl_xor_sync(0xffffffffu, before, o);
+  }
+  if (lane == 0) warp_near[warp] = near, below[0][warp] = before;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    nactive[0] = n, nactive[1] = near_s;
+  unsigned at = incl - mine, total = 0;
+  before = near = 0;
+  for (int w = 0; w < kWarps; ++w) {
+    if (w < warp) at += warp_active[w];
+    total += warp_active[w], near += warp_near[w], before += below[0][w];
+  }
+  const unsigned n = before + total;
+  // a block that has looked at every seed reports
+  if (threadIdx.x == 0 && blockIdx.x == (sort ? 0 : gridDim.x - 1)) {
+    nactive[0] = n, nactive[1] = near;
     if (iter && n) {
       if (*iter < trace_cap) trace[*iter] = n;
       ++*iter;
     }
+  }
+  if (!sort) {
+    at += before;
+    for (unsigned m = mask; m; m &= m - 1)
+      ids[at++] = int32_t(first + threadIdx.x * 8 + __ffs(int(m)) - 1);
+    return;
+  }
+  const unsigned r0 = blockIdx.x * kRankSeeds;
+  if (r0 >= n) return;  // the whole block
+  for (unsigned m = mask; m; m &= m - 1) seeds[at++] = uint16_t(threadIdx.x * 8 + __ffs(int(m)) - 1);
+  __syncthreads();
+  for (unsigned i = threadIdx.x; i < n; i += kRetileThreads) {
+    const uint64_t s = seeds[i];
+    float x[6];
+    for (int d = 0; d < 6; ++d) x[d] = float(means[s * 8 + d]);
+    keys[i] = morton6(x, box);
+  }
+  __syncthreads();
+  const unsigned i = r0 + lane;
+  const unsigned long long key = i < n ? keys[i] : 0;
+  const unsigned part = (n + kWarps - 1) / kWarps, j0 = warp * part, j1 = min(n, j0 + part);
+  unsigned count = 0;
+  for (unsigned j = j0; j < j1; ++j) {
+    const unsigned long long other = keys[j];
+    count += other < key || (other == key && j < i);  // equal keys: the listed order is seed order
+  }
+  below[warp][lane] = count;
+  __syncthreads();
+  if (warp == 0 && i < n) {
+    unsigned rank = 0;
+    for (int w = 0; w < kWarps; ++w) rank += below[w][lane];
+    ids[rank] = int32_t(seeds[i]);
   }
 }
 
@@ -947,7 +920,7 @@ int shift_impl(Call &call, const VoteSet &v, const T *desc, T *means, uint8_t *s
   TileWork work = tile_work<T>(call, v, k);
   int it = 0;
   for (; it < max_iter; ++it) {
-    retile<T><<<1, 1024, 0, st>>>(means, state, k, v.gbox, polish, ids, nact);
+    retile<T><<<retile_blocks(k), kRetileThreads, 0, st>>>(means, state, k, v.gbox, polish, ids, nact);
     check_launch();
     unsigned counts[2] = {0, 0};
     SYM_CUDA(cudaMemcpyAsync(counts, nact, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
@@ -1055,8 +1028,8 @@ int shift(Call &call, const VoteSet &v, double *means, uint8_t *state, uint64_t 
 void active_seeds_async(Call &call, const VoteSet &v, const float *means, const uint8_t *state,
                         uint64_t k, int32_t *ids, unsigned *nact, unsigned *iter, uint32_t *trace,
                         unsigned trace_cap) {
-  retile<float><<<1, 1024, 0, call.stream()>>>(means, state, k, v.gbox, false, ids, nact, iter,
-                                               trace, trace_cap);
+  retile<float><<<retile_blocks(k), kRetileThreads, 0, call.stream()>>>(means, state, k, v.gbox, false, ids,
+                                                                        nact, iter, trace, trace_cap);
   check_launch();
   call.launched();
 }
@@ -1069,7 +1042,7 @@ void count_within(Call &call, const VoteSet &v, const float *points, uint64_t nm
   SYM_CUDA(cudaMemsetAsync(state, 0, nm, st));
   int32_t *ids = call.alloc<int32_t>(nm);
   unsigned *nact = call.alloc<unsigned>(2);
-  retile<float><<<1, 1024, 0, st>>>(points, state, nm, v.gbox, false, ids, nact);
+  retile<float><<<retile_blocks(nm), kRetileThreads, 0, st>>>(points, state, nm, v.gbox, false, ids, nact);
   check_launch();
   const Grid g = grid_for(nm, v.nchunks, v.tuning.simt_blocks_per_sm);
   TileWork work = tile_work<float>(call, v, nm);

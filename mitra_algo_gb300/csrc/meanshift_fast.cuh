@@ -37,6 +37,35 @@ constexpr uint8_t kNearRetry1 = 5;  // kNear after one rejected Newton step
 __host__ __device__ inline bool is_near(uint8_t s) { return s == kNear || s == kNearRetry1; }
 constexpr double kSwitch2 = 4e-4, kNewtonStop2 = 1e-8, kTrust = 0.25;
 constexpr int kNewtonCap = 10;
+#ifdef __CUDACC__
+// a / b, correctly rounded, from r = 1 / b correctly rounded: two residual
+// corrections q + (a - b q) r.  The first leaves q within one unit in the last
+// place; from there the second rounds correctly (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990).  No
+// branch, unlike the general division, so several overlap.
+__device__ __forceinline__ float ratio(float a, float b, float r) {
+  float q = a * r;
+  q = fmaf(fmaf(-b, q, a), r, q);
+  return fmaf(fmaf(-b, q, a), r, q);
+}
+__device__ __forceinline__ double ratio(double a, double b, double) { return a / b; }
+__device__ __forceinline__ float reciprocal(float b) { return __frcp_rn(b); }
+__device__ __forceinline__ double reciprocal(double) { return 0.0; }
+
+// a / b for any a and b: by ratio where neither the quotient nor its residual
+// can leave FP32's range, a zero included, else by the division, out of line.
+// The 27 quotients of a Newton step (ms_update, one thread per seed, a chain):
+// 36 -> 12 us at 2,048 seeds.
+static __device__ __noinline__ float divide(float a, float b) { return a / b; }
+__device__ __forceinline__ float quotient(float a, float b) {
+  const float x = fabsf(a), y = fabsf(b);
+  if (!(y > 1e-14f && y < 1e12f && (x == 0.f || (x > 1e-20f && x < 1e20f)))) return divide(a, b);
+  const float r = reciprocal(b);
+  return x == 0.f ? a * r : ratio(a, b, r);
+}
+__device__ __forceinline__ double quotient(double a, double b) { return a / b; }
+#endif
+
 // Floats (or doubles) per partial sum of one seed: sum w (v - x) (6), sum w, pad,
 // then for kNear seeds the unweighted in-window sums of d = v - x: sum d
 // (6) and sum d d^T (21, upper triangle row by row), pad.

@@ -392,77 +392,104 @@ __device__ __forceinline__ uint32_t block_scan_1024(uint32_t v, uint32_t *warp_s
 // budget = sms - tiles (at least tiles), so the pieces fill one wave of the
 // GPU.  seg holds max_tiles + 1 entries.  A list longer than `cap` (which
 // the counts never give) records DS_CAPACITY and leaves an empty plan.
+// Every iteration waits for this one block, so it takes few rounds
+// (kScanEntries per thread), searches the tile of an entry in shared memory
+// and plans with a thread per tile (20,000-sample motif sphere, 16 tiles at
+// first: 7.1 us on average; with one entry per thread, the search in device
+// memory and a serial plan 9.2).
+constexpr int kScanEntries = 4, kScanTiles = 1024;
 __global__ void __launch_bounds__(1024) scan_lists(const uint32_t *bcount, const uint32_t *nsurv,
                                                    const unsigned *nact, uint32_t nblk, uint32_t sms,
                                                    uint64_t cap, uint32_t *seg, uint32_t *boff,
                                                    uint64_t *offsets, uint32_t *pieces,
                                                    int *status) {
   __shared__ uint32_t warp_sum[32];
-  __shared__ uint32_t carry_s;
+  __shared__ uint32_t seg_s[kScanTiles + 1];
   const uint32_t tiles = active_tiles(nact);
-  if (threadIdx.x == 0) carry_s = 0;
-  __syncthreads();
+  // exclusive scan over the rounds of a loop: the running total stays in a
+  // register, the same in every thread
+  uint32_t entries = 0;
+  const bool near = tiles <= kScanTiles;  // seg fits in shared memory
   for (uint32_t base = 0; base < tiles; base += blockDim.x) {  // segment starts
     const uint32_t t = base + threadIdx.x;
     const uint32_t v = t < tiles ? nsurv[t] : 0u;
     uint32_t total;
-    const uint32_t incl = block_scan_1024(v, warp_sum, total);
-    if (t < tiles) seg[t] = carry_s + incl - v;
-    __syncthreads();
-    if (threadIdx.x == 0) carry_s += total;
-    __syncthreads();
+    const uint32_t excl = entries + block_scan_1024(v, warp_sum, total) - v;
+    if (t < tiles) {
+      seg[t] = excl;
+      if (near) seg_s[t] = excl;
+    }
+    entries += total;
   }
-  const uint32_t entries = carry_s;
-  __syncthreads();  // every thread has read carry_s before it is reset
-  if (threadIdx.x == 0) seg[tiles] = entries, carry_s = 0;
+  if (threadIdx.x == 0) {
+    seg[tiles] = entries;
+    if (near) seg_s[tiles] = entries;
+  }
   __syncthreads();
-  for (uint32_t base = 0; base < entries; base += blockDim.x) {  // list positions
-    const uint32_t e = base + threadIdx.x;
-    uint32_t t = 0, v = 0;
-    if (e < entries) {  // the tile of entry e: the last t with seg[t] <= e
-      uint32_t lo = 0, hi = tiles;  // seg[lo] <= e < seg[hi]
+  const uint32_t *starts = near ? seg_s : seg;
+  uint32_t list_len = 0;
+  for (uint32_t base = 0; base < entries; base += blockDim.x * kScanEntries) {  // list positions
+    const uint32_t e0 = base + threadIdx.x * kScanEntries;
+    uint32_t at[kScanEntries], v[kScanEntries], tile[kScanEntries], sum = 0;
+    uint32_t t = 0;
+    if (e0 < entries) {  // the tile of entry e0: the last t with starts[t] <= e0
+      uint32_t lo = 0, hi = tiles;  // starts[lo] <= e0 < starts[hi]
       while (hi - lo > 1) {
         const uint32_t mid = (lo + hi) >> 1;
-        if (seg[mid] <= e) lo = mid;
+        if (starts[mid] <= e0) lo = mid;
         else hi = mid;
       }
       t = lo;
-      v = bcount[uint64_t(t) * nblk + (e - seg[t])];
+    }
+#pragma unroll
+    for (int k = 0; k < kScanEntries; ++k) {
+      const uint32_t e = e0 + k;
+      v[k] = 0, at[k] = 0, tile[k] = t;
+      if (e < entries) {
+        while (starts[t + 1] <= e) ++t;
+        tile[k] = t, at[k] = e - starts[t];
+        v[k] = bcount[uint64_t(t) * nblk + at[k]];
+      }
+      sum += v[k];
     }
     uint32_t total;
-    const uint32_t incl = block_scan_1024(v, warp_sum, total);
-    if (e < entries) boff[uint64_t(t) * nblk + (e - seg[t])] = carry_s + incl - v;
-    __syncthreads();
-    if (threadIdx.x == 0) carry_s += total;
-    __syncthreads();
+    uint32_t run = list_len + block_scan_1024(sum, warp_sum, total) - sum;
+#pragma unroll
+    for (int k = 0; k < kScanEntries; ++k) {
+      if (e0 + k < entries) {
+        boff[uint64_t(tile[k]) * nblk + at[k]] = run;
+        // a tile's first entry starts it, and the empty tiles before it
+        if (at[k] == 0)
+          for (uint32_t x = tile[k] + 1; x-- > 0 && starts[x] == e0 + k;) offsets[x] = run;
+      }
+      run += v[k];
+    }
+    list_len += total;
   }
-  const uint32_t list_len = carry_s;
-  for (uint32_t t = threadIdx.x; t < tiles; t += blockDim.x)  // a tile with no entry starts
-    offsets[t] = seg[t] < seg[t + 1] ? boff[uint64_t(t) * nblk] : 0u;  // fixed below
+  for (uint32_t t = threadIdx.x; t <= tiles; t += blockDim.x)
+    if (starts[t] == entries) offsets[t] = list_len;  // the empty tiles at the end, and the end
   __syncthreads();
-  if (threadIdx.x == 0 && list_len > cap) {
-    atomicExch(status, DS_CAPACITY);
-    for (uint32_t t = 0; t <= tiles; ++t) offsets[t] = 0, pieces[t] = 0;
+  if (list_len > cap) {
+    for (uint32_t t = threadIdx.x; t <= tiles; t += blockDim.x) offsets[t] = 0, pieces[t] = 0;
+    if (threadIdx.x == 0) atomicExch(status, DS_CAPACITY);
     return;
   }
-  if (threadIdx.x == 0) {
-    // empty tiles take the position where the next entries start
-    uint64_t next = list_len;
-    for (uint32_t t = tiles; t-- > 0;) {
-      if (seg[t] < seg[t + 1]) next = offsets[t];
-      else offsets[t] = next;
-    }
-    offsets[tiles] = list_len;
-    const uint32_t budget = tiles < sms ? sms - tiles : tiles;
-    uint32_t at = 0;
-    for (uint32_t t = 0; t < tiles; ++t) {
-      pieces[t] = at;
+  const uint32_t budget = tiles < sms ? sms - tiles : tiles;
+  uint32_t planned = 0;
+  for (uint32_t base = 0; base < tiles; base += blockDim.x) {
+    const uint32_t t = base + threadIdx.x;
+    uint32_t v = 0;
+    if (t < tiles) {
       const uint64_t len = offsets[t + 1] - offsets[t];
       const uint64_t want = list_len ? (len * budget + list_len - 1) / list_len : 1;
-      at += uint32_t(want ? want : 1);
+      v = uint32_t(want ? want : 1);
     }
-    pieces[tiles] = at;
+    uint32_t total;
+    const uint32_t excl = planned + block_scan_1024(v, warp_sum, total) - v;
+    if (t < tiles) pieces[t] = excl;
+    planned += total;
   }
+  if (threadIdx.x == 0) pieces[tiles] = planned;
 }
 
 // list[boff[t * nblk + j] + r] = t * nchunks + c for the r-th kept chunk c
@@ -991,20 +1018,48 @@ __global__ void __launch_bounds__(32, 1) wait_selftest(uint64_t limit_ns, int *s
 // Sum of a seed's pieces (fixed order), then the mean-shift step; a seed
 // leaves the bulk (kNear: the FP32 polish takes it on with Newton steps)
 // when its squared move falls under kSwitch2 h^2.
-__global__ void __launch_bounds__(256) ms_update_bulk(float *means, const float *partial,
-                                                       const uint32_t *pieces, const int32_t *ids,
-                                                       const unsigned *nact, float h2,
-                                                       uint8_t *state) {
-  // one warp per seed: the lanes stride over the tile's pieces, a fixed
-  // butterfly sums them, lane 0 takes the step
-  const uint64_t slot = uint64_t(blockIdx.x) * 8 + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (slot >= nact[0]) return;  // whole warp
-  const int32_t s = ids[slot];
-  const uint64_t tile = slot / kChunk, row = slot % kChunk;
+// A block serves kUpdateSeeds neighbouring seeds: thread (y, x) adds the
+// pieces y, y + 32, ... of seed x, so eight threads read one 32-byte sector of
+// the partial sums and kUpdateAhead rounds of loads are in flight; then
+// through shared memory warp x takes seed x, the lanes its 32 sums, and a
+// fixed butterfly adds them.  Latency-bound: 4 us at 128 seeds and 152 pieces, 6
+// at 2,048; a warp per seed, whose lanes read one float of 32 pieces each and
+// which stored each coordinate before it loaded the next, took 19 and 37.
+constexpr int kUpdateSeeds = 8, kUpdateAhead = 8;
+__global__ void __launch_bounds__(32 * kUpdateSeeds) ms_update_bulk(float *means, const float *partial,
+                                                                    const uint32_t *pieces,
+                                                                    const int32_t *ids,
+                                                                    const unsigned *nact, float h2,
+                                                                    uint8_t *state) {
+  __shared__ float sums[7][32][kUpdateSeeds + 1];
+  const uint64_t slot0 = uint64_t(blockIdx.x) * kUpdateSeeds;
+  const unsigned n = nact[0];
+  if (slot0 >= n) return;  // the whole block
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint64_t tile = slot0 / kChunk;
   float acc[7] = {0, 0, 0, 0, 0, 0, 0};
-  for (uint32_t p = pieces[tile] + lane; p < pieces[tile + 1]; p += 32)
-    for (int d = 0; d < 7; ++d) acc[d] += partial[(uint64_t(p) * 8 + d) * kChunk + row];
+  const uint32_t x = threadIdx.x % kUpdateSeeds, y = threadIdx.x / kUpdateSeeds;
+  const uint32_t p1 = pieces[tile + 1];
+  const float *in = partial + slot0 % kChunk + x;
+  for (uint32_t p = pieces[tile] + y; p < p1; p += 32 * kUpdateAhead) {
+    float v[kUpdateAhead][7];
+#pragma unroll
+    for (int r = 0; r < kUpdateAhead; ++r)
+      if (p + 32 * r < p1)
+#pragma unroll
+        for (int d = 0; d < 7; ++d) v[r][d] = in[(uint64_t(p + 32 * r) * 8 + d) * kChunk];
+#pragma unroll
+    for (int r = 0; r < kUpdateAhead; ++r)
+      if (p + 32 * r < p1)
+#pragma unroll
+        for (int d = 0; d < 7; ++d) acc[d] += v[r][d];
+  }
+  for (int d = 0; d < 7; ++d) sums[d][y][x] = acc[d];
+  __syncthreads();
+  const uint64_t slot = slot0 + warp;
+  if (slot >= n) return;  // whole warp
+  const int32_t s = ids[slot];
+  for (int d = 0; d < 7; ++d) acc[d] = sums[d][lane][warp];
   for (int d = 0; d < 7; ++d)
     for (int o = 16; o; o >>= 1) acc[d] += __shfl_xor_sync(0xffffffffu, acc[d], o);
   if (lane != 0) return;
@@ -1012,13 +1067,17 @@ __global__ void __launch_bounds__(256) ms_update_bulk(float *means, const float 
     state[s] = kExhausted;
     return;
   }
-  float move = 0;
+  // every load before the first store: a load behind a store to its own line
+  // waits for it (a store per coordinate between the loads took 14 us more)
+  float *mean = means + uint64_t(s) * 8;
+  float old[6], nx[6], move = 0;
+  for (int d = 0; d < 6; ++d) old[d] = mean[d];
   for (int d = 0; d < 6; ++d) {
-    float nx = acc[d] / acc[6];
-    float e = means[uint64_t(s) * 8 + d] - nx;
+    nx[d] = quotient(acc[d], acc[6]);
+    const float e = old[d] - nx[d];
     move += e * e;
-    means[uint64_t(s) * 8 + d] = nx;
   }
+  for (int d = 0; d < 6; ++d) mean[d] = nx[d];
   if (move < float(kSwitch2) * h2) state[s] = kNear;
 }
 
@@ -1112,8 +1171,8 @@ bool meanshift_bf16_bulk(Call &call, const VoteSet &v, float *means, uint8_t *st
     ms_tile_tc<<<unsigned(max_grid), kThreadsTc, kTcSmem, st>>>(args);
     check_launch();
     if (kernel_ms) mark_event();
-    ms_update_bulk<<<unsigned((k + 7) / 8), 256, 0, st>>>(means, partial, pieces, ids, nact,
-                                                          float(h2), state);
+    ms_update_bulk<<<unsigned((k + kUpdateSeeds - 1) / kUpdateSeeds), 32 * kUpdateSeeds, 0, st>>>(
+        means, partial, pieces, ids, nact, float(h2), state);
     check_launch();
     call.launched(6);
     if (it % kCheck == kCheck - 1) {
