@@ -62,6 +62,7 @@ __global__ void __launch_bounds__(kCullThreads) tile_boxes(const T *means, const
   __shared__ float part[kChunk / kGroupSeeds][12];
   __shared__ float tb[kBoxFloats];
   __shared__ uint32_t warp_cnt[kCullThreads / 32], base_s;
+  chained();
   if (blockIdx.x >= active_tiles(nact)) return;
   if (threadIdx.x < kChunk) {  // whole warps
     const uint64_t slot = uint64_t(blockIdx.x) * kChunk + threadIdx.x;

@@ -140,6 +140,31 @@ inline unsigned blocks_for(uint64_t n, int threads = kThreads) {
 }
 inline void check_launch() { cuda_check(cudaGetLastError(), "kernel launch"); }
 
+// Chained launches (programmatic dependent launch): launch_chained lets a
+// kernel's blocks take their places while the kernel before it on the stream
+// drains; its first statement, chained(), waits until that kernel has completed
+// and its writes are visible, so nothing else changes.  For runs of short
+// kernels, whose launch and drain are much of their time.  Every kernel of a
+// run starts with chained(): the next one's wait then covers all before it.
+// (In a kernel launched the ordinary way chained() does nothing.)
+#ifdef __CUDACC__
+__device__ __forceinline__ void chained() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+void launch_chained(cudaStream_t stream, void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem,
+                    A &&...args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config{};
+  config.gridDim = grid, config.blockDim = dim3(threads), config.dynamicSmemBytes = smem;
+  config.stream = stream, config.attrs = &attr, config.numAttrs = 1;
+  cuda_check(cudaLaunchKernelEx(&config, kernel, P(args)...), "chained kernel launch");
+}
+#endif
+
 // ------------------------------------------------------------- FP64 math
 struct D3 {
   double x, y, z;

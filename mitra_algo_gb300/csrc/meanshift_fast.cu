@@ -194,6 +194,7 @@ __global__ void __launch_bounds__(kListThreads) split_items(
     const float *bbox, uint32_t nchunks, const uint32_t *sblk, const uint32_t *nsurv, uint32_t nblk,
     float skip_gap2, uint32_t cps, uint32_t words, uint32_t bwords, uint32_t *bits,
     uint32_t *touched, uint2 *pairs, uint32_t *work) {
+  chained();
   __shared__ TileSeeds seeds;
   uint32_t t, sub, per;
   if (!list_share(nact, t, sub, per)) return;
@@ -219,6 +220,7 @@ __global__ void __launch_bounds__(256) weigh_items(const uint2 *pairs, const uns
                                                    const uint32_t *bits, uint32_t bwords,
                                                    uint32_t cps, uint32_t nchunks, uint32_t room,
                                                    uint2 *items, uint32_t *work) {
+  chained();
   const uint32_t n = work[kWorkPairs];
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const uint32_t t = pairs[i].x, p = pairs[i].y;
@@ -320,6 +322,7 @@ __global__ void __launch_bounds__(kChunk, sizeof(T) == 4 ? 8 : 2)
             const uint8_t *state, const int32_t *ids, uint32_t nactive, T h2, T gk, float skip_gap2,
             Grid grid, uint32_t *touched, const uint32_t *bits, uint32_t bwords, const uint2 *items,
             uint32_t room, uint32_t *work, T *partial, unsigned long long *counts, unsigned long long *evals) {
+  chained();
   constexpr int kWords = int(sizeof(T)) / 4;  // 16-byte words per lane of a run
   __shared__ __align__(16) T runs[kChunk / 32][2][kRunValues];
   __shared__ T nsum[NEWTON ? 27 * kChunk : 1];
@@ -580,6 +583,7 @@ constexpr int kReduceWords = 32;  // words of touched splits listed at a time
 template <typename T>
 __global__ void __launch_bounds__(2 * kChunk) ms_reduce(const T *partial, Grid grid, uint64_t nactive,
                                                         const uint32_t *touched, T *red) {
+  chained();
   __shared__ uint16_t list[2][kReduceWords * 16];
   __shared__ int count[2];
   __shared__ T other[kChunk];
@@ -629,6 +633,7 @@ template <typename T>
 __global__ void __launch_bounds__(kChunk) ms_update(T *means, const T *red, uint64_t slots,
                                                     const int32_t *ids, uint64_t nactive, T h2,
                                                     T gk, int polish_it, uint8_t *state) {
+  chained();
   const uint64_t slot = uint64_t(blockIdx.x) * kChunk + threadIdx.x;
   if (slot >= nactive) return;
   const int32_t s = ids[slot];
@@ -715,6 +720,7 @@ __global__ void __launch_bounds__(kRetileThreads) retile(const T *means, const u
   __shared__ unsigned long long keys[kRetile];
   __shared__ uint16_t seeds[kRetile];
   __shared__ unsigned warp_active[kWarps], warp_near[kWarps], below[kWarps][kRankSeeds];
+  chained();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool sort = k <= kRetile;
   const uint64_t first = sort ? 0 : uint64_t(blockIdx.x) * kRetile;
@@ -873,24 +879,20 @@ void run_tiles(Call &call, const VoteSet &v, const T *desc, const T *means, cons
   SYM_CUDA(cudaMemsetAsync(w.work, 0, (kWorkSize + touch_words + (list ? g.tiles * w.bwords : 0)) * 4, st));
   const T k = T(v.kernel_k);
   if (!list) {
-    ms_tile<T, COUNT, NEWTON, GAUSS><<<dim3(unsigned(g.tiles), unsigned(g.splits)), kChunk, 0, st>>>(
-        desc, v.sbox, uint32_t(v.nchunks), v.q, means, state, ids, uint32_t(n), T(h2), k, gap2, g,
-        w.touched, nullptr, 0, nullptr, 0, nullptr, partial, counts, evals);
-    check_launch();
+    launch_chained(st, ms_tile<T, COUNT, NEWTON, GAUSS>, dim3(unsigned(g.tiles), unsigned(g.splits)), kChunk, 0,
+                   desc, v.sbox, uint32_t(v.nchunks), v.q, means, state, ids, uint32_t(n), T(h2), k, gap2, g,
+                   w.touched, nullptr, 0u, nullptr, 0u, nullptr, partial, counts, evals);
     call.launched();
     return;
   }
-  tile_boxes<T><<<unsigned(g.tiles), kCullThreads, 0, st>>>(means, ids, nact, v.bbox, w.nblk, gap2,
-                                                            w.boxes, w.sblk, w.nsurv, nullptr);
-  check_launch();
-  split_items<T><<<w.list_ctas, kListThreads, 0, st>>>(
-      w.boxes, means, ids, nact, v.cbox, v.bbox, uint32_t(v.nchunks), w.sblk, w.nsurv, w.nblk, gap2,
-      uint32_t(g.cps), g.words, w.bwords, w.bits, w.touched, w.pairs, w.work);
-  check_launch();
+  launch_chained(st, tile_boxes<T>, unsigned(g.tiles), kCullThreads, 0, means, ids, nact, v.bbox, w.nblk, gap2,
+                 w.boxes, w.sblk, w.nsurv, nullptr);
+  launch_chained(st, split_items<T>, w.list_ctas, kListThreads, 0, w.boxes, means, ids, nact, v.cbox, v.bbox,
+                 uint32_t(v.nchunks), w.sblk, w.nsurv, w.nblk, gap2, uint32_t(g.cps), g.words, w.bwords,
+                 w.bits, w.touched, w.pairs, w.work);
   const uint32_t room = uint32_t(w.max_splits * (kChunk / 32));
-  weigh_items<<<blocks_for(g.tiles * g.splits), kThreads, 0, st>>>(
-      w.pairs, nact, w.bits, w.bwords, uint32_t(g.cps), uint32_t(v.nchunks), room, w.items, w.work);
-  check_launch();
+  launch_chained(st, weigh_items, blocks_for(g.tiles * g.splits), kThreads, 0, w.pairs, nact, w.bits, w.bwords,
+                 uint32_t(g.cps), uint32_t(v.nchunks), room, w.items, w.work);
   static const int per_sm = [] {
     int a = 0;
     SYM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, ms_tile<T, COUNT, NEWTON, GAUSS>,
@@ -898,10 +900,9 @@ void run_tiles(Call &call, const VoteSet &v, const T *desc, const T *means, cons
     return std::max(1, a);
   }();
   const unsigned ctas = unsigned(std::min<uint64_t>(g.tiles * g.splits, uint64_t(152) * per_sm));
-  ms_tile<T, COUNT, NEWTON, GAUSS><<<ctas, kChunk, 0, st>>>(
-      desc, v.sbox, uint32_t(v.nchunks), v.q, means, state, ids, uint32_t(n), T(h2), k, gap2, g,
-      w.touched, w.bits, w.bwords, w.items, room, w.work, partial, counts, evals);
-  check_launch();
+  launch_chained(st, ms_tile<T, COUNT, NEWTON, GAUSS>, ctas, kChunk, 0, desc, v.sbox, uint32_t(v.nchunks), v.q,
+                 means, state, ids, uint32_t(n), T(h2), k, gap2, g, w.touched, w.bits, w.bwords, w.items, room,
+                 w.work, partial, counts, evals);
   call.launched(4);
 }
 
@@ -920,8 +921,8 @@ int shift_impl(Call &call, const VoteSet &v, const T *desc, T *means, uint8_t *s
   TileWork work = tile_work<T>(call, v, k);
   int it = 0;
   for (; it < max_iter; ++it) {
-    retile<T><<<retile_blocks(k), kRetileThreads, 0, st>>>(means, state, k, v.gbox, polish, ids, nact);
-    check_launch();
+    launch_chained(st, retile<T>, retile_blocks(k), kRetileThreads, 0, means, state, k, v.gbox, polish, ids, nact,
+                   nullptr, nullptr, 0u);
     unsigned counts[2] = {0, 0};
     SYM_CUDA(cudaMemcpyAsync(counts, nact, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
     call.sync();
@@ -937,12 +938,10 @@ int shift_impl(Call &call, const VoteSet &v, const T *desc, T *means, uint8_t *s
     const auto tiles = counts[1] ? (gauss ? run_tiles<T, false, true, true> : run_tiles<T, false, true, false>)
                                  : (gauss ? run_tiles<T, false, false, true> : run_tiles<T, false, false, false>);
     tiles(call, v, desc, means, state, ids, nact, n, h2, g, work, partial, nullptr, evals);
-    ms_reduce<T><<<dim3(unsigned(g.tiles), counts[1] ? 34u : 7u, kGroups), 2 * kChunk, 0, st>>>(
-        partial, g, n, work.touched, red);
-    check_launch();
-    ms_update<T><<<unsigned(g.tiles), kChunk, 0, st>>>(means, red, g.slots, ids, n, T(h2),
-                                                       T(v.kernel_k), polish ? it : -1, state);
-    check_launch();
+    launch_chained(st, ms_reduce<T>, dim3(unsigned(g.tiles), counts[1] ? 34u : 7u, kGroups), 2 * kChunk, 0,
+                   partial, g, n, work.touched, red);
+    launch_chained(st, ms_update<T>, unsigned(g.tiles), kChunk, 0, means, red, g.slots, ids, n, T(h2),
+                   T(v.kernel_k), polish ? it : -1, state);
     call.launched(2);
   }
   return it;
@@ -1028,9 +1027,8 @@ int shift(Call &call, const VoteSet &v, double *means, uint8_t *state, uint64_t 
 void active_seeds_async(Call &call, const VoteSet &v, const float *means, const uint8_t *state,
                         uint64_t k, int32_t *ids, unsigned *nact, unsigned *iter, uint32_t *trace,
                         unsigned trace_cap) {
-  retile<float><<<retile_blocks(k), kRetileThreads, 0, call.stream()>>>(means, state, k, v.gbox, false, ids,
-                                                                        nact, iter, trace, trace_cap);
-  check_launch();
+  launch_chained(call.stream(), retile<float>, retile_blocks(k), kRetileThreads, 0, means, state, k, v.gbox,
+                 false, ids, nact, iter, trace, trace_cap);
   call.launched();
 }
 

@@ -338,6 +338,7 @@ __global__ void __launch_bounds__(kListThreads) tile_count(const float *boxes, c
                                                            float skip_gap2, uint8_t *need,
                                                            uint32_t *bcount) {
   __shared__ TileSeeds seeds;
+  chained();
   uint32_t t, sub, per;
   if (!list_share(nact, t, sub, per)) return;
   const uint32_t ns = nsurv[t];
@@ -405,6 +406,7 @@ __global__ void __launch_bounds__(1024) scan_lists(const uint32_t *bcount, const
                                                    int *status) {
   __shared__ uint32_t warp_sum[32];
   __shared__ uint32_t seg_s[kScanTiles + 1];
+  chained();
   const uint32_t tiles = active_tiles(nact);
   // exclusive scan over the rounds of a loop: the running total stays in a
   // register, the same in every thread
@@ -504,6 +506,7 @@ __global__ void __launch_bounds__(kListThreads) scatter_lists(const uint8_t *nee
                                                               uint64_t nchunks, uint64_t cap,
                                                               int32_t *list, int *status) {
   __shared__ uint32_t warp_cnt[kListThreads / 32];
+  chained();
   uint32_t t, sub, per;
   if (!list_share(nact, t, sub, per)) return;
   const uint32_t ns = nsurv[t];
@@ -632,6 +635,7 @@ __device__ __forceinline__ void mma2_chunk(uint32_t acc, uint32_t w_tmem, const 
 }
 
 __global__ void __launch_bounds__(kThreadsTc, 1) ms_tile_tc(TcArgs a) {
+  chained();
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t *stage = smem + kTcStage;
   float *U = reinterpret_cast<float *>(smem + kTcU);
@@ -1032,6 +1036,7 @@ __global__ void __launch_bounds__(32 * kUpdateSeeds) ms_update_bulk(float *means
                                                                     const unsigned *nact, float h2,
                                                                     uint8_t *state) {
   __shared__ float sums[7][32][kUpdateSeeds + 1];
+  chained();
   const uint64_t slot0 = uint64_t(blockIdx.x) * kUpdateSeeds;
   const unsigned n = nact[0];
   if (slot0 >= n) return;  // the whole block
@@ -1154,26 +1159,19 @@ bool meanshift_bf16_bulk(Call &call, const VoteSet &v, float *means, uint8_t *st
   int it = 0;
   for (; it < max_iter; ++it) {
     active_seeds_async(call, v, means, state, k, ids, nact, iter, trace_dev, trace_cap);
-    tile_boxes<<<unsigned(max_tiles), kCullThreads, 0, st>>>(means, ids, nact, v.bbox, nblk,
-                                                              gap * gap, boxes, sblk, nsurv, bcount);
-    check_launch();
-    tile_count<<<list_ctas, kListThreads, 0, st>>>(boxes, means, ids, nact, v.cbox, v.bbox,
-                                                   v.nchunks, sblk, nsurv, nblk, gap * gap, need,
-                                                   bcount);
-    check_launch();
-    scan_lists<<<1, 1024, 0, st>>>(bcount, nsurv, nact, nblk, sms, list_cap, seg, boff, offsets,
-                                   pieces, call.status());
-    check_launch();
-    scatter_lists<<<list_ctas, kListThreads, 0, st>>>(need, boff, bcount, sblk, nsurv, nblk, nact,
-                                                      v.nchunks, list_cap, list, call.status());
-    check_launch();
+    launch_chained(st, tile_boxes<float>, unsigned(max_tiles), kCullThreads, 0, means, ids, nact, v.bbox, nblk,
+                   gap * gap, boxes, sblk, nsurv, bcount);
+    launch_chained(st, tile_count, list_ctas, kListThreads, 0, boxes, means, ids, nact, v.cbox, v.bbox,
+                   v.nchunks, sblk, nsurv, nblk, gap * gap, need, bcount);
+    launch_chained(st, scan_lists, 1, 1024, 0, bcount, nsurv, nact, nblk, sms, list_cap, seg, boff, offsets,
+                   pieces, call.status());
+    launch_chained(st, scatter_lists, list_ctas, kListThreads, 0, need, boff, bcount, sblk, nsurv, nblk, nact,
+                   v.nchunks, list_cap, list, call.status());
     if (kernel_ms) mark_event();
-    ms_tile_tc<<<unsigned(max_grid), kThreadsTc, kTcSmem, st>>>(args);
-    check_launch();
+    launch_chained(st, ms_tile_tc, unsigned(max_grid), kThreadsTc, kTcSmem, args);
     if (kernel_ms) mark_event();
-    ms_update_bulk<<<unsigned((k + kUpdateSeeds - 1) / kUpdateSeeds), 32 * kUpdateSeeds, 0, st>>>(
-        means, partial, pieces, ids, nact, float(h2), state);
-    check_launch();
+    launch_chained(st, ms_update_bulk, unsigned((k + kUpdateSeeds - 1) / kUpdateSeeds), 32 * kUpdateSeeds, 0,
+                   means, partial, pieces, ids, nact, float(h2), state);
     call.launched(6);
     if (it % kCheck == kCheck - 1) {
       unsigned n = 0;

@@ -36,6 +36,7 @@ __device__ uint64_t block_exclusive(uint64_t v, uint64_t &total) {
 }
 
 __global__ void tile_sums(const uint64_t *in, uint64_t n, uint64_t *partial) {
+  chained();
   uint64_t base = uint64_t(blockIdx.x) * kScanTile + threadIdx.x * kScanItems;
   uint64_t s = 0;
   for (int k = 0; k < kScanItems; ++k)
@@ -48,6 +49,7 @@ __global__ void tile_sums(const uint64_t *in, uint64_t n, uint64_t *partial) {
 // One block scans `count` partial sums in place (exclusive) sequentially in
 // chunks of blockDim.
 __global__ void scan_partials(uint64_t *partial, uint64_t count) {
+  chained();
   __shared__ uint64_t carry;
   if (threadIdx.x == 0) carry = 0;
   __syncthreads();
@@ -64,6 +66,7 @@ __global__ void scan_partials(uint64_t *partial, uint64_t count) {
 
 __global__ void tile_scan(const uint64_t *in, uint64_t n, const uint64_t *partial,
                           uint64_t *out) {
+  chained();
   uint64_t base = uint64_t(blockIdx.x) * kScanTile + threadIdx.x * kScanItems;
   uint64_t v[kScanItems], s = 0;
   for (int k = 0; k < kScanItems; ++k) {
@@ -86,6 +89,7 @@ constexpr int kSortTile = kSortWarps * kSortRounds * 32;  // 2048 keys per block
 
 __global__ void radix_histogram(const uint64_t *keys, uint64_t n, int shift, uint64_t *hist,
                                 unsigned blocks) {
+  chained();
   __shared__ unsigned counts[256];
   for (int d = threadIdx.x; d < 256; d += blockDim.x) counts[d] = 0;
   __syncthreads();
@@ -104,6 +108,7 @@ __global__ void radix_histogram(const uint64_t *keys, uint64_t n, int shift, uin
 __global__ void __launch_bounds__(kSortWarps * 32) radix_scatter(
     const uint64_t *keys, const int32_t *vals, uint64_t n, int shift, const uint64_t *offsets,
     unsigned blocks, uint64_t *keys_out, int32_t *vals_out) {
+  chained();
   __shared__ unsigned warp_count[kSortWarps][256];
   __shared__ unsigned digit_start[256];
   __shared__ uint64_t skey[kSortTile];
@@ -167,12 +172,14 @@ __global__ void __launch_bounds__(kSortWarps * 32) radix_scatter(
 }
 
 __global__ void flags_to_counts(const uint8_t *flags, uint64_t n, uint64_t *counts) {
+  chained();
   uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i < n) counts[i] = flags[i] != 0;
 }
 
 __global__ void scatter_flagged(const uint8_t *flags, const int32_t *values, uint64_t n,
                                 const uint64_t *pos, int32_t *out, uint64_t *count) {
+  chained();
   uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i < n && flags[i]) out[pos[i]] = values ? values[i] : int32_t(i);
   if (i == 0) *count = pos[n];
@@ -187,12 +194,9 @@ void exclusive_scan(Call &call, const uint64_t *in, uint64_t *out, uint64_t n) {
   }
   unsigned tiles = static_cast<unsigned>((n + kScanTile - 1) / kScanTile);
   uint64_t *partial = call.alloc<uint64_t>(tiles);
-  tile_sums<<<tiles, kScanThreads, 0, call.stream()>>>(in, n, partial);
-  check_launch();
-  scan_partials<<<1, 1024, 0, call.stream()>>>(partial, tiles);
-  check_launch();
-  tile_scan<<<tiles, kScanThreads, 0, call.stream()>>>(in, n, partial, out);
-  check_launch();
+  launch_chained(call.stream(), tile_sums, tiles, kScanThreads, 0, in, n, partial);
+  launch_chained(call.stream(), scan_partials, 1, 1024, 0, partial, tiles);
+  launch_chained(call.stream(), tile_scan, tiles, kScanThreads, 0, in, n, partial, out);
   call.launched(3);
 }
 
@@ -214,12 +218,10 @@ void radix_sort_pairs(Call &call, const uint64_t *keys, const int32_t *values,
     uint64_t *kdst = last_to_out ? keys_out : kbuf;
     int32_t *vdst = last_to_out ? values_out : vbuf;
     int shift = 8 * p;
-    radix_histogram<<<blocks, 256, 0, call.stream()>>>(ksrc, n, shift, hist, blocks);
-    check_launch();
+    launch_chained(call.stream(), radix_histogram, blocks, 256, 0, ksrc, n, shift, hist, blocks);
     exclusive_scan(call, hist, offsets, hist_n);
-    radix_scatter<<<blocks, kSortWarps * 32, 0, call.stream()>>>(ksrc, vsrc, n, shift, offsets,
-                                                                 blocks, kdst, vdst);
-    check_launch();
+    launch_chained(call.stream(), radix_scatter, blocks, kSortWarps * 32, 0, ksrc, vsrc, n, shift, offsets,
+                   blocks, kdst, vdst);
     call.launched(2);
     ksrc = kdst;
     vsrc = vdst;
@@ -234,11 +236,9 @@ void compact_values(Call &call, const uint8_t *flags, const int32_t *values, uin
   }
   uint64_t *counts = call.alloc<uint64_t>(n);
   uint64_t *pos = call.alloc<uint64_t>(n + 1);
-  flags_to_counts<<<blocks_for(n), kThreads, 0, call.stream()>>>(flags, n, counts);
-  check_launch();
+  launch_chained(call.stream(), flags_to_counts, blocks_for(n), kThreads, 0, flags, n, counts);
   exclusive_scan(call, counts, pos, n);
-  scatter_flagged<<<blocks_for(n), kThreads, 0, call.stream()>>>(flags, values, n, pos, out, count);
-  check_launch();
+  launch_chained(call.stream(), scatter_flagged, blocks_for(n), kThreads, 0, flags, values, n, pos, out, count);
   call.launched(2);
 }
 
