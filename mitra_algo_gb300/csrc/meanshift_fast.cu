@@ -166,6 +166,30 @@ struct Grid {
   uint32_t words;  // 32-bit words of `touched` per group of a tile
 };
 
+// The layout for `nactive` seeds; without seeds all zero.
+__device__ inline Grid grid_for(uint64_t nactive, uint64_t nchunks, int blocks_per_sm) {
+  Grid g{};
+  if (!nactive) return g;
+  g.tiles = (nactive + kChunk - 1) / kChunk;
+  const uint64_t want = (uint64_t(blocks_per_sm) * 152 + g.tiles - 1) / g.tiles;
+  g.splits = max(uint64_t(1), min(nchunks, want));
+  g.cps = (nchunks + g.splits - 1) / g.splits;
+  g.splits = (nchunks + g.cps - 1) / g.cps;
+  g.slots = g.tiles * kChunk;
+  g.words = uint32_t(((g.splits + kGroups - 1) / kGroups + 31) / 32);
+  return g;
+}
+
+// What retile leaves behind for a SIMT iteration: its layout, and `clear`
+// zeroed (the iteration's work counters, touched and chunk bits).
+struct Plan {
+  Grid *grid = nullptr;
+  uint64_t nchunks = 0;
+  int blocks_per_sm = 0;
+  uint32_t *clear = nullptr;
+  uint64_t clear_words = 0;
+};
+
 __device__ __forceinline__ bool touch(uint32_t *touched, uint32_t words, uint32_t tile, uint32_t p) {
   uint32_t *w = touched + (uint64_t(tile) * kGroups + p % kGroups) * words + (p / kGroups) / 32;
   const uint32_t bit = 1u << ((p / kGroups) % 32);
@@ -192,8 +216,8 @@ template <typename T>
 __global__ void __launch_bounds__(kListThreads) split_items(
     const float *boxes, const T *means, const int32_t *ids, const unsigned *nact, const float *cbox,
     const float *bbox, uint32_t nchunks, const uint32_t *sblk, const uint32_t *nsurv, uint32_t nblk,
-    float skip_gap2, uint32_t cps, uint32_t words, uint32_t bwords, uint32_t *bits,
-    uint32_t *touched, uint2 *pairs, uint32_t *work) {
+    float skip_gap2, const Grid *grid, uint32_t bwords, uint32_t *bits, uint32_t *touched, uint2 *pairs,
+    uint32_t *work) {
   chained();
   __shared__ TileSeeds seeds;
   uint32_t t, sub, per;
@@ -201,6 +225,7 @@ __global__ void __launch_bounds__(kListThreads) split_items(
   const uint32_t ns = nsurv[t];
   if (sub >= ns) return;
   load_tile(seeds, t, nact[0], boxes, means, ids);
+  const uint32_t cps = uint32_t(grid->cps), words = grid->words;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (uint32_t j = sub; j < ns; j += per) {
     const uint32_t blk = sblk[uint64_t(t) * nblk + j];
@@ -218,9 +243,10 @@ __global__ void __launch_bounds__(kListThreads) split_items(
 
 __global__ void __launch_bounds__(256) weigh_items(const uint2 *pairs, const unsigned *nact,
                                                    const uint32_t *bits, uint32_t bwords,
-                                                   uint32_t cps, uint32_t nchunks, uint32_t room,
+                                                   const Grid *grid, uint32_t nchunks, uint32_t room,
                                                    uint2 *items, uint32_t *work) {
   chained();
+  const uint32_t cps = uint32_t(grid->cps);
   const uint32_t n = work[kWorkPairs];
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const uint32_t t = pairs[i].x, p = pairs[i].y;
@@ -319,10 +345,13 @@ constexpr int kPairStride = 20, kRunValues = kSubVotes / 2 * kPairStride;
 template <typename T, bool COUNT, bool NEWTON, bool GAUSS>
 __global__ void __launch_bounds__(kChunk, sizeof(T) == 4 ? 8 : 2)
     ms_tile(const T *desc, const float *sbox, uint32_t nchunks, uint64_t q, const T *means,
-            const uint8_t *state, const int32_t *ids, uint32_t nactive, T h2, T gk, float skip_gap2,
-            Grid grid, uint32_t *touched, const uint32_t *bits, uint32_t bwords, const uint2 *items,
+            const uint8_t *state, const int32_t *ids, const unsigned *nact, T h2, T gk, float skip_gap2,
+            const Grid *plan, uint32_t *touched, const uint32_t *bits, uint32_t bwords, const uint2 *items,
             uint32_t room, uint32_t *work, T *partial, unsigned long long *counts, unsigned long long *evals) {
   chained();
+  const Grid grid = *plan;
+  const uint32_t nactive = nact[0];
+  if (!nactive) return;
   constexpr int kWords = int(sizeof(T)) / 4;  // 16-byte words per lane of a run
   __shared__ __align__(16) T runs[kChunk / 32][2][kRunValues];
   __shared__ T nsum[NEWTON ? 27 * kChunk : 1];
@@ -333,7 +362,7 @@ __global__ void __launch_bounds__(kChunk, sizeof(T) == 4 ? 8 : 2)
   T *const ns = nsum + threadIdx.x;
   const T rcp = reciprocal(h2), floor_w = GAUSS ? exp2(-gk) : T(0);
   for (;;) {
-    uint32_t tile = blockIdx.x, split = blockIdx.y, quarter = warp;
+    uint32_t tile = blockIdx.x % uint32_t(grid.tiles), split = blockIdx.x / uint32_t(grid.tiles), quarter = warp;
     if (items) {
       uint32_t it = 0;
       if (lane == 0) it = atomicAdd(&work[kWorkNext], 1u);
@@ -344,6 +373,8 @@ __global__ void __launch_bounds__(kChunk, sizeof(T) == 4 ? 8 : 2)
         if (it >= queue_end[k - 1]) at = uint64_t(k) * room + (it - queue_end[k - 1]);
       const uint2 x = items[at];
       tile = x.x / (kChunk / 32), quarter = x.x % (kChunk / 32), split = x.y;
+    } else if (split >= grid.splits) {
+      return;
     }
     const uint32_t slot = tile * kChunk + quarter * 32 + lane;
     const bool live = slot < nactive;
@@ -581,9 +612,13 @@ __device__ bool solve6(T (&M)[6][6], T (&b)[6], T tiny) {
 // mostly; 21 us now.)
 constexpr int kReduceWords = 32;  // words of touched splits listed at a time
 template <typename T>
-__global__ void __launch_bounds__(2 * kChunk) ms_reduce(const T *partial, Grid grid, uint64_t nactive,
-                                                        const uint32_t *touched, T *red) {
+__global__ void __launch_bounds__(2 * kChunk) ms_reduce(const T *partial, const Grid *plan,
+                                                        const unsigned *nact, const uint32_t *touched,
+                                                        T *red) {
   chained();
+  const Grid grid = *plan;
+  if (blockIdx.x >= grid.tiles) return;
+  const unsigned nactive = nact[0];
   __shared__ uint16_t list[2][kReduceWords * 16];
   __shared__ int count[2];
   __shared__ T other[kChunk];
@@ -630,10 +665,12 @@ __global__ void __launch_bounds__(2 * kChunk) ms_reduce(const T *partial, Grid g
 
 // One thread per seed: the step from the summed values (ms_reduce).
 template <typename T>
-__global__ void __launch_bounds__(kChunk) ms_update(T *means, const T *red, uint64_t slots,
-                                                    const int32_t *ids, uint64_t nactive, T h2,
+__global__ void __launch_bounds__(kChunk) ms_update(T *means, const T *red, const Grid *grid,
+                                                    const int32_t *ids, const unsigned *nact, T h2,
                                                     T gk, int polish_it, uint8_t *state) {
   chained();
+  const uint64_t slots = grid->slots;
+  const unsigned nactive = nact[0];
   const uint64_t slot = uint64_t(blockIdx.x) * kChunk + threadIdx.x;
   if (slot >= nactive) return;
   const int32_t s = ids[slot];
@@ -693,6 +730,7 @@ constexpr uint64_t kListedPairs = 32768;  // (tile, chunk) pairs from which the 
 // nactive[0] = the number of active seeds, nactive[1] = how many of them are
 // kNear.  With `iter`, an iteration that finds active seeds records their
 // number in trace[*iter] (while *iter < trace_cap) and counts itself in *iter.
+// `plan` as above.
 //
 // Runs in every iteration between two kernels that wait for it, so its own
 // latency counts.  A block lists the active seeds for itself from their state
@@ -715,12 +753,15 @@ __global__ void __launch_bounds__(kRetileThreads) retile(const T *means, const u
                                                          int32_t *ids, unsigned *nactive,
                                                          unsigned *iter = nullptr,
                                                          uint32_t *trace = nullptr,
-                                                         unsigned trace_cap = 0) {
+                                                         unsigned trace_cap = 0, Plan plan = Plan()) {
   constexpr int kWarps = kRetileThreads / 32;
   __shared__ unsigned long long keys[kRetile];
   __shared__ uint16_t seeds[kRetile];
   __shared__ unsigned warp_active[kWarps], warp_near[kWarps], below[kWarps][kRankSeeds];
   chained();
+  for (uint64_t i = uint64_t(blockIdx.x) * kRetileThreads + threadIdx.x; i < plan.clear_words;
+       i += uint64_t(gridDim.x) * kRetileThreads)
+    plan.clear[i] = 0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool sort = k <= kRetile;
   const uint64_t first = sort ? 0 : uint64_t(blockIdx.x) * kRetile;
@@ -765,6 +806,7 @@ __global__ void __launch_bounds__(kRetileThreads) retile(const T *means, const u
   // a block that has looked at every seed reports
   if (threadIdx.x == 0 && blockIdx.x == (sort ? 0 : gridDim.x - 1)) {
     nactive[0] = n, nactive[1] = near;
+    if (plan.grid) *plan.grid = grid_for(n, plan.nchunks, plan.blocks_per_sm);
     if (iter && n) {
       if (*iter < trace_cap) trace[*iter] = n;
       ++*iter;
@@ -811,28 +853,18 @@ __global__ void gather_seeds(const T *desc, const int64_t *pos, uint64_t k, T *m
   for (int d = 0; d < 8; ++d) means[i * 8 + d] = desc[uint64_t(pos[i]) * 8 + d];
 }
 
-Grid grid_for(uint64_t nactive, uint64_t nchunks, int blocks_per_sm) {
-  Grid g;
-  g.tiles = (nactive + kChunk - 1) / kChunk;
-  uint64_t want = (uint64_t(blocks_per_sm) * 152 + g.tiles - 1) / g.tiles;
-  g.splits = std::max<uint64_t>(1, std::min<uint64_t>(nchunks, want));
-  g.cps = (nchunks + g.splits - 1) / g.splits;
-  g.splits = (nchunks + g.cps - 1) / g.cps;
-  g.slots = g.tiles * kChunk;
-  g.words = uint32_t(((g.splits + kGroups - 1) / kGroups + 31) / 32);
-  return g;
-}
-
 // Whether an iteration draws its work from split_items' list: with few
 // (tile, chunk) pairs the direct grid's own tests cost less than the three list
 // kernels (us per iteration, direct and listed: 44 and 61 at 940 pairs, 71 and
 // 80 at 18,750 pairs, 300 and 160 at 160,000 pairs).
-bool listed(const Grid &g, uint64_t nchunks) { return g.tiles * nchunks >= kListedPairs; }
+// The sums are the same either way.
+bool listed(uint64_t tiles, uint64_t nchunks) { return tiles * nchunks >= kListedPairs; }
 
-// Scratch of one ms_tile launch, sized for `k` seeds.
+// Scratch of the SIMT iterations, sized for `k` seeds.
 struct TileWork {
   uint32_t *work = nullptr;     // [items, next item], then `touched`, then `bits`: zeroed together
   uint32_t *touched = nullptr, *bits = nullptr;
+  Grid *grid = nullptr;         // of the iteration, by retile
   uint32_t bwords = 0, nblk = 0;
   uint64_t max_splits = 0;      // tiles x splits never exceeds it
   float *boxes = nullptr;
@@ -852,6 +884,8 @@ TileWork tile_work(Call &call, const VoteSet &v, uint64_t k) {
   const uint64_t touch_words = w.max_splits / 32 + (tiles + 1) * kGroups * 2;
   w.work = call.alloc<uint32_t>(kWorkSize + touch_words + tiles * w.bwords);
   w.touched = w.work + kWorkSize;
+  w.bits = w.touched + touch_words;
+  w.grid = call.alloc<Grid>(1);
   w.boxes = call.alloc<float>(tiles * kBoxFloats);
   w.sblk = call.alloc<uint32_t>(tiles * w.nblk);
   w.nsurv = call.alloc<uint32_t>(tiles);
@@ -866,85 +900,126 @@ TileWork tile_work(Call &call, const VoteSet &v, uint64_t k) {
   return w;
 }
 
-// One ms_tile launch (and, listed, the work items before it) over n seeds.
+// What retile is to prepare for an iteration of at most `tiles` tiles.
+template <typename T>
+Plan plan_of(const VoteSet &v, const TileWork &w, uint64_t tiles) {
+  Plan p;
+  p.grid = w.grid, p.nchunks = v.nchunks, p.blocks_per_sm = v.tuning.simt_blocks_per_sm;
+  p.clear = w.work;
+  p.clear_words = uint64_t(w.bits - w.work) + (listed(tiles, v.nchunks) ? tiles * w.bwords : 0);
+  return p;
+}
+
+// One ms_tile launch (and, listed, the work items before it) over the active
+// seeds, at most `tiles` tiles of them.
 template <typename T, bool COUNT, bool NEWTON, bool GAUSS>
 void run_tiles(Call &call, const VoteSet &v, const T *desc, const T *means, const uint8_t *state,
-               const int32_t *ids, const unsigned *nact, uint64_t n, double h2, const Grid &g,
-               TileWork &w, T *partial, unsigned long long *counts, unsigned long long *evals) {
+               const int32_t *ids, const unsigned *nact, uint64_t tiles, double h2, const TileWork &w,
+               T *partial, unsigned long long *counts, unsigned long long *evals) {
   cudaStream_t st = call.stream();
   const float gap = float(std::sqrt(h2)) + 1e-6f, gap2 = gap * gap;
-  const uint64_t touch_words = g.tiles * kGroups * g.words;
-  const bool list = listed(g, v.nchunks);
-  w.bits = w.touched + touch_words;
-  SYM_CUDA(cudaMemsetAsync(w.work, 0, (kWorkSize + touch_words + (list ? g.tiles * w.bwords : 0)) * 4, st));
   const T k = T(v.kernel_k);
-  if (!list) {
-    launch_chained(st, ms_tile<T, COUNT, NEWTON, GAUSS>, dim3(unsigned(g.tiles), unsigned(g.splits)), kChunk, 0,
-                   desc, v.sbox, uint32_t(v.nchunks), v.q, means, state, ids, uint32_t(n), T(h2), k, gap2, g,
-                   w.touched, nullptr, 0u, nullptr, 0u, nullptr, partial, counts, evals);
+  // (tile, split) pairs of any number of tiles up to that: tiles x splits
+  const uint64_t pairs =
+      std::min<uint64_t>(tiles * v.nchunks, uint64_t(v.tuning.simt_blocks_per_sm) * 152 + tiles);
+  if (!listed(tiles, v.nchunks)) {
+    launch_chained(st, ms_tile<T, COUNT, NEWTON, GAUSS>, unsigned(pairs), kChunk, 0, desc, v.sbox,
+                   uint32_t(v.nchunks), v.q, means, state, ids, nact, T(h2), k, gap2, w.grid, w.touched,
+                   nullptr, 0u, nullptr, 0u, nullptr, partial, counts, evals);
     call.launched();
     return;
   }
-  launch_chained(st, tile_boxes<T>, unsigned(g.tiles), kCullThreads, 0, means, ids, nact, v.bbox, w.nblk, gap2,
+  launch_chained(st, tile_boxes<T>, unsigned(tiles), kCullThreads, 0, means, ids, nact, v.bbox, w.nblk, gap2,
                  w.boxes, w.sblk, w.nsurv, nullptr);
   launch_chained(st, split_items<T>, w.list_ctas, kListThreads, 0, w.boxes, means, ids, nact, v.cbox, v.bbox,
-                 uint32_t(v.nchunks), w.sblk, w.nsurv, w.nblk, gap2, uint32_t(g.cps), g.words, w.bwords,
-                 w.bits, w.touched, w.pairs, w.work);
+                 uint32_t(v.nchunks), w.sblk, w.nsurv, w.nblk, gap2, w.grid, w.bwords, w.bits, w.touched,
+                 w.pairs, w.work);
   const uint32_t room = uint32_t(w.max_splits * (kChunk / 32));
-  launch_chained(st, weigh_items, blocks_for(g.tiles * g.splits), kThreads, 0, w.pairs, nact, w.bits, w.bwords,
-                 uint32_t(g.cps), uint32_t(v.nchunks), room, w.items, w.work);
+  launch_chained(st, weigh_items, blocks_for(pairs), kThreads, 0, w.pairs, nact, w.bits, w.bwords, w.grid,
+                 uint32_t(v.nchunks), room, w.items, w.work);
   static const int per_sm = [] {
     int a = 0;
     SYM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, ms_tile<T, COUNT, NEWTON, GAUSS>,
                                                            kChunk, 0));
     return std::max(1, a);
   }();
-  const unsigned ctas = unsigned(std::min<uint64_t>(g.tiles * g.splits, uint64_t(152) * per_sm));
+  const unsigned ctas = unsigned(std::min<uint64_t>(pairs, uint64_t(152) * per_sm));
   launch_chained(st, ms_tile<T, COUNT, NEWTON, GAUSS>, ctas, kChunk, 0, desc, v.sbox, uint32_t(v.nchunks), v.q,
-                 means, state, ids, uint32_t(n), T(h2), k, gap2, g, w.touched, w.bits, w.bwords, w.items, room,
+                 means, state, ids, nact, T(h2), k, gap2, w.grid, w.touched, w.bits, w.bwords, w.items, room,
                  w.work, partial, counts, evals);
   call.launched(4);
 }
 
+// Iterations are launched back to back: the number of active seeds and the
+// layout that goes with it stay on the device, and an iteration that finds no
+// active seed returns at once.  The number only falls, so the last one the
+// host saw bounds the launches; it looks before the first iteration and after
+// every kShiftCheck (an iteration of the mirror planes' approach: 34 us with a
+// look at each, 25 now).  A polish with kMoving seeds
+// left looks at each: the instance without Newton sums serves an iteration
+// without kNear seeds, and rounds distances otherwise.
+constexpr int kShiftCheck = 4, kPolishCheck = 2;  // (a polish ends after a few)
 template <typename T>
 int shift_impl(Call &call, const VoteSet &v, const T *desc, T *means, uint8_t *state, uint64_t k,
                double h2, int max_iter, bool polish, double *seed_iterations,
                unsigned long long *evals, uint32_t *trace = nullptr, int trace_len = 0) {
   cudaStream_t st = call.stream();
   int32_t *ids = call.alloc<int32_t>(k);
-  unsigned *nact = call.alloc<unsigned>(2);
+  // active seeds, kNear ones, iterations done, then the active seeds of each
+  const unsigned trace_cap = unsigned(std::max(max_iter, 1));
+  unsigned *nact = call.alloc<unsigned>(3 + size_t(trace_cap)), *iter = nact + 2, *trace_dev = nact + 3;
+  std::vector<unsigned> seen(3 + (trace || seed_iterations ? size_t(trace_cap) : 0), 0u);
   // partial capacity: splits x slots is at most ~blocks*152*kChunk (+ one tile)
   const int bps = v.tuning.simt_blocks_per_sm;
   uint64_t cap = (uint64_t(bps) * 152 + 2) * uint64_t(kChunk) + std::max<uint64_t>(k, kChunk) * 2;
   T *partial = call.alloc<T>(cap * kPartial);
   T *red = call.alloc<T>(uint64_t(kGroups) * kPartial * std::max<uint64_t>(k, kChunk) * 2);
   TileWork work = tile_work<T>(call, v, k);
-  int it = 0;
-  for (; it < max_iter; ++it) {
-    launch_chained(st, retile<T>, retile_blocks(k), kRetileThreads, 0, means, state, k, v.gbox, polish, ids, nact,
-                   nullptr, nullptr, 0u);
-    unsigned counts[2] = {0, 0};
-    SYM_CUDA(cudaMemcpyAsync(counts, nact, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+  SYM_CUDA(cudaMemsetAsync(iter, 0, sizeof(unsigned), st));
+  uint64_t tiles = (k + kChunk - 1) / kChunk;  // at most, as the host knows
+  const unsigned *const counts = seen.data();
+  const bool gauss = v.kernel_k > 0;
+  bool finished = false;
+  auto look = [&]() {
+    // what a call without a long limit asks for arrives with the counts
+    call.d2h(seen.data(), nact, std::min<size_t>(seen.size(), 512) * sizeof(unsigned));
     call.sync();
+  };
+  const int check = polish ? kPolishCheck : kShiftCheck;
+  for (int it = 0; it < max_iter; ++it) {
+    launch_chained(st, retile<T>, retile_blocks(k), kRetileThreads, 0, means, state, k, v.gbox, polish, ids, nact,
+                   iter, trace_dev, trace_cap, plan_of<T>(v, work, tiles));
     call.launched();
-    const unsigned n = counts[0];
-    if (!n) break;
-    if (seed_iterations) *seed_iterations += n;
-    if (trace && it < trace_len) trace[it] = n;
-    const Grid g = grid_for(n, v.nchunks, bps);
-    if (g.splits * g.slots > cap || g.splits * g.tiles > work.max_splits)
+    if (it % check == 0 || (polish && counts[1] != counts[0])) {
+      look();
+      finished = !counts[0];
+      if (finished) break;
+      tiles = (counts[0] + kChunk - 1) / kChunk;
+    }
+    if ((uint64_t(bps) * 152 + tiles) * kChunk > cap || uint64_t(bps) * 152 + tiles > work.max_splits)
       fail(SYM_RUNTIME_ERROR, "mean-shift partial buffer too small");
-    const bool gauss = v.kernel_k > 0;
-    const auto tiles = counts[1] ? (gauss ? run_tiles<T, false, true, true> : run_tiles<T, false, true, false>)
-                                 : (gauss ? run_tiles<T, false, false, true> : run_tiles<T, false, false, false>);
-    tiles(call, v, desc, means, state, ids, nact, n, h2, g, work, partial, nullptr, evals);
-    launch_chained(st, ms_reduce<T>, dim3(unsigned(g.tiles), counts[1] ? 34u : 7u, kGroups), 2 * kChunk, 0,
-                   partial, g, n, work.touched, red);
-    launch_chained(st, ms_update<T>, unsigned(g.tiles), kChunk, 0, means, red, g.slots, ids, n, T(h2),
+    const auto run = counts[1] ? (gauss ? run_tiles<T, false, true, true> : run_tiles<T, false, true, false>)
+                               : (gauss ? run_tiles<T, false, false, true> : run_tiles<T, false, false, false>);
+    run(call, v, desc, means, state, ids, nact, tiles, h2, work, partial, nullptr, evals);
+    launch_chained(st, ms_reduce<T>, dim3(unsigned(tiles), counts[1] ? 34u : 7u, kGroups), 2 * kChunk, 0,
+                   partial, work.grid, nact, work.touched, red);
+    launch_chained(st, ms_update<T>, unsigned(tiles), kChunk, 0, means, red, work.grid, ids, nact, T(h2),
                    T(v.kernel_k), polish ? it : -1, state);
     call.launched(2);
   }
-  return it;
+  if (!finished) look();
+  const unsigned done = seen[2];
+  if (seen.size() > 3) {
+    if (3 + size_t(done) > 512) {
+      call.d2h(seen.data(), nact, (3 + size_t(std::min(done, trace_cap))) * sizeof(unsigned));
+      call.sync();
+    }
+    for (unsigned i = 0; i < done && i < trace_cap; ++i) {
+      if (seed_iterations) *seed_iterations += seen[3 + i];
+      if (trace && int(i) < trace_len) trace[i] = seen[3 + i];
+    }
+  }
+  return int(done);
 }
 
 }  // namespace
@@ -1028,7 +1103,7 @@ void active_seeds_async(Call &call, const VoteSet &v, const float *means, const 
                         uint64_t k, int32_t *ids, unsigned *nact, unsigned *iter, uint32_t *trace,
                         unsigned trace_cap) {
   launch_chained(call.stream(), retile<float>, retile_blocks(k), kRetileThreads, 0, means, state, k, v.gbox,
-                 false, ids, nact, iter, trace, trace_cap);
+                 false, ids, nact, iter, trace, trace_cap, Plan());
   call.launched();
 }
 
@@ -1040,13 +1115,13 @@ void count_within(Call &call, const VoteSet &v, const float *points, uint64_t nm
   SYM_CUDA(cudaMemsetAsync(state, 0, nm, st));
   int32_t *ids = call.alloc<int32_t>(nm);
   unsigned *nact = call.alloc<unsigned>(2);
-  retile<float><<<retile_blocks(nm), kRetileThreads, 0, st>>>(points, state, nm, v.gbox, false, ids, nact);
-  check_launch();
-  const Grid g = grid_for(nm, v.nchunks, v.tuning.simt_blocks_per_sm);
+  const uint64_t tiles = (nm + kChunk - 1) / kChunk;
   TileWork work = tile_work<float>(call, v, nm);
   SYM_CUDA(cudaMemsetAsync(counts, 0, nm * sizeof(*counts), st));
-  run_tiles<float, true, false, false>(call, v, v.desc, points, nullptr, ids, nact, nm, h2, g, work,
-                                static_cast<float *>(nullptr), counts, nullptr);
+  launch_chained(st, retile<float>, retile_blocks(nm), kRetileThreads, 0, points, state, nm, v.gbox, false, ids,
+                 nact, nullptr, nullptr, 0u, plan_of<float>(v, work, tiles));
+  run_tiles<float, true, false, false>(call, v, v.desc, points, nullptr, ids, nact, tiles, h2, work,
+                                       static_cast<float *>(nullptr), counts, nullptr);
   call.launched();
 }
 

@@ -59,3 +59,29 @@ def test_vote_counts(gpu, votes):
         near = np.abs(means[:, None] - centres[None]).max(-1)
         assert np.array_equal(near.argmin(1), np.abs(v[pick][:, None] - centres[None]).max(-1).argmin(1))
         assert near.min(1).max() < 1e-5
+
+
+@pytest.mark.parametrize("precision,kernel", [("fp32", "epanechnikov"), ("fp32", "gaussian"),
+                                              ("fp64", "epanechnikov"), ("bf16", "epanechnikov")])
+@pytest.mark.parametrize("votes", [3000, 40000])  # direct, and by work items
+def test_iteration_limits(gpu, votes, precision, kernel):
+    """The host looks at the seeds every few iterations only: whatever the limit
+    relative to that, it is kept, and a limit past the last iteration changes
+    nothing, also with a polish that finds seeds still moving."""
+    g = np.random.default_rng(votes)
+    v = g.normal(size=(votes, 6)) * 0.2
+    pick = g.choice(votes, 300, replace=False)
+    long = gpu.meanshift6(v, pick, 0.3, precision, 500, 0, kernel)
+    total = long[2][0]
+    assert 3 < total < 500
+    for limit in [1, 2, 3, 4, 5, 6, 7, 8, 9, total - 1, total, total + 1, total + 9]:
+        out = gpu.meanshift6(v, pick, 0.3, precision, limit, 0, kernel)
+        assert out[2][0] == min(limit, total)
+        if limit >= total:
+            assert np.array_equal(out[0], long[0]) and np.array_equal(out[1], long[1])
+    for limit in (1, 2, 5):  # the polish goes on with moving seeds
+        ends = [gpu.meanshift6(v, pick, 0.3, precision, limit, polish, kernel) for polish in (200, 201, 203)]
+        assert ends[0][2][1] < 200
+        for e in ends[1:]:
+            assert e[2] == ends[0][2]
+            assert np.array_equal(e[0], ends[0][0]) and np.array_equal(e[1], ends[0][1])
