@@ -11,10 +11,12 @@ namespace sym {
 // alias `in` only if in == out is not required: in and out must differ.
 void exclusive_scan(Call &call, const uint64_t *in, uint64_t *out, uint64_t n);
 
-// Stable sort of `keys`/`values` by the low `key_bits` bits of the keys
-// (8-bit digits).  Results land in keys_out/values_out.
+// Stable sort of `keys`/`values` by bits first_bit .. key_bits - 1 of the keys
+// (8-bit digits; bits up to the next whole digit must order the same way).
+// Results land in keys_out/values_out.
 void radix_sort_pairs(Call &call, const uint64_t *keys, const int32_t *values,
-                      uint64_t *keys_out, int32_t *values_out, uint64_t n, int key_bits = 64);
+                      uint64_t *keys_out, int32_t *values_out, uint64_t n, int key_bits = 64,
+                      int first_bit = 0);
 
 // Writes the indices i (ascending) with flags[i] != 0 to `out`
 // (capacity n) and their number to *count (device).

@@ -1436,7 +1436,8 @@ Lbvh lbvh_build(Call &call, const double *xyz, const double *vn, uint64_t nv,
   lbvh_keys<<<blocks_for(nf), kThreads, 0, st>>>(b.xyz, nv, faces, nf, make_float3(lo[0], lo[1], lo[2]),
                                                  make_float3(1 / ext, 1 / ext, 1 / ext), keys, ids);
   check_launch();
-  radix_sort_pairs(call, keys, ids, skeys, sids, nf, 64);
+  // the keys arrive in the order of their low halves, the ids: the codes alone are sorted
+  radix_sort_pairs(call, keys, ids, skeys, sids, nf, 62, 32);
   {  // the query order of the verification: neighbouring vertices in a warp
     uint64_t *vkeys = call.alloc<uint64_t>(nv), *svkeys = call.alloc<uint64_t>(nv);
     int32_t *vids = call.alloc<int32_t>(nv);
@@ -1445,7 +1446,7 @@ Lbvh lbvh_build(Call &call, const double *xyz, const double *vn, uint64_t nv,
         vids);
     check_launch();
     call.launched();
-    radix_sort_pairs(call, vkeys, vids, svkeys, b.order, nv, 64);
+    radix_sort_pairs(call, vkeys, vids, svkeys, b.order, nv, 62, 32);
   }
   if (ni) {
     int32_t *parent_in = call.alloc<int32_t>(ni), *parent_leaf = call.alloc<int32_t>(nf);
