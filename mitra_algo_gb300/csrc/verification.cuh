@@ -356,6 +356,7 @@ struct Lbvh {
   float4 *node = nullptr;          // (nf - 1) x 4: the two children's lo[3], hi[3], then their
                                    // ids (>= 0 internal node, < 0 leaf ~face) and padding
   float4 *face = nullptr;          // nf x 4: corners, edge and normal data (verify_fast.cu, Face)
+  float4 *flat = nullptr;          // nf x 4: the faces in their planes (verify_fast.cu, FlatFace)
   float *vn = nullptr;             // 3 x nv, FP32 copy of the vertex normals
   int32_t *order = nullptr;        // nv: the vertices in Morton order of their position
   double *fn64 = nullptr;          // nf x 3: unit(cross(b - a, c - a)) of each face, FP64

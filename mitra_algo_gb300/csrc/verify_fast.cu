@@ -227,6 +227,7 @@ struct BvhView {
   const float *xyz;
   const float4 *node;    // nf - 1 records of four (lbvh_internal)
   const float4 *face;    // nf records of four: (a, inv_ab), (b, inv_bc), (c, inv_ca), (n, reach)
+  const float4 *flat;    // nf records of four, for the candidate search (FlatFace)
   const int32_t *order;  // nv: query order of the vertices (Morton order of their position)
   const double *fn64;    // nf x 3: the faces' FP64 unit normals of the normal test
 };
@@ -356,6 +357,62 @@ constexpr float kErr = 1.0f / 32768.0f;
 constexpr float kNormalBand = 1.0f / 1024.0f;
 constexpr int kCandidates = 16;
 
+// A face as the candidate search reads it, 64 bytes: the triangle in its own
+// plane.  Corner a, the unit normal n and the unit direction e of ab (both
+// rounded from FP64), and with x along e and y along n x e the corners b = (l, 0)
+// and c = (cx, cy), the reciprocal lengths of the three edges, and `reach`, a
+// bound on the edge lengths; reach 0: no usable normal; reach < 0: a face longer
+// than a quarter of the mesh's largest coordinate, or with an edge outside 1e-15 ..
+// 1e15, for which face_d2n decides.
+struct FlatFace {
+  F3 a, n, e;
+  float l, cx, cy, rab, rbc, rca, reach;
+};
+__device__ __forceinline__ FlatFace load_flat(const BvhView &b, int32_t f) {
+  const float4 *r = b.flat + 4 * int64_t(f);
+  const float4 x = r[0], y = r[1], z = r[2], w = r[3];
+  return {{x.x, x.y, x.z}, {y.x, y.y, y.z}, {z.x, z.y, z.z}, x.w, y.w, z.w, w.x, w.y, w.z, w.w};
+}
+__device__ __forceinline__ float dot_fma(F3 a, F3 b) { return fmaf(a.x, b.x, fmaf(a.y, b.y, a.z * b.z)); }
+
+// FP32 squared distance from p to a face with reach > 0, within 64 u M of its
+// FP64 distance; only the plane distance when that is above `lim` already.
+// The in-plane distance is 0 when p projects inside the three edge lines by
+// more than the rounding of those tests (band), else that to the nearest edge
+// segment: of a p that projects inside by less, whose in-plane distance is 0, the
+// nearest segment is within two bands.
+// Error, with M the largest coordinate magnitude of mesh, image and translation
+// and at least 2 tau, and w = p - a, |w| <= tau + reach <= 0.75 M: the image (30
+// u M) and a (1.8 u M) move w by 32 u M + u |w|; n, e and n x e are within u,
+// u and 4 u of their directions, and the products round by 3 u |w| each, which
+// moves (h, x, y) by sqrt(4^2 + 4^2 + 8^2) u |w| <= 8 u M; b and c by 2 u reach
+// <= u M; the line tests, 5 u (|x| + |y| + reach) <= 6.5 u M each, enter twice; the
+// rest is rounding of the distance, 4 u (0.5 M): 32 + 8 + 1 + 13 + 2 = 56 u M.
+// In the plane a distance takes some 45 instructions where face_d2n's, from the
+// corners and with a band of its own per edge function, take some 120: verify_fp32
+// on the 1e6-triangle torus (2e7 queries) 35 ms, 41 with face_d2n; 31 with five
+// CTAs per SM instead of four (it waits for memory most of the time).
+__device__ __forceinline__ float flat_d2(F3 p, const FlatFace &f, float lim) {
+  const F3 w = p - f.a;
+  const float h = dot_fma(f.n, w), h2 = h * h;
+  if (h2 > lim) return h2;
+  const F3 m{fmaf(f.n.y, f.e.z, -(f.n.z * f.e.y)), fmaf(f.n.z, f.e.x, -(f.n.x * f.e.z)),
+             fmaf(f.n.x, f.e.y, -(f.n.y * f.e.x))};
+  const float x = dot_fma(f.e, w), y = dot_fma(m, w);
+  const float bx = f.cx - f.l, rx = x - f.l;  // b to c, b to p
+  const float sbc = fmaf(bx, y, -(f.cy * rx)) * f.rbc, sca = fmaf(f.cy, x, -(f.cx * y)) * f.rca;
+  const float band = 5.f * kUnit * (fabsf(x) + fabsf(y) + f.reach);
+  if (fminf(y, fminf(sbc, sca)) > band) return h2;
+  const float tab = __saturatef(x * f.rab);
+  const float tbc = __saturatef(fmaf(rx, bx, y * f.cy) * f.rbc * f.rbc);
+  const float tca = __saturatef(fmaf(x, f.cx, y * f.cy) * f.rca * f.rca);
+  const float ax = fmaf(-f.l, tab, x);
+  const float ux = fmaf(-bx, tbc, rx), uy = fmaf(-f.cy, tbc, y);
+  const float vx = fmaf(-f.cx, tca, x), vy = fmaf(-f.cy, tca, y);
+  const float g2 = fminf(fmaf(ax, ax, y * y), fminf(fmaf(ux, ux, uy * uy), fmaf(vx, vx, vy * vy)));
+  return h2 + g2;
+}
+
 // Faces whose FP64 distance to the image can be the smallest: every face
 // whose FP32 distance (or, for a face face_d2n leaves undecided or one
 // without a usable normal, a lower bound: the face_d2n bound or the box
@@ -382,10 +439,11 @@ __device__ int candidate_faces(const BvhView &b, F3 p, float tau_err, float err,
   bool overflow = false;
   const float um = err * (1.f / 512.f);  // err = kErr M = 512 u M
   auto consider = [&](int32_t f, float box) {
-    const Face face = load_face(b, f);
+    const FlatFace face = load_flat(b, f);
     float key = box;
     int32_t id = ~f;
-    if (face.reach != 0.f && face_d2n(p, face, um, lim, key)) id = f;
+    if (face.reach > 0.f) key = flat_d2(p, face, lim), id = f;
+    else if (face.reach < 0.f && face_d2n(p, load_face(b, f), um, lim, key)) id = f;
     if (id >= 0) {
       if (key < best) {
         best = key;
@@ -486,7 +544,7 @@ struct RowLists {
 // candidates that disagree on the normal test, or a candidate overflow send
 // the row to the FP64 decisions.  An accepted forward row is listed with its
 // candidates, the faces its FP64 distance is the smallest of.
-__global__ void __launch_bounds__(kThreads, 4)
+__global__ void __launch_bounds__(kThreads, 5)
     verify_fp32(BvhView b, const float *vn32, const MotionF *motions, uint64_t nc, float tau,
                 float scale, uint8_t *flags, double *err, RowLists lists, int *status) {
   // query q = (c, direction, j) takes vertex i = order[j]: the warps walk
@@ -509,7 +567,7 @@ __global__ void __launch_bounds__(kThreads, 4)
   F3 q{r[0] * u.x + r[1] * u.y + r[2] * u.z, r[3] * u.x + r[4] * u.y + r[5] * u.z,
        r[6] * u.x + r[7] * u.y + r[8] * u.z};
   if (!inverse) q = q + F3{m.t[0], m.t[1], m.t[2]};
-  const float mag = fmaxf(scale, fmaxf(fabsf(q.x), fmaxf(fabsf(q.y), fabsf(q.z))));
+  const float mag = fmaxf(fmaxf(scale, 2.f * tau), fmaxf(fabsf(q.x), fmaxf(fabsf(q.y), fabsf(q.z))));
   const float e = kErr * fmaxf(mag, fmaxf(fabsf(m.t[0]), fmaxf(fabsf(m.t[1]), fabsf(m.t[2]))));
   auto to_fp64 = [&]() {
     lists.mark[qid] = 1;
@@ -605,7 +663,7 @@ __device__ int hybrid_query(const BvhView &b, const Surface &s, const double *vn
   D3 q;
   if (query_skipped(m, r, inverse, p, tau, q)) return 0;
   const F3 qf{float(q.x), float(q.y), float(q.z)};
-  const float mag = fmaxf(scale, fmaxf(fabsf(qf.x), fmaxf(fabsf(qf.y), fabsf(qf.z))));
+  const float mag = fmaxf(fmaxf(scale, 2.f * float(tau)), fmaxf(fabsf(qf.x), fmaxf(fabsf(qf.y), fabsf(qf.z))));
   const float e = kErr * mag;
   int32_t faces[N];
   float keys[N];
@@ -1391,6 +1449,29 @@ __global__ void lbvh_face_records(const double *xyz, uint64_t nv, const int32_t 
                                 usable ? fmaxf(sqrtf(longest) * 1.0001f, 1e-30f) : 0.f);
 }
 
+// The FlatFace records: one thread per face, in FP64 (a face's quotients and
+// square roots are some 150 FP64 operations, 0.2 ms for 1e6 faces, once per mesh).
+__global__ void lbvh_flat_records(const double *xyz, uint64_t nv, const int32_t *faces, uint64_t nf,
+                                  const float4 *face, float longest, float4 *flat) {
+  const uint64_t f = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (f >= nf) return;
+  D3 c[3];
+  for (int i = 0; i < 3; ++i) {
+    const int32_t v = faces[i * nf + f];
+    c[i] = D3{xyz[v], xyz[nv + v], xyz[2 * nv + v]};
+  }
+  const D3 ab = c[1] - c[0], ac = c[2] - c[0], bc = c[2] - c[1];
+  const double lab = norm(ab), lbc = norm(bc), lca = norm(ac);
+  const D3 n = unit(cross(ab, ac)), e = div(ab, lab), m = cross(n, e);
+  const float4 normal = face[4 * f + 3];
+  const bool plain = normal.w <= longest && fmin(lab, fmin(lbc, lca)) > 1e-15 && fmax(lab, fmax(lbc, lca)) < 1e15;
+  const float reach = plain ? normal.w : -normal.w;
+  flat[4 * f] = make_float4(float(c[0].x), float(c[0].y), float(c[0].z), float(lab));
+  flat[4 * f + 1] = make_float4(float(n.x), float(n.y), float(n.z), float(dot(ac, e)));
+  flat[4 * f + 2] = make_float4(float(e.x), float(e.y), float(e.z), float(dot(ac, m)));
+  flat[4 * f + 3] = make_float4(float(1.0 / lab), float(1.0 / lbc), float(1.0 / lca), reach);
+}
+
 Lbvh lbvh_build(Call &call, const double *xyz, const double *vn, uint64_t nv,
                 const int32_t *faces, uint64_t nf) {
   Lbvh b;
@@ -1401,7 +1482,7 @@ Lbvh lbvh_build(Call &call, const double *xyz, const double *vn, uint64_t nv,
   auto pad = [](uint64_t x) { return (x + 255) & ~uint64_t(255); };
   const uint64_t s_xyz = pad(12 * nv), s_node = pad(4 * kNodeWords * (ni + 1)),
                  s_face = pad(64 * nf), s_order = pad(4 * nv), s_fn64 = pad(24 * nf);
-  SYM_CUDA(cudaMalloc(&b.block, 2 * s_xyz + s_node + s_face + s_order + s_fn64));
+  SYM_CUDA(cudaMalloc(&b.block, 2 * s_xyz + s_node + 2 * s_face + s_order + s_fn64));
   char *at = b.block;
   auto take = [&](uint64_t bytes) {
     char *r = at;
@@ -1410,6 +1491,7 @@ Lbvh lbvh_build(Call &call, const double *xyz, const double *vn, uint64_t nv,
   };
   b.node = reinterpret_cast<float4 *>(take(s_node));
   b.face = reinterpret_cast<float4 *>(take(s_face));
+  b.flat = reinterpret_cast<float4 *>(take(s_face));
   b.xyz = reinterpret_cast<float *>(take(s_xyz));
   b.vn = reinterpret_cast<float *>(take(s_xyz));
   b.order = reinterpret_cast<int32_t *>(take(s_order));
@@ -1431,6 +1513,9 @@ Lbvh lbvh_build(Call &call, const double *xyz, const double *vn, uint64_t nv,
   }
   float ext = std::max({hi[0] - lo[0], hi[1] - lo[1], hi[2] - lo[2], 1e-30f});
   for (int a = 0; a < 3; ++a) b.scale = std::max({b.scale, std::fabs(lo[a]), std::fabs(hi[a])});
+  lbvh_flat_records<<<blocks_for(nf), kThreads, 0, st>>>(xyz, nv, faces, nf, b.face, 0.25f * b.scale, b.flat);
+  check_launch();
+  call.launched();
   uint64_t *keys = call.alloc<uint64_t>(nf), *skeys = call.alloc<uint64_t>(nf);
   int32_t *ids = call.alloc<int32_t>(nf), *sids = call.alloc<int32_t>(nf);
   lbvh_keys<<<blocks_for(nf), kThreads, 0, st>>>(b.xyz, nv, faces, nf, make_float3(lo[0], lo[1], lo[2]),
@@ -1473,7 +1558,7 @@ void lbvh_free(Lbvh &b) {
 namespace {
 
 BvhView view_of(const Lbvh &b) {
-  return {b.nv, b.nf, b.faces, b.xyz, b.node, b.face, b.order, b.fn64};
+  return {b.nv, b.nf, b.faces, b.xyz, b.node, b.face, b.flat, b.order, b.fn64};
 }
 
 // `refine` passes of FP64 least-squares refinement of the nc modes' motions
