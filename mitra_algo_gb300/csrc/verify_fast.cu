@@ -413,6 +413,19 @@ __device__ __forceinline__ float flat_d2(F3 p, const FlatFace &f, float lim) {
   return h2 + g2;
 }
 
+// The region of the face p's nearest point seems to lie in (0, 1, 2: nearest to
+// the segment ab, bc, ca; 3: inside) and its squared distance `d2` (flat_d2).
+__device__ __forceinline__ int flat_region(F3 p, const FlatFace &f, float &d2) {
+  d2 = flat_d2(p, f, INFINITY);
+  const F3 w = p - f.a;
+  const F3 m{fmaf(f.n.y, f.e.z, -(f.n.z * f.e.y)), fmaf(f.n.z, f.e.x, -(f.n.x * f.e.z)),
+             fmaf(f.n.x, f.e.y, -(f.n.y * f.e.x))};
+  const float x = dot_fma(f.e, w), y = dot_fma(m, w);
+  const float sbc = fmaf(f.cx - f.l, y, -(f.cy * (x - f.l))) * f.rbc, sca = fmaf(f.cy, x, -(f.cx * y)) * f.rca;
+  const float least = fminf(y, fminf(sbc, sca));
+  return least >= 0.f ? 3 : least == y ? 0 : least == sbc ? 1 : 2;
+}
+
 // Faces whose FP64 distance to the image can be the smallest: every face
 // whose FP32 distance (or, for a face face_d2n leaves undecided or one
 // without a usable normal, a lower bound: the face_d2n bound or the box
@@ -697,6 +710,12 @@ __device__ int hybrid_query(const BvhView &b, const Surface &s, const double *vn
   return agree ? 1 : 0;
 }
 
+// u M of a query whose image is q, M as the error of a FlatFace distance has it.
+__device__ __forceinline__ float search_unit(const ClusterMotion &m, F3 q, float scale, float tau) {
+  const float t = fmaxf(fabsf(float(m.t[0])), fmaxf(fabsf(float(m.t[1])), fabsf(float(m.t[2]))));
+  return kUnit * fmaxf(fmaxf(fmaxf(scale, 2.f * tau), t), fmaxf(fabsf(q.x), fmaxf(fabsf(q.y), fabsf(q.z))));
+}
+
 // Which corner of the face is the nearest point to p, by the region tests of
 // triangle_d2, when FP32 decides them: 0, 1, 2 for a, b, c, else -1.  p is
 // within 1.8 u M of its FP64 value, as the corners are, so a product e . (p - v)
@@ -720,204 +739,352 @@ __device__ __forceinline__ int corner_region(F3 p, const Face &f, float um) {
   return -1;
 }
 
-// The reference's FP64 squared distance of each listed forward row: the
-// smallest over its candidate faces (the face it keeps is among them).
-__global__ void forward_errors(Surface s, const ClusterMotion *motions, RowLists lists,
-                               unsigned long long count, double *err) {
-  const uint64_t k = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k >= count) return;
-  const uint64_t row = lists.forward[k], nv = s.nv;
-  const uint64_t c = row / (2 * nv), i = row % (2 * nv);
-  const ClusterMotion &m = motions[c];
-  const M3 r = query_rotation(m, false);
-  const D3 q = mul(r, vertex(s, int32_t(i))) + D3{m.t[0], m.t[1], m.t[2]};
+// FP64 distances of a block's rows, one per thread.  FP64 runs at 1/64 of the
+// FP32 rate, and a warp pays for an FP64 operation whether one of its lanes needs
+// it or all: FP64 is kept to what FP32 cannot decide, and what is left is sorted
+// so that the lanes of a warp need the same.
+//  * A face whose nearest point is one of its corners (most of a rough mesh's
+//    rows: the faces around a vertex at exactly one distance) takes that vertex's
+//    |q - v|^2, eight FP64 operations and none for the next face around the
+//    same vertex.
+//  * Another face is evaluated only when its FP32 distance does not already put it
+//    beyond the smallest of those.
+//  * What remains goes by the region its nearest point seems to lie in (an edge
+//    of the three, or inside) into one of four lists, and whole warps take 32
+//    distances of one list: triangle_d2 returns early for the edges, and its
+//    divisions, a fifth of its operations, are those of one region.  A wrong
+//    guess costs time only.
+constexpr int kRowThreads = 256, kRegions = 4, kRegionItems = 384;
+struct RowBlock {
+  double q[kRowThreads][3], d[kRegions][kRegionItems];
+  unsigned long long dmin[kRowThreads];  // as bits: no distance is negative
+  const int32_t *list[kRowThreads];
+  unsigned at_min[kRowThreads];
+  unsigned count[kRegions];
+  uint16_t item[kRegions][kRegionItems];  // row * 16 + candidate
+};
+static_assert(kCandidates == 16 && kRowThreads * 16 <= 65536, "an item is 16 bits");
+
+// The candidates of a row seen in FP32: bit sets of those at the smallest
+// distance so far, in no corner's region, and of the normal test's outcome.
+struct RowFaces {
+  unsigned at_min = 0, open = 0, agrees = 0, unsure = 0;
   double dmin = INFINITY;
-  for (int j = 0; j < kCandidates; ++j) {
-    const int32_t f = lists.faces[k * kCandidates + j];
-    if (f < 0) break;
-    dmin = fmin(dmin, triangle_d2(q, corner(s, f, 0), corner(s, f, 1), corner(s, f, 2)));
+  __device__ __forceinline__ void take(double d, int j) {
+    if (d < dmin) dmin = d, at_min = 0;
+    if (d == dmin) at_min |= 1u << j;
   }
-  err[c * nv + i] = dmin;
+};
+__device__ __forceinline__ int32_t listed_face(int32_t x) { return x < 0 ? ~x : x; }
+
+// The candidates cl (up to `end`) of a row whose image is q: their corner
+// distances, and with NORMALS their normal tests.
+template <bool NORMALS>
+__device__ __forceinline__ RowFaces corner_distances(const BvhView &b, const Surface &s, D3 q, F3 qf, float um,
+                                                     const int32_t *cl, int32_t end, F3 rn) {
+  RowFaces r;
+  double dv = 0;
+  int32_t at_vertex = -1;  // of which dv is the squared distance
+  for (int j = 0; j < kCandidates && cl[j] != end; ++j) {
+    const int32_t f = listed_face(cl[j]);
+    const Face face = load_face(b, f);
+    if (NORMALS) {
+      const float cosine = dotf(rn, face.n);
+      if (face.reach == 0.f || !(fabsf(cosine - 0.5f) > kNormalBand)) r.unsure |= 1u << j;
+      else if (cosine > 0.5f) r.agrees |= 1u << j;
+    }
+    const int v = face.reach == 0.f ? -1 : corner_region(qf, face, um);
+    if (v < 0) {
+      r.open |= 1u << j;
+      continue;
+    }
+    const int32_t id = s.faces[uint64_t(v) * s.nf + f];
+    if (id != at_vertex) {
+      const D3 e = q - vertex(s, id);
+      dv = dot(e, e), at_vertex = id;
+    }
+    r.take(dv, j);
+  }
+  return r;
 }
 
-// The FP64 decisions of the rows verify_fp32 listed.  Where the faces at
-// the minimum disagree on the normal test, the first of them the reference's
-// search reaches takes the test (first_in_reference_order); rows whose
-// candidates overflow the list are listed for verify_listed_ref.
-//
-// FP64 runs at 1/64 of the FP32 rate, and a warp pays for an FP64 operation
-// whether one of its lanes needs it or all: a lane serves a row (so the image
-// costs a warp its twenty operations once per 32 rows), and FP64 is kept to
-// what FP32 cannot decide.  A face whose nearest point is one of its corners
-// (most of a rough mesh's rows: the faces around a vertex at exactly one
-// distance) takes that vertex's |q - v|^2, eight FP64 operations and none for
-// the next face around the same vertex; another face is evaluated only when
-// its FP32 distance does not already put it beyond the smallest of those; the
-// normal test and the visiting order go through FP32 with a band.  Rows with a
-// face to evaluate, and those without candidates, are left by the first pass
-// (ALL = false) in lists.open for a second pass over them alone, from its two
-// ends: the searches of the latter take much longer and fill warps of their own.
-// On the 1e6-triangle torus (1.1e7 rows, 3.3e6 of them in the second pass) the
-// two take 4.4 and 4.2 ms; with eight lanes per row, each with its own copy of the
-// image, they took 17 and 11.
-template <bool ALL>
+// Whether face f is farther than dmin in FP32 already (a decided FP32 distance is
+// within 64 u M of FP64's); `region`: the list its distance belongs to.
+__device__ __forceinline__ bool beyond(const BvhView &b, F3 p, int32_t f, float um, double dmin, int &region) {
+  const FlatFace face = load_flat(b, f);
+  region = 3;
+  if (!(face.reach > 0.f)) return false;
+  float key;
+  region = flat_region(p, face, key);
+  return dmin < INFINITY && sqrtf(key) > sqrtf(float(dmin)) + 128.f * um;
+}
+
+// The smallest FP64 distance of the row of each thread (`live` ones) over the
+// faces `r` left open and the corners it has, and the candidates at exactly that
+// distance (TIES).  Called by the whole block; `cl` and `end` as above.
+template <bool TIES>
+__device__ __forceinline__ void block_distances(RowBlock &sh, const BvhView &b, const Surface &s, bool live,
+                                                D3 q, F3 qf, float um, const int32_t *cl, RowFaces &r) {
+  const int t = threadIdx.x;
+  if (t < kRegions) sh.count[t] = 0;
+  __syncthreads();
+  if (live) {
+    sh.q[t][0] = q.x, sh.q[t][1] = q.y, sh.q[t][2] = q.z;
+    sh.list[t] = cl, sh.at_min[t] = 0;
+    for (unsigned rest = r.open; rest; rest &= rest - 1) {
+      const int j = __ffs(int(rest)) - 1;
+      const int32_t f = listed_face(cl[j]);
+      int region;
+      if (beyond(b, qf, f, um, r.dmin, region)) continue;
+      const unsigned at = atomicAdd(&sh.count[region], 1u);
+      if (at < kRegionItems) sh.item[region][at] = uint16_t(t * 16 + j);
+      else r.take(triangle_d2(q, corner(s, f, 0), corner(s, f, 1), corner(s, f, 2)), j);  // no room left
+    }
+    sh.dmin[t] = __double_as_longlong(r.dmin);
+  }
+  __syncthreads();
+  const int lane = t & 31, warp = t >> 5;
+  unsigned chunks[kRegions + 1];
+  chunks[0] = 0;
+  for (int k = 0; k < kRegions; ++k) chunks[k + 1] = chunks[k] + (min(sh.count[k], unsigned(kRegionItems)) + 31) / 32;
+  for (unsigned c = warp; c < chunks[kRegions]; c += kRowThreads / 32) {
+    int k = 0;
+    while (c >= chunks[k + 1]) ++k;
+    const unsigned at = (c - chunks[k]) * 32 + lane;
+    if (at < min(sh.count[k], unsigned(kRegionItems))) {
+      const int row = sh.item[k][at] >> 4;
+      const int32_t f = listed_face(sh.list[row][sh.item[k][at] & 15]);
+      const D3 x{sh.q[row][0], sh.q[row][1], sh.q[row][2]};
+      const double d = triangle_d2(x, corner(s, f, 0), corner(s, f, 1), corner(s, f, 2));
+      if (TIES) sh.d[k][at] = d;
+      atomicMin(&sh.dmin[row], (unsigned long long)__double_as_longlong(d));
+    }
+  }
+  __syncthreads();
+  if (TIES) {
+    for (int k = 0; k < kRegions; ++k)
+      for (unsigned at = t; at < min(sh.count[k], unsigned(kRegionItems)); at += kRowThreads) {
+        const int row = sh.item[k][at] >> 4;
+        if ((unsigned long long)__double_as_longlong(sh.d[k][at]) == sh.dmin[row])
+          atomicOr(&sh.at_min[row], 1u << (sh.item[k][at] & 15));
+      }
+    __syncthreads();
+  }
+  if (live) {
+    const double d = __longlong_as_double((long long)sh.dmin[t]);
+    if (d < r.dmin) r.dmin = d, r.at_min = 0;
+    r.at_min |= sh.at_min[t];
+  }
+  __syncthreads();  // the lists are free again
+}
+
+// The reference's FP64 squared distance of each listed forward row: the
+// smallest over its candidate faces (the face it keeps is among them).
+// 3.3e6 rows of the 180,000-vertex torus: 1.6 ms; a lane per row that evaluated
+// every candidate took 2.9.
+__global__ void __launch_bounds__(kRowThreads) forward_errors(BvhView b, Surface s, const ClusterMotion *motions,
+                                                              RowLists lists, unsigned long long count,
+                                                              float scale, float tau, double *err) {
+  __shared__ RowBlock sh;
+  const uint64_t k = uint64_t(blockIdx.x) * kRowThreads + threadIdx.x;
+  const uint64_t nv = s.nv;
+  const bool live = k < count;
+  uint64_t at = 0;
+  D3 q{0, 0, 0};
+  F3 qf{0, 0, 0};
+  float um = 0;
+  RowFaces r;
+  const int32_t *cl = nullptr;
+  if (live) {
+    const uint64_t row = lists.forward[k], c = row / (2 * nv), i = row % (2 * nv);
+    const ClusterMotion &m = motions[c];
+    at = c * nv + i;
+    q = mul(query_rotation(m, false), vertex(s, int32_t(i))) + D3{m.t[0], m.t[1], m.t[2]};
+    qf = F3{float(q.x), float(q.y), float(q.z)};
+    um = search_unit(m, qf, scale, tau);
+    cl = lists.faces + k * kCandidates;
+    r = corner_distances<false>(b, s, q, qf, um, cl, -1, F3{0, 0, 0});
+  }
+  block_distances<false>(sh, b, s, live, q, qf, um, cl, r);
+  if (live) err[at] = r.dmin;
+}
+
+// A query of the FP64 rows.
+struct Query {
+  uint64_t c, i, row;
+  bool inverse;
+};
+__device__ __forceinline__ Query query_of(const BvhView &b, uint64_t qid) {
+  const uint64_t nv = b.nv, rem = qid % (2 * nv);
+  Query x;
+  x.c = qid / (2 * nv), x.inverse = rem >= nv;
+  x.i = uint64_t(b.order[rem % nv]);
+  x.row = qid - rem % nv + x.i;
+  return x;
+}
+// Its vertex's image and the unit of the FP32 search there (verify_fp32 decided
+// the 2 tau and side tests of a row with candidates), and its turned normal.
+__device__ __forceinline__ void query_image(const Surface &s, const ClusterMotion *motions,
+                                            const MotionF *motions32, const float *vn32, const Query &x,
+                                            float scale, float tau, D3 &q, F3 &qf, float &um, F3 &rn) {
+  const ClusterMotion &m = motions[x.c];
+  const M3 r = query_rotation(m, x.inverse);
+  const D3 p = vertex(s, int32_t(x.i)), mt{m.t[0], m.t[1], m.t[2]};
+  q = x.inverse ? mul(r, p - mt) : mul(r, p) + mt;
+  qf = F3{float(q.x), float(q.y), float(q.z)};
+  um = search_unit(m, qf, scale, tau);
+  const MotionF &mf = motions32[x.c];
+  float rf[9];
+  for (int j = 0; j < 9; ++j) rf[j] = x.inverse ? mf.r[(j % 3) * 3 + j / 3] : mf.r[j];
+  const F3 ni{vn32[x.i], vn32[s.nv + x.i], vn32[2 * s.nv + x.i]};
+  rn = F3{rf[0] * ni.x + rf[1] * ni.y + rf[2] * ni.z, rf[3] * ni.x + rf[4] * ni.y + rf[5] * ni.z,
+          rf[6] * ni.x + rf[7] * ni.y + rf[8] * ni.z};
+}
+// The decision of a row whose faces at the minimum are known: the normal test of
+// those, and where they disagree (`tie`) that of the one the reference's search
+// visits first (its visiting order is a total order on the faces for this query).
+__device__ __forceinline__ bool decide_row(const BvhView &b, const RefBvh &t, const double *vn,
+                                           const ClusterMotion &m, const Query &x, double tau, D3 q, float um,
+                                           const int32_t *cl, RowFaces &r, bool &tie) {
+  if (!(r.dmin <= tau * tau)) return false;
+  for (unsigned rest = r.at_min & r.unsure; rest; rest &= rest - 1) {
+    const int j = __ffs(int(rest)) - 1;
+    if (normal_agrees_t(b, listed_face(cl[j]), query_rotation(m, x.inverse),
+                        D3{vn[x.i], vn[b.nv + x.i], vn[2 * b.nv + x.i]}))
+      r.agrees |= 1u << j;
+  }
+  tie = (r.at_min & r.agrees) && (r.at_min & ~r.agrees);
+  if (!tie) return (r.at_min & r.agrees) != 0;
+  int jf = __ffs(int(r.at_min)) - 1;
+  int32_t first = listed_face(cl[jf]);
+  for (unsigned rest = r.at_min & (r.at_min - 1); rest; rest &= rest - 1) {
+    const int j = __ffs(int(rest)) - 1;
+    const int32_t f = listed_face(cl[j]);
+    if (first_in_reference_order_f(t, q, um, first, f) != first) first = f, jf = j;
+  }
+  return r.agrees >> jf & 1u;
+}
+
+// The FP64 decisions of the rows verify_fp32 listed, a lane per row, where the
+// corners decide (block_distances); the others, with a face left to evaluate or
+// without candidates, are left in lists.open for verify_rows_open, from its two
+// ends: the searches of the latter take much longer.  Rows whose candidates
+// overflowed stay marked for verify_rows_wide.  On the 1e6-triangle torus 1.1e7
+// rows take 4.3 ms and the 3.3e6 left to the second kernel 3.4 (4.2 with a lane per
+// row that evaluates its open faces in turn); eight lanes per
+// row, each with its own copy of the image, took 17 and 11.
 __global__ void verify_rows_fp64(BvhView b, Surface s, RefBvh t, const double *vn, const float *vn32,
                                  const ClusterMotion *motions, const MotionF *motions32, double tau,
                                  float scale, uint8_t *flags, double *err, RowLists lists,
-                                 unsigned long long rows, int *status) {
-  const unsigned long long searches = ALL ? lists.counts[4] : 0;
-  // the second pass's warps hold searches or rows with candidates, not both
-  const unsigned long long listed_from = (searches + 31) / 32 * 32;
-  const unsigned long long count = ALL ? listed_from + lists.counts[2] : rows;
-  const uint64_t nv = b.nv;
+                                 unsigned long long rows) {
+  const uint64_t k = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
-  for (uint64_t k0 = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32 * 32; k0 < count;
-       k0 += uint64_t(gridDim.x) * blockDim.x) {  // whole warps
-    const uint64_t k = k0 + lane;
-    int32_t left = -1;      // the row to list for the second pass
-    bool search = false;    // ... which has to search
-    bool tie = false;
-    if (k < count && !(ALL && k >= searches && k < listed_from)) {
-      const uint64_t qid =  // a query, as verify_fp32's
-          uint64_t(!ALL              ? lists.fp64[k]
-                   : k < searches    ? lists.open[lists.capacity - 1 - k]
-                                     : lists.open[k - listed_from]);
-      const uint64_t c = qid / (2 * nv), rem = qid % (2 * nv);
-      const bool inverse = rem >= nv;
-      const uint64_t i = uint64_t(b.order[rem % nv]);
-      const uint64_t row = qid - rem % nv + i;
-      const uint32_t slot = lists.slot_of[qid];
-      if (slot == kWideSlot) {
-        // left marked for verify_rows_wide
-      } else if (slot == kNoSlot) {  // no candidates yet
-        if (!ALL) {
-          left = int32_t(qid), search = true;
-        } else {
-          double d = 0;
-          int32_t tied[kCandidates];
-          int v = hybrid_query(b, s, vn, motions[c], inverse, i, tau, scale, d, tied, status);
-          if (v == 3) {
-            tie = true;
-            const M3 r = query_rotation(motions[c], inverse);
-            D3 q;
-            query_skipped(motions[c], r, inverse, vertex(s, int32_t(i)), tau, q);
-            int32_t first = tied[0];
-            for (int x = 1; x < kCandidates && tied[x] >= 0; ++x)
-              first = first_in_reference_order(t, q, first, tied[x]);
-            v = normal_agrees_t(b, first, r, D3{vn[i], vn[nv + i], vn[2 * nv + i]}) ? 1 : 0;
-          }
-          flags[row] = v == 1;
-          if (!inverse) err[c * nv + i] = v == 1 ? d : 0.0;
-          if (v != 2) lists.mark[qid] = 0;  // marked queries go on to the reference-order search
-        }
-      } else {
-        // the image; verify_fp32 decided the 2 tau and side tests of a row with candidates
-        const ClusterMotion &m = motions[c];
-        const M3 r = query_rotation(m, inverse);
-        const D3 p = vertex(s, int32_t(i)), mt{m.t[0], m.t[1], m.t[2]};
-        const D3 q = inverse ? mul(r, p - mt) : mul(r, p) + mt;
-        const F3 qf{float(q.x), float(q.y), float(q.z)};
-        const float mag = fmaxf(scale, fmaxf(fabsf(qf.x), fmaxf(fabsf(qf.y), fabsf(qf.z))));
-        const float um = kErr * (1.f / 512.f) * mag;
-        const MotionF &mf = motions32[c];
-        float rf[9];
-        for (int j = 0; j < 9; ++j) rf[j] = inverse ? mf.r[(j % 3) * 3 + j / 3] : mf.r[j];
-        const F3 ni{vn32[i], vn32[nv + i], vn32[2 * nv + i]};
-        const F3 rn{rf[0] * ni.x + rf[1] * ni.y + rf[2] * ni.z, rf[3] * ni.x + rf[4] * ni.y + rf[5] * ni.z,
-                    rf[6] * ni.x + rf[7] * ni.y + rf[8] * ni.z};
-        const int32_t *cl = lists.cand + uint64_t(slot) * kCandidates;
-        auto candidate = [&](int j) {
-          const int32_t x = cl[j];
-          return x < 0 ? ~x : x;
-        };
-        // sets of candidates, a bit each: at the smallest distance so far, in
-        // no corner's region, with the normal, with the normal test undecided
-        unsigned at_min = 0, open = 0, agrees = 0, unsure = 0;
-        double dmin = INFINITY, dv = 0;
-        int32_t at_vertex = -1;  // of which dv is the squared distance
-        auto take = [&](double d, int j) {
-          if (d < dmin) dmin = d, at_min = 0;
-          if (d == dmin) at_min |= 1u << j;
-        };
-        for (int j = 0; j < kCandidates && cl[j] != kNoFace; ++j) {
-          const int32_t f = candidate(j);
-          const Face face = load_face(b, f);
-          const float cosine = dotf(rn, face.n);
-          if (face.reach == 0.f || !(fabsf(cosine - 0.5f) > kNormalBand)) unsure |= 1u << j;
-          else if (cosine > 0.5f) agrees |= 1u << j;
-          const int v = face.reach == 0.f ? -1 : corner_region(qf, face, um);
-          if (v < 0) {
-            open |= 1u << j;
-            continue;
-          }
-          const int32_t id = s.faces[uint64_t(v) * s.nf + f];
-          if (id != at_vertex) {
-            const D3 e = q - vertex(s, id);
-            dv = dot(e, e), at_vertex = id;
-          }
-          take(dv, j);
-        }
-        bool leave = false;
-        for (unsigned rest = open; rest && !leave; rest &= rest - 1) {
-          const int j = __ffs(rest) - 1;
-          const int32_t f = candidate(j);
-          if (dmin < INFINITY) {  // a decided FP32 distance is within 32 u M of FP64's
-            const Face face = load_face(b, f);
-            float key;
-            if (face.reach != 0.f && face_d2n(qf, face, um, INFINITY, key) &&
-                sqrtf(key) > sqrtf(float(dmin)) + 64.f * um)
-              continue;
-          }
-          if (ALL) take(triangle_d2(q, corner(s, f, 0), corner(s, f, 1), corner(s, f, 2)), j);
-          else leave = true;
-        }
-        if (leave) {
+  int32_t left = -1;      // the row to list for the second kernel
+  bool search = false;    // ... which has to search
+  bool tie = false;
+  if (k < rows) {
+    const uint64_t qid = uint64_t(lists.fp64[k]);  // a query, as verify_fp32's
+    const uint32_t slot = lists.slot_of[qid];
+    if (slot == kNoSlot) {
+      left = int32_t(qid), search = true;
+    } else if (slot != kWideSlot) {
+      const Query x = query_of(b, qid);
+      D3 q;
+      F3 qf, rn;
+      float um;
+      query_image(s, motions, motions32, vn32, x, scale, float(tau), q, qf, um, rn);
+      const int32_t *cl = lists.cand + uint64_t(slot) * kCandidates;
+      RowFaces r = corner_distances<true>(b, s, q, qf, um, cl, kNoFace, rn);
+      for (unsigned rest = r.open; rest && left < 0; rest &= rest - 1) {
+        int region;
+        if (r.dmin == INFINITY || !beyond(b, qf, listed_face(cl[__ffs(int(rest)) - 1]), um, r.dmin, region))
           left = int32_t(qid);
-        } else {
-          bool ok = false;
-          if (dmin <= tau * tau) {  // the normal test of the faces at exactly the minimum
-            for (unsigned rest = at_min & unsure; rest; rest &= rest - 1) {
-              const int j = __ffs(rest) - 1;
-              if (normal_agrees_t(b, candidate(j), r, D3{vn[i], vn[nv + i], vn[2 * nv + i]}))
-                agrees |= 1u << j;
-            }
-            tie = (at_min & agrees) && (at_min & ~agrees);
-            if (tie) {
-              // they disagree: the one the reference visits first (its
-              // visiting order is a total order on the faces for this query)
-              int jf = __ffs(at_min) - 1;
-              int32_t first = candidate(jf);
-              for (unsigned rest = at_min & (at_min - 1); rest; rest &= rest - 1) {
-                const int j = __ffs(rest) - 1;
-                const int32_t f = candidate(j);
-                if (first_in_reference_order_f(t, q, um, first, f) != first) first = f, jf = j;
-              }
-              ok = agrees >> jf & 1u;
-            } else {
-              ok = (at_min & agrees) != 0;
-            }
-          }
-          flags[row] = ok;
-          if (!inverse) err[c * nv + i] = ok ? dmin : 0.0;
-          lists.mark[qid] = 0;
+      }
+      if (left < 0) {
+        const bool ok = decide_row(b, t, vn, motions[x.c], x, tau, q, um, cl, r, tie);
+        flags[x.row] = ok;
+        if (!x.inverse) err[x.c * b.nv + x.i] = ok ? r.dmin : 0.0;
+        lists.mark[qid] = 0;
+      }
+    }
+  }
+  const unsigned ties = __ballot_sync(0xffffffffu, tie);
+  if (ties && lane == 0) atomicAdd(&lists.counts[3], (unsigned long long)__popc(ties));
+  // one atomic per warp and list
+  const unsigned rows_left = __ballot_sync(0xffffffffu, left >= 0 && !search),
+                 to_search = __ballot_sync(0xffffffffu, left >= 0 && search);
+  unsigned long long at = 0;
+  if (lane == 0 && rows_left) at = atomicAdd(&lists.counts[2], (unsigned long long)__popc(rows_left));
+  if (lane == 1 && to_search) at = atomicAdd(&lists.counts[4], (unsigned long long)__popc(to_search));
+  const unsigned long long rows_at = __shfl_sync(0xffffffffu, at, 0),
+                           search_at = __shfl_sync(0xffffffffu, at, 1);
+  const unsigned lt = (1u << lane) - 1;
+  if (left >= 0 && !search) lists.open[rows_at + __popc(rows_left & lt)] = left;
+  if (left >= 0 && search) lists.open[lists.capacity - 1 - (search_at + __popc(to_search & lt))] = left;
+}
+
+// The rows verify_rows_fp64 left: those that search (whole blocks of them, on one
+// lane each), then those with candidates.
+__global__ void __launch_bounds__(kRowThreads) verify_rows_open(
+    BvhView b, Surface s, RefBvh t, const double *vn, const float *vn32, const ClusterMotion *motions,
+    const MotionF *motions32, double tau, float scale, uint8_t *flags, double *err, RowLists lists,
+    int *status) {
+  __shared__ RowBlock sh;
+  const unsigned long long searches = lists.counts[4], open = lists.counts[2];
+  const unsigned long long listed_from = (searches + kRowThreads - 1) / kRowThreads * kRowThreads;
+  const int lane = threadIdx.x & 31;
+  for (uint64_t k0 = uint64_t(blockIdx.x) * kRowThreads; k0 < listed_from + open;
+       k0 += uint64_t(gridDim.x) * kRowThreads) {  // whole blocks of one kind
+    const uint64_t k = k0 + threadIdx.x;
+    bool tie = false;
+    if (k0 < listed_from) {
+      if (k < searches) {
+        const uint64_t qid = uint64_t(lists.open[lists.capacity - 1 - k]);
+        const Query x = query_of(b, qid);
+        const ClusterMotion &m = motions[x.c];
+        double d = 0;
+        int32_t tied[kCandidates];
+        int v = hybrid_query(b, s, vn, m, x.inverse, x.i, tau, scale, d, tied, status);
+        if (v == 3) {
+          tie = true;
+          const M3 r = query_rotation(m, x.inverse);
+          D3 q;
+          query_skipped(m, r, x.inverse, vertex(s, int32_t(x.i)), tau, q);
+          int32_t first = tied[0];
+          for (int j = 1; j < kCandidates && tied[j] >= 0; ++j)
+            first = first_in_reference_order(t, q, first, tied[j]);
+          v = normal_agrees_t(b, first, r, D3{vn[x.i], vn[b.nv + x.i], vn[2 * b.nv + x.i]}) ? 1 : 0;
         }
+        flags[x.row] = v == 1;
+        if (!x.inverse) err[x.c * b.nv + x.i] = v == 1 ? d : 0.0;
+        if (v != 2) lists.mark[qid] = 0;  // marked queries go on to the reference-order search
+      }
+    } else {
+      const bool live = k < listed_from + open;
+      uint64_t qid = 0;
+      Query x{};
+      D3 q{0, 0, 0};
+      F3 qf{0, 0, 0}, rn{0, 0, 0};
+      float um = 0;
+      RowFaces r;
+      const int32_t *cl = nullptr;
+      if (live) {
+        qid = uint64_t(lists.open[k - listed_from]);
+        x = query_of(b, qid);
+        query_image(s, motions, motions32, vn32, x, scale, float(tau), q, qf, um, rn);
+        cl = lists.cand + uint64_t(lists.slot_of[qid]) * kCandidates;
+        r = corner_distances<true>(b, s, q, qf, um, cl, kNoFace, rn);
+      }
+      block_distances<true>(sh, b, s, live, q, qf, um, cl, r);
+      if (live) {
+        const bool ok = decide_row(b, t, vn, motions[x.c], x, tau, q, um, cl, r, tie);
+        flags[x.row] = ok;
+        if (!x.inverse) err[x.c * b.nv + x.i] = ok ? r.dmin : 0.0;
+        lists.mark[qid] = 0;
       }
     }
     const unsigned ties = __ballot_sync(0xffffffffu, tie);
     if (ties && lane == 0) atomicAdd(&lists.counts[3], (unsigned long long)__popc(ties));
-    if (!ALL) {  // one atomic per warp and list
-      const unsigned rows_left = __ballot_sync(0xffffffffu, left >= 0 && !search),
-                     to_search = __ballot_sync(0xffffffffu, left >= 0 && search);
-      unsigned long long at = 0;
-      if (lane == 0 && rows_left) at = atomicAdd(&lists.counts[2], (unsigned long long)__popc(rows_left));
-      if (lane == 1 && to_search) at = atomicAdd(&lists.counts[4], (unsigned long long)__popc(to_search));
-      const unsigned long long rows_at = __shfl_sync(0xffffffffu, at, 0),
-                               search_at = __shfl_sync(0xffffffffu, at, 1);
-      const unsigned lt = (1u << lane) - 1;
-      if (left >= 0 && !search) lists.open[rows_at + __popc(rows_left & lt)] = left;
-      if (left >= 0 && search)
-        lists.open[lists.capacity - 1 - (search_at + __popc(to_search & lt))] = left;
-    }
   }
 }
 
@@ -1668,7 +1835,8 @@ uint64_t exact_flags(Call &call, const ResidentSurface &m, const ClusterMotion *
   call.sync();
   call.launched();
   if (counts[0]) {
-    forward_errors<<<blocks_for(counts[0]), kThreads, 0, st>>>(s, dm, lists, counts[0], err);
+    forward_errors<<<blocks_for(counts[0], kRowThreads), kRowThreads, 0, st>>>(view, s, dm, lists, counts[0],
+                                                                             bvh.scale, float(tau), err);
     check_launch();
     call.launched();
   }
@@ -1676,13 +1844,12 @@ uint64_t exact_flags(Call &call, const ResidentSurface &m, const ClusterMotion *
     ensure_ref_bvh(call, m);
     s.nodes = m.ref->dev.nodes, s.ids = m.ref->dev.ids;
     lists.open = lists.reference;  // free until the next compaction
-    verify_rows_fp64<false><<<blocks_for(counts[1]), kThreads, 0, st>>>(
-        view, s, m.ref->dev, m.vn, bvh.vn, dm, dmf, tau, bvh.scale, flags, err, lists, counts[1],
-        call.status());
+    verify_rows_fp64<<<blocks_for(counts[1]), kThreads, 0, st>>>(view, s, m.ref->dev, m.vn, bvh.vn, dm, dmf, tau,
+                                                                 bvh.scale, flags, err, lists, counts[1]);
     check_launch();
-    verify_rows_fp64<true><<<unsigned(std::min<uint64_t>(blocks_for(counts[1] + 32), 152 * 8)), kThreads,
-                             0, st>>>(view, s, m.ref->dev, m.vn, bvh.vn, dm, dmf, tau, bvh.scale, flags,
-                                      err, lists, 0, call.status());
+    verify_rows_open<<<unsigned(std::min<uint64_t>(blocks_for(counts[1] + kRowThreads, kRowThreads), 152 * 8)),
+                       kRowThreads, 0, st>>>(view, s, m.ref->dev, m.vn, bvh.vn, dm, dmf, tau, bvh.scale, flags,
+                                             err, lists, call.status());
     check_launch();
     call.launched(2);
     compact_indices(call, lists.mark, rows, lists.reference, listed + 1);
