@@ -382,8 +382,9 @@ typedef struct sym_fast_result {
    * position), 0 when only by seeds that settled on a ridge or ran out of
    * iterations */
   uint8_t precise[SYM_FAST_MAX_CLUSTERS];
-  /* the BF16 tensor-core kernel alone: launches, summed device time (CUDA
-   * events around each launch) and the seed-vote evaluations it made */
+  /* the BF16 tensor-core kernel alone: launches, summed device time (from the
+   * start of a launch's first CTA to the end of its last by the device's clock)
+   * and the seed-vote evaluations it made */
   uint64_t tc_launches;
   double tc_kernel_ms, tc_evaluations;
   /* verification queries that the FP32 search and its FP64 rechecks left

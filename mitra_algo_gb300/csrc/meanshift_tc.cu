@@ -583,6 +583,9 @@ struct TcArgs {
   float gauss_k2;           // 0: Epanechnikov; k > 0 (a power of 2): 2^(-k d^2/h^2) - 2^-k
   float *partial;
   unsigned long long *evals;
+  const unsigned *iter;       // iterations with active seeds, this one included
+  unsigned long long *began, *ended;  // per iteration (while *iter <= span_cap): device clock, ns
+  unsigned span_cap;
   int *status;
 };
 
@@ -651,6 +654,10 @@ __global__ void __launch_bounds__(kThreadsTc, 1) ms_tile_tc(TcArgs a) {
   const uint32_t piece = blockIdx.x;
   const uint32_t ntiles = active_tiles(a.nact);
   if (piece >= a.pieces[ntiles]) return;
+  // the launch's own time: its first CTA's start to its last CTA's end by the
+  // device's clock (events around the launch kept it from being chained and cost
+  // 9 us per iteration)
+  if (tid == 0 && *a.iter <= a.span_cap) atomicMin(&a.began[*a.iter - 1], (unsigned long long)global_ns());
   const uint64_t nactive = a.nact[0];
   uint64_t lo_t = 0, hi_t = ntiles;  // last tile whose first piece is <= piece
   while (hi_t - lo_t > 1) {
@@ -901,6 +908,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) ms_tile_tc(TcArgs a) {
   tc_fence_before();
   __syncthreads();
   if (warp == 0 && n) tmem_dealloc(tmem, kTcCols);
+  if (tid == 0 && *a.iter <= a.span_cap) atomicMax(&a.ended[*a.iter - 1], (unsigned long long)global_ns());
 }
 
 // ------------------------------------------------------ tensor self-test
@@ -1140,18 +1148,15 @@ bool meanshift_bf16_bulk(Call &call, const VoteSet &v, float *means, uint8_t *st
   unsigned long long *evals = call.alloc<unsigned long long>(1);
   SYM_CUDA(cudaMemsetAsync(evals, 0, 8, st));
   SYM_CUDA(cudaMemsetAsync(iter, 0, 4, st));
+  const unsigned span_cap = kernel_ms ? trace_cap : 0;
+  unsigned long long *spans = call.alloc<unsigned long long>(2 * size_t(span_cap));
+  SYM_CUDA(cudaMemsetAsync(spans, 0xff, 8 * size_t(span_cap), st));
+  SYM_CUDA(cudaMemsetAsync(spans + span_cap, 0, 8 * size_t(span_cap), st));
   const float gap = float(std::sqrt(h2)) + 1e-6f;
   call.launched();
   TcArgs args{images, v.nchunks, list, offsets, pieces, nact, means, ids, v.gbox,
-              float(1.0 / std::sqrt(h2)), float(v.kernel_k), partial, evals, call.status()};
-  // CUDA events around every launch of the tensor kernel (its own time)
-  std::vector<cudaEvent_t> marks;
-  auto mark_event = [&]() {
-    cudaEvent_t e;
-    SYM_CUDA(cudaEventCreate(&e));
-    SYM_CUDA(cudaEventRecord(e, st));
-    marks.push_back(e);
-  };
+              float(1.0 / std::sqrt(h2)), float(v.kernel_k), partial, evals, iter, spans, spans + span_cap,
+              span_cap, call.status()};
   // Iterations are launched back to back: each reads the active-seed count
   // that the previous one left on the device, and one whose count is zero
   // returns at once.  The host looks at the count every kCheck iterations.
@@ -1167,9 +1172,7 @@ bool meanshift_bf16_bulk(Call &call, const VoteSet &v, float *means, uint8_t *st
                    pieces, call.status());
     launch_chained(st, scatter_lists, list_ctas, kListThreads, 0, need, boff, bcount, sblk, nsurv, nblk, nact,
                    v.nchunks, list_cap, list, call.status());
-    if (kernel_ms) mark_event();
     launch_chained(st, ms_tile_tc, unsigned(max_grid), kThreadsTc, kTcSmem, args);
-    if (kernel_ms) mark_event();
     launch_chained(st, ms_update_bulk, unsigned((k + kUpdateSeeds - 1) / kUpdateSeeds), 32 * kUpdateSeeds, 0,
                    means, partial, pieces, ids, nact, float(h2), state);
     call.launched(6);
@@ -1201,15 +1204,15 @@ bool meanshift_bf16_bulk(Call &call, const VoteSet &v, float *means, uint8_t *st
     for (unsigned i = 0; seed_iterations && i < active_iterations && i < trace_cap; ++i)
       *seed_iterations += tr[i];
   }
-  // launches after the last iteration with active seeds found none and
-  // returned at once: only the active ones are timed
-  for (size_t i = 0; i + 1 < marks.size() && i / 2 < active_iterations; i += 2) {
-    float ms = 0;
-    SYM_CUDA(cudaEventElapsedTime(&ms, marks[i], marks[i + 1]));
-    *kernel_ms += ms;
+  const unsigned timed = std::min(active_iterations, span_cap);
+  if (timed) {
+    std::vector<unsigned long long> began(timed), ended(timed);
+    call.d2h(began.data(), spans, 8 * size_t(timed));
+    call.d2h(ended.data(), spans + span_cap, 8 * size_t(timed));
+    call.sync();
+    for (unsigned i = 0; i < timed; ++i) *kernel_ms += double(ended[i] - began[i]) * 1e-6;
   }
-  if (kernel_launches) *kernel_launches = std::min<uint64_t>(marks.size() / 2, active_iterations);
-  for (auto e : marks) cudaEventDestroy(e);
+  if (kernel_launches) *kernel_launches = timed;
   return true;
 }
 

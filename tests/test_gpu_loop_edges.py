@@ -85,3 +85,17 @@ def test_iteration_limits(gpu, votes, precision, kernel):
         for e in ends[1:]:
             assert e[2] == ends[0][2]
             assert np.array_equal(e[0], ends[0][0]) and np.array_equal(e[1], ends[0][1])
+
+
+def test_tensor_kernel_time(gpu):
+    """The tensor kernel's own time is taken on the device, launch by launch:
+    positive, below the phase's, as many launches as iterations."""
+    from mitra_algo_gb300.mesh import motif_sphere, prepare
+    from mitra_algo_gb300.types import Options
+    mesh = motif_sphere(level=4, bumps=12, folds=5, partial_shift=0.4, noise=1e-3, seed=0)
+    o = Options(sample_ratio=0.5, pair_threshold=0.25, bandwidth=0.1, max_pairs=10 ** 7, max_votes=10 ** 8)
+    r = gpu.load_mesh(prepare(mesh, o))
+    d = gpu.detect_fast(r, None, o, precision="bf16", seeds=128, max_iterations=60, polish_iterations=30)
+    r.close()
+    assert d["tc_launches"] == d["iterations"] > 0
+    assert 0 < d["tc_kernel_ms"] < d["bulk_ms"]
