@@ -83,7 +83,7 @@ __global__ void tile_scan(const uint64_t *in, uint64_t n, const uint64_t *partia
 }
 
 // The whole scan in one block, for the short ones (a radix pass over up to
-// 131,072 keys scans its histogram of 256 digits per 2,048 keys): warp w takes
+// 81,920 keys scans its histogram of 256 digits per 1,280 keys): warp w takes
 // 32 x kBlockItems consecutive values, round by round, and two barriers join the
 // warps.  One launch of 4 us in place of three of 2.5 to 4 each.
 constexpr int kBlockItems = 16, kBlockScan = 1024 * kBlockItems;
@@ -132,9 +132,13 @@ __global__ void __launch_bounds__(1024) scan_block(const uint64_t *in, unsigned 
 }
 
 // ---------------------------------------------------------------- radix sort
+// Keys per block: more make longer runs of a digit (coalescing), fewer leave
+// registers and shared memory for more warps, which is what the scatter waits
+// for.  2.5e7 votes, a pass's scatter and histogram: 58 us with 4 rounds or 5, 67
+// with 8 (2,048 keys), 72 with 12; 4 make the histograms' scan larger.
 constexpr int kSortWarps = 8;
-constexpr int kSortRounds = 8;                       // 32-key rounds per warp
-constexpr int kSortTile = kSortWarps * kSortRounds * 32;  // 2048 keys per block
+constexpr int kSortRounds = 5;                       // 32-key rounds per warp
+constexpr int kSortTile = kSortWarps * kSortRounds * 32;  // 1280 keys per block
 
 __global__ void radix_histogram(const uint64_t *keys, uint64_t n, int shift, uint64_t *hist,
                                 unsigned blocks) {
@@ -150,7 +154,7 @@ __global__ void radix_histogram(const uint64_t *keys, uint64_t n, int shift, uin
     hist[uint64_t(d) * blocks + blockIdx.x] = counts[d];
 }
 
-// Stable scatter: warp w ranks its 256 keys round by round (in input order),
+// Stable scatter: warp w ranks its 160 keys round by round (in input order),
 // warps are then ordered by their index, blocks by the scanned histogram.
 // The block's keys are first placed in digit order in shared memory, so the
 // global writes of each digit are one consecutive run.

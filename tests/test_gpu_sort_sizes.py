@@ -48,7 +48,7 @@ def test_preparation(gpu, nf):
         assert np.array_equal(x, y, equal_nan=True)
 
 
-@pytest.mark.parametrize("samples", [2, 31, 1023, 1024, 1025, 2049, 4096, 8191, 8192, 8193, 16385])
+@pytest.mark.parametrize("samples", [2, 31, 1023, 1024, 1025, 2049, 4096, 8191, 8192, 8193, 12800, 12801, 16385])
 def test_pairs(gpu, samples):
     rng = np.random.default_rng(samples)
     n = samples + 17
