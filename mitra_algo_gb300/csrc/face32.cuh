@@ -54,8 +54,7 @@ constexpr float kUnit = 1.0f / 16777216.0f;
 // band serves the three, 64 u M (|p - a|_1 + 2 reach) with |p - v| <= |p - a| +
 // reach and |e| <= reach (a band too wide only leaves more to FP64): six
 // square roots and three divisions fewer per face than bands and segments of
-// their own (verify_fp32 on the 1e6-triangle torus, 2e7 queries, with the
-// 64-byte nodes and faces: 72 -> 48 ms, 41 with four CTAs per SM).
+// their own.
 __device__ __forceinline__ bool face_d2n(F3 p, const Face &f, float um, float lim, float &d2) {
   const F3 ap = p - f.a;
   const float h = dotf(f.n, ap), h2 = h * h;

@@ -339,20 +339,15 @@ __device__ __forceinline__ int32_t support_query(const BvhView &b, const double 
 // ------------------------------------------- exact decisions, FP32 search
 // Error bound of the FP32 search, in distance units: kErr (512 FP32 units u)
 // times M, the largest coordinate magnitude of the vertex, its image, the
-// translation and the mesh.  The FP32 corners and image are within a few
-// u M of their FP64 values, and the distance is 1-Lipschitz in each; the
-// face's unit normal comes from the FP64 corners (rounded once to FP32), so
-// the plane distance n . (p - a) and the three edge functions
-// (n x e) . (p - v) carry errors of a few u (M + |p - v|) whatever the
-// face's shape, and the segment distances of a few u M as well -- far below
-// kErr M.  A face decided by face_d2n therefore has its FP32 distance within
-// kErr M of the reference's FP64 distance; a face without a usable normal
-// (its FP64 normal not accurate to well below u: no area, or a corner angle
-// with sin below 1e-6), or whose projection falls within the rounding band
-// of an edge line, enters the candidates by a lower bound and leaves the
-// decision to FP64.  The same bound serves as the band of the FP32 threshold
-// tests (2 tau, the plane side, tau), and kNormalBand (on the cosine) as
-// that of the normal test, whose FP32 error is a few u.
+// translation and the mesh, at least 2 tau.  A decided FP32 distance (flat_d2,
+// face_d2n) is within 64 u M of the reference's FP64 distance whatever the
+// face's shape, far inside kErr M; a face without a usable normal (its FP64
+// normal not accurate to well below u: no area, or a corner angle with sin
+// below 1e-6), or one that face_d2n leaves undecided (a projection within the
+// rounding band of an edge line), enters the candidates by a lower bound and
+// leaves the decision to FP64.  The same bound serves as the band of the FP32
+// threshold tests (2 tau, the plane side, tau), and kNormalBand (on the cosine)
+// as that of the normal test, whose FP32 error is a few u.
 constexpr float kErr = 1.0f / 32768.0f;
 constexpr float kNormalBand = 1.0f / 1024.0f;
 constexpr int kCandidates = 16;
@@ -434,9 +429,7 @@ __device__ __forceinline__ int flat_region(F3 p, const FlatFace &f, float &d2) {
 // in FP32 than the best FP32 face.  Nodes are pruned with a slightly larger
 // radius, for the rounding of their boxes' distances.  The search's window is
 // generous; the faces returned are held to the error of a decided distance
-// itself: 30 u M for the image, 2 u M for the corners, 14 u M for the normal and
-// the rounding of the products, 64 u M taken, so 128 u M from the best (with
-// the search's window, 1,024 u M, eight times as many queries found
+// itself, 64 u M, so 128 u M from the best (with the search's window, 1,024 u M, eight times as many queries found
 // neighbouring faces in it that disagree on the normal test, and went to
 // FP64).  Undecided faces are listed as ~face.  Returns the count (N + 1 on
 // overflow: faces and keys hold N entries); `best` receives the smallest FP32
