@@ -254,7 +254,9 @@ namespace {
 // above the best by more than the errors of both; children are ordered in FP32
 // only when their distances differ by more; the rest goes to FP64, which runs at
 // 1/64 of the rate.  (16 boxes and some 30 faces per query were FP64: 8.7 ms for 8
-// clusters of the 128 x 128 height field, 2.0 ms now.)
+// clusters of the 128 x 128 height field, 1.8 ms now; 2.0 when each face within
+// reach went to FP64 in turn, without a look at the rest of its leaf.)
+constexpr int kLeafFaces = 8;
 __device__ double nearest_face_f(const Surface &s, const float4 *face32, const float4 *boxes32,
                                  float um, D3 p, double limit, int32_t &face, int *status) {
   double best = limit;
@@ -282,17 +284,32 @@ __device__ double nearest_face_f(const Surface &s, const float4 *face32, const f
     if ((at.d < 0.f || !(at.d <= reach - 128.f * um - 4e-6f * reach)) && box_d2(p, n) > best) continue;
     const int32_t left = n.left;
     if (left < 0) {
+      // FP32 distances (or lower bounds) of up to kLeafFaces of the leaf's faces at
+      // a time; those that another of them beats by more than the errors are out
+      // as well: in order they could be the best only until that one's turn
       const int32_t end = n.end;
-      for (int32_t i = n.begin; i < end; ++i) {
-        const int32_t f = s.ids[i];
-        const Face r = load_face(face32, f);
-        if (r.reach != 0.f) {
-          float d2;
-          face_d2n(pf, r, um, reach2, d2);
-          if (d2 > reach2) continue;
+      for (int32_t i0 = n.begin; i0 < end; i0 += kLeafFaces) {
+        float d2[kLeafFaces], least = INFINITY;
+#pragma unroll
+        for (int k = 0; k < kLeafFaces; ++k) {
+          d2[k] = INFINITY;
+          if (i0 + k >= end) continue;
+          const Face r = load_face(face32, s.ids[i0 + k]);
+          d2[k] = 0.f;
+          if (r.reach != 0.f && face_d2n(pf, r, um, reach2, d2[k])) least = fminf(least, d2[k]);
         }
-        const double d = triangle_d2(p, corner(s, f, 0), corner(s, f, 1), corner(s, f, 2));
-        if (d < best) best = d, face = f, bound();
+        float within2 = reach2;
+        if (least > 1e-30f && least < 1e30f) {
+          const float within = sqrtf(least) * (1.f + 2e-6f) + 128.f * um;
+          within2 = fminf(reach2, within * within);
+        }
+#pragma unroll
+        for (int k = 0; k < kLeafFaces; ++k) {
+          if (i0 + k >= end || d2[k] > within2 || d2[k] > reach2) continue;
+          const int32_t f = s.ids[i0 + k];
+          const double d = triangle_d2(p, corner(s, f, 0), corner(s, f, 1), corner(s, f, 2));
+          if (d < best) best = d, face = f, bound();
+        }
       }
     } else {
       const int32_t right = n.right;
@@ -319,7 +336,8 @@ __device__ double nearest_face_f(const Surface &s, const float4 *face32, const f
 // Query (c, direction, j) takes vertex i = order[j], the vertices in Morton
 // order of their position, so a warp walks neighbouring vertices through
 // nearly the same BVH nodes; flags and errors stay per vertex (row).
-__global__ void verify_vertices(Surface s, const float4 *face32, const float4 *boxes32, float scale,
+__global__ void __launch_bounds__(kThreads, 3)
+    verify_vertices(Surface s, const float4 *face32, const float4 *boxes32, float scale,
                                 const double *vn, const int32_t *order,
                                 const ClusterMotion *clusters, uint64_t nc, double tau,
                                 double limit, uint8_t *flags, double *err, int *status) {
