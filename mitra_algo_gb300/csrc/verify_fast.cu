@@ -873,9 +873,10 @@ __device__ __forceinline__ void block_distances(RowBlock &sh, const BvhView &b, 
 
 // The reference's FP64 squared distance of each listed forward row: the
 // smallest over its candidate faces (the face it keeps is among them).
-// 3.3e6 rows of the 180,000-vertex torus: 1.6 ms; a lane per row that evaluated
+// 3.3e6 rows of the 180,000-vertex torus: 1.4 ms (1.6 with two CTAs per SM in
+// place of four); a lane per row that evaluated
 // every candidate took 2.9.
-__global__ void __launch_bounds__(kRowThreads) forward_errors(BvhView b, Surface s, const ClusterMotion *motions,
+__global__ void __launch_bounds__(kRowThreads, 4) forward_errors(BvhView b, Surface s, const ClusterMotion *motions,
                                                               RowLists lists, unsigned long long count,
                                                               float scale, float tau, double *err) {
   __shared__ RowBlock sh;
@@ -963,10 +964,12 @@ __device__ __forceinline__ bool decide_row(const BvhView &b, const RefBvh &t, co
 // without candidates, are left in lists.open for verify_rows_open, from its two
 // ends: the searches of the latter take much longer.  Rows whose candidates
 // overflowed stay marked for verify_rows_wide.  On the 1e6-triangle torus 1.1e7
-// rows take 4.3 ms and the 3.3e6 left to the second kernel 3.4 (4.2 with a lane per
-// row that evaluates its open faces in turn); eight lanes per
-// row, each with its own copy of the image, took 17 and 11.
-__global__ void verify_rows_fp64(BvhView b, Surface s, RefBvh t, const double *vn, const float *vn32,
+// rows take 3.0 ms and the 3.3e6 left to the second kernel 2.8 (4.2 with a lane per
+// row that evaluates its open faces in turn); eight lanes per row, each with its
+// own copy of the image, took 17 and 11.  Both wait for the faces' records as much
+// as for FP64, so the launch bounds leave room for four and three CTAs per SM (two
+// each: 4.3 and 3.4 ms).
+__global__ void __launch_bounds__(kThreads, 4) verify_rows_fp64(BvhView b, Surface s, RefBvh t, const double *vn, const float *vn32,
                                  const ClusterMotion *motions, const MotionF *motions32, double tau,
                                  float scale, uint8_t *flags, double *err, RowLists lists,
                                  unsigned long long rows) {
@@ -1018,7 +1021,7 @@ __global__ void verify_rows_fp64(BvhView b, Surface s, RefBvh t, const double *v
 
 // The rows verify_rows_fp64 left: those that search (whole blocks of them, on one
 // lane each), then those with candidates.
-__global__ void __launch_bounds__(kRowThreads) verify_rows_open(
+__global__ void __launch_bounds__(kRowThreads, 3) verify_rows_open(
     BvhView b, Surface s, RefBvh t, const double *vn, const float *vn32, const ClusterMotion *motions,
     const MotionF *motions32, double tau, float scale, uint8_t *flags, double *err, RowLists lists,
     int *status) {
