@@ -1,6 +1,6 @@
 """The FP64 decisions of the resident verification where most of them are
 made: images at, next to and between the corners of faces, around vertices of
-4 to 17 faces (the lists hold 16, eight lanes take two each) whose normals
+4 to 17 faces (the lists hold 16) whose normals
 disagree, at three scales.  Everything must equal sym_verification bit for
 bit, as in tests/test_gpu_verify_resident.py."""
 import numpy as np
