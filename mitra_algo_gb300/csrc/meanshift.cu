@@ -11,21 +11,26 @@
 // reference evaluator only reads the seed descriptor and the vote set), so:
 //   1. one launch runs the trajectory of EVERY vote as a seed, a warp per
 //      seed, and records its final mean, its converged/exhausted flags and
-//      per same-kind vote the iterations that counted it (its support);
+//      its support (the same-kind votes that some iteration counted);
 //   2. the host replays the reference's host loop verbatim (RNG draw per seed,
 //      visited set, merge test, budgets) on those results - no device round
 //      trip per trajectory;
-//   3. the hits of the trajectories the host loop used are added up per
-//      cluster, and each vote takes the cluster with the most (the first
-//      cluster on ties).
+//   3. the hits (iterations that counted a vote) of the trajectories the host
+//      loop used are added up per cluster, and each vote takes the cluster with
+//      the most (the first cluster on ties).
 // Distances, weights and products are the reference's FP64 expressions (no
 // FMA contraction), and the weighted sums add the members' contributions in
 // vote order, as the reference's serial loop does: each lane evaluates one
-// vote of a group of 32, then a lane per sum adds the members' values in order.  The means are therefore the reference's bit
-// for bit, and so is every decision that depends on them (d^2 < h^2, the
-// stop test, the merge test): no rounding band exists to be checked.
-// Memory: seeds run in batches whose hit counts fit a fixed device budget (the
-// supports are kept as sparse lists), and so do the clusters' hit counts.
+// vote of a group of 32, then a lane per sum adds the members' values in
+// order.  The means are therefore the reference's bit for bit, and so is every
+// decision that depends on them (d^2 < h^2, the stop test, the merge test): no
+// rounding band exists to be checked.
+// Memory: every device array whose size grows with the square of the votes or
+// with the supports fits kBatchBytes.  Where a row of hit counts for every seed
+// of a kind does, step 1 writes those, and step 3 adds the used ones; above
+// that (16,384 votes of a kind) step 1 writes rows of bits, batch by batch, and
+// step 3 runs the used trajectories again.  The supports go to the host as lists,
+// piece by piece, and the clusters' hit counts are made batch by batch.
 #include "common.cuh"
 #include "primitives.cuh"
 #include "rng.hpp"
@@ -57,9 +62,10 @@ __global__ void round_desc(const double *desc, uint64_t n, float *out) {
   for (int k = 0; k < D; ++k) out[uint64_t(k) * n + j] = float(desc[j * D + k]);
 }
 
-// The trajectory of every vote of [first, first + nseeds) as a seed, a warp
-// each; counts[s * n + j] += the iterations in which vote j was within the
-// bandwidth (the support is where it is not 0).
+// Trajectories, a warp each: the i-th from vote seeds[i] (or first + i), into
+// row rows[i] (or i) of `out`, `pitch` words apart.  BITS: bit j of the row is
+// set when some iteration had vote j within the bandwidth; else word j of the row
+// gains the number of iterations that had.  final_mean and flags may be null.
 //
 // Culling: `lanes32` holds the descriptors rounded to FP32 and `reach` the
 // bandwidth plus a bound on how far an FP32 distance can fall below the FP64
@@ -80,10 +86,11 @@ __global__ void round_desc(const double *desc, uint64_t n, float *out) {
 // (8,900 votes of the mirrored 128 x 128 height field, 1,500 of them planes:
 // trajectories and counts 15.7 ms, 1.0 ms now.)
 constexpr int kListed = 1024, kTrajWarps = 4;
-template <int D>
+template <int D, bool BITS>
 __global__ void __launch_bounds__(32 * kTrajWarps) trajectories(
-    const double *desc, const float *lanes32, float reach, float slack, uint64_t n, uint64_t first,
-    uint64_t nseeds, double h2, int max_iter, double *final_mean, uint8_t *flags, uint32_t *counts) {
+    const double *desc, const float *lanes32, float reach, float slack, uint64_t n, const int32_t *seeds,
+    uint64_t first, const int32_t *rows, uint64_t nseeds, double h2, int max_iter, double *final_mean,
+    uint8_t *flags, uint32_t *out, uint64_t pitch) {
   __shared__ uint32_t list_s[kTrajWarps][kListed];
   __shared__ uint32_t near_s[kTrajWarps][64];
   __shared__ double term_s[kTrajWarps][32 * (D + 1)];
@@ -92,10 +99,11 @@ __global__ void __launch_bounds__(32 * kTrajWarps) trajectories(
   if (si >= nseeds) return;
   uint32_t *list = list_s[warp], *near = near_s[warp];
   double *term = term_s[warp];
-  uint32_t *row = counts + si * n;
+  const uint64_t from = seeds ? uint64_t(seeds[si]) : first + si;
+  uint32_t *row = out + (rows ? uint64_t(rows[si]) : si) * pitch;
   double mean[D];  // the same in every lane, as `converged` and `exhausted`
   float mean32[D], listed32[D];
-  for (int k = 0; k < D; ++k) mean[k] = desc[(first + si) * D + k], listed32[k] = INFINITY;
+  for (int k = 0; k < D; ++k) mean[k] = desc[from * D + k], listed32[k] = INFINITY;
   bool converged = false, exhausted = false;
   const double stop = 1e-6 * h2;
   const float reach2 = reach * reach, wide = (reach + slack) * (1 + 1e-5f), wide2 = wide * wide;
@@ -159,10 +167,15 @@ __global__ void __launch_bounds__(32 * kTrajWarps) trajectories(
           const double w = 1 - dist / h2;
           term[lane * (D + 1)] = w;
           for (int k = 0; k < D; ++k) term[lane * (D + 1) + 1 + k] = w * x[k];
-          atomicAdd(&row[j], 1u);
+          if (!BITS) atomicAdd(&row[j], 1u);
         }
       }
       const unsigned bits = __ballot_sync(0xffffffffu, in);
+      if (BITS && in) {  // the lanes of one word set it together
+        const unsigned peers = __match_any_sync(bits, uint32_t(j >> 5));
+        const uint32_t set = __reduce_or_sync(peers, 1u << (j & 31));
+        if (lane == __ffs(int(peers)) - 1) atomicOr(&row[j >> 5], set);
+      }
       __syncwarp();
       for (unsigned m = bits; m; m &= m - 1)  // in vote order
         if (lane <= D) sum += term[(__ffs(int(m)) - 1) * (D + 1) + lane];
@@ -211,59 +224,79 @@ __global__ void __launch_bounds__(32 * kTrajWarps) trajectories(
       break;
     }
   }
-  if (lane == 0) {
+  if (lane == 0 && final_mean) {
     for (int k = 0; k < D; ++k) final_mean[si * D + k] = mean[k];
     flags[si] = uint8_t((converged ? 1 : 0) | (exhausted ? 2 : 0));
   }
 }
 
-// Row s of the counts as a list: the votes with hits, ascending, and their
-// hits; a warp per row.  size[s] (entries null) or entries[off[s] ..].
-__global__ void list_hits(const uint32_t *counts, uint64_t n, uint64_t nseeds, uint64_t *size,
-                          const uint64_t *off, uint2 *entries) {
+// Row s of the supports (bits, or hit counts) as a list: the votes in it,
+// ascending; a warp per row.  size[s] (members null), or members[off[s] - off[0]
+// ..].
+template <bool BITS>
+__global__ void list_support(const uint32_t *rows, uint64_t pitch, uint64_t n, uint64_t nseeds,
+                             uint64_t *size, const uint64_t *off, uint32_t *members) {
   const uint64_t s = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (s >= nseeds) return;
-  uint64_t at = entries ? off[s] : 0;
-  for (uint64_t base = 0; base < n; base += 32) {
-    const uint64_t j = base + lane;
-    const uint32_t hits = j < n ? counts[s * n + j] : 0u;
-    const unsigned bits = __ballot_sync(0xffffffffu, hits != 0);
-    if (entries && hits) entries[at + __popc(bits & ((1u << lane) - 1u))] = make_uint2(uint32_t(j), hits);
-    at += __popc(bits);
+  const uint32_t *row = rows + s * pitch;
+  uint64_t at = members ? off[s] - off[0] : 0;
+  if (BITS) {
+    for (uint64_t base = 0; base < pitch; base += 32) {
+      uint32_t word = base + lane < pitch ? row[base + lane] : 0u;
+      const uint32_t mine = __popc(word);
+      uint32_t incl = mine;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      if (members)
+        for (uint64_t to = at + incl - mine; word; word &= word - 1)
+          members[to++] = uint32_t((base + lane) * 32) + __ffs(int(word)) - 1;
+      at += __shfl_sync(0xffffffffu, incl, 31);
+    }
+  } else {
+    for (uint64_t base = 0; base < n; base += 32) {
+      const uint64_t j = base + lane;
+      const bool in = j < n && row[j];
+      const unsigned bits = __ballot_sync(0xffffffffu, in);
+      if (members && in) members[at + __popc(bits & ((1u << lane) - 1u))] = uint32_t(j);
+      at += __popc(bits);
+    }
   }
-  if (!entries && lane == 0) size[s] = at;
+  if (!members && lane == 0) size[s] = at;
 }
 
-// The used seeds' hits added up per cluster (PICK = false), then per vote the
-// cluster with the most, the earliest on ties (PICK): best[j] = the count, then
-// the complement of the cluster's id, so a plain maximum decides.
-template <bool PICK>
-__global__ void cluster_hits(const uint2 *used, uint64_t nused, const uint64_t *off,
-                             const uint2 *entries, const int32_t *cluster_id, uint64_t n,
-                             uint32_t *counts, unsigned long long *best) {
-  const uint64_t i = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  if (i >= nused) return;
-  const uint32_t s = used[i].x, c = used[i].y;  // seed of the batch, cluster of the batch
-  for (uint64_t e = off[s] + (threadIdx.x & 31); e < off[s + 1]; e += 32) {
-    const uint2 x = entries[e];
-    uint32_t *sum = &counts[uint64_t(c) * n + x.x];
-    if (!PICK) atomicAdd(sum, x.y);
-    else atomicMax(&best[x.x], (unsigned long long)*sum << 32 | (0xffffffffu - uint32_t(cluster_id[c])));
-  }
+// counts[cluster[i] * n ..] += the hit counts of seed seeds[i]; a block each.
+__global__ void add_hits(const uint32_t *rows, uint64_t n, const int32_t *seeds, const int32_t *cluster,
+                         uint32_t *counts) {
+  const uint32_t *row = rows + uint64_t(seeds[blockIdx.x]) * n;
+  uint32_t *sum = counts + uint64_t(cluster[blockIdx.x]) * n;
+  for (uint64_t j = threadIdx.x; j < n; j += blockDim.x)
+    if (const uint32_t hits = row[j]) atomicAdd(&sum[j], hits);
 }
 
-// Device bytes for one batch of seeds' hit counts, and for one batch of
-// clusters'.
+// Per vote the cluster with the most hits among kPick of a batch's, the earliest
+// on ties: best[j] = the count, then the complement of the cluster's id, so a
+// plain maximum decides over all of them.
+constexpr int kPick = 64;
+__global__ void pick_cluster(const uint32_t *counts, uint64_t nclusters, uint64_t n,
+                             const int32_t *cluster_id, unsigned long long *best) {
+  const uint64_t j = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (j >= n) return;
+  const uint64_t c0 = uint64_t(blockIdx.y) * kPick, c1 = c0 + kPick < nclusters ? c0 + kPick : nclusters;
+  unsigned long long most = 0;
+  for (uint64_t c = c0; c < c1; ++c)
+    if (const uint32_t hits = counts[c * n + j]) {
+      const unsigned long long x = (unsigned long long)hits << 32 | (0xffffffffu - uint32_t(cluster_id[c]));
+      most = x > most ? x : most;
+    }
+  if (most) atomicMax(&best[j], most);
+}
+
+// Device bytes of one batch of seeds' rows, of a piece of their lists, and of one
+// batch of clusters' hit counts.
 constexpr uint64_t kBatchBytes = uint64_t(1) << 30;
-
-// A batch of seeds' supports on the device: off[s] .. off[s + 1] of entries
-// (vote, hits).
-struct SeedBatch {
-  uint64_t first = 0, count = 0;
-  const uint64_t *off = nullptr;
-  const uint2 *entries = nullptr;
-};
 
 struct KindData {
   int dim = 0;
@@ -275,49 +308,65 @@ struct KindData {
   std::vector<double> mean;          // n x dim final means
   std::vector<uint8_t> flags;        // bit0 converged, bit1 exhausted
   std::vector<uint64_t> sup_off;     // n + 1: each seed's support (kind-local
-  std::vector<uint2> sup;            //   member ids, ascending, and their hits)
-  std::vector<SeedBatch> batches;
+  std::vector<uint32_t> sup;         //   member ids, ascending)
+  uint32_t *hits = nullptr;          // device: every seed's hit counts (n x n), where they fit
 };
+
+float slack_of(double h2) { return float(0.5 * std::sqrt(h2)); }
 
 template <int D>
 void run_all_seeds(Call &call, KindData &k, double h2, int max_iter) {
   if (!k.n) return;
   cudaStream_t st = call.stream();
-  const uint64_t batch = std::max<uint64_t>(1, std::min<uint64_t>(k.n, kBatchBytes / (k.n * 4)));
+  const bool counted = k.n * k.n * 4 <= kBatchBytes;
+  const uint64_t pitch = counted ? k.n : (k.n + 31) / 32;
+  const uint64_t batch = std::max<uint64_t>(1, std::min<uint64_t>(k.n, kBatchBytes / (pitch * 4)));
+  if (counted) k.hits = call.alloc<uint32_t>(k.n * k.n);
+  const Arena::Mark kept = call.ctx->arena.mark();  // the rest is given back
+  uint32_t *rows = counted ? k.hits : call.alloc<uint32_t>(batch * pitch);
   double *mean = call.alloc<double>(batch * D);
   uint8_t *flags = call.alloc<uint8_t>(batch);
-  uint32_t *counts = call.alloc<uint32_t>(batch * k.n);
-  uint64_t *size = call.alloc<uint64_t>(batch);
+  uint64_t *size = call.alloc<uint64_t>(batch), *off = call.alloc<uint64_t>(batch + 1);
   k.mean.resize(k.n * D);
   k.flags.resize(k.n);
   k.sup_off.assign(1, 0);
   k.sup.clear();
+  const auto run = counted ? trajectories<D, false> : trajectories<D, true>;
+  const auto list = counted ? list_support<false> : list_support<true>;
+  std::vector<uint64_t> hoff(batch + 1);
   for (uint64_t first = 0; first < k.n; first += batch) {
+    const Arena::Mark before = call.ctx->arena.mark();
     const uint64_t cnt = std::min(batch, k.n - first);
-    SYM_CUDA(cudaMemsetAsync(counts, 0, cnt * k.n * 4, st));
-    trajectories<D><<<blocks_for(cnt, kTrajWarps), 32 * kTrajWarps, 0, st>>>(
-        k.desc, k.lanes32, k.reach, float(0.5 * std::sqrt(h2)), k.n, first, cnt, h2, max_iter, mean,
-        flags, counts);
+    SYM_CUDA(cudaMemsetAsync(rows, 0, cnt * pitch * 4, st));
+    run<<<blocks_for(cnt, kTrajWarps), 32 * kTrajWarps, 0, st>>>(k.desc, k.lanes32, k.reach, slack_of(h2), k.n,
+                                                                 nullptr, first, nullptr, cnt, h2, max_iter,
+                                                                 mean, flags, rows, pitch);
     check_launch();
-    uint64_t *off = call.alloc<uint64_t>(cnt + 1);
-    list_hits<<<blocks_for(cnt * 32), kThreads, 0, st>>>(counts, k.n, cnt, size, nullptr, nullptr);
+    list<<<blocks_for(cnt * 32), kThreads, 0, st>>>(rows, pitch, k.n, cnt, size, nullptr, nullptr);
     check_launch();
     exclusive_scan(call, size, off, cnt);
-    std::vector<uint64_t> hoff(cnt + 1);
     call.d2h(hoff.data(), off, (cnt + 1) * 8);
     call.d2h(k.mean.data() + first * D, mean, cnt * D * 8);
     call.d2h(k.flags.data() + first, flags, cnt);
     call.sync();
-    const uint64_t total = hoff[cnt], at = k.sup.size();
-    uint2 *entries = call.alloc<uint2>(total);
-    list_hits<<<blocks_for(cnt * 32), kThreads, 0, st>>>(counts, k.n, cnt, nullptr, off, entries);
-    check_launch();
-    call.launched(3);
-    k.sup.resize(at + total);
-    call.d2h(k.sup.data() + at, entries, total * sizeof(uint2));
+    call.launched(2);
+    const uint64_t at = k.sup.size(), room = std::min(hoff[cnt], std::max(kBatchBytes / 4, k.n));
+    uint32_t *members = call.alloc<uint32_t>(room);
+    k.sup.resize(at + hoff[cnt]);
     for (uint64_t s = 0; s < cnt; ++s) k.sup_off.push_back(at + hoff[s + 1]);
-    k.batches.push_back({first, cnt, off, entries});
+    for (uint64_t s0 = 0, s1; s0 < cnt; s0 = s1) {  // as many rows as fit the piece; one always does
+      s1 = uint64_t(std::upper_bound(hoff.begin() + s0, hoff.begin() + cnt + 1, hoff[s0] + room) - hoff.begin()) - 1;
+      if (hoff[s1] == hoff[s0]) continue;
+      list<<<blocks_for((s1 - s0) * 32), kThreads, 0, st>>>(rows + s0 * pitch, pitch, k.n, s1 - s0, nullptr,
+                                                            off + s0, members);
+      check_launch();
+      call.launched();
+      call.d2h(k.sup.data() + at + hoff[s0], members, (hoff[s1] - hoff[s0]) * 4);
+    }
+    call.sync();
+    call.ctx->arena.rewind(before);
   }
+  call.ctx->arena.rewind(kept);
 }
 
 struct Center {
@@ -328,8 +377,9 @@ struct Center {
   std::vector<int32_t> seeds;  // kind-local seeds merged into this cluster
 };
 
+template <int D>
 void count_members(Call &call, const KindData &k, const std::vector<Center> &centers, int kind_index,
-                   std::vector<int32_t> &winner_global) {
+                   double h2, int max_iter, std::vector<int32_t> &winner_global) {
   std::vector<int32_t> cluster_ids;
   for (size_t c = 0; c < centers.size(); ++c)
     if (centers[c].kind == kind_index) cluster_ids.push_back(int32_t(c));
@@ -337,38 +387,39 @@ void count_members(Call &call, const KindData &k, const std::vector<Center> &cen
   cudaStream_t st = call.stream();
   const uint64_t batch = std::max<uint64_t>(1, std::min<uint64_t>(cluster_ids.size(),
                                                                    kBatchBytes / (k.n * 4)));
+  const Arena::Mark before = call.ctx->arena.mark();
   uint32_t *counts = call.alloc<uint32_t>(batch * k.n);
   unsigned long long *best = call.alloc<unsigned long long>(k.n);
+  int32_t *dids = call.upload(cluster_ids.data(), cluster_ids.size());
   SYM_CUDA(cudaMemsetAsync(best, 0, k.n * 8, st));
-  std::vector<std::vector<uint2>> used(k.batches.size());  // kept until the copies are done
+  std::vector<int32_t> seeds, cluster;  // kept until the copies are done
   for (uint64_t first = 0; first < cluster_ids.size(); first += batch) {
+    const Arena::Mark per_batch = call.ctx->arena.mark();
     const uint64_t nc = std::min<uint64_t>(batch, cluster_ids.size() - first);
     if (first) call.sync();
-    for (auto &u : used) u.clear();
+    seeds.clear(), cluster.clear();
     for (uint64_t c = 0; c < nc; ++c)
-      for (int32_t s : centers[cluster_ids[first + c]].seeds) {
-        const uint64_t b = uint64_t(s) / k.batches[0].count;
-        used[b].push_back(make_uint2(uint32_t(uint64_t(s) - k.batches[b].first), uint32_t(c)));
-      }
+      for (int32_t s : centers[cluster_ids[first + c]].seeds) seeds.push_back(s), cluster.push_back(int32_t(c));
     SYM_CUDA(cudaMemsetAsync(counts, 0, nc * k.n * 4, st));
-    const int32_t *dids = call.upload(cluster_ids.data() + first, nc);
-    std::vector<const uint2 *> dused(used.size(), nullptr);
-    for (size_t b = 0; b < used.size(); ++b)
-      if (!used[b].empty()) dused[b] = call.upload(used[b].data(), used[b].size());
-    for (int pick = 0; pick < 2; ++pick)
-      for (size_t b = 0; b < used.size(); ++b) {
-        if (used[b].empty()) continue;
-        const uint64_t m = used[b].size();
-        const auto kernel = pick ? cluster_hits<true> : cluster_hits<false>;
-        kernel<<<blocks_for(m * 32), kThreads, 0, st>>>(dused[b], m, k.batches[b].off,
-                                                        k.batches[b].entries, dids, k.n, counts, best);
-        check_launch();
-        call.launched();
-      }
+    const int32_t *dseeds = call.upload(seeds.data(), seeds.size());
+    const int32_t *dcluster = call.upload(cluster.data(), cluster.size());
+    if (k.hits)
+      add_hits<<<unsigned(seeds.size()), kThreads, 0, st>>>(k.hits, k.n, dseeds, dcluster, counts);
+    else
+      trajectories<D, false><<<blocks_for(seeds.size(), kTrajWarps), 32 * kTrajWarps, 0, st>>>(
+          k.desc, k.lanes32, k.reach, slack_of(h2), k.n, dseeds, 0, dcluster, seeds.size(), h2, max_iter,
+          nullptr, nullptr, counts, k.n);
+    check_launch();
+    pick_cluster<<<dim3(blocks_for(k.n), blocks_for(nc, kPick)), kThreads, 0, st>>>(counts, nc, k.n, dids + first,
+                                                                                    best);
+    check_launch();
+    call.launched(2);
+    call.ctx->arena.rewind(per_batch);
   }
   std::vector<unsigned long long> local(k.n);
   call.d2h(local.data(), best, k.n * 8);
   call.sync();
+  call.ctx->arena.rewind(before);
   for (uint64_t j = 0; j < k.n; ++j)
     winner_global[k.ids[j]] = local[j] >> 32 ? int32_t(0xffffffffu - uint32_t(local[j])) : -1;
 }
@@ -549,9 +600,9 @@ void clustering_host(Call &call, const sym_votes_view &votes, const sym_model_co
     int t = kind_of[seed];
     KindData &k = kinds[t];
     uint64_t s = uint64_t(local_of[seed]);
-    const uint2 *members = k.sup.data() + k.sup_off[s];
+    const uint32_t *members = k.sup.data() + k.sup_off[s];
     const uint64_t size = k.sup_off[s + 1] - k.sup_off[s];
-    for (uint64_t m = 0; m < size; ++m) visit(uint64_t(k.ids[members[m].x]));
+    for (uint64_t m = 0; m < size; ++m) visit(uint64_t(k.ids[members[m]]));
     bool converged = k.flags[s] & 1, exhausted = k.flags[s] & 2;
     if (exhausted) visit(seed);
     if (!converged) ++limited;
@@ -562,8 +613,8 @@ void clustering_host(Call &call, const sym_votes_view &votes, const sym_model_co
     auto add_keys = [&](Center &c, uint64_t seed_of) {  // a support's members into the union
       uint64_t added = 0;
       for (uint64_t m = k.sup_off[seed_of]; m < k.sup_off[seed_of + 1]; ++m) {
-        uint64_t &w = c.keys[k.sup[m].x >> 6];
-        const uint64_t bit = uint64_t(1) << (k.sup[m].x & 63);
+        uint64_t &w = c.keys[k.sup[m] >> 6];
+        const uint64_t bit = uint64_t(1) << (k.sup[m] & 63);
         if (!(w & bit)) w |= bit, ++added;
       }
       return added;
@@ -603,8 +654,8 @@ void clustering_host(Call &call, const sym_votes_view &votes, const sym_model_co
 
   // ---- support counts and winners (clustering.cpp:97-108) on the GPU
   std::vector<int32_t> winner(q, -1);
-  count_members(call, kinds[0], centers, 0, winner);
-  count_members(call, kinds[1], centers, 1, winner);
+  count_members<4>(call, kinds[0], centers, 0, h2, o.max_iterations, winner);
+  count_members<12>(call, kinds[1], centers, 1, h2, o.max_iterations, winner);
   std::vector<std::vector<int32_t>> members(centers.size());
   for (uint64_t i = 0; i < q; ++i)
     if (winner[i] >= 0) members[winner[i]].push_back(int32_t(i));
