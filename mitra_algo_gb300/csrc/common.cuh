@@ -100,6 +100,9 @@ struct sym_context {
   int *host_status = nullptr;   // pinned host mirror for cheap reads
   sym::Metrics metrics;
   cudaDeviceProp prop{};
+  // kernels this context has asked to take more than 48 KB of dynamic shared
+  // memory (Call::allow_shared)
+  std::vector<const void *> large_shared;
   // contexts of the same device this one runs independent per-mesh work on
   // (the fused batch's modes and verification), created on first use
   std::vector<sym_context *> helpers;
@@ -124,6 +127,13 @@ public:
     if (n) h2d(d, src, n * sizeof(T));
     return d;
   }
+  // Lets `kernel` be launched with `bytes` of dynamic shared memory (always the
+  // same for a kernel).  The limit belongs to the current device, so every
+  // context asks for its own, once.
+  template <class... P> void allow_shared(void (*kernel)(P...), size_t bytes) {
+    allow_shared(reinterpret_cast<const void *>(kernel), bytes);
+  }
+  void allow_shared(const void *kernel, size_t bytes);
   void launched(int n = 1) { ctx->metrics.current.custom_launches += n; }
   void sync();
   // Synchronises and turns a nonzero device status word into an Error.

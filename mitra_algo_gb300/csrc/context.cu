@@ -90,6 +90,14 @@ void Call::d2h(void *dst, const void *src, size_t bytes) {
   ctx->metrics.current.d2h_bytes += bytes;
 }
 
+void Call::allow_shared(const void *kernel, size_t bytes) {
+  auto &done = ctx->large_shared;
+  if (std::find(done.begin(), done.end(), kernel) != done.end()) return;
+  cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)),
+             "shared memory limit");
+  done.push_back(kernel);
+}
+
 void Call::sync() { cuda_check(cudaStreamSynchronize(ctx->stream), "stream sync"); }
 
 void Call::check_status(const char *stage) {

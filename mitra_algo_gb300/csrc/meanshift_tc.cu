@@ -1108,12 +1108,7 @@ bool meanshift_bf16_bulk(Call &call, const VoteSet &v, float *means, uint8_t *st
   const uint64_t max_tiles = (k + kChunk - 1) / kChunk;
   if (max_tiles * v.nchunks >= (uint64_t(1) << 31)) return false;  // list entries are int32
   cudaStream_t st = call.stream();
-  // once per process (thread-safe: calls from several host threads may race)
-  static const bool configured = [] {
-    SYM_CUDA(cudaFuncSetAttribute(ms_tile_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
-    return true;
-  }();
-  (void)configured;
+  call.allow_shared(ms_tile_tc, kTcSmem);
   uint8_t *images = call.alloc<uint8_t>(v.nchunks * kImage);
   build_images<<<unsigned(v.nchunks), kChunk, 0, st>>>(v.desc, v.q, v.nchunks, v.cbox, v.gbox,
                                                        float(1.0 / std::sqrt(h2)), images);
@@ -1225,12 +1220,7 @@ void wait_selftest_host(Call &call, uint64_t limit_ns) {
 
 void tc_selftest_host(Call &call, const uint16_t *a1, const uint16_t *b1, const uint16_t *a2,
                       const uint16_t *b2, float *d_out, float *acc_out) {
-  static const bool configured = [] {
-    SYM_CUDA(cudaFuncSetAttribute(tc_selftest, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  kSmemRequest));
-    return true;
-  }();
-  (void)configured;
+  call.allow_shared(tc_selftest, kSmemRequest);
   auto up = [&](const uint16_t *p, size_t n) {
     return reinterpret_cast<const __nv_bfloat16 *>(call.upload(p, n));
   };

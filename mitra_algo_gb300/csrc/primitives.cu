@@ -314,11 +314,7 @@ template <int ITEMS>
 void launch_sort_block(Call &call, const uint64_t *keys, const int32_t *values, uint64_t *keys_out,
                        int32_t *values_out, uint64_t n, int begin_bit, int end_bit) {
   constexpr size_t smem = size_t(1024) * ITEMS * 12 + (32 + 1) * 256 * sizeof(unsigned);
-  static const bool configured = [] {
-    SYM_CUDA(cudaFuncSetAttribute(sort_block<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    return true;
-  }();
-  (void)configured;
+  call.allow_shared(sort_block<ITEMS>, smem);
   launch_chained(call.stream(), sort_block<ITEMS>, 1, 1024, smem, keys, values, unsigned(n), begin_bit, end_bit,
                  keys_out, values_out);
   call.launched();
