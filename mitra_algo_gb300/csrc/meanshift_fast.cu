@@ -345,7 +345,7 @@ constexpr int kPairStride = 20, kRunValues = kSubVotes / 2 * kPairStride;
 template <typename T, bool COUNT, bool NEWTON, bool GAUSS>
 __global__ void __launch_bounds__(kChunk, sizeof(T) == 4 ? 8 : 2)
     ms_tile(const T *desc, const float *sbox, uint32_t nchunks, uint64_t q, const T *means,
-            const uint8_t *state, const int32_t *ids, const unsigned *nact, T h2, T gk, float skip_gap2,
+            const uint8_t *state, const int32_t *ids, const unsigned *nact, T h2, Window<T> win, T gk, float skip_gap2,
             const Grid *plan, uint32_t *touched, const uint32_t *bits, uint32_t bwords, const uint2 *items,
             uint32_t room, uint32_t *work, T *partial, unsigned long long *counts, unsigned long long *evals) {
   chained();
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(kChunk, sizeof(T) == 4 ? 8 : 2)
   for (int k = 0; k < kQueues; ++k)
     queue_end[k] = (k ? queue_end[k - 1] : 0u) + (items ? work[kWorkQueue + k] : 0u);
   T *const ns = nsum + threadIdx.x;
-  const T rcp = reciprocal(h2), floor_w = GAUSS ? exp2(-gk) : T(0);
+  const T floor_w = GAUSS ? exp2(-gk) : T(0);
   for (;;) {
     uint32_t tile = blockIdx.x % uint32_t(grid.tiles), split = blockIdx.x / uint32_t(grid.tiles), quarter = warp;
     if (items) {
@@ -461,7 +461,7 @@ __global__ void __launch_bounds__(kChunk, sizeof(T) == 4 ? 8 : 2)
             const T e = vs[at[k] + 2 * d] - m[d];
             d2 = NEWTON && !GAUSS ? add_rn(d2, mul_rn(e, e)) : fma(e, e, d2);
           }
-          const T x = ratio(d2, h2, rcp);
+          const T x = over(d2, win);
           w[k] = GAUSS ? exp2(-gk * x) - floor_w : T(1) - x;
           if (k >= n) w[k] = T(0);  // adds nothing
         }
@@ -924,7 +924,7 @@ void run_tiles(Call &call, const VoteSet &v, const T *desc, const T *means, cons
       std::min<uint64_t>(tiles * v.nchunks, uint64_t(v.tuning.simt_blocks_per_sm) * 152 + tiles);
   if (!listed(tiles, v.nchunks)) {
     launch_chained(st, ms_tile<T, COUNT, NEWTON, GAUSS>, unsigned(pairs), kChunk, 0, desc, v.sbox,
-                   uint32_t(v.nchunks), v.q, means, state, ids, nact, T(h2), k, gap2, w.grid, w.touched,
+                   uint32_t(v.nchunks), v.q, means, state, ids, nact, T(h2), window(T(h2)), k, gap2, w.grid, w.touched,
                    nullptr, 0u, nullptr, 0u, nullptr, partial, counts, evals);
     call.launched();
     return;
@@ -945,7 +945,7 @@ void run_tiles(Call &call, const VoteSet &v, const T *desc, const T *means, cons
   }();
   const unsigned ctas = unsigned(std::min<uint64_t>(pairs, uint64_t(152) * per_sm));
   launch_chained(st, ms_tile<T, COUNT, NEWTON, GAUSS>, ctas, kChunk, 0, desc, v.sbox, uint32_t(v.nchunks), v.q,
-                 means, state, ids, nact, T(h2), k, gap2, w.grid, w.touched, w.bits, w.bwords, w.items, room,
+                 means, state, ids, nact, T(h2), window(T(h2)), k, gap2, w.grid, w.touched, w.bits, w.bwords, w.items, room,
                  w.work, partial, counts, evals);
   call.launched(4);
 }

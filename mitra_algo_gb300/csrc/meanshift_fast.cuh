@@ -42,15 +42,34 @@ constexpr int kNewtonCap = 10;
 // corrections q + (a - b q) r.  The first leaves q within one unit in the last
 // place; from there the second rounds correctly (P. Markstein, "Computation of
 // elementary functions on the IBM RISC System/6000 processor", 1990).  No
-// branch, unlike the general division, so several overlap.
+// branch, unlike the general division, so several overlap.  For b, r and a b's
+// size or less whose residuals stay in FP32's normal range (window and quotient
+// see to that); an a so small that they do not gives a quotient off in its last
+// places, below 2^-40.
 __device__ __forceinline__ float ratio(float a, float b, float r) {
   float q = a * r;
   q = fmaf(fmaf(-b, q, a), r, q);
   return fmaf(fmaf(-b, q, a), r, q);
 }
-__device__ __forceinline__ double ratio(double a, double b, double) { return a / b; }
-__device__ __forceinline__ float reciprocal(float b) { return __frcp_rn(b); }
-__device__ __forceinline__ double reciprocal(double) { return 0.0; }
+
+// d^2 / h^2 of a vote within the bandwidth (0 <= d2 < h2), by ratio.  Any
+// bandwidth is accepted, so one whose square lies outside 2^-60 .. 2^60 is
+// brought into the range by a power of two, and d2 with it (exact, but where the
+// quotient is below 2^-120); a square beyond FP32 gives 0, as the division would.
+// Made on the host, for the kernels to read it from their parameters: as values
+// of each thread it spilled registers of the polish.
+template <typename T>
+struct Window {
+  T b, r, scale;
+};
+template <typename T>
+inline Window<T> window(T h2) {
+  if (sizeof(T) == 8 || !(h2 < INFINITY)) return {sizeof(T) == 8 ? h2 : T(1), T(0), T(1)};
+  const T scale = h2 < T(0x1p-60) ? T(0x1p100) : h2 > T(0x1p60) ? T(0x1p-64) : T(1);
+  return {h2 * scale, T(1) / (h2 * scale), scale};
+}
+__device__ __forceinline__ float over(float d2, const Window<float> &w) { return ratio(d2 * w.scale, w.b, w.r); }
+__device__ __forceinline__ double over(double d2, const Window<double> &w) { return d2 / w.b; }
 
 // a / b for any a and b: by ratio where neither the quotient nor its residual
 // can leave FP32's range, a zero included, else by the division, out of line.
@@ -60,7 +79,7 @@ static __device__ __noinline__ float divide(float a, float b) { return a / b; }
 __device__ __forceinline__ float quotient(float a, float b) {
   const float x = fabsf(a), y = fabsf(b);
   if (!(y > 1e-14f && y < 1e12f && (x == 0.f || (x > 1e-20f && x < 1e20f)))) return divide(a, b);
-  const float r = reciprocal(b);
+  const float r = __frcp_rn(b);
   return x == 0.f ? a * r : ratio(a, b, r);
 }
 __device__ __forceinline__ double quotient(double a, double b) { return a / b; }
