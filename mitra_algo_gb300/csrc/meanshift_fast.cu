@@ -324,7 +324,10 @@ constexpr int kPairStride = 20, kRunValues = kSubVotes / 2 * kPairStride;
 // GAUSS: the shifted Gaussian weights instead of Epanechnikov's.
 // With `items`, the warps draw (quarter, split) items of split_items' list
 // and take the chunks whose bits are set; without, block
-// (tile, split) takes every chunk of its split, a quarter per warp.
+// (tile, split) takes the chunks of its split that some seed of the warp's
+// quarter can reach.
+// evals gains the seed-vote pairs of the (tile, chunk) pairs taken: a chunk
+// within the bandwidth of some seed of the tile, whichever quarter's, counts once.
 //
 // Of the chunks, the lanes test the boxes of four chunks' runs of kSubVotes
 // votes (kSubs each) against the box of the warp's seeds at once; a run that
@@ -342,9 +345,13 @@ constexpr int kPairStride = 20, kRunValues = kSubVotes / 2 * kPairStride;
 // the tail of its CTAs (first Newton iteration of the 20,000-sample motif
 // sphere, 2,048 seeds, 2.5e7 votes: 5.2 ms, 2.9 ms here).  The next run's
 // 512 bytes are loaded while the current one is evaluated.
+constexpr uint64_t kListedPairs = 32768;  // (tile, chunk) pairs from which the items pay (listed)
+// words that hold the chunks of a direct split: at least 152 / tiles splits, so at
+// most kListedPairs / 152 chunks (rounded up), starting anywhere in a word
+constexpr int kDirectWords = (31 + int((kListedPairs + 151) / 152) + 31) / 32;
 template <typename T, bool COUNT, bool NEWTON, bool GAUSS>
 __global__ void __launch_bounds__(kChunk, sizeof(T) == 4 ? 8 : 2)
-    ms_tile(const T *desc, const float *sbox, uint32_t nchunks, uint64_t q, const T *means,
+    ms_tile(const T *desc, const float *cbox, const float *sbox, uint32_t nchunks, uint64_t q, const T *means,
             const uint8_t *state, const int32_t *ids, const unsigned *nact, T h2, Window<T> win, T gk, float skip_gap2,
             const Grid *plan, uint32_t *touched, const uint32_t *bits, uint32_t bwords, const uint2 *items,
             uint32_t room, uint32_t *work, T *partial, unsigned long long *counts, unsigned long long *evals) {
@@ -359,6 +366,11 @@ __global__ void __launch_bounds__(kChunk, sizeof(T) == 4 ? 8 : 2)
   uint32_t queue_end[kQueues];  // items of the queues up to and including each
   for (int k = 0; k < kQueues; ++k)
     queue_end[k] = (k ? queue_end[k - 1] : 0u) + (items ? work[kWorkQueue + k] : 0u);
+  __shared__ uint32_t counted[kDirectWords];  // chunks of the direct split in evals already
+  if (!items) {
+    if (threadIdx.x < kDirectWords) counted[threadIdx.x] = 0;
+    __syncthreads();
+  }
   T *const ns = nsum + threadIdx.x;
   const T floor_w = GAUSS ? exp2(-gk) : T(0);
   for (;;) {
@@ -508,12 +520,33 @@ __global__ void __launch_bounds__(kChunk, sizeof(T) == 4 ? 8 : 2)
       pending = more;
     };
     for (uint32_t base = c0 & ~31u; base < c1; base += 32) {
-      uint32_t word = mine ? mine[base / 32] : ~0u;
-      if (base < c0) word &= ~0u << (c0 - base);
-      if (c1 - base < 32) word &= (1u << (c1 - base)) - 1u;
-      if (quarter == 0 && evals && lane == 0 && word) {
-        done += uint64_t(__popc(word)) * kChunk;
-        if (c1 == nchunks && c1 - base <= 32 && (word >> (nchunks - 1 - base) & 1u) && q % kChunk)
+      uint32_t word, fresh;  // the chunks to take, those of them to count
+      if (mine) {
+        word = mine[base / 32];
+        if (base < c0) word &= ~0u << (c0 - base);
+        if (c1 - base < 32) word &= (1u << (c1 - base)) - 1u;
+        fresh = quarter == 0 ? word : 0u;
+      } else {  // a chunk per lane against the box of the warp's seeds, then each seed
+        const uint32_t c = base + lane;
+        bool near = false;
+        if (c >= c0 && c < c1) {
+          const float4 *b4 = reinterpret_cast<const float4 *>(cbox + uint64_t(c) * 12);
+          const float4 x = b4[0], y = b4[1], z = b4[2];
+          const float box[12] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w, z.x, z.y, z.z, z.w};
+          near = box_gap2(lo, hi, box) <= skip_gap2;
+        }
+        word = __ballot_sync(0xffffffffu, near);
+        for (uint32_t rest = word; rest; rest &= rest - 1) {
+          const int k = __ffs(int(rest)) - 1;
+          const bool reach = live && point_gap2_16(mf, cbox + uint64_t(base + k) * 12) <= skip_gap2;
+          if (!__any_sync(0xffffffffu, reach)) word &= ~(1u << k);
+        }
+        fresh = 0;
+        if (evals && lane == 0 && word) fresh = word & ~atomicOr(&counted[(base - (c0 & ~31u)) / 32], word);
+      }
+      if (evals && lane == 0 && fresh) {
+        done += uint64_t(__popc(fresh)) * kChunk;
+        if (c1 == nchunks && c1 - base <= 32 && (fresh >> (nchunks - 1 - base) & 1u) && q % kChunk)
           done -= kChunk - q % kChunk;  // the last chunk is not full
       }
       while (word) {  // four chunks at a time: a run box per lane
@@ -723,8 +756,6 @@ __global__ void __launch_bounds__(kChunk) ms_update(T *means, const T *red, cons
   }
 }
 
-constexpr uint64_t kListedPairs = 32768;  // (tile, chunk) pairs from which the items pay (listed)
-
 // Active seeds (kMoving, and kNear when include_near): in seed order, sorted
 // by the Morton key of their current mean (ties by seed id) when k <= kRetile.
 // nactive[0] = the number of active seeds, nactive[1] = how many of them are
@@ -923,7 +954,7 @@ void run_tiles(Call &call, const VoteSet &v, const T *desc, const T *means, cons
   const uint64_t pairs =
       std::min<uint64_t>(tiles * v.nchunks, uint64_t(v.tuning.simt_blocks_per_sm) * 152 + tiles);
   if (!listed(tiles, v.nchunks)) {
-    launch_chained(st, ms_tile<T, COUNT, NEWTON, GAUSS>, unsigned(pairs), kChunk, 0, desc, v.sbox,
+    launch_chained(st, ms_tile<T, COUNT, NEWTON, GAUSS>, unsigned(pairs), kChunk, 0, desc, v.cbox, v.sbox,
                    uint32_t(v.nchunks), v.q, means, state, ids, nact, T(h2), window(T(h2)), k, gap2, w.grid, w.touched,
                    nullptr, 0u, nullptr, 0u, nullptr, partial, counts, evals);
     call.launched();
@@ -944,7 +975,7 @@ void run_tiles(Call &call, const VoteSet &v, const T *desc, const T *means, cons
     return std::max(1, a);
   }();
   const unsigned ctas = unsigned(std::min<uint64_t>(pairs, uint64_t(152) * per_sm));
-  launch_chained(st, ms_tile<T, COUNT, NEWTON, GAUSS>, ctas, kChunk, 0, desc, v.sbox, uint32_t(v.nchunks), v.q,
+  launch_chained(st, ms_tile<T, COUNT, NEWTON, GAUSS>, ctas, kChunk, 0, desc, v.cbox, v.sbox, uint32_t(v.nchunks), v.q,
                  means, state, ids, nact, T(h2), window(T(h2)), k, gap2, w.grid, w.touched, w.bits, w.bwords, w.items, room,
                  w.work, partial, counts, evals);
   call.launched(4);
