@@ -15,16 +15,17 @@
 // How the decisions stay the reference's: the LBVH (Karras 2012: 30-bit
 // Morton codes of the face centroids, radix sort, longest-common-prefix
 // splits, boxes merged bottom-up, built once per resident mesh) is searched
-// in FP32 for every face whose FP32 distance lies within a margin of the
-// nearest one -- a margin several hundred times the FP32 error of a
-// distance, so the face of smallest FP64 distance is always among them.
-// Those candidates are re-evaluated with the reference's FP64 distance, and
-// the FP64 nearest face takes the reference's FP64 distance and normal
-// tests.  A query whose FP64 minimum is shared by faces that disagree on the
-// normal test (the reference then keeps the face its BVH visits first), or
-// whose candidates overflow the list, is re-run through the reference-order
-// BVH (verification.cuh), built on the host once per resident mesh when the
-// first such query appears.  Sums use the reference's serial order.
+// in FP32 with a window of 1,024 u M (u the FP32 unit, M the query's magnitude),
+// and of the faces met those within 128 u M of the nearest are kept, more than the
+// errors of two FP32 distances together (flat_d2 and face_d2n derive them), so the
+// face of smallest FP64 distance is always among them.  That holds for any
+// motion: a matrix that is not orthonormal widens M by its row sums (motion32).
+// What FP32 leaves open is decided in FP64 over those candidates.  Where faces at
+// the FP64 minimum disagree on the normal test, the one the reference's BVH visits
+// first is found from the tree's order (first_in_reference_order); candidates
+// that overflow the list go to a list of 64, and those that overflow that to the
+// reference-order search (verification.cuh).  That tree is built on the host
+// from the time the mesh is loaded.  Sums are the reference's serial ones.
 #include "face32.cuh"
 #include "primitives.cuh"
 #include "verification.cuh"
@@ -339,15 +340,15 @@ __device__ __forceinline__ int32_t support_query(const BvhView &b, const double 
 // ------------------------------------------- exact decisions, FP32 search
 // Error bound of the FP32 search, in distance units: kErr (512 FP32 units u)
 // times M, the largest coordinate magnitude of the vertex, its image, the
-// translation and the mesh, at least 2 tau.  A decided FP32 distance (flat_d2,
-// face_d2n) is within 64 u M of the reference's FP64 distance whatever the
-// face's shape, far inside kErr M; a face without a usable normal (its FP64
+// translation and the mesh, at least 2 tau, times the motion's gain (motion32).
+// A decided FP32 distance is far inside kErr M of the reference's FP64 distance
+// whatever the face's shape, 56 u M (flat_d2) to 73 (face_d2n); a face without a usable normal (its FP64
 // normal not accurate to well below u: no area, or a corner angle with sin
 // below 1e-6), or one that face_d2n leaves undecided (a projection within the
 // rounding band of an edge line), enters the candidates by a lower bound and
 // leaves the decision to FP64.  The same bound serves as the band of the FP32
 // threshold tests (2 tau, the plane side, tau), and kNormalBand (on the cosine)
-// as that of the normal test, whose FP32 error is a few u.
+// as that of the normal test, whose FP32 error is a few u times the gain.
 constexpr float kErr = 1.0f / 32768.0f;
 constexpr float kNormalBand = 1.0f / 1024.0f;
 constexpr int kCandidates = 16;
@@ -377,7 +378,8 @@ __device__ __forceinline__ float dot_fma(F3 a, F3 b) { return fmaf(a.x, b.x, fma
 // segment: of a p that projects inside by less, whose in-plane distance is 0, the
 // nearest segment is within two bands.
 // Error, with M the largest coordinate magnitude of mesh, image and translation
-// and at least 2 tau, and w = p - a, |w| <= tau + reach <= 0.75 M: the image (30
+// and at least 2 tau (times the motion's gain, which the image's share needs), and w
+// = p - a, |w| <= tau + reach <= 0.75 M: the image (30
 // u M) and a (1.8 u M) move w by 32 u M + u |w|; n, e and n x e are within u,
 // u and 4 u of their directions, and the products round by 3 u |w| each, which
 // moves (h, x, y) by sqrt(4^2 + 4^2 + 8^2) u |w| <= 8 u M; b and c by 2 u reach
@@ -428,10 +430,11 @@ __device__ __forceinline__ int flat_region(F3 p, const FlatFace &f, float &d2) {
 // bound) -- the face of smallest FP64 distance is at most 2 bounds farther
 // in FP32 than the best FP32 face.  Nodes are pruned with a slightly larger
 // radius, for the rounding of their boxes' distances.  The search's window is
-// generous; the faces returned are held to the error of a decided distance
-// itself, 64 u M, so 128 u M from the best (with the search's window, 1,024 u M, eight times as many queries found
-// neighbouring faces in it that disagree on the normal test, and went to
-// FP64).  Undecided faces are listed as ~face.  Returns the count (N + 1 on
+// generous; the faces returned are held to the errors of decided distances
+// themselves, at most 73 u M too long for one and 51 too short for the other of two:
+// within 128 u M of the best (with the search's window, 1,024 u M,
+// eight times as many queries found neighbouring faces in it that disagree on
+// the normal test, and went to FP64).  Undecided faces are listed as ~face.  Returns the count (N + 1 on
 // overflow: faces and keys hold N entries); `best` receives the smallest FP32
 // squared distance of a decided face (INFINITY when none lies within tau + 3
 // bounds).
@@ -495,7 +498,7 @@ __device__ int candidate_faces(const BvhView &b, F3 p, float tau_err, float err,
     }
   }
   if (overflow) return N + 1;
-  // what is left by a decided distance's own error, 64 u M
+  // what is left by the errors of two decided distances
   radius = fminf(tau_err, sqrtf(best)) + 128.f * um;
   lim = fminf(lim, radius * radius);
   int m = 0;
@@ -508,7 +511,36 @@ __device__ int candidate_faces(const BvhView &b, F3 p, float tau_err, float err,
 struct MotionF {
   float r[9], t[3], n[3], offset;
   int32_t reflection;
+  float gain;  // the largest row or column sum of |r| (and |n|_1) over an orthonormal one's bound
+  float reach;  // the largest magnitude among t and, of a reflection, offset
 };
+
+// A record's matrix need not be orthonormal: one whose products cancel brings an
+// image of ordinary size with the rounding of large terms.  The error bounds are
+// those of row sums up to sqrt(3), an orthonormal matrix's most, and grow with
+// the sum beyond.  (A matrix or plane that is not finite keeps them: its
+// images are not finite either.)
+MotionF motion32(const sym_cluster_record &r) {
+  MotionF m{};
+  double most = 0;
+  for (int k = 0; k < 3; ++k) {
+    double row = 0, column = 0;
+    for (int j = 0; j < 3; ++j) row += std::fabs(r.rotation[3 * k + j]), column += std::fabs(r.rotation[3 * j + k]);
+    most = std::max(most, std::max(row, column));
+  }
+  m.reflection = r.reflection != 0;
+  if (m.reflection)
+    most = std::max(most, std::fabs(r.plane_normal[0]) + std::fabs(r.plane_normal[1]) + std::fabs(r.plane_normal[2]));
+  m.gain = std::isfinite(most) ? std::max(1.f, float(most / 1.7320508 * (1 - 1e-6))) : 1.f;
+  for (int k = 0; k < 9; ++k) m.r[k] = float(r.rotation[k]);
+  for (int k = 0; k < 3; ++k) {
+    m.t[k] = float(r.translation[k]), m.n[k] = float(r.plane_normal[k]);
+    m.reach = std::fmax(m.reach, std::fabs(m.t[k]));
+  }
+  m.offset = float(r.plane_offset);
+  if (m.reflection) m.reach = std::fmax(m.reach, std::fabs(m.offset));
+  return m;
+}
 
 // Row lists between the verification kernels.
 // A row (c, direction, vertex i) holds the flag and error of one query;
@@ -574,7 +606,7 @@ __global__ void __launch_bounds__(kThreads, 5)
        r[6] * u.x + r[7] * u.y + r[8] * u.z};
   if (!inverse) q = q + F3{m.t[0], m.t[1], m.t[2]};
   const float mag = fmaxf(fmaxf(scale, 2.f * tau), fmaxf(fabsf(q.x), fmaxf(fabsf(q.y), fabsf(q.z))));
-  const float e = kErr * fmaxf(mag, fmaxf(fabsf(m.t[0]), fmaxf(fabsf(m.t[1]), fabsf(m.t[2]))));
+  const float e = kErr * m.gain * fmaxf(mag, m.reach);
   auto to_fp64 = [&]() {
     lists.mark[qid] = 1;
     lists.slot_of[qid] = kNoSlot;
@@ -627,7 +659,7 @@ __global__ void __launch_bounds__(kThreads, 5)
     // has one): the cosine is good to a few u
     const float4 fn = b.face[4 * int64_t(faces[j]) + 3];
     const float v = dotf(rn, F3{fn.x, fn.y, fn.z});
-    if (fabsf(v - 0.5f) <= kNormalBand) return to_fp64_listed();
+    if (fabsf(v - 0.5f) <= kNormalBand * m.gain) return to_fp64_listed();
     if (v >= 0.5f) ++agree;
     else ++disagree;
   }
@@ -771,10 +803,10 @@ struct RowFaces {
 __device__ __forceinline__ int32_t listed_face(int32_t x) { return x < 0 ? ~x : x; }
 
 // The candidates cl (up to `end`) of a row whose image is q: their corner
-// distances, and with NORMALS their normal tests.
+// distances, and with NORMALS their normal tests (turned normal rn, `band`).
 template <bool NORMALS>
 __device__ __forceinline__ RowFaces corner_distances(const BvhView &b, const Surface &s, D3 q, F3 qf, float um,
-                                                     const int32_t *cl, int32_t end, F3 rn) {
+                                                     const int32_t *cl, int32_t end, F3 rn, float band) {
   RowFaces r;
   double dv = 0;
   int32_t at_vertex = -1;  // of which dv is the squared distance
@@ -783,7 +815,7 @@ __device__ __forceinline__ RowFaces corner_distances(const BvhView &b, const Sur
     const Face face = load_face(b, f);
     if (NORMALS) {
       const float cosine = dotf(rn, face.n);
-      if (face.reach == 0.f || !(fabsf(cosine - 0.5f) > kNormalBand)) r.unsure |= 1u << j;
+      if (face.reach == 0.f || !(fabsf(cosine - 0.5f) > band)) r.unsure |= 1u << j;
       else if (cosine > 0.5f) r.agrees |= 1u << j;
     }
     const int v = face.reach == 0.f ? -1 : corner_region(qf, face, um);
@@ -801,8 +833,8 @@ __device__ __forceinline__ RowFaces corner_distances(const BvhView &b, const Sur
   return r;
 }
 
-// Whether face f is farther than dmin in FP32 already (a decided FP32 distance is
-// within 64 u M of FP64's); `region`: the list its distance belongs to.
+// Whether face f is farther than dmin in FP32 already (its decided FP32
+// distance is within 64 u M of FP64's); `region`: the list its distance belongs to.
 __device__ __forceinline__ bool beyond(const BvhView &b, F3 p, int32_t f, float um, double dmin, int &region) {
   const FlatFace face = load_flat(b, f);
   region = 3;
@@ -897,7 +929,7 @@ __global__ void __launch_bounds__(kRowThreads, 4) forward_errors(BvhView b, Surf
     qf = F3{float(q.x), float(q.y), float(q.z)};
     um = search_unit(m, qf, scale, tau);
     cl = lists.faces + k * kCandidates;
-    r = corner_distances<false>(b, s, q, qf, um, cl, -1, F3{0, 0, 0});
+    r = corner_distances<false>(b, s, q, qf, um, cl, -1, F3{0, 0, 0}, 0.f);
   }
   block_distances<false>(sh, b, s, live, q, qf, um, cl, r);
   if (live) err[at] = r.dmin;
@@ -917,10 +949,12 @@ __device__ __forceinline__ Query query_of(const BvhView &b, uint64_t qid) {
   return x;
 }
 // Its vertex's image and the unit of the FP32 search there (verify_fp32 decided
-// the 2 tau and side tests of a row with candidates), and its turned normal.
+// the 2 tau and side tests of a row with candidates), its turned normal, and the
+// band of the normal test.
 __device__ __forceinline__ void query_image(const Surface &s, const ClusterMotion *motions,
                                             const MotionF *motions32, const float *vn32, const Query &x,
-                                            float scale, float tau, D3 &q, F3 &qf, float &um, F3 &rn) {
+                                            float scale, float tau, D3 &q, F3 &qf, float &um, F3 &rn,
+                                            float &band) {
   const ClusterMotion &m = motions[x.c];
   const M3 r = query_rotation(m, x.inverse);
   const D3 p = vertex(s, int32_t(x.i)), mt{m.t[0], m.t[1], m.t[2]};
@@ -928,6 +962,7 @@ __device__ __forceinline__ void query_image(const Surface &s, const ClusterMotio
   qf = F3{float(q.x), float(q.y), float(q.z)};
   um = search_unit(m, qf, scale, tau);
   const MotionF &mf = motions32[x.c];
+  band = kNormalBand * mf.gain;
   float rf[9];
   for (int j = 0; j < 9; ++j) rf[j] = x.inverse ? mf.r[(j % 3) * 3 + j / 3] : mf.r[j];
   const F3 ni{vn32[x.i], vn32[s.nv + x.i], vn32[2 * s.nv + x.i]};
@@ -987,10 +1022,10 @@ __global__ void __launch_bounds__(kThreads, 4) verify_rows_fp64(BvhView b, Surfa
       const Query x = query_of(b, qid);
       D3 q;
       F3 qf, rn;
-      float um;
-      query_image(s, motions, motions32, vn32, x, scale, float(tau), q, qf, um, rn);
+      float um, band;
+      query_image(s, motions, motions32, vn32, x, scale, float(tau), q, qf, um, rn, band);
       const int32_t *cl = lists.cand + uint64_t(slot) * kCandidates;
-      RowFaces r = corner_distances<true>(b, s, q, qf, um, cl, kNoFace, rn);
+      RowFaces r = corner_distances<true>(b, s, q, qf, um, cl, kNoFace, rn, band);
       for (unsigned rest = r.open; rest && left < 0; rest &= rest - 1) {
         int region;
         if (r.dmin == INFINITY || !beyond(b, qf, listed_face(cl[__ffs(int(rest)) - 1]), um, r.dmin, region))
@@ -1061,15 +1096,15 @@ __global__ void __launch_bounds__(kRowThreads, 3) verify_rows_open(
       Query x{};
       D3 q{0, 0, 0};
       F3 qf{0, 0, 0}, rn{0, 0, 0};
-      float um = 0;
+      float um = 0, band = 0;
       RowFaces r;
       const int32_t *cl = nullptr;
       if (live) {
         qid = uint64_t(lists.open[k - listed_from]);
         x = query_of(b, qid);
-        query_image(s, motions, motions32, vn32, x, scale, float(tau), q, qf, um, rn);
+        query_image(s, motions, motions32, vn32, x, scale, float(tau), q, qf, um, rn, band);
         cl = lists.cand + uint64_t(lists.slot_of[qid]) * kCandidates;
-        r = corner_distances<true>(b, s, q, qf, um, cl, kNoFace, rn);
+        r = corner_distances<true>(b, s, q, qf, um, cl, kNoFace, rn, band);
       }
       block_distances<true>(sh, b, s, live, q, qf, um, cl, r);
       if (live) {
@@ -1798,13 +1833,7 @@ uint64_t exact_flags(Call &call, const ResidentSurface &m, const ClusterMotion *
   }
   const Lbvh &bvh = *m.lbvh;
   std::vector<MotionF> mf(nc);
-  for (uint64_t c = 0; c < nc; ++c) {
-    const sym_cluster_record &r = records[c];
-    for (int k = 0; k < 9; ++k) mf[c].r[k] = float(r.rotation[k]);
-    for (int k = 0; k < 3; ++k) mf[c].t[k] = float(r.translation[k]), mf[c].n[k] = float(r.plane_normal[k]);
-    mf[c].offset = float(r.plane_offset);
-    mf[c].reflection = r.reflection != 0;
-  }
+  for (uint64_t c = 0; c < nc; ++c) mf[c] = motion32(records[c]);
   const MotionF *dmf = call.upload(mf.data(), nc);
   RowLists lists;
   lists.forward = call.alloc<uint32_t>(nc * nv);
