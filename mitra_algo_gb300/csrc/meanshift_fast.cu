@@ -758,10 +758,8 @@ __global__ void __launch_bounds__(kChunk) ms_update(T *means, const T *red, cons
 
 // Active seeds (kMoving, and kNear when include_near): in seed order, sorted
 // by the Morton key of their current mean (ties by seed id) when k <= kRetile.
-// nactive[0] = the number of active seeds, nactive[1] = how many of them are
-// kNear.  With `iter`, an iteration that finds active seeds records their
-// number in trace[*iter] (while *iter < trace_cap) and counts itself in *iter.
-// `plan` as above.
+// The number of active seeds and what else `progress` holds goes there; `plan` as
+// above.
 //
 // Runs in every iteration between two kernels that wait for it, so its own
 // latency counts.  A block lists the active seeds for itself from their state
@@ -781,10 +779,7 @@ unsigned retile_blocks(uint64_t k) {
 template <typename T>
 __global__ void __launch_bounds__(kRetileThreads) retile(const T *means, const uint8_t *state, uint64_t k,
                                                          const float *box, bool include_near,
-                                                         int32_t *ids, unsigned *nactive,
-                                                         unsigned *iter = nullptr,
-                                                         uint32_t *trace = nullptr,
-                                                         unsigned trace_cap = 0, Plan plan = Plan()) {
+                                                         int32_t *ids, Progress *progress, Plan plan) {
   constexpr int kWarps = kRetileThreads / 32;
   __shared__ unsigned long long keys[kRetile];
   __shared__ uint16_t seeds[kRetile];
@@ -795,6 +790,13 @@ __global__ void __launch_bounds__(kRetileThreads) retile(const T *means, const u
     plan.clear[i] = 0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool sort = k <= kRetile;
+  // a block that looks at every seed reports; its loads come ahead of its stores
+  const bool reports = threadIdx.x == 0 && blockIdx.x == (sort ? 0 : gridDim.x - 1);
+  unsigned done = 0;
+  unsigned long long served = 0, began = 0, ended = 0, busy = 0;
+  if (reports)
+    done = progress->iterations, served = progress->seeds, began = progress->began, ended = progress->ended,
+    busy = progress->busy;
   const uint64_t first = sort ? 0 : uint64_t(blockIdx.x) * kRetile;
   // the states of seeds s..s + 7 (zero bits: not active), `near` of them
   unsigned mask = 0, near = 0, before = 0;
@@ -834,14 +836,15 @@ __global__ void __launch_bounds__(kRetileThreads) retile(const T *means, const u
     total += warp_active[w], near += warp_near[w], before += below[0][w];
   }
   const unsigned n = before + total;
-  // a block that has looked at every seed reports
-  if (threadIdx.x == 0 && blockIdx.x == (sort ? 0 : gridDim.x - 1)) {
-    nactive[0] = n, nactive[1] = near;
+  if (reports) {
+    progress->nact[0] = n, progress->nact[1] = near;
     if (plan.grid) *plan.grid = grid_for(n, plan.nchunks, plan.blocks_per_sm);
-    if (iter && n) {
-      if (*iter < trace_cap) trace[*iter] = n;
-      ++*iter;
+    if (n) {
+      if (done < kTraced) progress->trace[done] = n;
+      progress->iterations = done + 1, progress->seeds = served + n;
     }
+    if (ended) progress->busy = busy + (ended - began);
+    progress->began = ~0ull, progress->ended = 0;
   }
   if (!sort) {
     at += before;
@@ -996,30 +999,27 @@ int shift_impl(Call &call, const VoteSet &v, const T *desc, T *means, uint8_t *s
                unsigned long long *evals, uint32_t *trace = nullptr, int trace_len = 0) {
   cudaStream_t st = call.stream();
   int32_t *ids = call.alloc<int32_t>(k);
-  // active seeds, kNear ones, iterations done, then the active seeds of each
-  const unsigned trace_cap = unsigned(std::max(max_iter, 1));
-  unsigned *nact = call.alloc<unsigned>(3 + size_t(trace_cap)), *iter = nact + 2, *trace_dev = nact + 3;
-  std::vector<unsigned> seen(3 + (trace || seed_iterations ? size_t(trace_cap) : 0), 0u);
+  Progress *progress = call.alloc<Progress>(1), seen{};
+  const unsigned *const nact = progress->nact;  // on the device
   // partial capacity: splits x slots is at most ~blocks*152*kChunk (+ one tile)
   const int bps = v.tuning.simt_blocks_per_sm;
   uint64_t cap = (uint64_t(bps) * 152 + 2) * uint64_t(kChunk) + std::max<uint64_t>(k, kChunk) * 2;
   T *partial = call.alloc<T>(cap * kPartial);
   T *red = call.alloc<T>(uint64_t(kGroups) * kPartial * std::max<uint64_t>(k, kChunk) * 2);
   TileWork work = tile_work<T>(call, v, k);
-  SYM_CUDA(cudaMemsetAsync(iter, 0, sizeof(unsigned), st));
+  SYM_CUDA(cudaMemsetAsync(progress, 0, sizeof(Progress), st));
   uint64_t tiles = (k + kChunk - 1) / kChunk;  // at most, as the host knows
-  const unsigned *const counts = seen.data();
+  const unsigned *const counts = seen.nact;
   const bool gauss = v.kernel_k > 0;
   bool finished = false;
   auto look = [&]() {
-    // what a call without a long limit asks for arrives with the counts
-    call.d2h(seen.data(), nact, std::min<size_t>(seen.size(), 512) * sizeof(unsigned));
+    call.d2h(&seen, progress, sizeof(Progress));
     call.sync();
   };
   const int check = polish ? kPolishCheck : kShiftCheck;
   for (int it = 0; it < max_iter; ++it) {
-    launch_chained(st, retile<T>, retile_blocks(k), kRetileThreads, 0, means, state, k, v.gbox, polish, ids, nact,
-                   iter, trace_dev, trace_cap, plan_of<T>(v, work, tiles));
+    launch_chained(st, retile<T>, retile_blocks(k), kRetileThreads, 0, means, state, k, v.gbox, polish, ids,
+                   progress, plan_of<T>(v, work, tiles));
     call.launched();
     if (it % check == 0 || (polish && counts[1] != counts[0])) {
       look();
@@ -1039,18 +1039,9 @@ int shift_impl(Call &call, const VoteSet &v, const T *desc, T *means, uint8_t *s
     call.launched(2);
   }
   if (!finished) look();
-  const unsigned done = seen[2];
-  if (seen.size() > 3) {
-    if (3 + size_t(done) > 512) {
-      call.d2h(seen.data(), nact, (3 + size_t(std::min(done, trace_cap))) * sizeof(unsigned));
-      call.sync();
-    }
-    for (unsigned i = 0; i < done && i < trace_cap; ++i) {
-      if (seed_iterations) *seed_iterations += seen[3 + i];
-      if (trace && int(i) < trace_len) trace[i] = seen[3 + i];
-    }
-  }
-  return int(done);
+  if (seed_iterations) *seed_iterations += double(seen.seeds);
+  for (int i = 0; trace && i < std::min(trace_len, kTraced) && i < int(seen.iterations); ++i) trace[i] = seen.trace[i];
+  return int(seen.iterations);
 }
 
 }  // namespace
@@ -1131,10 +1122,9 @@ int shift(Call &call, const VoteSet &v, double *means, uint8_t *state, uint64_t 
 }
 
 void active_seeds_async(Call &call, const VoteSet &v, const float *means, const uint8_t *state,
-                        uint64_t k, int32_t *ids, unsigned *nact, unsigned *iter, uint32_t *trace,
-                        unsigned trace_cap) {
+                        uint64_t k, int32_t *ids, Progress *progress) {
   launch_chained(call.stream(), retile<float>, retile_blocks(k), kRetileThreads, 0, means, state, k, v.gbox,
-                 false, ids, nact, iter, trace, trace_cap, Plan());
+                 false, ids, progress, Plan());
   call.launched();
 }
 
@@ -1145,12 +1135,14 @@ void count_within(Call &call, const VoteSet &v, const float *points, uint64_t nm
   uint8_t *state = call.alloc<uint8_t>(nm);
   SYM_CUDA(cudaMemsetAsync(state, 0, nm, st));
   int32_t *ids = call.alloc<int32_t>(nm);
-  unsigned *nact = call.alloc<unsigned>(2);
+  Progress *progress = call.alloc<Progress>(1);
+  SYM_CUDA(cudaMemsetAsync(progress, 0, sizeof(Progress), st));
+  const unsigned *const nact = progress->nact;  // on the device
   const uint64_t tiles = (nm + kChunk - 1) / kChunk;
   TileWork work = tile_work<float>(call, v, nm);
   SYM_CUDA(cudaMemsetAsync(counts, 0, nm * sizeof(*counts), st));
   launch_chained(st, retile<float>, retile_blocks(nm), kRetileThreads, 0, points, state, nm, v.gbox, false, ids,
-                 nact, nullptr, nullptr, 0u, plan_of<float>(v, work, tiles));
+                 progress, plan_of<float>(v, work, tiles));
   run_tiles<float, true, false, false>(call, v, v.desc, points, nullptr, ids, nact, tiles, h2, work,
                                        static_cast<float *>(nullptr), counts, nullptr);
   call.launched();

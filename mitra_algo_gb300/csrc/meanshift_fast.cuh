@@ -159,13 +159,23 @@ int shift(Call &call, const VoteSet &v, float *means, uint8_t *state, uint64_t k
 int shift(Call &call, const VoteSet &v, double *means, uint8_t *state, uint64_t k, double h2,
           int max_iter, bool polish, double *seed_iterations, unsigned long long *evals);
 
+// What the iterations of one loop leave on the device (zeroed before the first).
+// Its size does not depend on the iteration limit: a caller may give any.
+constexpr int kTraced = 320;  // iterations whose active seeds are kept (a result's traces)
+struct Progress {
+  unsigned nact[2];  // active seeds of the last iteration, kNear ones among them
+  unsigned iterations, unused;  // that found active seeds
+  unsigned long long seeds;  // active seeds over all of them
+  // the tensor kernel by the device's clock (ns): start of the first CTA and end of
+  // the last since the last retile, and the time of the launches before
+  unsigned long long began, ended, busy;
+  uint32_t trace[kTraced];  // active seeds of the first ones
+};
+
 // kMoving seeds, Morton-sorted by position when k <= 2048, with their
-// number left on the device (nact[0]); an iteration that finds active seeds
-// records their number in trace[*iter] (while *iter < trace_cap) and
-// increments *iter.  No synchronisation.
+// number left on the device (progress->nact[0]).  No synchronisation.
 void active_seeds_async(Call &call, const VoteSet &v, const float *means, const uint8_t *state,
-                        uint64_t k, int32_t *ids, unsigned *nact, unsigned *iter, uint32_t *trace,
-                        unsigned trace_cap);
+                        uint64_t k, int32_t *ids, Progress *progress);
 
 // Number of votes within the bandwidth of each of `nm` points (nm x 8).
 void count_within(Call &call, const VoteSet &v, const float *points, uint64_t nm, double h2,

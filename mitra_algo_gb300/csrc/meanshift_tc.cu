@@ -583,9 +583,8 @@ struct TcArgs {
   float gauss_k2;           // 0: Epanechnikov; k > 0 (a power of 2): 2^(-k d^2/h^2) - 2^-k
   float *partial;
   unsigned long long *evals;
-  const unsigned *iter;       // iterations with active seeds, this one included
-  unsigned long long *began, *ended;  // per iteration (while *iter <= span_cap): device clock, ns
-  unsigned span_cap;
+  Progress *progress;
+  bool timed;  // began and ended of it
   int *status;
 };
 
@@ -657,7 +656,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) ms_tile_tc(TcArgs a) {
   // the launch's own time: its first CTA's start to its last CTA's end by the
   // device's clock (events around the launch kept it from being chained and cost
   // 9 us per iteration)
-  if (tid == 0 && *a.iter <= a.span_cap) atomicMin(&a.began[*a.iter - 1], (unsigned long long)global_ns());
+  if (tid == 0 && a.timed) atomicMin(&a.progress->began, (unsigned long long)global_ns());
   const uint64_t nactive = a.nact[0];
   uint64_t lo_t = 0, hi_t = ntiles;  // last tile whose first piece is <= piece
   while (hi_t - lo_t > 1) {
@@ -908,7 +907,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) ms_tile_tc(TcArgs a) {
   tc_fence_before();
   __syncthreads();
   if (warp == 0 && n) tmem_dealloc(tmem, kTcCols);
-  if (tid == 0 && *a.iter <= a.span_cap) atomicMax(&a.ended[*a.iter - 1], (unsigned long long)global_ns());
+  if (tid == 0 && a.timed) atomicMax(&a.progress->ended, (unsigned long long)global_ns());
 }
 
 // ------------------------------------------------------ tensor self-test
@@ -1137,28 +1136,23 @@ bool meanshift_bf16_bulk(Call &call, const VoteSet &v, float *means, uint8_t *st
   const uint32_t sms = 152 * uint32_t(v.tuning.tc_ctas_per_sm);
   const uint64_t max_grid = std::max<uint64_t>(sms, 2 * max_tiles);
   float *partial = call.alloc<float>(max_grid * kChunk * 8);
-  unsigned *nact = call.alloc<unsigned>(2), *iter = call.alloc<unsigned>(1);
-  const unsigned trace_cap = unsigned(std::max(max_iter, 1));
-  uint32_t *trace_dev = call.alloc<uint32_t>(trace_cap);
+  Progress *progress = call.alloc<Progress>(1);
+  const unsigned *const nact = progress->nact;  // on the device
   unsigned long long *evals = call.alloc<unsigned long long>(1);
   SYM_CUDA(cudaMemsetAsync(evals, 0, 8, st));
-  SYM_CUDA(cudaMemsetAsync(iter, 0, 4, st));
-  const unsigned span_cap = kernel_ms ? trace_cap : 0;
-  unsigned long long *spans = call.alloc<unsigned long long>(2 * size_t(span_cap));
-  SYM_CUDA(cudaMemsetAsync(spans, 0xff, 8 * size_t(span_cap), st));
-  SYM_CUDA(cudaMemsetAsync(spans + span_cap, 0, 8 * size_t(span_cap), st));
+  SYM_CUDA(cudaMemsetAsync(progress, 0, sizeof(Progress), st));
   const float gap = float(std::sqrt(h2)) + 1e-6f;
   call.launched();
   TcArgs args{images, v.nchunks, list, offsets, pieces, nact, means, ids, v.gbox,
-              float(1.0 / std::sqrt(h2)), float(v.kernel_k), partial, evals, iter, spans, spans + span_cap,
-              span_cap, call.status()};
+              float(1.0 / std::sqrt(h2)), float(v.kernel_k), partial, evals, progress, kernel_ms != nullptr,
+              call.status()};
   // Iterations are launched back to back: each reads the active-seed count
   // that the previous one left on the device, and one whose count is zero
   // returns at once.  The host looks at the count every kCheck iterations.
   const int kCheck = v.tuning.check_interval;
   int it = 0;
   for (; it < max_iter; ++it) {
-    active_seeds_async(call, v, means, state, k, ids, nact, iter, trace_dev, trace_cap);
+    active_seeds_async(call, v, means, state, k, ids, progress);
     launch_chained(st, tile_boxes<float>, unsigned(max_tiles), kCullThreads, 0, means, ids, nact, v.bbox, nblk,
                    gap * gap, boxes, sblk, nsurv, bcount);
     launch_chained(st, tile_count, list_ctas, kListThreads, 0, boxes, means, ids, nact, v.cbox, v.bbox,
@@ -1183,31 +1177,16 @@ bool meanshift_bf16_bulk(Call &call, const VoteSet &v, float *means, uint8_t *st
   }
   call.check_status("mean_shift (tensor)");
   unsigned long long ev = 0;
-  unsigned active_iterations = 0;
+  Progress seen;
   call.d2h(&ev, evals, 8);
-  call.d2h(&active_iterations, iter, sizeof(unsigned));
+  call.d2h(&seen, progress, sizeof(seen));
   call.sync();
-  *iterations = int(active_iterations);
+  *iterations = int(seen.iterations);
   *evaluations = double(ev);
-  if ((trace && trace_len > 0) || seed_iterations) {
-    std::vector<uint32_t> tr(trace_cap);
-    call.d2h(tr.data(), trace_dev, trace_cap * sizeof(uint32_t));
-    call.sync();
-    for (int i = 0; trace && i < trace_len && i < int(active_iterations) && i < int(trace_cap); ++i)
-      trace[i] = tr[i];
-    // every iteration with active seeds is recorded (trace_cap = max_iter)
-    for (unsigned i = 0; seed_iterations && i < active_iterations && i < trace_cap; ++i)
-      *seed_iterations += tr[i];
-  }
-  const unsigned timed = std::min(active_iterations, span_cap);
-  if (timed) {
-    std::vector<unsigned long long> began(timed), ended(timed);
-    call.d2h(began.data(), spans, 8 * size_t(timed));
-    call.d2h(ended.data(), spans + span_cap, 8 * size_t(timed));
-    call.sync();
-    for (unsigned i = 0; i < timed; ++i) *kernel_ms += double(ended[i] - began[i]) * 1e-6;
-  }
-  if (kernel_launches) *kernel_launches = timed;
+  for (int i = 0; trace && i < std::min(trace_len, kTraced) && i < int(seen.iterations); ++i) trace[i] = seen.trace[i];
+  if (seed_iterations) *seed_iterations += double(seen.seeds);
+  if (kernel_ms) *kernel_ms = double(seen.busy + (seen.ended ? seen.ended - seen.began : 0)) * 1e-6;
+  if (kernel_launches) *kernel_launches = kernel_ms ? seen.iterations : 0;
   return true;
 }
 
