@@ -324,8 +324,8 @@ constexpr int kPairStride = 20, kRunValues = kSubVotes / 2 * kPairStride;
 // GAUSS: the shifted Gaussian weights instead of Epanechnikov's.
 // With `items`, the warps draw (quarter, split) items of split_items' list
 // and take the chunks whose bits are set; without, block
-// (tile, split) takes the chunks of its split that some seed of the warp's
-// quarter can reach.
+// (tile, split) takes every chunk of its split, a quarter per warp, or, where they
+// are counted, those that some seed of the quarter can reach.
 // evals gains the seed-vote pairs of the (tile, chunk) pairs taken: a chunk
 // within the bandwidth of some seed of the tile, whichever quarter's, counts once.
 //
@@ -520,13 +520,11 @@ __global__ void __launch_bounds__(kChunk, sizeof(T) == 4 ? 8 : 2)
       pending = more;
     };
     for (uint32_t base = c0 & ~31u; base < c1; base += 32) {
-      uint32_t word, fresh;  // the chunks to take, those of them to count
-      if (mine) {
-        word = mine[base / 32];
-        if (base < c0) word &= ~0u << (c0 - base);
-        if (c1 - base < 32) word &= (1u << (c1 - base)) - 1u;
-        fresh = quarter == 0 ? word : 0u;
-      } else {  // a chunk per lane against the box of the warp's seeds, then each seed
+      uint32_t word = mine ? mine[base / 32] : ~0u;  // the chunks to take
+      if (base < c0) word &= ~0u << (c0 - base);
+      if (c1 - base < 32) word &= (1u << (c1 - base)) - 1u;
+      uint32_t fresh = quarter == 0 ? word : 0u;  // those of them to count
+      if (!mine && evals) {  // a chunk per lane against the box of the warp's seeds, then each seed
         const uint32_t c = base + lane;
         bool near = false;
         if (c >= c0 && c < c1) {
@@ -542,7 +540,7 @@ __global__ void __launch_bounds__(kChunk, sizeof(T) == 4 ? 8 : 2)
           if (!__any_sync(0xffffffffu, reach)) word &= ~(1u << k);
         }
         fresh = 0;
-        if (evals && lane == 0 && word) fresh = word & ~atomicOr(&counted[(base - (c0 & ~31u)) / 32], word);
+        if (lane == 0 && word) fresh = word & ~atomicOr(&counted[(base - (c0 & ~31u)) / 32], word);
       }
       if (evals && lane == 0 && fresh) {
         done += uint64_t(__popc(fresh)) * kChunk;
