@@ -887,9 +887,11 @@ __global__ void gather_seeds(const T *desc, const int64_t *pos, uint64_t k, T *m
 
 // Whether an iteration draws its work from split_items' list: with few
 // (tile, chunk) pairs the direct grid's own tests cost less than the three list
-// kernels (us per iteration, direct and listed: 44 and 61 at 940 pairs, 71 and
-// 80 at 18,750 pairs, 300 and 160 at 160,000 pairs).
-// The sums are the same either way.
+// kernels.  Us per approach iteration, direct and listed: 23 and 34 at 40 pairs
+// (mirror planes), on the motif sphere 24 and 37 at 2,800, 48 and 65 at 18,900, 68
+// and 84 at 38,000, 147 and 169 at 170,000; on the 1e7-vote Gaussian torus, whose
+// tiles reach fewer of their chunks, 50 and 51 at 7,300, 68 and 62 at 11,400, 85 and
+// 79 at 45,600.  The line lies between the two.  The sums are the same either way.
 bool listed(uint64_t tiles, uint64_t nchunks) { return tiles * nchunks >= kListedPairs; }
 
 // Scratch of the SIMT iterations, sized for `k` seeds.

@@ -16,7 +16,7 @@
 //  6. the edge table: the corner edges stably sorted by (lo, hi), one edge per
 //     run of equal keys with its first two corners - the order and content of
 //     the reference's std::map, plus its non-manifold / winding checks;
-//  7. the vertex centroid as one sequential sum (on the host, meanwhile).
+//  7. the vertex centroid as one sequential sum (on the host).
 // FP64 without FMA contraction in the reference's operation order, so every
 // output is bit-exact with the CPU path.
 #include "common.cuh"
@@ -325,8 +325,8 @@ PreparedDevice prepare_device(Call &call, const sym_mesh_view &m, const sym_opti
                                                     p.edges, diag, diag + 1);
   check_launch();
   // 7. centroid: one addition waits for the one before, so the host, which has
-  // the vertices, takes the serial sums while the device works (500,000
-  // vertices: 33 ms in a kernel of three threads)
+  // the vertices, takes the serial sums (500,000 vertices: 33 ms in a kernel of
+  // three threads, about 1 on the host; only the edge records run meanwhile)
   double hc[3] = {0, 0, 0};
   for (uint64_t v = 0; v < nv; ++v)
     hc[0] += m.vertices.x[v], hc[1] += m.vertices.y[v], hc[2] += m.vertices.z[v];
